@@ -10,7 +10,8 @@
 // x . w^T reads (engine/model.py:303-320 of the reference calls F.linear on the same
 // layout). Every output element sums its K products in the same order whatever M is, so
 // a token's result does not depend on what else is in the batch. When activations, weights
-// and output are all float32 the K products are summed in double and rounded once: a
+// and output are all float32 (kernels of their own below, unless K is not a multiple of 4 or an
+// operand is not 16-byte aligned) the K products are summed in double and rounded once: a
 // sequential float32 sum over a long K loses several bits against what a float32 result
 // can hold, and a model whose layers cancel (a recurrent state read out by a near-orthogonal
 // vector) amplifies exactly that.
@@ -112,7 +113,331 @@ int launch(void* out, const void* x, const void* w, const float* bias, const voi
   return check_launch("linear_simt");
 }
 
+// ---------------------------------------------------------------------------------------
+// The float32 products (activations, weights and output all float32, K a multiple of 4, 16-byte
+// aligned operands): K is cut into segments of SEGMENT; a segment's products are added one after
+// the other in double, the segments' sums one after the other to the total, bias and residual
+// to that, and the result is rounded once. Both kernels below keep exactly this order, whatever
+// M is and however K is shared out, so a token's result does not depend on its batch.
+//
+// f32_few_kernel, up to 16 tokens: bound by the weights' bytes (up to about 8 tokens; beyond, by
+// the double multiply-adds, 64 a clock and SM). A lane owns a weight row, a warp a segment of
+// 32 rows; a warp's weights pass through a ring of cp.async stages of its own (32 k of 32 rows, rows
+// 144 bytes apart so that the lanes' 16-byte reads meet no bank twice), the tokens' values of a
+// chunk are widened once per warp and read by all lanes at once. The tile kernel before ran 64 x 64
+// tiles with a token's row repeated over nothing: one token, K = 1,536, N = 1,536 took 24 blocks.
+//
+// f32_tile_kernel, more tokens: bound by the double multiply-adds. 64 x 64 outputs a block, 4 x 4 a
+// thread, operands widened when they are put into shared memory (not at every use), the next
+// tile's loads under this tile's arithmetic. While the tiles are fewer than half of the SMs the
+// segments are shared out over blocks, each of which leaves its segments' sums in planes of double that
+// f32_planes_kernel adds up.
+// ---------------------------------------------------------------------------------------
+constexpr int SEGMENT = 256;
+
+__device__ __forceinline__ void copy16(uint32_t dst, const float* src, bool valid) {
+  const int bytes = valid ? 16 : 0;         // 0: the destination is filled with zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+namespace few {
+constexpr int WARPS = 8;
+constexpr int ROWS = 32;                    // weight rows of a block: one a lane
+constexpr int CHUNK = 32;                   // k of a stage
+constexpr int PITCH = CHUNK + 4;            // floats between the rows of a stage
+
+template <int MT>
+struct Layout {
+  static constexpr int STAGES = MT > 8 ? 3 : 4;                 // what eight warps' rings leave room for
+  static constexpr int W_FLOATS = ROWS * PITCH;
+  static constexpr int X_FLOATS = MT * CHUNK;
+  static constexpr int STAGE_FLOATS = W_FLOATS + X_FLOATS;
+  static constexpr int RING_BYTES = STAGES * STAGE_FLOATS * 4;
+  static constexpr int WIDE_BYTES = MT * CHUNK * 8;             // the tokens' values of a chunk in double, [token][k]
+  static constexpr int WARP_BYTES = RING_BYTES + WIDE_BYTES;
+  static constexpr int PART_BYTES = MT * ROWS * 8;              // a warp's segment sums, [token][row]
+  static size_t bytes(int warps) { return (size_t)warps * (WARP_BYTES + PART_BYTES); }
+};
+}  // namespace few
+
+template <int MT>
+__global__ void __launch_bounds__(32 * few::WARPS) f32_few_kernel(float* __restrict__ out, const float* __restrict__ x,
+                                                                  const float* __restrict__ w, const float* __restrict__ bias,
+                                                                  const float* __restrict__ residual, int M, int N, int K) {
+  using L = few::Layout<MT>;
+  constexpr int CHUNK = few::CHUNK, PITCH = few::PITCH, STAGES = L::STAGES;
+  constexpr int CHUNKS_PER_SEGMENT = SEGMENT / CHUNK;
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* ring = (float*)(smem + (size_t)warp * L::WARP_BYTES);
+  double* wide = (double*)(smem + (size_t)warp * L::WARP_BYTES + L::RING_BYTES);
+  double* parts = (double*)(smem + (size_t)warps * L::WARP_BYTES);
+  const int n0 = blockIdx.x * few::ROWS;
+  const int segments = (K + SEGMENT - 1) / SEGMENT;
+  // This warp's segments are warp, warp + warps, ...; its chunks run through all of them in order.
+  const int mine = warp < segments ? (segments - warp + warps - 1) / warps : 0;
+  // The last segment may be short: its chunks behind K are left out.
+  const int chunks = mine * CHUNKS_PER_SEGMENT -
+                     (mine > 0 && warp + (mine - 1) * warps == segments - 1 ? (segments * SEGMENT - K) / CHUNK : 0);
+  auto chunk_k = [&](int c) { return (warp + (c / CHUNKS_PER_SEGMENT) * warps) * SEGMENT + (c % CHUNKS_PER_SEGMENT) * CHUNK; };
+  const uint32_t ring_address = (uint32_t)__cvta_generic_to_shared(ring);
+  auto fetch = [&](int c) {
+    if (c < chunks) {
+      const int k0 = chunk_k(c);
+      const uint32_t stage = ring_address + (c % STAGES) * L::STAGE_FLOATS * 4;
+      const int piece = (lane & 7) * 4;       // eight lanes bring a row's 32 k
+#pragma unroll
+      for (int i = 0; i < few::ROWS / 4; ++i) {
+        const int row = i * 4 + (lane >> 3);
+        const bool valid = n0 + row < N && k0 + piece < K;
+        copy16(stage + (row * PITCH + piece) * 4, valid ? w + (size_t)(n0 + row) * K + k0 + piece : w, valid);
+      }
+#pragma unroll
+      for (int i = 0; i < (MT + 3) / 4; ++i) {
+        const int m = i * 4 + (lane >> 3);
+        const bool valid = m < M && k0 + piece < K;
+        if (m < MT) copy16(stage + (L::W_FLOATS + m * CHUNK + piece) * 4, valid ? x + (size_t)m * K + k0 + piece : x, valid);
+      }
+    }
+    copy_commit();                            // one group per chunk, empty ones too: the waits count groups
+  };
+  dependent_launch_prologue();
+#pragma unroll
+  for (int c = 0; c < STAGES - 1; ++c) fetch(c);
+
+  // The outputs that this thread adds up, a round's segments in their order.
+  constexpr int OUTPUTS = (MT * few::ROWS + 31) / 32;          // at most, when one warp runs
+  double total[OUTPUTS];
+#pragma unroll
+  for (int i = 0; i < OUTPUTS; ++i) total[i] = 0.0;
+  const int rounds = (segments + warps - 1) / warps;
+  int c = 0;
+  for (int round = 0; round < rounds; ++round) {
+    if (round < mine) {
+      double acc[MT];
+#pragma unroll
+      for (int m = 0; m < MT; ++m) acc[m] = 0.0;
+      for (int i = 0; i < CHUNKS_PER_SEGMENT && c < chunks; ++i, ++c) {
+        copy_wait<STAGES - 2>();
+        __syncwarp();                         // every lane's copies of this chunk are there, and all are done with the chunk before
+        fetch(c + STAGES - 1);
+        const float* stage = ring + (c % STAGES) * L::STAGE_FLOATS;
+#pragma unroll
+        for (int m = 0; m < MT; ++m) wide[m * CHUNK + lane] = (double)stage[L::W_FLOATS + m * CHUNK + lane];
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < CHUNK; k += 4) {
+          const float4 w4 = *(const float4*)(stage + lane * PITCH + k);
+          const double w0 = (double)w4.x, w1 = (double)w4.y, w2 = (double)w4.z, w3 = (double)w4.w;
+#pragma unroll
+          for (int m = 0; m < MT; ++m) {
+            const double2 x01 = *(const double2*)(wide + m * CHUNK + k), x23 = *(const double2*)(wide + m * CHUNK + k + 2);
+            acc[m] = fma(x23.y, w3, fma(x23.x, w2, fma(x01.y, w1, fma(x01.x, w0, acc[m]))));
+          }
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < MT; ++m) parts[(warp * MT + m) * few::ROWS + lane] = acc[m];
+    }
+    __syncthreads();
+    const int present = min(warps, segments - round * warps);
+#pragma unroll
+    for (int i = 0; i < OUTPUTS; ++i) {
+      const int o = threadIdx.x + i * blockDim.x;
+      if (o < MT * few::ROWS)
+        for (int s = 0; s < present; ++s) total[i] += parts[s * MT * few::ROWS + o];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < OUTPUTS; ++i) {
+    const int o = threadIdx.x + i * blockDim.x;
+    const int m = o / few::ROWS, n = n0 + o % few::ROWS;
+    if (o >= MT * few::ROWS || m >= M || n >= N) continue;
+    double v = total[i];
+    if (bias != nullptr) v += (double)bias[n];
+    if (residual != nullptr) v += (double)residual[(size_t)m * N + n];
+    out[(size_t)m * N + n] = (float)v;
+  }
+}
+
+template <int MT>
+int launch_few(float* out, const float* x, const float* w, const float* bias, const float* residual, int M, int N, int K, cudaStream_t s) {
+  using L = few::Layout<MT>;
+  const int segments = (K + SEGMENT - 1) / SEGMENT;
+  const int warps = segments < few::WARPS ? segments : few::WARPS;
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(f32_few_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::bytes(few::WARPS));
+  if (configured != cudaSuccess) return fail(100, "linear_f32: %s", cudaGetErrorString(configured));
+  launch_kernel(f32_few_kernel<MT>, dim3((N + few::ROWS - 1) / few::ROWS), 32 * warps, L::bytes(warps), s, out, x, w, bias, residual, M, N, K);
+  return check_launch("linear_f32");
+}
+
+namespace tiled {
+constexpr int TILE = 64, STEP = 16;         // outputs of a block along M and along N; k of a step
+constexpr int PITCH = TILE + 2;             // doubles between the k of a step
+}  // namespace tiled
+
+// planes (double [segments, M, N]): null, or where this block's segments' sums go instead of the output.
+__global__ void __launch_bounds__(256, 2) f32_tile_kernel(float* __restrict__ out, double* __restrict__ planes, const float* __restrict__ x,
+                                                       const float* __restrict__ w, const float* __restrict__ bias,
+                                                       const float* __restrict__ residual, int M, int N, int K, int segments_per_block) {
+  constexpr int TILE = tiled::TILE, STEP = tiled::STEP, PITCH = tiled::PITCH;
+  __shared__ __align__(16) double xs[2][STEP][PITCH];
+  __shared__ __align__(16) double ws[2][STEP][PITCH];
+  dependent_launch_prologue();
+  const int tid = threadIdx.x;
+  const int m0 = blockIdx.y * TILE, n0 = blockIdx.x * TILE;
+  const int segments = (K + SEGMENT - 1) / SEGMENT;
+  const int first_segment = blockIdx.z * segments_per_block, end_segment = min(segments, first_segment + segments_per_block);
+  // Threads of a warp: eight groups of four columns x four groups of four rows.
+  const int warp = tid >> 5, lane = tid & 31;
+  const int col = ((warp & 1) * 8 + (lane & 7)) * 4, row = ((warp >> 1) * 4 + (lane >> 3)) * 4;
+  const int load_row = tid >> 2, load_k = (tid & 3) * 4;
+  const float* x_src = x + (size_t)(m0 + load_row) * K + load_k;
+  const float* w_src = w + (size_t)(n0 + load_row) * K + load_k;
+  const bool x_valid = m0 + load_row < M, w_valid = n0 + load_row < N;
+  const int k_begin = first_segment * SEGMENT, k_end = min(K, end_segment * SEGMENT);
+  float4 xr, wr;
+  auto read = [&](int k) {
+    const bool inside = k + load_k < k_end;
+    xr = x_valid && inside ? *(const float4*)(x_src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    wr = w_valid && inside ? *(const float4*)(w_src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  auto put = [&](int b) {
+    xs[b][load_k][load_row] = xr.x; xs[b][load_k + 1][load_row] = xr.y;
+    xs[b][load_k + 2][load_row] = xr.z; xs[b][load_k + 3][load_row] = xr.w;
+    ws[b][load_k][load_row] = wr.x; ws[b][load_k + 1][load_row] = wr.y;
+    ws[b][load_k + 2][load_row] = wr.z; ws[b][load_k + 3][load_row] = wr.w;
+  };
+  double acc[4][4], total[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = total[i][j] = 0.0;
+  read(k_begin);
+  put(0);
+  __syncthreads();
+  int b = 0;
+  for (int k0 = k_begin; k0 < k_end; k0 += STEP) {
+    if (k0 + STEP < k_end) read(k0 + STEP);
+#pragma unroll
+    for (int k = 0; k < STEP; ++k) {
+      const double2 a01 = *(const double2*)&xs[b][k][row], a23 = *(const double2*)&xs[b][k][row + 2];
+      const double2 b01 = *(const double2*)&ws[b][k][col], b23 = *(const double2*)&ws[b][k][col + 2];
+      const double a[4] = {a01.x, a01.y, a23.x, a23.y}, v[4] = {b01.x, b01.y, b23.x, b23.y};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], v[j], acc[i][j]);
+    }
+    if ((k0 + STEP) % SEGMENT == 0 || k0 + STEP >= k_end) {       // a segment ends
+      if (planes != nullptr) {
+        double* plane = planes + (size_t)(k0 / SEGMENT) * M * N;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (m0 + row + i < M && n0 + col + j < N) plane[(size_t)(m0 + row + i) * N + n0 + col + j] = acc[i][j];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          total[i][j] += acc[i][j];
+          acc[i][j] = 0.0;
+        }
+    }
+    if (k0 + STEP < k_end) put(b ^ 1);      // everyone has left that buffer: the barrier of the step before
+    __syncthreads();
+    b ^= 1;
+  }
+  if (planes != nullptr) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + row + i;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int n = n0 + col + j;
+      if (m >= M || n >= N) continue;
+      double v = total[i][j];
+      if (bias != nullptr) v += (double)bias[n];
+      if (residual != nullptr) v += (double)residual[(size_t)m * N + n];
+      out[(size_t)m * N + n] = (float)v;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) f32_planes_kernel(float* __restrict__ out, const double* __restrict__ planes,
+                                                         const float* __restrict__ bias, const float* __restrict__ residual,
+                                                         int segments, long long count, int N) {
+  dependent_launch_prologue();
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= count) return;
+  double v = 0.0;
+#pragma unroll 8
+  for (int s = 0; s < segments; ++s) v += planes[(size_t)s * count + i];
+  if (bias != nullptr) v += (double)bias[i % N];
+  if (residual != nullptr) v += (double)residual[i];
+  out[i] = (float)v;
+}
+
+int sm_count() {
+  static const int count = [] {
+    int device = 0, n = 148;
+    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+    return n;
+  }();
+  return count;
+}
+
 }  // namespace
+
+constexpr int F32_FEW_TOKENS = 16;
+
+// How many planes of doubles [M, N] `pae_linear_f32` needs as scratch (0: none): the K segments, when the
+// tiles would leave more than half of the SMs idle.
+PAE_EXPORT int pae_linear_f32_planes(int M, int N, int K) {
+  const int segments = (K + SEGMENT - 1) / SEGMENT;
+  if (M <= F32_FEW_TOKENS || segments < 2) return 0;
+  const long long tiles = (long long)((M + tiled::TILE - 1) / tiled::TILE) * ((N + tiled::TILE - 1) / tiled::TILE);
+  return tiles * 2 <= sm_count() ? segments : 0;
+}
+
+// out[M, N] = x[M, K] . w[N, K]^T (+ bias[N]) (+ residual[M, N]), all float32, sums in double; K a multiple of 4,
+// x and w on 16-byte boundaries. planes: double scratch [pae_linear_f32_planes(M, N, K), M, N], or null when that is 0.
+PAE_EXPORT int pae_linear_f32(float* out, const float* x, const float* w, const float* bias, const float* residual, int M, int N, int K,
+                              double* planes, void* stream) {
+  if (M == 0 || N == 0) return 0;
+  if (K % 4 || K < 4) return fail(2, "linear_f32: K = %d is not a positive multiple of 4", K);
+  if (((uintptr_t)x | (uintptr_t)w) & 15) return fail(2, "linear_f32: an operand does not start on a 16-byte boundary");
+  cudaStream_t s = (cudaStream_t)stream;
+  if (M == 1) return launch_few<1>(out, x, w, bias, residual, M, N, K, s);
+  if (M == 2) return launch_few<2>(out, x, w, bias, residual, M, N, K, s);
+  if (M <= 4) return launch_few<4>(out, x, w, bias, residual, M, N, K, s);
+  if (M <= 8) return launch_few<8>(out, x, w, bias, residual, M, N, K, s);
+  if (M <= F32_FEW_TOKENS) return launch_few<16>(out, x, w, bias, residual, M, N, K, s);
+  const int tiles_m = (M + tiled::TILE - 1) / tiled::TILE, tiles_n = (N + tiled::TILE - 1) / tiled::TILE;
+  if (tiles_m > 65535) return fail(3, "linear_f32: %d rows are more than one launch takes", M);
+  const int segments = (K + SEGMENT - 1) / SEGMENT;
+  const bool split = pae_linear_f32_planes(M, N, K) > 0;
+  if (split && planes == nullptr) return fail(2, "linear_f32: [%d, %d] x [%d, %d] needs scratch planes", M, K, N, K);
+  int blocks_k = split ? (int)(2LL * sm_count() / ((long long)tiles_m * tiles_n)) : 1;
+  blocks_k = blocks_k > segments ? segments : blocks_k;
+  const int per = (segments + blocks_k - 1) / blocks_k;
+  launch_kernel(f32_tile_kernel, dim3(tiles_n, tiles_m, (segments + per - 1) / per), 256, 0, s, out, split ? planes : nullptr, x, w, bias,
+                residual, M, N, K, per);
+  if (split) {
+    const long long count = (long long)M * N;
+    launch_kernel(f32_planes_kernel, dim3((unsigned)((count + 255) / 256)), 256, 0, s, out, planes, bias, residual, segments, count, N);
+  }
+  return check_launch("linear_f32");
+}
 
 // x_dtype, w_dtype, out_dtype: 0 float32, 1 bfloat16. bias (float32) and residual
 // (out_dtype, may be `out` itself) may be null.

@@ -1,0 +1,52 @@
+"""The float32 products: tokens on both sides of every kernel's range, K and N off every tile, against
+the same sums in float64; and a token's bits whatever else is in its batch."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(m, n, k, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(m, k, device="cuda", generator=gen)
+    w = torch.randn(n, k, device="cuda", generator=gen) * 0.02
+    bias = torch.randn(n, device="cuda", generator=gen)
+    residual = torch.randn(m, n, device="cuda", generator=gen)
+    return x, w, bias, residual
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8, 9, 16, 17, 64, 65, 130])
+@pytest.mark.parametrize("n,k", [(1, 4), (31, 96), (33, 252), (96, 256), (70, 260), (65, 2308), (1537, 1536), (4801, 512), (48, 97)])
+@pytest.mark.parametrize("extras", [False, True])
+def test_float32_product_is_the_rounded_float64_product(m, n, k, extras):
+    from paged_attention_engine_b200.kernels import ops
+
+    x, w, bias, residual = _operands(m, n, k)
+    got = ops.linear(x, w, bias if extras else None, residual if extras else None)
+    want = x.double() @ w.double().T
+    if extras:
+        want = want + bias.double() + residual.double()
+    # One rounding to float32 of a sum in double: half a unit in the last place of the result, and the
+    # sums' own error (2^-53 a step relative to the terms' absolute sum) far below it.
+    terms = x.double().abs() @ w.double().abs().T + (bias.abs().double() + residual.abs().double() if extras else 0.0)
+    assert bool(((got.double() - want).abs() <= want.abs() * 2**-24 + terms * (k + 2) * 2**-52).all())
+
+
+@pytest.mark.parametrize("n,k", [(96, 96), (256, 1536), (1536, 2052), (9600, 512)])
+def test_a_token_has_the_same_bits_in_every_batch(n, k):
+    from paged_attention_engine_b200.kernels import ops
+
+    x, w, bias, residual = _operands(200, n, k, seed=1)
+    whole = ops.linear(x, w, bias, residual)
+    for m in (1, 2, 4, 7, 16, 17, 64, 100):
+        assert torch.equal(ops.linear(x[:m], w, bias, residual[:m]), whole[:m])
+
+
+def test_misaligned_operands_are_taken():
+    from paged_attention_engine_b200.kernels import ops
+
+    x, w, _, _ = _operands(3, 40, 64)
+    shifted = torch.empty(3 * 64 + 1, device="cuda")[1:].view(3, 64).copy_(x)
+    want = x.double() @ w.double().T
+    assert torch.allclose(ops.linear(shifted, w).double(), want, rtol=1e-6, atol=1e-6)
