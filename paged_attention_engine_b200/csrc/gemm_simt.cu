@@ -115,25 +115,29 @@ int launch(void* out, const void* x, const void* w, const float* bias, const voi
 
 // ---------------------------------------------------------------------------------------
 // The float32 products (activations, weights and output all float32, K a multiple of 4, 16-byte
-// aligned operands): K is cut into segments of SEGMENT; a segment's products are added one after
-// the other in double, the segments' sums one after the other to the total, bias and residual
-// to that, and the result is rounded once. Both kernels below keep exactly this order, whatever
-// M is and however K is shared out, so a token's result does not depend on its batch.
+// aligned operands). K is cut into segments of SEGMENT; a segment's products are added one after the other in
+// double, the segments' sums one after the other to the total, bias and residual to that, and the result is rounded
+// once. All kernels below keep exactly this order, whatever M is and however K is shared out (the tensor
+// cores' double-precision instruction adds its four products like four fused multiply-adds in a row; a test of
+// sums that cancel compares them), so a token's result does not depend on its batch.
 //
-// f32_few_kernel, up to 16 tokens: bound by the weights' bytes (up to about 8 tokens; beyond, by
-// the double multiply-adds, 64 a clock and SM). A lane owns a weight row, a warp a segment of
-// 32 rows; a warp's weights pass through a ring of cp.async stages of its own (32 k of 32 rows, rows
-// 144 bytes apart so that the lanes' 16-byte reads meet no bank twice), the tokens' values of a
-// chunk are widened once per warp and read by all lanes at once. The tile kernel before ran 64 x 64
-// tiles with a token's row repeated over nothing: one token, K = 1,536, N = 1,536 took 24 blocks.
+// f32_lane_kernel, one or two tokens: a lane owns a weight row, a warp a segment of 32 rows, plain double
+// multiply-adds. f32_few_kernel, 3 to 32 tokens: the same split, with mma.m8n8k4.f64 (eight weight rows x eight
+// tokens; operands widened from float32, which is exact). Both are bound by the weights' bytes at few tokens and
+// by the chain of a segment's sums; weights pass through a ring of cp.async stages per warp (32 k; rows 144 bytes
+// apart, so that a fragment's reads meet no bank twice).
+// f32_tile_kernel, more tokens: bound by the double products. 64 tokens x 64 weight rows a block, 32 x 32 a warp. While
+// the tiles are fewer than half of the SMs the segments are shared out over blocks, each of which leaves its
+// segments' sums in planes of double that f32_planes_kernel adds up.
 //
-// f32_tile_kernel, more tokens: bound by the double multiply-adds. 64 x 64 outputs a block, 4 x 4 a
-// thread, operands widened when they are put into shared memory (not at every use), the next
-// tile's loads under this tile's arithmetic. While the tiles are fewer than half of the SMs the
-// segments are shared out over blocks, each of which leaves its segments' sums in planes of double that
-// f32_planes_kernel adds up.
+// Measured, us, [17,920, 1,536] and [1,536, 8,960] weights: 1 token 24.0 and 26.0 (16.8 and 8.4 at the copy bandwidth;
+// the eight-token kernel 36 and 40), 8 tokens 37 and 43 (63 and 78 with plain multiply-adds, whose operands meet the shared memory's
+// bandwidth), 60 tokens 168 and 75 (313 and 171), 256 tokens 450 and 574 (1,232 and 1,496): 31 of 37 TFLOP/s.
 // ---------------------------------------------------------------------------------------
-constexpr int SEGMENT = 256;
+constexpr int SEGMENT = 128;
+constexpr int CHUNK = 32;                   // k of a stage
+constexpr int CHUNKS_PER_SEGMENT = SEGMENT / CHUNK;
+constexpr int PITCH = CHUNK + 4;            // floats between the rows of a stage
 
 __device__ __forceinline__ void copy16(uint32_t dst, const float* src, bool valid) {
   const int bytes = valid ? 16 : 0;         // 0: the destination is filled with zeros
@@ -145,39 +149,38 @@ __device__ __forceinline__ void copy_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// c[8 x 8] += a[8 x 4] b[4 x 8]: this lane holds a[lane / 4][lane % 4], b[lane % 4][lane / 4] and
+// c[lane / 4][2 (lane % 4)], c[lane / 4][2 (lane % 4) + 1].
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+
 namespace few {
 constexpr int WARPS = 8;
-constexpr int ROWS = 32;                    // weight rows of a block: one a lane
-constexpr int CHUNK = 32;                   // k of a stage
-constexpr int PITCH = CHUNK + 4;            // floats between the rows of a stage
+constexpr int ROWS = 32;                    // weight rows of a block
 
-template <int MT>
+template <int T>                            // groups of eight tokens
 struct Layout {
-  static constexpr int STAGES = MT > 8 ? 3 : 4;                 // what eight warps' rings leave room for
-  static constexpr int W_FLOATS = ROWS * PITCH;
-  static constexpr int X_FLOATS = MT * CHUNK;
-  static constexpr int STAGE_FLOATS = W_FLOATS + X_FLOATS;
+  static constexpr int TOKENS = 8 * T;
+  static constexpr int STAGES = T == 1 ? 4 : (T == 2 ? 3 : 2);  // what eight warps' rings leave room for
+  static constexpr int STAGE_FLOATS = (ROWS + TOKENS) * PITCH;
   static constexpr int RING_BYTES = STAGES * STAGE_FLOATS * 4;
-  static constexpr int WIDE_BYTES = MT * CHUNK * 8;             // the tokens' values of a chunk in double, [token][k]
-  static constexpr int WARP_BYTES = RING_BYTES + WIDE_BYTES;
-  static constexpr int PART_BYTES = MT * ROWS * 8;              // a warp's segment sums, [token][row]
-  static size_t bytes(int warps) { return (size_t)warps * (WARP_BYTES + PART_BYTES); }
+  static constexpr int PART_BYTES = TOKENS * ROWS * 8;          // a warp's segment sums, [token][row]
+  static size_t bytes(int warps) { return (size_t)warps * (RING_BYTES + PART_BYTES); }
 };
 }  // namespace few
 
-template <int MT>
+template <int T>
 __global__ void __launch_bounds__(32 * few::WARPS) f32_few_kernel(float* __restrict__ out, const float* __restrict__ x,
                                                                   const float* __restrict__ w, const float* __restrict__ bias,
                                                                   const float* __restrict__ residual, int M, int N, int K) {
-  using L = few::Layout<MT>;
-  constexpr int CHUNK = few::CHUNK, PITCH = few::PITCH, STAGES = L::STAGES;
-  constexpr int CHUNKS_PER_SEGMENT = SEGMENT / CHUNK;
+  using L = few::Layout<T>;
+  constexpr int STAGES = L::STAGES, TOKENS = L::TOKENS, ROWS = few::ROWS;
   extern __shared__ __align__(16) uint8_t smem[];
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* ring = (float*)(smem + (size_t)warp * L::WARP_BYTES);
-  double* wide = (double*)(smem + (size_t)warp * L::WARP_BYTES + L::RING_BYTES);
-  double* parts = (double*)(smem + (size_t)warps * L::WARP_BYTES);
-  const int n0 = blockIdx.x * few::ROWS;
+  float* ring = (float*)(smem + (size_t)warp * L::RING_BYTES);
+  double* parts = (double*)(smem + (size_t)warps * L::RING_BYTES);
+  const int n0 = blockIdx.x * ROWS;
   const int segments = (K + SEGMENT - 1) / SEGMENT;
   // This warp's segments are warp, warp + warps, ...; its chunks run through all of them in order.
   const int mine = warp < segments ? (segments - warp + warps - 1) / warps : 0;
@@ -188,20 +191,19 @@ __global__ void __launch_bounds__(32 * few::WARPS) f32_few_kernel(float* __restr
   const uint32_t ring_address = (uint32_t)__cvta_generic_to_shared(ring);
   auto fetch = [&](int c) {
     if (c < chunks) {
-      const int k0 = chunk_k(c);
-      const uint32_t stage = ring_address + (c % STAGES) * L::STAGE_FLOATS * 4;
-      const int piece = (lane & 7) * 4;       // eight lanes bring a row's 32 k
+      const int k = chunk_k(c) + (lane & 7) * 4;                // eight lanes bring a row's 32 k
+      const uint32_t dst = ring_address + ((c % STAGES) * L::STAGE_FLOATS + (lane >> 3) * PITCH + (lane & 7) * 4) * 4;
 #pragma unroll
-      for (int i = 0; i < few::ROWS / 4; ++i) {
-        const int row = i * 4 + (lane >> 3);
-        const bool valid = n0 + row < N && k0 + piece < K;
-        copy16(stage + (row * PITCH + piece) * 4, valid ? w + (size_t)(n0 + row) * K + k0 + piece : w, valid);
+      for (int i = 0; i < ROWS / 4; ++i) {
+        const int n = n0 + i * 4 + (lane >> 3);
+        const bool valid = n < N && k < K;
+        copy16(dst + i * 4 * PITCH * 4, valid ? w + (size_t)n * K + k : w, valid);
       }
 #pragma unroll
-      for (int i = 0; i < (MT + 3) / 4; ++i) {
+      for (int i = 0; i < TOKENS / 4; ++i) {
         const int m = i * 4 + (lane >> 3);
-        const bool valid = m < M && k0 + piece < K;
-        if (m < MT) copy16(stage + (L::W_FLOATS + m * CHUNK + piece) * 4, valid ? x + (size_t)m * K + k0 + piece : x, valid);
+        const bool valid = m < M && k < K;
+        copy16(dst + (ROWS + i * 4) * PITCH * 4, valid ? x + (size_t)m * K + k : x, valid);
       }
     }
     copy_commit();                            // one group per chunk, empty ones too: the waits count groups
@@ -211,10 +213,133 @@ __global__ void __launch_bounds__(32 * few::WARPS) f32_few_kernel(float* __restr
   for (int c = 0; c < STAGES - 1; ++c) fetch(c);
 
   // The outputs that this thread adds up, a round's segments in their order.
-  constexpr int OUTPUTS = (MT * few::ROWS + 31) / 32;          // at most, when one warp runs
+  constexpr int OUTPUTS = TOKENS * ROWS / 32;                  // when one warp runs; an eighth when eight do
   double total[OUTPUTS];
 #pragma unroll
   for (int i = 0; i < OUTPUTS; ++i) total[i] = 0.0;
+  const int rounds = (segments + warps - 1) / warps;
+  int c = 0;
+  for (int round = 0; round < rounds; ++round) {
+    if (round < mine) {
+      double acc[ROWS / 8][T][2];
+#pragma unroll
+      for (int i = 0; i < ROWS / 8; ++i)
+#pragma unroll
+        for (int j = 0; j < T; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+      for (int i = 0; i < CHUNKS_PER_SEGMENT && c < chunks; ++i, ++c) {
+        copy_wait<STAGES - 2>();
+        __syncwarp();                         // every lane's copies of this chunk are there, and all are done with the chunk before
+        fetch(c + STAGES - 1);
+        const float* from = ring + (c % STAGES) * L::STAGE_FLOATS + (lane >> 2) * PITCH + (lane & 3);
+#pragma unroll
+        for (int k = 0; k < CHUNK; k += 4) {
+          double a[ROWS / 8], b[T];
+#pragma unroll
+          for (int r = 0; r < ROWS / 8; ++r) a[r] = (double)from[r * 8 * PITCH + k];
+#pragma unroll
+          for (int j = 0; j < T; ++j) b[j] = (double)from[(ROWS + j * 8) * PITCH + k];
+#pragma unroll
+          for (int r = 0; r < ROWS / 8; ++r)
+#pragma unroll
+            for (int j = 0; j < T; ++j) mma_f64(acc[r][j], a[r], b[j]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < ROWS / 8; ++r)
+#pragma unroll
+        for (int j = 0; j < T; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            parts[(warp * TOKENS + j * 8 + 2 * (lane & 3) + e) * ROWS + r * 8 + (lane >> 2)] = acc[r][j][e];
+    }
+    __syncthreads();
+    const int present = min(warps, segments - round * warps);
+#pragma unroll
+    for (int i = 0; i < OUTPUTS; ++i) {
+      const int o = threadIdx.x + i * blockDim.x;
+      if (o < M * ROWS)
+        for (int s = 0; s < present; ++s) total[i] += parts[s * TOKENS * ROWS + o];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < OUTPUTS; ++i) {
+    const int o = threadIdx.x + i * blockDim.x;
+    const int m = o / ROWS, n = n0 + o % ROWS;
+    if (m >= M || n >= N) continue;
+    double v = total[i];
+    if (bias != nullptr) v += (double)bias[n];
+    if (residual != nullptr) v += (double)residual[(size_t)m * N + n];
+    out[(size_t)m * N + n] = (float)v;
+  }
+}
+
+template <int T>
+int launch_few(float* out, const float* x, const float* w, const float* bias, const float* residual, int M, int N, int K, cudaStream_t s) {
+  using L = few::Layout<T>;
+  const int segments = (K + SEGMENT - 1) / SEGMENT;
+  const int warps = segments < few::WARPS ? segments : few::WARPS;
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(f32_few_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::bytes(few::WARPS));
+  if (configured != cudaSuccess) return fail(100, "linear_f32: %s", cudaGetErrorString(configured));
+  launch_kernel(f32_few_kernel<T>, dim3((N + few::ROWS - 1) / few::ROWS), 32 * warps, L::bytes(warps), s, out, x, w, bias, residual, M, N, K);
+  return check_launch("linear_f32");
+}
+
+namespace lane_rows {
+constexpr int WARPS = 16;
+constexpr int ROWS = 32;                    // weight rows of a block: one a lane
+constexpr int STAGES = 2;
+
+template <int MT>
+struct Layout {
+  static constexpr int STAGE_FLOATS = ROWS * PITCH + MT * CHUNK;
+  static constexpr int WARP_BYTES = STAGES * STAGE_FLOATS * 4 + MT * CHUNK * 8;    // the ring, and a chunk's token values in double
+  static constexpr int PART_BYTES = MT * ROWS * 8;              // a warp's segment sums, [token][row]
+  static size_t bytes(int warps) { return (size_t)warps * (WARP_BYTES + PART_BYTES); }
+};
+}  // namespace lane_rows
+
+template <int MT>
+__global__ void __launch_bounds__(32 * lane_rows::WARPS) f32_lane_kernel(float* __restrict__ out, const float* __restrict__ x,
+                                                                         const float* __restrict__ w, const float* __restrict__ bias,
+                                                                         const float* __restrict__ residual, int M, int N, int K) {
+  using L = lane_rows::Layout<MT>;
+  constexpr int STAGES = lane_rows::STAGES, ROWS = lane_rows::ROWS;
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* ring = (float*)(smem + (size_t)warp * L::WARP_BYTES);
+  double* wide = (double*)(ring + STAGES * L::STAGE_FLOATS);
+  double* parts = (double*)(smem + (size_t)warps * L::WARP_BYTES);
+  const int n0 = blockIdx.x * ROWS;
+  const int segments = (K + SEGMENT - 1) / SEGMENT;
+  const int mine = warp < segments ? (segments - warp + warps - 1) / warps : 0;
+  const int chunks = mine * CHUNKS_PER_SEGMENT -
+                     (mine > 0 && warp + (mine - 1) * warps == segments - 1 ? (segments * SEGMENT - K) / CHUNK : 0);
+  auto chunk_k = [&](int c) { return (warp + (c / CHUNKS_PER_SEGMENT) * warps) * SEGMENT + (c % CHUNKS_PER_SEGMENT) * CHUNK; };
+  const uint32_t ring_address = (uint32_t)__cvta_generic_to_shared(ring);
+  auto fetch = [&](int c) {
+    if (c < chunks) {
+      const int k = chunk_k(c) + (lane & 7) * 4;
+      const uint32_t stage = ring_address + (c % STAGES) * L::STAGE_FLOATS * 4;
+#pragma unroll
+      for (int i = 0; i < ROWS / 4; ++i) {
+        const int row = i * 4 + (lane >> 3);
+        const bool valid = n0 + row < N && k < K;
+        copy16(stage + (row * PITCH + (lane & 7) * 4) * 4, valid ? w + (size_t)(n0 + row) * K + k : w, valid);
+      }
+      const int m = lane >> 3;
+      const bool valid = m < M && k < K;
+      if (m < MT) copy16(stage + (ROWS * PITCH + m * CHUNK + (lane & 7) * 4) * 4, valid ? x + (size_t)m * K + k : x, valid);
+    }
+    copy_commit();
+  };
+  dependent_launch_prologue();
+#pragma unroll
+  for (int c = 0; c < STAGES; ++c) fetch(c);
+  double total[MT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) total[m] = 0.0;
   const int rounds = (segments + warps - 1) / warps;
   int c = 0;
   for (int round = 0; round < rounds; ++round) {
@@ -223,43 +348,45 @@ __global__ void __launch_bounds__(32 * few::WARPS) f32_few_kernel(float* __restr
 #pragma unroll
       for (int m = 0; m < MT; ++m) acc[m] = 0.0;
       for (int i = 0; i < CHUNKS_PER_SEGMENT && c < chunks; ++i, ++c) {
-        copy_wait<STAGES - 2>();
-        __syncwarp();                         // every lane's copies of this chunk are there, and all are done with the chunk before
-        fetch(c + STAGES - 1);
-        const float* stage = ring + (c % STAGES) * L::STAGE_FLOATS;
-#pragma unroll
-        for (int m = 0; m < MT; ++m) wide[m * CHUNK + lane] = (double)stage[L::W_FLOATS + m * CHUNK + lane];
+        copy_wait<STAGES - 1>();
         __syncwarp();
+        const float* stage = ring + (c % STAGES) * L::STAGE_FLOATS;
+        float4 w4[CHUNK / 4];                 // the chunk leaves its stage at once, which is then filled again
 #pragma unroll
-        for (int k = 0; k < CHUNK; k += 4) {
-          const float4 w4 = *(const float4*)(stage + lane * PITCH + k);
-          const double w0 = (double)w4.x, w1 = (double)w4.y, w2 = (double)w4.z, w3 = (double)w4.w;
+        for (int q = 0; q < CHUNK / 4; ++q) w4[q] = *(const float4*)(stage + lane * PITCH + 4 * q);
+#pragma unroll
+        for (int m = 0; m < MT; ++m) wide[m * CHUNK + lane] = (double)stage[ROWS * PITCH + m * CHUNK + lane];
+        __syncwarp();
+        fetch(c + STAGES);
+#pragma unroll
+        for (int q = 0; q < CHUNK / 4; ++q) {
+          const double w0 = (double)w4[q].x, w1 = (double)w4[q].y, w2 = (double)w4[q].z, w3 = (double)w4[q].w;
 #pragma unroll
           for (int m = 0; m < MT; ++m) {
-            const double2 x01 = *(const double2*)(wide + m * CHUNK + k), x23 = *(const double2*)(wide + m * CHUNK + k + 2);
+            const double2 x01 = *(const double2*)(wide + m * CHUNK + 4 * q), x23 = *(const double2*)(wide + m * CHUNK + 4 * q + 2);
             acc[m] = fma(x23.y, w3, fma(x23.x, w2, fma(x01.y, w1, fma(x01.x, w0, acc[m]))));
           }
         }
       }
 #pragma unroll
-      for (int m = 0; m < MT; ++m) parts[(warp * MT + m) * few::ROWS + lane] = acc[m];
+      for (int m = 0; m < MT; ++m) parts[(warp * MT + m) * ROWS + lane] = acc[m];
     }
     __syncthreads();
-    const int present = min(warps, segments - round * warps);
+    // The first warp adds a round's segments up in their order.
+    if (warp == 0) {
+      const int present = min(warps, segments - round * warps);
 #pragma unroll
-    for (int i = 0; i < OUTPUTS; ++i) {
-      const int o = threadIdx.x + i * blockDim.x;
-      if (o < MT * few::ROWS)
-        for (int s = 0; s < present; ++s) total[i] += parts[s * MT * few::ROWS + o];
+      for (int m = 0; m < MT; ++m)
+        for (int s = 0; s < present; ++s) total[m] += parts[(s * MT + m) * ROWS + lane];
     }
-    __syncthreads();
+    if (round + 1 < rounds) __syncthreads();
   }
+  const int n = n0 + lane;
+  if (warp != 0 || n >= N) return;
 #pragma unroll
-  for (int i = 0; i < OUTPUTS; ++i) {
-    const int o = threadIdx.x + i * blockDim.x;
-    const int m = o / few::ROWS, n = n0 + o % few::ROWS;
-    if (o >= MT * few::ROWS || m >= M || n >= N) continue;
-    double v = total[i];
+  for (int m = 0; m < MT; ++m) {
+    if (m >= M) continue;
+    double v = total[m];
     if (bias != nullptr) v += (double)bias[n];
     if (residual != nullptr) v += (double)residual[(size_t)m * N + n];
     out[(size_t)m * N + n] = (float)v;
@@ -267,109 +394,109 @@ __global__ void __launch_bounds__(32 * few::WARPS) f32_few_kernel(float* __restr
 }
 
 template <int MT>
-int launch_few(float* out, const float* x, const float* w, const float* bias, const float* residual, int M, int N, int K, cudaStream_t s) {
-  using L = few::Layout<MT>;
+int launch_lane(float* out, const float* x, const float* w, const float* bias, const float* residual, int M, int N, int K, cudaStream_t s) {
+  using L = lane_rows::Layout<MT>;
   const int segments = (K + SEGMENT - 1) / SEGMENT;
-  const int warps = segments < few::WARPS ? segments : few::WARPS;
+  const int warps = segments < lane_rows::WARPS ? segments : lane_rows::WARPS;
   static const cudaError_t configured =
-      cudaFuncSetAttribute(f32_few_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::bytes(few::WARPS));
+      cudaFuncSetAttribute(f32_lane_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::bytes(lane_rows::WARPS));
   if (configured != cudaSuccess) return fail(100, "linear_f32: %s", cudaGetErrorString(configured));
-  launch_kernel(f32_few_kernel<MT>, dim3((N + few::ROWS - 1) / few::ROWS), 32 * warps, L::bytes(warps), s, out, x, w, bias, residual, M, N, K);
+  launch_kernel(f32_lane_kernel<MT>, dim3((N + lane_rows::ROWS - 1) / lane_rows::ROWS), 32 * warps, L::bytes(warps), s, out, x, w, bias, residual, M, N, K);
   return check_launch("linear_f32");
 }
 
 namespace tiled {
-constexpr int TILE = 64, STEP = 16;         // outputs of a block along M and along N; k of a step
-constexpr int PITCH = TILE + 2;             // doubles between the k of a step
+constexpr int TILE = 64;                    // tokens and weight rows of a block
+constexpr int STAGES = 3;
+constexpr int STAGE_FLOATS = 2 * TILE * PITCH;
+constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_FLOATS * 4;
 }  // namespace tiled
 
 // planes (double [segments, M, N]): null, or where this block's segments' sums go instead of the output.
-__global__ void __launch_bounds__(256, 2) f32_tile_kernel(float* __restrict__ out, double* __restrict__ planes, const float* __restrict__ x,
+__global__ void __launch_bounds__(128, 3) f32_tile_kernel(float* __restrict__ out, double* __restrict__ planes, const float* __restrict__ x,
                                                        const float* __restrict__ w, const float* __restrict__ bias,
                                                        const float* __restrict__ residual, int M, int N, int K, int segments_per_block) {
-  constexpr int TILE = tiled::TILE, STEP = tiled::STEP, PITCH = tiled::PITCH;
-  __shared__ __align__(16) double xs[2][STEP][PITCH];
-  __shared__ __align__(16) double ws[2][STEP][PITCH];
-  dependent_launch_prologue();
-  const int tid = threadIdx.x;
+  constexpr int TILE = tiled::TILE, STAGES = tiled::STAGES;
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * TILE, n0 = blockIdx.x * TILE;
   const int segments = (K + SEGMENT - 1) / SEGMENT;
   const int first_segment = blockIdx.z * segments_per_block, end_segment = min(segments, first_segment + segments_per_block);
-  // Threads of a warp: eight groups of four columns x four groups of four rows.
-  const int warp = tid >> 5, lane = tid & 31;
-  const int col = ((warp & 1) * 8 + (lane & 7)) * 4, row = ((warp >> 1) * 4 + (lane >> 3)) * 4;
-  const int load_row = tid >> 2, load_k = (tid & 3) * 4;
-  const float* x_src = x + (size_t)(m0 + load_row) * K + load_k;
-  const float* w_src = w + (size_t)(n0 + load_row) * K + load_k;
-  const bool x_valid = m0 + load_row < M, w_valid = n0 + load_row < N;
   const int k_begin = first_segment * SEGMENT, k_end = min(K, end_segment * SEGMENT);
-  float4 xr, wr;
-  auto read = [&](int k) {
-    const bool inside = k + load_k < k_end;
-    xr = x_valid && inside ? *(const float4*)(x_src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-    wr = w_valid && inside ? *(const float4*)(w_src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-  };
-  auto put = [&](int b) {
-    xs[b][load_k][load_row] = xr.x; xs[b][load_k + 1][load_row] = xr.y;
-    xs[b][load_k + 2][load_row] = xr.z; xs[b][load_k + 3][load_row] = xr.w;
-    ws[b][load_k][load_row] = wr.x; ws[b][load_k + 1][load_row] = wr.y;
-    ws[b][load_k + 2][load_row] = wr.z; ws[b][load_k + 3][load_row] = wr.w;
-  };
-  double acc[4][4], total[4][4];
+  const int chunks = (k_end - k_begin + CHUNK - 1) / CHUNK;
+  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem);
+  auto fetch = [&](int c) {
+    if (c < chunks) {
+      const int k = k_begin + c * CHUNK + (tid & 7) * 4;
+      const uint32_t dst = ring + ((c % STAGES) * tiled::STAGE_FLOATS + (tid >> 3) * PITCH + (tid & 7) * 4) * 4;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = total[i][j] = 0.0;
-  read(k_begin);
-  put(0);
-  __syncthreads();
-  int b = 0;
-  for (int k0 = k_begin; k0 < k_end; k0 += STEP) {
-    if (k0 + STEP < k_end) read(k0 + STEP);
-#pragma unroll
-    for (int k = 0; k < STEP; ++k) {
-      const double2 a01 = *(const double2*)&xs[b][k][row], a23 = *(const double2*)&xs[b][k][row + 2];
-      const double2 b01 = *(const double2*)&ws[b][k][col], b23 = *(const double2*)&ws[b][k][col + 2];
-      const double a[4] = {a01.x, a01.y, a23.x, a23.y}, v[4] = {b01.x, b01.y, b23.x, b23.y};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], v[j], acc[i][j]);
-    }
-    if ((k0 + STEP) % SEGMENT == 0 || k0 + STEP >= k_end) {       // a segment ends
-      if (planes != nullptr) {
-        double* plane = planes + (size_t)(k0 / SEGMENT) * M * N;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (m0 + row + i < M && n0 + col + j < N) plane[(size_t)(m0 + row + i) * N + n0 + col + j] = acc[i][j];
+      for (int i = 0; i < TILE / 16; ++i) {
+        const int n = n0 + i * 16 + (tid >> 3), m = m0 + i * 16 + (tid >> 3);
+        const bool w_valid = n < N && k < k_end, x_valid = m < M && k < k_end;
+        copy16(dst + i * 16 * PITCH * 4, w_valid ? w + (size_t)n * K + k : w, w_valid);
+        copy16(dst + (TILE + i * 16) * PITCH * 4, x_valid ? x + (size_t)m * K + k : x, x_valid);
       }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          total[i][j] += acc[i][j];
-          acc[i][j] = 0.0;
-        }
     }
-    if (k0 + STEP < k_end) put(b ^ 1);      // everyone has left that buffer: the barrier of the step before
-    __syncthreads();
-    b ^= 1;
+    copy_commit();
+  };
+  dependent_launch_prologue();
+#pragma unroll
+  for (int c = 0; c < STAGES - 1; ++c) fetch(c);
+  const int row0 = (warp & 1) * 32, token0 = (warp >> 1) * 32;      // this warp's quarter of the tile
+  double acc[4][4][2], total[4][4][2];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[r][j][0] = acc[r][j][1] = total[r][j][0] = total[r][j][1] = 0.0;
+  for (int c = 0; c < chunks; ++c) {
+    copy_wait<STAGES - 2>();
+    __syncthreads();                          // this chunk is there, and all are done with the chunk before
+    fetch(c + STAGES - 1);
+    const float* from = (const float*)smem + (c % STAGES) * tiled::STAGE_FLOATS + (lane >> 2) * PITCH + (lane & 3);
+#pragma unroll
+    for (int k = 0; k < CHUNK; k += 4) {
+      double a[4], b[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) a[r] = (double)from[(row0 + r * 8) * PITCH + k];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = (double)from[(TILE + token0 + j * 8) * PITCH + k];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_f64(acc[r][j], a[r], b[j]);
+    }
+    if ((c + 1) % CHUNKS_PER_SEGMENT == 0 || c + 1 == chunks) {     // a segment ends
+      double* plane = planes != nullptr ? planes + (size_t)(first_segment + c / CHUNKS_PER_SEGMENT) * M * N : nullptr;
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            if (plane != nullptr) {
+              const int n = n0 + row0 + r * 8 + (lane >> 2), m = m0 + token0 + j * 8 + 2 * (lane & 3) + e;
+              if (m < M && n < N) plane[(size_t)m * N + n] = acc[r][j][e];
+            }
+            total[r][j][e] += acc[r][j][e];
+            acc[r][j][e] = 0.0;
+          }
+    }
   }
   if (planes != nullptr) return;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + row + i;
+  for (int r = 0; r < 4; ++r) {
+    const int n = n0 + row0 + r * 8 + (lane >> 2);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + col + j;
-      if (m >= M || n >= N) continue;
-      double v = total[i][j];
-      if (bias != nullptr) v += (double)bias[n];
-      if (residual != nullptr) v += (double)residual[(size_t)m * N + n];
-      out[(size_t)m * N + n] = (float)v;
-    }
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int m = m0 + token0 + j * 8 + 2 * (lane & 3) + e;
+        if (m >= M || n >= N) continue;
+        double v = total[r][j][e];
+        if (bias != nullptr) v += (double)bias[n];
+        if (residual != nullptr) v += (double)residual[(size_t)m * N + n];
+        out[(size_t)m * N + n] = (float)v;
+      }
   }
 }
 
@@ -398,7 +525,7 @@ int sm_count() {
 
 }  // namespace
 
-constexpr int F32_FEW_TOKENS = 16;
+constexpr int F32_FEW_TOKENS = 32;
 
 // How many planes of doubles [M, N] `pae_linear_f32` needs as scratch (0: none): the K segments, when the
 // tiles would leave more than half of the SMs idle.
@@ -417,20 +544,22 @@ PAE_EXPORT int pae_linear_f32(float* out, const float* x, const float* w, const 
   if (K % 4 || K < 4) return fail(2, "linear_f32: K = %d is not a positive multiple of 4", K);
   if (((uintptr_t)x | (uintptr_t)w) & 15) return fail(2, "linear_f32: an operand does not start on a 16-byte boundary");
   cudaStream_t s = (cudaStream_t)stream;
-  if (M == 1) return launch_few<1>(out, x, w, bias, residual, M, N, K, s);
-  if (M == 2) return launch_few<2>(out, x, w, bias, residual, M, N, K, s);
-  if (M <= 4) return launch_few<4>(out, x, w, bias, residual, M, N, K, s);
-  if (M <= 8) return launch_few<8>(out, x, w, bias, residual, M, N, K, s);
-  if (M <= F32_FEW_TOKENS) return launch_few<16>(out, x, w, bias, residual, M, N, K, s);
+  if (M <= 2) return M == 1 ? launch_lane<1>(out, x, w, bias, residual, M, N, K, s) : launch_lane<2>(out, x, w, bias, residual, M, N, K, s);
+  if (M <= 8) return launch_few<1>(out, x, w, bias, residual, M, N, K, s);
+  if (M <= 16) return launch_few<2>(out, x, w, bias, residual, M, N, K, s);
+  if (M <= F32_FEW_TOKENS) return launch_few<4>(out, x, w, bias, residual, M, N, K, s);
   const int tiles_m = (M + tiled::TILE - 1) / tiled::TILE, tiles_n = (N + tiled::TILE - 1) / tiled::TILE;
   if (tiles_m > 65535) return fail(3, "linear_f32: %d rows are more than one launch takes", M);
   const int segments = (K + SEGMENT - 1) / SEGMENT;
   const bool split = pae_linear_f32_planes(M, N, K) > 0;
   if (split && planes == nullptr) return fail(2, "linear_f32: [%d, %d] x [%d, %d] needs scratch planes", M, K, N, K);
-  int blocks_k = split ? (int)(2LL * sm_count() / ((long long)tiles_m * tiles_n)) : 1;
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(f32_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiled::SMEM_BYTES);
+  if (configured != cudaSuccess) return fail(100, "linear_f32: %s", cudaGetErrorString(configured));
+  int blocks_k = split ? (int)(3LL * sm_count() / ((long long)tiles_m * tiles_n)) : 1;
   blocks_k = blocks_k > segments ? segments : blocks_k;
   const int per = (segments + blocks_k - 1) / blocks_k;
-  launch_kernel(f32_tile_kernel, dim3(tiles_n, tiles_m, (segments + per - 1) / per), 256, 0, s, out, split ? planes : nullptr, x, w, bias,
+  launch_kernel(f32_tile_kernel, dim3(tiles_n, tiles_m, (segments + per - 1) / per), 128, tiled::SMEM_BYTES, s, out, split ? planes : nullptr, x, w, bias,
                 residual, M, N, K, per);
   if (split) {
     const long long count = (long long)M * N;
