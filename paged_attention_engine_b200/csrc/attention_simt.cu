@@ -160,6 +160,182 @@ int launch(void* out, const void* qkv, const void* keys, const void* values, con
   return check_launch("paged_attention_simt");
 }
 
+// ---------------------------------------------------------------------------------------
+// The float32 form for head sizes 32, 64 and 128. A block owns ROWS query tokens of one request and one
+// query head; its eight warps take the 16-key tiles of the context in turn (tile number modulo 8, whatever
+// the step's shape, so a query's result depends on its own keys only). A lane holds D / 32 dimensions:
+// a warp asks for the 16 keys and the 16 values of a tile at once, straight into registers, forms the lanes' parts
+// of the 16 scores and adds them across the lanes in 16 exchanges (each halves what a lane holds), so a score
+// ends in a lane of its own. Running maximum, sum and output are a warp's own and are merged in the warps'
+// order at the end. Bound by the trips to memory of a warp's tiles, one after the other. The form above walks 32
+// keys at a time with one chain of D multiply-adds per score and a block of 16 query rows for a single one:
+// one token over 68 keys 56.7 us, over 250 keys 157 (12 heads of 128).
+// ---------------------------------------------------------------------------------------
+namespace wide {
+constexpr int WARPS = 8;
+constexpr int KEYS = 16;                     // keys of a tile
+
+template <int DL>
+struct Vec {
+  float v[DL];
+};
+template <int DL>
+__device__ __forceinline__ Vec<DL> load(const float* p) {
+  Vec<DL> r;
+  if constexpr (DL == 4) {
+    const float4 t = *(const float4*)p;
+    r.v[0] = t.x; r.v[1] = t.y; r.v[2] = t.z; r.v[3] = t.w;
+  } else if constexpr (DL == 2) {
+    const float2 t = *(const float2*)p;
+    r.v[0] = t.x; r.v[1] = t.y;
+  } else {
+    r.v[0] = *p;
+  }
+  return r;
+}
+
+// The sum over the lanes of s[k], k = 0..15, ends in the lanes 2 k and 2 k + 1 (lane bits 4..1 are k's bits 3..0).
+__device__ __forceinline__ float sum_across(float (&s)[KEYS], int lane) {
+#pragma unroll
+  for (int width = KEYS / 2; width >= 1; width >>= 1) {
+    const bool upper = (lane & (2 * width)) != 0;
+#pragma unroll
+    for (int i = 0; i < width; ++i) {
+      const float give = upper ? s[i] : s[i + width];
+      const float keep = upper ? s[i + width] : s[i];
+      s[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * width);
+    }
+  }
+  return s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);
+}
+
+template <int DL, int ROWS>
+__global__ void __launch_bounds__(32 * WARPS) paged_attention_f32_kernel(
+    float* __restrict__ out, const float* __restrict__ qkv, const float* __restrict__ keys, const float* __restrict__ values,
+    const int* __restrict__ block_table, int table_width, const int* __restrict__ q_start, const int* __restrict__ q_pos0,
+    const int* __restrict__ kv_len, int heads, int kv_heads, int page_size, float scale, int window) {
+  constexpr int D = 32 * DL;
+  dependent_launch_prologue();
+  __shared__ float merged_max[WARPS][ROWS], merged_sum[WARPS][ROWS];
+  __shared__ __align__(16) float merged_out[WARPS][ROWS][D];
+  const int b = blockIdx.z, h = blockIdx.y;
+  const int first_token = q_start[b];
+  const int q_count = q_start[b + 1] - first_token;
+  const int row0 = blockIdx.x * ROWS;
+  if (row0 >= q_count) return;
+  const int rows = min(ROWS, q_count - row0);
+  const int p0 = q_pos0[b] + row0;                       // position of the first query
+  const int kv_end = min(kv_len[b], p0 + rows);
+  const int kv_begin = window > 0 ? max(0, p0 - window + 1) : 0;
+  const int g = h / (heads / kv_heads);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int* table = block_table + (size_t)b * table_width;
+
+  Vec<DL> q[ROWS];
+  float acc[ROWS][DL], row_max[ROWS], row_sum[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    row_max[r] = -FLT_MAX;
+    row_sum[r] = 0.f;
+#pragma unroll
+    for (int i = 0; i < DL; ++i) acc[r][i] = q[r].v[i] = 0.f;
+    if (r < rows) q[r] = load<DL>(qkv + ((size_t)(first_token + row0 + r) * (heads + 2 * kv_heads) + h) * D + lane * DL);
+  }
+  const int first_tile = kv_begin / KEYS, end_tile = (kv_end + KEYS - 1) / KEYS;
+  const int my_key = lane >> 1;                          // the key of a tile whose score ends in this lane
+  for (int tile = first_tile + (warp - first_tile % WARPS + WARPS) % WARPS; tile < end_tile; tile += WARPS) {
+    const int j = tile * KEYS + my_key;
+    int place = -1;                                      // row of the key in the cache, -1: not seen by any query here
+    if (j >= kv_begin && j < kv_end) {
+      const int page = checked_page(table[checked_table_index(j / page_size, table_width)]);
+      place = (page * kv_heads + g) * page_size + j % page_size;
+    }
+    Vec<DL> k[KEYS], v[KEYS];
+#pragma unroll
+    for (int i = 0; i < KEYS; ++i) {
+      const int at = __shfl_sync(0xffffffffu, place, 2 * i);
+#pragma unroll
+      for (int e = 0; e < DL; ++e) k[i].v[e] = v[i].v[e] = 0.f;
+      if (at >= 0) {
+        k[i] = load<DL>(keys + (size_t)at * D + lane * DL);
+        v[i] = load<DL>(values + (size_t)at * D + lane * DL);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      if (r >= rows) break;
+      float s[KEYS];
+#pragma unroll
+      for (int i = 0; i < KEYS; ++i) {
+        s[i] = q[r].v[0] * k[i].v[0];
+#pragma unroll
+        for (int e = 1; e < DL; ++e) s[i] = fmaf(q[r].v[e], k[i].v[e], s[i]);
+      }
+      const float dot = sum_across(s, lane);
+      const int pos = p0 + r;
+      const bool seen = place >= 0 && j <= pos && (window <= 0 || pos - j < window);
+      const float score = seen ? dot * scale : -FLT_MAX;
+      float tile_max = score;
+#pragma unroll
+      for (int o = 16; o > 1; o >>= 1) tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, o));
+      const float new_max = fmaxf(row_max[r], tile_max);
+      const float rescale = row_max[r] == -FLT_MAX ? 0.f : expf(row_max[r] - new_max);
+      const float p = seen ? expf(score - new_max) : 0.f;
+      float tile_sum = p;
+#pragma unroll
+      for (int o = 16; o > 1; o >>= 1) tile_sum += __shfl_xor_sync(0xffffffffu, tile_sum, o);
+      row_sum[r] = row_sum[r] * rescale + tile_sum;
+      row_max[r] = new_max;
+#pragma unroll
+      for (int e = 0; e < DL; ++e) acc[r][e] *= rescale;
+#pragma unroll
+      for (int i = 0; i < KEYS; ++i) {
+        const float weight = __shfl_sync(0xffffffffu, p, 2 * i);
+#pragma unroll
+        for (int e = 0; e < DL; ++e) acc[r][e] = fmaf(weight, v[i].v[e], acc[r][e]);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    if (lane == 0) {
+      merged_max[warp][r] = row_max[r];
+      merged_sum[warp][r] = row_sum[r];
+    }
+#pragma unroll
+    for (int e = 0; e < DL; ++e) merged_out[warp][r][lane * DL + e] = acc[r][e];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < rows * D; i += 32 * WARPS) {
+    const int r = i / D, dim = i % D;
+    float top = -FLT_MAX;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) top = fmaxf(top, merged_max[w][r]);
+    float sum = 0.f, value = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+      const float factor = merged_max[w][r] == -FLT_MAX ? 0.f : expf(merged_max[w][r] - top);
+      sum += merged_sum[w][r] * factor;
+      value = fmaf(merged_out[w][r][dim], factor, value);
+    }
+    out[((size_t)(first_token + row0 + r) * heads + h) * D + dim] = sum > 0.f ? value * (1.f / sum) : 0.f;
+  }
+}
+
+template <int DL>
+int launch(float* out, const float* qkv, const float* keys, const float* values, const int* block_table, int table_width,
+           const int* q_start, const int* q_pos0, const int* kv_len, int seqs, int max_q_len, int heads, int kv_heads,
+           int page_size, float scale, int window, cudaStream_t s) {
+  if (max_q_len == 1)
+    launch_kernel(paged_attention_f32_kernel<DL, 1>, dim3(1, heads, seqs), 32 * WARPS, 0, s, out, qkv, keys, values, block_table, table_width,
+                  q_start, q_pos0, kv_len, heads, kv_heads, page_size, scale, window);
+  else
+    launch_kernel(paged_attention_f32_kernel<DL, 4>, dim3((max_q_len + 3) / 4, heads, seqs), 32 * WARPS, 0, s, out, qkv, keys, values,
+                  block_table, table_width, q_start, q_pos0, kv_len, heads, kv_heads, page_size, scale, window);
+  return check_launch("paged_attention_simt");
+}
+}  // namespace wide
+
 }  // namespace
 
 // out [tokens, heads, d]; qkv [tokens, heads + 2 kv_heads, d] (queries are read from it);
@@ -175,6 +351,13 @@ PAE_EXPORT int pae_paged_attention_simt(void* out, const void* qkv, const void* 
   if (heads > 65535 || seqs > 65535) return fail(3, "paged_attention_simt: %d heads x %d requests exceed one launch", heads, seqs);
   if (page_size < 1) return fail(2, "paged_attention_simt: page size %d", page_size);
   cudaStream_t s = (cudaStream_t)stream;
+  // The wide form reads 16 bytes at a time: operands of other alignments, and other head sizes, take the general one.
+  const bool aligned = (((uintptr_t)qkv | (uintptr_t)keys | (uintptr_t)values) & 15) == 0;
+  if (dtype == kF32 && aligned && (d == 32 || d == 64 || d == 128)) {
+    const auto launch_wide = d == 32 ? wide::launch<1> : (d == 64 ? wide::launch<2> : wide::launch<4>);
+    return launch_wide((float*)out, (const float*)qkv, (const float*)keys, (const float*)values, block_table, table_width, q_start, q_pos0,
+                       kv_len, seqs, max_q_len, heads, kv_heads, page_size, scale, window, s);
+  }
   if (dtype == kF32)
     return launch<float>(out, qkv, keys, values, block_table, table_width, q_start, q_pos0, kv_len, seqs, max_q_len, heads, kv_heads, d, page_size, scale, window, s);
   if (dtype == kBF16)
