@@ -468,6 +468,62 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// One thread's part of a tile's epilogue: its row of the accumulator at `lane_address`, and of the tile's PBN columns
+// the range of its warp (`share`: which of the warps of its quarter of the rows).
+template <int PBN, int GATE>
+__device__ __forceinline__ void tile_epilogue(const Params& p, uint32_t lane_address, int share, int row, int rows_end, int tile_b,
+                                              size_t plane_offset, bool rotating, float (&cs_a)[16], float (&sn_a)[16], int slot) {
+  // The warps of a quarter of the rows share the tile's columns in equal ranges that end
+  // on a multiple of 32 columns (a gate block with its up block) or of the head size.
+  const int unit = p.rotary ? p.head_dim : 32;
+  const int range = ((PBN + EPILOGUE_SHARES - 1) / EPILOGUE_SHARES + unit - 1) / unit * unit;
+  const int col_begin = min(share * range, PBN), col_end = min(col_begin + range, PBN);
+  if (p.rotary) {
+    // 16 columns of each half of a head at a time; the token's cosines and sines of those
+    // 16 frequencies are read once and serve every head of the tile, and those of the next
+    // 16 are on their way while these are used.
+    const int d = p.head_dim, half = d >> 1;
+    auto heads_of = [&](int f0, const float* cs, const float* sn) {
+#pragma unroll 1
+      for (int head0 = col_begin; head0 < col_end; head0 += d) {
+        float lo[16], hi[16];
+        tmem_load16(lane_address + head0 + f0, lo);
+        tmem_load16(lane_address + head0 + half + f0, hi);
+        if (row < p.rows_a && tile_b * PBN + head0 < p.rows_b)
+          store_rotary_chunks(p, row, (tile_b * PBN + head0) / d, f0, lo, hi, cs, sn, slot);
+      }
+    };
+#pragma unroll 1
+    for (int f0 = 0; f0 < half; f0 += 32) {
+      float cs_b[16], sn_b[16];
+      const bool second = f0 + 16 < half;
+      if (second && rotating) load_angles(p, row, f0 + 16, cs_b, sn_b);
+      heads_of(f0, cs_a, sn_a);
+      if (second) {
+        if (f0 + 32 < half && rotating) load_angles(p, row, f0 + 32, cs_a, sn_a);
+        heads_of(f0 + 16, cs_b, sn_b);
+      }
+    }
+  } else if (p.swiglu) {
+#pragma unroll 1
+    for (int c0 = col_begin; c0 < col_end; c0 += 32) {
+      float gate[16], up[16];
+      tmem_load16(lane_address + c0, gate);
+      tmem_load16(lane_address + c0 + 16, up);
+      const int col0 = tile_b * PBN + c0;
+      if (row < rows_end && col0 < p.rows_b) store_swiglu_chunk<GATE>(p, row, col0, gate, up);
+    }
+  } else {
+#pragma unroll 1
+    for (int c0 = col_begin; c0 < col_end; c0 += 16) {
+      float v[16];
+      tmem_load16(lane_address + c0, v);
+      const int col0 = tile_b * PBN + c0;
+      if (row < rows_end && col0 < p.rows_b) store_row_chunk(p, row, col0, v, plane_offset);
+    }
+  }
+}
+
 // GATE: the gate's activation of the gated epilogue, known when compiled (a choice at run time in that
 // epilogue cost the SiLU models 1 % of a step).
 template <int PBN, int GATE>
@@ -639,55 +695,7 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
       if (!ok) break;
       tcgen05_fence_after();
       const uint32_t lane_address = tmem_base + ((uint32_t)(quadrant * 32) << 16) + acc * ACC;
-      // The warps of a quarter of the rows share the tile's columns in equal ranges that end
-      // on a multiple of 32 columns (a gate block with its up block) or of the head size.
-      const int unit = p.rotary ? p.head_dim : 32;
-      const int range = ((PBN + EPILOGUE_SHARES - 1) / EPILOGUE_SHARES + unit - 1) / unit * unit;
-      const int col_begin = min(share * range, PBN), col_end = min(col_begin + range, PBN);
-      if (p.rotary) {
-        // 16 columns of each half of a head at a time; the token's cosines and sines of those
-        // 16 frequencies are read once and serve every head of the tile, and those of the next
-        // 16 are on their way while these are used.
-        const int d = p.head_dim, half = d >> 1;
-        auto heads_of = [&](int f0, const float* cs, const float* sn) {
-#pragma unroll 1
-          for (int head0 = col_begin; head0 < col_end; head0 += d) {
-            float lo[16], hi[16];
-            tmem_load16(lane_address + head0 + f0, lo);
-            tmem_load16(lane_address + head0 + half + f0, hi);
-            if (row < p.rows_a && tile_b * PBN + head0 < p.rows_b)
-              store_rotary_chunks(p, row, (tile_b * PBN + head0) / d, f0, lo, hi, cs, sn, slot);
-          }
-        };
-#pragma unroll 1
-        for (int f0 = 0; f0 < half; f0 += 32) {
-          float cs_b[16], sn_b[16];
-          const bool second = f0 + 16 < half;
-          if (second && rotating) load_angles(p, row, f0 + 16, cs_b, sn_b);
-          heads_of(f0, cs_a, sn_a);
-          if (second) {
-            if (f0 + 32 < half && rotating) load_angles(p, row, f0 + 32, cs_a, sn_a);
-            heads_of(f0 + 16, cs_b, sn_b);
-          }
-        }
-      } else if (p.swiglu) {
-#pragma unroll 1
-        for (int c0 = col_begin; c0 < col_end; c0 += 32) {
-          float gate[16], up[16];
-          tmem_load16(lane_address + c0, gate);
-          tmem_load16(lane_address + c0 + 16, up);
-          const int col0 = tile_b * PBN + c0;
-          if (row < rows_end && col0 < p.rows_b) store_swiglu_chunk<GATE>(p, row, col0, gate, up);
-        }
-      } else {
-#pragma unroll 1
-        for (int c0 = col_begin; c0 < col_end; c0 += 16) {
-          float v[16];
-          tmem_load16(lane_address + c0, v);
-          const int col0 = tile_b * PBN + c0;
-          if (row < rows_end && col0 < p.rows_b) store_row_chunk(p, row, col0, v, plane_offset);
-        }
-      }
+      tile_epilogue<PBN, GATE>(p, lane_address, share, row, rows_end, tile_b, plane_offset, rotating, cs_a, sn_a, slot);
       tcgen05_fence_before();
       mbar_arrive(tmem_empty_bar(acc));        // this thread has read its part of the accumulator
     }
@@ -698,6 +706,213 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
   if (warp == 1) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, 2 * ACC);
+  }
+}
+
+// ---------------------------------------------------------------------------------------
+// The many-token product by pairs of SMs (cta_group::2): a cluster of two blocks computes 256 x PBN outputs,
+// each block holding 128 of the tokens and half of the weight rows in its shared memory and 128 rows of the
+// accumulator in its tensor memory. The one-block kernel above is held up by what its blocks draw from L2 (48 KB for
+// 128 x 256 x 64 multiply-adds: 15 TB/s at 1.3 PFLOP/s); a pair draws a third less for the same work, and six
+// stages fit instead of four. Both blocks load their own halves, without multicast, and report to the first
+// block's barrier; the first block issues the MMAs for both; commits report to both blocks' barriers. Walk,
+// double-buffered accumulator and epilogue are those of the one-block kernel.
+// ---------------------------------------------------------------------------------------
+template <int PBN>
+struct PairTile {
+  static constexpr int A_BYTES = BM * BK * 2;                 // this block's 128 tokens
+  static constexpr int B_BYTES = PBN / 2 * BK * 2;            // this block's half of the weight rows
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGES = (200 * 1024 / STAGE_BYTES) > 8 ? 8 : 200 * 1024 / STAGE_BYTES;
+  static constexpr int ACC_COLUMNS = 256;
+  static constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_BYTES + 1024 + 256;
+  static_assert(B_BYTES % 1024 == 0, "stages start on 1024 bytes");
+};
+
+__device__ __forceinline__ uint32_t in_block(uint32_t address, uint32_t rank) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(address), "r"(rank));
+  return remote;
+}
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// A load into this block's shared memory that reports to a barrier of either block of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// All MMAs issued so far, reported to the barrier at this offset in both blocks.
+__device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
+               : "memory");
+}
+
+template <int PBN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PERSISTENT_THREADS)
+    gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p,
+                             int tiles_a, int tiles_b) {
+  using T = PairTile<PBN>;
+  constexpr int STAGES = T::STAGES, ACC = T::ACC_COLUMNS;
+  dependent_launch_trigger();
+  if (threadIdx.x == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+  }
+  extern __shared__ uint8_t raw_smem[];
+  const uint32_t raw = smem_u32(raw_smem);
+  const uint32_t base = (raw + 1023u) & ~1023u;               // the same offset in both blocks
+  uint8_t* generic_base = raw_smem + (base - raw);
+  const uint32_t bars = base + STAGES * T::STAGE_BYTES;       // full[S], empty[S], tmem_full[2], tmem_empty[2]
+  volatile uint32_t* tmem_holder = (volatile uint32_t*)(generic_base + STAGES * T::STAGE_BYTES + 8 * (2 * STAGES + 4));
+  volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = blockIdx.x & 1;                            // the first block of the pair issues the MMAs
+  auto full_bar = [&](int s) { return bars + 8u * s; };       // the first block's count for both blocks' loads
+  auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
+  auto tmem_full_bar = [&](int a) { return bars + 8u * (2 * STAGES + a); };
+  auto tmem_empty_bar = [&](int a) { return bars + 8u * (2 * STAGES + 2 + a); };   // the first block's count for both blocks' warps
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(tmem_full_bar(a), 1);
+      mbar_init(tmem_empty_bar(a), 2 * (PERSISTENT_THREADS / 32 - 2));
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_holder)), "r"(2 * ACC) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  cluster_sync();                  // the other block's barriers are set up, too
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
+
+  const int total = tiles_a * tiles_b, step = (int)gridDim.x >> 1;
+  const int k_blocks = p.k_blocks;
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0, issued_b = 0;
+      bool ok = true;
+      // The weights of the first stages are asked for before the wait for the kernel before: they are not written in a step.
+      if ((int)(blockIdx.x >> 1) < total) {
+        const int b_row = (int)(blockIdx.x >> 1) / tiles_a * PBN + rank * (PBN / 2);
+        for (; issued_b < STAGES && issued_b < k_blocks; ++issued_b) {
+          if (rank == 0) mbar_expect_tx(full_bar(issued_b), 2 * T::STAGE_BYTES);
+          tma_load_2d_pair(base + issued_b * T::STAGE_BYTES + T::A_BYTES, &map_b, in_block(full_bar(issued_b), 0), issued_b * BK, b_row);
+        }
+      }
+      dependent_launch_wait();
+      for (int tile = blockIdx.x >> 1; tile < total && ok; tile += step) {
+        const int a_row = (tile % tiles_a * 2 + rank) * BM, b_row = tile / tiles_a * PBN + rank * (PBN / 2);
+        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+          const int s = it % STAGES;
+          if (it >= STAGES && !mbar_wait(empty_bar(s), ((it / STAGES) - 1) & 1, abort_flag, p.error, 1)) {
+            ok = false;
+            break;
+          }
+          const uint32_t a_dst = base + s * T::STAGE_BYTES, report = in_block(full_bar(s), 0);
+          if (it >= issued_b && rank == 0) mbar_expect_tx(full_bar(s), 2 * T::STAGE_BYTES);
+          tma_load_2d_pair(a_dst, &map_a, report, kb * BK, a_row);
+          if (it >= issued_b) tma_load_2d_pair(a_dst + T::A_BYTES, &map_b, report, kb * BK, b_row);
+        }
+      }
+      if (*abort_flag && rank == 0) {      // both blocks' loads report here; the other block waits for this one at the end
+        for (int i = max(0, it - STAGES); i < it; ++i)
+          for (uint32_t t = 0; t < WAIT_LIMIT && !mbar_try_wait(full_bar(i % STAGES), (i / STAGES) & 1); ++t) __nanosleep(64);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc = instruction_descriptor(2 * BM, PBN);
+      const uint64_t a_desc0 = smem_descriptor(base);
+      const uint64_t b_desc0 = smem_descriptor(base + T::A_BYTES);
+      int local = 0, s = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x >> 1; tile < total && ok; tile += step) {
+        const int acc = local & 1, use = local >> 1;
+        ++local;
+        if (local > 2) ok = mbar_wait(tmem_empty_bar(acc), (use - 1) & 1, abort_flag, p.error, 4);
+        if (!ok) break;
+        tcgen05_fence_after();
+        const uint32_t tmem_acc = tmem_base + acc * ACC;
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          if (!mbar_try_wait(full_bar(s), phase)) ok = mbar_wait(full_bar(s), phase, abort_flag, p.error, 2);
+          if (!ok) break;
+          tcgen05_fence_after();
+          const uint64_t stage_offset = (uint64_t)(uint32_t)(s * (T::STAGE_BYTES >> 4));
+          const uint64_t a_desc = a_desc0 + stage_offset, b_desc = b_desc0 + stage_offset;
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_bf16_pair(tmem_acc, a_desc + (uint64_t)(k * UMMA_K * 2 >> 4), b_desc + (uint64_t)(k * UMMA_K * 2 >> 4), idesc,
+                           (kb > 0 || k > 0) ? 1u : 0u);
+          tcgen05_commit_pair(empty_bar(s));
+          if (++s == STAGES) {
+            s = 0;
+            phase ^= 1u;
+          }
+        }
+        if (ok) tcgen05_commit_pair(tmem_full_bar(acc));
+      }
+    }
+  } else {
+    dependent_launch_wait();
+    const int quadrant = warp & 3, share = (warp - 2) >> 2;
+    const int row_in_tile = quadrant * 32 + lane;
+    int local = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x >> 1; tile < total; tile += step) {
+      const int tile_b = tile / tiles_a;
+      const int acc = local & 1, use = local >> 1;
+      ++local;
+      const int row = (tile % tiles_a * 2 + rank) * BM + row_in_tile;
+      const bool rotating = p.rotary && p.rotary_table != nullptr && row < p.rows_a;
+      float cs_a[16], sn_a[16];
+      int slot = -1;
+      if (rotating) load_angles(p, row, 0, cs_a, sn_a);
+      if (p.rotary && p.slots != nullptr && row < p.rows_a) slot = p.slots[row];
+      ok = ok && mbar_wait(tmem_full_bar(acc), use & 1, abort_flag, p.error, 3);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tcgen05_fence_after();
+      const uint32_t lane_address = tmem_base + ((uint32_t)(quadrant * 32) << 16) + acc * ACC;
+      tile_epilogue<PBN, kGateSilu>(p, lane_address, share, row, p.rows_a, tile_b, 0, rotating, cs_a, sn_a, slot);
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_remote(in_block(tmem_empty_bar(acc), 0));     // this warp has read its part of the accumulator
+    }
+  }
+
+  tcgen05_fence_before();
+  __syncthreads();
+  cluster_sync();                  // nobody leaves while the other block may still report to its barriers or read its shared memory
+  if (warp == 1) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * ACC) : "memory");
   }
 }
 
@@ -750,6 +965,30 @@ int launch_persistent_with(const Params& p, const void* a, const void* b, int k,
   return check_launch("linear_tcgen05");
 }
 
+template <int PBN>
+int launch_pair_with(const Params& p, const void* a, const void* b, int k, cudaStream_t stream) {
+  using T = PairTile<PBN>;
+  CUtensorMap map_a, map_b;
+  if (int err = tensor_map(&map_a, a, p.rows_a, k, BM)) return err;
+  if (int err = tensor_map(&map_b, b, p.rows_b, k, PBN / 2)) return err;
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<PBN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM_BYTES);
+  if (configured != cudaSuccess) return fail(100, "linear_tcgen05: %s", cudaGetErrorString(configured));
+  const int tiles_a = (p.rows_a + 2 * BM - 1) / (2 * BM), tiles_b = (p.rows_b + PBN - 1) / PBN;
+  const int pairs = sm_count() / 2;
+  const int clusters = tiles_a * tiles_b < pairs ? tiles_a * tiles_b : pairs;
+  launch_kernel(gemm_tcgen05_pair_kernel<PBN>, dim3(2 * clusters), PERSISTENT_THREADS, T::SMEM_BYTES, stream, map_a, map_b, p, tiles_a, tiles_b);
+  return check_launch("linear_tcgen05");
+}
+
+int launch_pair(const Params& p, int width, const void* a, const void* b, int k, cudaStream_t stream) {
+  if (width == 224) return launch_pair_with<224>(p, a, b, k, stream);
+  if (width == 192) return launch_pair_with<192>(p, a, b, k, stream);
+  if (width == 160) return launch_pair_with<160>(p, a, b, k, stream);
+  if (width == 128) return launch_pair_with<128>(p, a, b, k, stream);
+  return launch_pair_with<256>(p, a, b, k, stream);
+}
+
 // The tile width whose walk over the output costs least: rounds of tiles over the SMs
 // times (width + a fixed share for a tile's first loads and its epilogue). The narrow widths
 // serve a portion of a few hundred tokens, whose few wide tiles would leave most SMs idle
@@ -778,6 +1017,33 @@ int persistent_width(const Params& p) {
   return best;
 }
 
+// The tile width of the pair kernel where it is expected to be the quicker one, else 0. Both kernels' times follow
+// rounds of tiles over the SMs x k-blocks x (width + 200), 0.87 ns a unit for pairs and 6 % more for single blocks (all SMs drawing
+// from L2), plus 1 us of a cluster's set-up. Measured, us, single / pair, 1536- and 3584-wide layers: gate|up of 512, 2,048,
+// 8,192 tokens 29.9 / 27.3, 85.6 / 78.2, 316 / 294 and 104 / 93, 367 / 337, 1,481 / 1,369 (1.62 PFLOP/s); down of 8,192
+// 202 / 169 and 935 / 758; but down of 2,048 at K = 8,960 (one round either way, 144 blocks of 176 columns against 64
+// pairs of 192) 50.4 / 52.4, o there 16.8 / 18.0 and q|k|v 23.9 / 24.4. Grouped products, planes of K and
+// gates other than SiLU stay with single blocks.
+int pair_width(const Params& p) {
+  if (p.group_tiles != nullptr || p.planes > 1 || (p.swiglu && p.gate_kind != kGateSilu)) return 0;
+  auto units = [&](int rows, int w, int at_once) {
+    const long tiles = (long)((p.rows_a + rows - 1) / rows) * ((p.rows_b + w - 1) / w);
+    return (tiles + at_once - 1) / at_once * p.k_blocks * (w + 200);
+  };
+  const long single = units(BM, persistent_width(p), sm_count());
+  long best = single + single * 6 / 100;
+  int width = 0;
+  for (int w : {256, 224, 192, 160, 128}) {
+    if (p.rotary && w % p.head_dim) continue;        // a tile must not cut a head
+    const long cost = units(2 * BM, w, sm_count() / 2) + 1150;
+    if (cost < best) {
+      best = cost;
+      width = w;
+    }
+  }
+  return width;
+}
+
 template <int GATE>
 int launch_gated(const Params& p, int width, const void* a, const void* b, int k, cudaStream_t stream) {
   if (width == 192) return launch_persistent_with<192, GATE>(p, a, b, k, stream);
@@ -787,6 +1053,7 @@ int launch_gated(const Params& p, int width, const void* a, const void* b, int k
 }
 
 int launch_persistent(const Params& p, const void* a, const void* b, int k, cudaStream_t stream) {
+  if (const int width = pair_width(p)) return launch_pair(p, width, a, b, k, stream);
   const int best = persistent_width(p);
   if (p.swiglu && p.gate_kind == kGateRelu) return launch_gated<kGateRelu>(p, best, a, b, k, stream);
   if (p.swiglu && p.gate_kind == kGateGeluTanh) return launch_gated<kGateGeluTanh>(p, best, a, b, k, stream);
@@ -804,6 +1071,19 @@ int check_operands(const void* x, const void* w, int k) {
 }
 
 }  // namespace
+
+// The width of the tiles that pairs of SMs compute for a product of this shape (head_dim: of q|k|v with rotation, else 0;
+// swiglu: with SiLU x up), 0 where single blocks do.
+PAE_EXPORT int pae_linear_pair_width(int tokens, int n, int k, int head_dim, int swiglu) {
+  Params p{};
+  p.rows_a = tokens;
+  p.rows_b = n;
+  p.k_blocks = (k + BK - 1) / BK;
+  p.head_dim = head_dim;
+  p.rotary = head_dim > 0;
+  p.swiglu = swiglu;
+  return n >= 256 ? pair_width(p) : 0;
+}
 
 // out[tokens, n] = x[tokens, k] . w[n, k]^T (+ bias[n]) (+ residual[tokens, n]); x, w, residual
 // bfloat16, bias float32, out bfloat16 or float32 (then residual is float32 too).
