@@ -470,15 +470,15 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 
 // One thread's part of a tile's epilogue: its row of the accumulator at `lane_address`, and of the tile's PBN columns
 // the range of its warp (`share`: which of the warps of its quarter of the rows).
-template <int PBN, int GATE>
+template <int PBN, int GATE, bool ROTARY>
 __device__ __forceinline__ void tile_epilogue(const Params& p, uint32_t lane_address, int share, int row, int rows_end, int tile_b,
                                               size_t plane_offset, bool rotating, float (&cs_a)[16], float (&sn_a)[16], int slot) {
   // The warps of a quarter of the rows share the tile's columns in equal ranges that end
   // on a multiple of 32 columns (a gate block with its up block) or of the head size.
-  const int unit = p.rotary ? p.head_dim : 32;
+  const int unit = ROTARY ? p.head_dim : 32;
   const int range = ((PBN + EPILOGUE_SHARES - 1) / EPILOGUE_SHARES + unit - 1) / unit * unit;
   const int col_begin = min(share * range, PBN), col_end = min(col_begin + range, PBN);
-  if (p.rotary) {
+  if constexpr (ROTARY) {
     // 16 columns of each half of a head at a time; the token's cosines and sines of those
     // 16 frequencies are read once and serve every head of the tile, and those of the next
     // 16 are on their way while these are used.
@@ -525,8 +525,10 @@ __device__ __forceinline__ void tile_epilogue(const Params& p, uint32_t lane_add
 }
 
 // GATE: the gate's activation of the gated epilogue, known when compiled (a choice at run time in that
-// epilogue cost the SiLU models 1 % of a step).
-template <int PBN, int GATE>
+// epilogue cost the SiLU models 1 % of a step). ROTARY: whether the epilogue rotates, likewise: its angles take 168 registers a thread,
+// the others 60, and a block of 60 may start beside the blocks of the kernel before and ask for its first weights there (a
+// 100-token prompt of 8 layers of the 1.5B sizes 628 -> 611 us).
+template <int PBN, int GATE, bool ROTARY>
 __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                           const __grid_constant__ CUtensorMap map_b,
                                                                           const Params p, int tiles_a, int tiles_b) {
@@ -572,13 +574,25 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  dependent_launch_wait();
 
   // A work item is an output tile, or one of the `planes` ranges of K of an output tile when a
   // launch of few tiles and a long K shares each tile out over several blocks.
   const int planes = p.planes > 1 ? p.planes : 1;
   const int total_items = tiles_a * tiles_b * planes;
   const int k_blocks = p.k_blocks;
+  // The weights of the first item's first stages are asked for before the wait for the kernel before, which never writes
+  // them (grouped: which matrix a tile multiplies is that kernel's output, so nothing is): they are a large
+  // part of what a block reads when the tokens are few.
+  int early = 0;
+  if (threadIdx.x == 0 && p.group_tiles == nullptr && (int)blockIdx.x < total_items) {
+    const int item = blockIdx.x, kb_first = (item % planes) * p.kb_per_split;
+    const int count = min(kb_first + p.kb_per_split, k_blocks) - kb_first;
+    for (; early < PSTAGES && early < count; ++early) {
+      mbar_expect_tx(full_bar(early), P_STAGE_BYTES);
+      tma_load_2d(base + early * P_STAGE_BYTES + P_A_BYTES, &map_b, full_bar(early), (kb_first + early) * BK, item / planes / tiles_a * PBN);
+    }
+  }
+  dependent_launch_wait();
   // Grouped: how many of the table's tiles are in use, read once by the thread or warp of each role.
   auto used_tiles = [&]() { return p.group_tiles != nullptr ? min(tiles_a, p.group_tiles[2 * tiles_a]) : tiles_a; };
   // Which tile of the A rows and which of the B rows a tile index means. Plain: neighbouring
@@ -611,9 +625,9 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
             break;
           }
           const uint32_t a_dst = base + s * P_STAGE_BYTES;
-          mbar_expect_tx(full_bar(s), P_STAGE_BYTES);
+          if (it >= early) mbar_expect_tx(full_bar(s), P_STAGE_BYTES);
           tma_load_2d(a_dst, &map_a, full_bar(s), kb * BK, tile_a * BM);
-          tma_load_2d(a_dst + P_A_BYTES, &map_b, full_bar(s), kb * BK, b_row);
+          if (it >= early) tma_load_2d(a_dst + P_A_BYTES, &map_b, full_bar(s), kb * BK, b_row);
         }
       }
       if (*abort_flag) {
@@ -685,17 +699,17 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
       const int row = tile_a * BM + row_in_tile;
       // What the rotation needs of this thread's token is asked for before the wait for the
       // tile's MMAs: its place in its page and its first 16 cosines and sines.
-      const bool rotating = p.rotary && p.rotary_table != nullptr && row < p.rows_a;
+      const bool rotating = ROTARY && p.rotary_table != nullptr && row < p.rows_a;
       float cs_a[16], sn_a[16];
       int slot = -1;
       if (rotating) load_angles(p, row, 0, cs_a, sn_a);
-      if (p.rotary && p.slots != nullptr && row < p.rows_a) slot = p.slots[row];
+      if (ROTARY && p.slots != nullptr && row < p.rows_a) slot = p.slots[row];
       ok = ok && mbar_wait(tmem_full_bar(acc), use & 1, abort_flag, p.error, 3);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tcgen05_fence_after();
       const uint32_t lane_address = tmem_base + ((uint32_t)(quadrant * 32) << 16) + acc * ACC;
-      tile_epilogue<PBN, GATE>(p, lane_address, share, row, rows_end, tile_b, plane_offset, rotating, cs_a, sn_a, slot);
+      tile_epilogue<PBN, GATE, ROTARY>(p, lane_address, share, row, rows_end, tile_b, plane_offset, rotating, cs_a, sn_a, slot);
       tcgen05_fence_before();
       mbar_arrive(tmem_empty_bar(acc));        // this thread has read its part of the accumulator
     }
@@ -764,7 +778,7 @@ __device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar) {
                : "memory");
 }
 
-template <int PBN>
+template <int PBN, bool ROTARY>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PERSISTENT_THREADS)
     gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p,
                              int tiles_a, int tiles_b) {
@@ -890,17 +904,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PERSISTENT_THREADS)
       const int acc = local & 1, use = local >> 1;
       ++local;
       const int row = (tile % tiles_a * 2 + rank) * BM + row_in_tile;
-      const bool rotating = p.rotary && p.rotary_table != nullptr && row < p.rows_a;
+      const bool rotating = ROTARY && p.rotary_table != nullptr && row < p.rows_a;
       float cs_a[16], sn_a[16];
       int slot = -1;
       if (rotating) load_angles(p, row, 0, cs_a, sn_a);
-      if (p.rotary && p.slots != nullptr && row < p.rows_a) slot = p.slots[row];
+      if (ROTARY && p.slots != nullptr && row < p.rows_a) slot = p.slots[row];
       ok = ok && mbar_wait(tmem_full_bar(acc), use & 1, abort_flag, p.error, 3);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tcgen05_fence_after();
       const uint32_t lane_address = tmem_base + ((uint32_t)(quadrant * 32) << 16) + acc * ACC;
-      tile_epilogue<PBN, kGateSilu>(p, lane_address, share, row, p.rows_a, tile_b, 0, rotating, cs_a, sn_a, slot);
+      tile_epilogue<PBN, kGateSilu, ROTARY>(p, lane_address, share, row, p.rows_a, tile_b, 0, rotating, cs_a, sn_a, slot);
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(in_block(tmem_empty_bar(acc), 0));     // this warp has read its part of the accumulator
@@ -946,7 +960,7 @@ int sm_count() {
   return count;
 }
 
-template <int PBN, int GATE>
+template <int PBN, int GATE, bool ROTARY = false>
 int launch_persistent_with(const Params& p, const void* a, const void* b, int k, cudaStream_t stream) {
   using T = PTile<PBN>;
   CUtensorMap map_a, map_b;
@@ -954,34 +968,41 @@ int launch_persistent_with(const Params& p, const void* a, const void* b, int k,
   if (int err = tensor_map(&map_b, b, p.group_tiles != nullptr ? p.rows_b * p.groups : p.rows_b, k, PBN)) return err;
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(gemm_tcgen05_persistent_kernel<PBN, GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM_BYTES);
+    cudaError_t err = cudaFuncSetAttribute(gemm_tcgen05_persistent_kernel<PBN, GATE, ROTARY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM_BYTES);
     if (err != cudaSuccess) return fail(100, "linear_tcgen05: %s", cudaGetErrorString(err));
     configured = true;
   }
   const int tiles_a = (p.rows_a + BM - 1) / BM, tiles_b = (p.rows_b + PBN - 1) / PBN;
   const int items = tiles_a * tiles_b * (p.planes > 1 ? p.planes : 1);
   const int blocks = items < sm_count() ? items : sm_count();
-  launch_kernel(gemm_tcgen05_persistent_kernel<PBN, GATE>, dim3(blocks), PERSISTENT_THREADS, T::SMEM_BYTES, stream, map_a, map_b, p, tiles_a, tiles_b);
+  launch_kernel(gemm_tcgen05_persistent_kernel<PBN, GATE, ROTARY>, dim3(blocks), PERSISTENT_THREADS, T::SMEM_BYTES, stream, map_a, map_b, p, tiles_a, tiles_b);
   return check_launch("linear_tcgen05");
 }
 
-template <int PBN>
+template <int PBN, bool ROTARY = false>
 int launch_pair_with(const Params& p, const void* a, const void* b, int k, cudaStream_t stream) {
   using T = PairTile<PBN>;
   CUtensorMap map_a, map_b;
   if (int err = tensor_map(&map_a, a, p.rows_a, k, BM)) return err;
   if (int err = tensor_map(&map_b, b, p.rows_b, k, PBN / 2)) return err;
   static const cudaError_t configured =
-      cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<PBN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM_BYTES);
+      cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<PBN, ROTARY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM_BYTES);
   if (configured != cudaSuccess) return fail(100, "linear_tcgen05: %s", cudaGetErrorString(configured));
   const int tiles_a = (p.rows_a + 2 * BM - 1) / (2 * BM), tiles_b = (p.rows_b + PBN - 1) / PBN;
   const int pairs = sm_count() / 2;
   const int clusters = tiles_a * tiles_b < pairs ? tiles_a * tiles_b : pairs;
-  launch_kernel(gemm_tcgen05_pair_kernel<PBN>, dim3(2 * clusters), PERSISTENT_THREADS, T::SMEM_BYTES, stream, map_a, map_b, p, tiles_a, tiles_b);
+  launch_kernel(gemm_tcgen05_pair_kernel<PBN, ROTARY>, dim3(2 * clusters), PERSISTENT_THREADS, T::SMEM_BYTES, stream, map_a, map_b, p, tiles_a, tiles_b);
   return check_launch("linear_tcgen05");
 }
 
 int launch_pair(const Params& p, int width, const void* a, const void* b, int k, cudaStream_t stream) {
+  if (p.rotary) {                 // a tile holds whole heads: widths that divide 256
+    if (width == 192) return launch_pair_with<192, true>(p, a, b, k, stream);
+    if (width == 160) return launch_pair_with<160, true>(p, a, b, k, stream);
+    if (width == 224) return launch_pair_with<224, true>(p, a, b, k, stream);
+    if (width == 128) return launch_pair_with<128, true>(p, a, b, k, stream);
+    return launch_pair_with<256, true>(p, a, b, k, stream);
+  }
   if (width == 224) return launch_pair_with<224>(p, a, b, k, stream);
   if (width == 192) return launch_pair_with<192>(p, a, b, k, stream);
   if (width == 160) return launch_pair_with<160>(p, a, b, k, stream);
@@ -1055,6 +1076,12 @@ int launch_gated(const Params& p, int width, const void* a, const void* b, int k
 int launch_persistent(const Params& p, const void* a, const void* b, int k, cudaStream_t stream) {
   if (const int width = pair_width(p)) return launch_pair(p, width, a, b, k, stream);
   const int best = persistent_width(p);
+  if (p.rotary) {
+    if (best == 192) return launch_persistent_with<192, kGateSilu, true>(p, a, b, k, stream);
+    if (best == 128) return launch_persistent_with<128, kGateSilu, true>(p, a, b, k, stream);
+    if (best == 64) return launch_persistent_with<64, kGateSilu, true>(p, a, b, k, stream);
+    return launch_persistent_with<256, kGateSilu, true>(p, a, b, k, stream);
+  }
   if (p.swiglu && p.gate_kind == kGateRelu) return launch_gated<kGateRelu>(p, best, a, b, k, stream);
   if (p.swiglu && p.gate_kind == kGateGeluTanh) return launch_gated<kGateGeluTanh>(p, best, a, b, k, stream);
   if (best == 192) return launch_persistent_with<192, kGateSilu>(p, a, b, k, stream);
