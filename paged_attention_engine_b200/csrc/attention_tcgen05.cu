@@ -612,11 +612,19 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
 }
 
 // ---------------------------------------------------------------------------------------
-// The paired form, for launches of at least two blocks per SM (long prompts, many requests or
-// heads). A block walks the keys 64 at a time with one softmax thread per query row, and
+// The paired form, for launches of many blocks (long prompts, many requests or heads) and for short ones
+// (`takes_paired`). A block walks the keys 64 at a time with one softmax thread per query row, and
 // keeps O in tensor memory over all tiles instead of reading each tile's product back:
-// 113 KB of shared memory, 256 columns of tensor memory and 192 threads, so two blocks share
+// 97 KB of shared memory, 256 columns of tensor memory and 192 threads, so two blocks share
 // an SM and the softmax of one overlaps the products and the waits of the other.
+//
+// The probabilities of a tile go into tensor memory, over the scores they came from, and are the second product's A
+// operand there: no trip through shared memory (sixteen-byte stores into the swizzled layout, a proxy fence, and 16 KB that
+// the tensor core reads back), and the softmax never waits for a product unless a reference moves. The thread that issues the MMAs
+// waits for the product of the tile before last before the next scores are written over the probabilities it reads. Scale
+// and sum take two scores an instruction. The kernel is bound by the chain of a tile's steps (a special-function unit
+// working a third of the time, tensor cores half): 8,192 tokens, 12 heads of 128: 277 -> 258 us (800 TFLOP/s), 28 heads:
+// 596 -> 547 us (880); with the probabilities still in shared memory 266 and 568, without the instructions on pairs 268 and 570.
 //
 // The reference of a row is its running maximum, but it only moves when the maximum has grown
 // by more than 2^8 since it was set: probabilities then stay below 256, which float32 sums and
@@ -632,23 +640,55 @@ constexpr int SOFTMAX_WARPS = 4;
 constexpr int KV_STAGES = 2;
 constexpr float REFERENCE_SLACK = 8.f;   // a row's reference follows its maximum in steps of more than 2^8
 
-// The same 32 columns written back (the whole warp calls it).
-__device__ __forceinline__ void tmem_store32(uint32_t address, const float* v) {
+// 64 consecutive float32 columns of this thread's lane of tensor memory.
+__device__ __forceinline__ void tmem_load64(uint32_t address, float* v) {
+  uint32_t r[64];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x64.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
+      : "r"(address)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
+}
+// 32 columns written (the whole warp calls it).
+__device__ __forceinline__ void tmem_store32(uint32_t address, const uint32_t* v) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-      ::"r"(address), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-        "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])),
-        "r"(__float_as_uint(v[7])), "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])),
-        "r"(__float_as_uint(v[11])), "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])),
-        "r"(__float_as_uint(v[15])), "r"(__float_as_uint(v[16])), "r"(__float_as_uint(v[17])), "r"(__float_as_uint(v[18])),
-        "r"(__float_as_uint(v[19])), "r"(__float_as_uint(v[20])), "r"(__float_as_uint(v[21])), "r"(__float_as_uint(v[22])),
-        "r"(__float_as_uint(v[23])), "r"(__float_as_uint(v[24])), "r"(__float_as_uint(v[25])), "r"(__float_as_uint(v[26])),
-        "r"(__float_as_uint(v[27])), "r"(__float_as_uint(v[28])), "r"(__float_as_uint(v[29])), "r"(__float_as_uint(v[30])),
-        "r"(__float_as_uint(v[31]))
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n"
+      "tcgen05.wait::st.sync.aligned;"
+      ::"r"(address), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
       : "memory");
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// D[tmem] (+)= A[tmem] . B[smem]^T: a lane of A is a row, a column holds two neighbouring bfloat16 of K.
+__device__ __forceinline__ void umma_bf16_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// Two floats side by side: one instruction for both, each rounded as the single one rounds.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 template <int D>
 struct Layout {
@@ -657,24 +697,22 @@ struct Layout {
   static constexpr int KV_HALF_BYTES = BKEYS * 128;           // 64 rows x 64 bfloat16
   static constexpr int Q_BYTES = HALVES * Q_HALF_BYTES;
   static constexpr int KV_BYTES = HALVES * KV_HALF_BYTES;     // one stage of K, or of V
-  static constexpr int P_BYTES = BQ * BKEYS * 2;              // 128 rows x 64 keys: one swizzle row each
   static constexpr int Q_OFFSET = 0;
   static constexpr int K_OFFSET = Q_BYTES;                    // two stages
   static constexpr int V_OFFSET = K_OFFSET + KV_STAGES * KV_BYTES;
-  static constexpr int P_OFFSET = V_OFFSET + KV_STAGES * KV_BYTES;
-  static constexpr int BAR_OFFSET = P_OFFSET + P_BYTES;
+  static constexpr int BAR_OFFSET = V_OFFSET + KV_STAGES * KV_BYTES;
   static constexpr int USED_BYTES = BAR_OFFSET + 256;
   // 768 bytes of slack for the 1024-byte alignment of the tiles: with it two blocks of head
   // size 128 still fit on one SM. The kernel checks that the slack was enough.
   static constexpr size_t SMEM_BYTES = (size_t)USED_BYTES + 768;
-  static constexpr int S_COLUMNS = BKEYS;                     // per score buffer
+  static constexpr int S_COLUMNS = BKEYS;                     // per score buffer; its first half holds the tile's probabilities later
   static constexpr int O_COLUMN = 2 * S_COLUMNS;              // O behind the two score buffers
   static constexpr int TMEM_COLUMNS = 256;
 };
 
 enum Bar : int {
-  Q_FULL = 0, O_FULL = 1, S_FULL = 2, S_EMPTY = 4, P_READY = 6, P_EMPTY = 7,
-  K_FULL = 8, K_EMPTY = K_FULL + KV_STAGES, V_FULL = K_EMPTY + KV_STAGES, V_EMPTY = V_FULL + KV_STAGES, NUM_BARS = V_EMPTY + KV_STAGES
+  Q_FULL = 0, O_FULL = 1, S_FULL = 2, P_READY = 4, O_REST = 6,
+  K_FULL = 7, K_EMPTY = K_FULL + KV_STAGES, V_FULL = K_EMPTY + KV_STAGES, V_EMPTY = V_FULL + KV_STAGES, NUM_BARS = V_EMPTY + KV_STAGES
 };
 
 template <int D>
@@ -713,10 +751,11 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar(S_FULL, i), 1);
-      mbar_init(bar(S_EMPTY, i), SOFTMAX_WARPS);     // one arrival per warp
+      // One arrival per warp. Two of them, like the score buffers: the softmax may finish a tile before the MMA thread has
+      // looked at the tile before, but not two (the scores of tile t + 2 follow the product of tile t).
+      mbar_init(bar(P_READY, i), SOFTMAX_WARPS);
     }
-    mbar_init(bar(P_READY), SOFTMAX_WARPS);
-    mbar_init(bar(P_EMPTY), 1);                      // by tcgen05.commit: the second product has read P
+    mbar_init(bar(O_REST), 1);                       // by tcgen05.commit: the second product of a tile has completed
     mbar_init(bar(O_FULL), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -840,7 +879,8 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
       auto issue_scores = [&](int t) {
         const int st = t & 1, stage = t % KV_STAGES;
         ok = ok && mbar_wait(bar(K_FULL, stage), (t / KV_STAGES) & 1, abort_flag, p.error, 3);
-        if (t >= 2) ok = ok && mbar_wait(bar(S_EMPTY, st), ((t >> 1) - 1) & 1, abort_flag, p.error, 4);
+        // These scores go where the probabilities of tile t - 2 lay.
+        if (t >= 2) ok = ok && mbar_wait(bar(O_REST), (t - 2) & 1, abort_flag, p.error, 4);
         if (!ok) return;
         tcgen05_fence_after();
         const uint32_t q_addr = base + L::Q_OFFSET, k_addr = base + L::K_OFFSET + stage * L::KV_BYTES;
@@ -858,15 +898,15 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
         if (t + 1 < n_tiles) issue_scores(t + 1);
         const int stage = t % KV_STAGES;
         ok = ok && mbar_wait(bar(V_FULL, stage), (t / KV_STAGES) & 1, abort_flag, p.error, 5);
-        ok = ok && mbar_wait(bar(P_READY), t & 1, abort_flag, p.error, 6);
+        ok = ok && mbar_wait(bar(P_READY, t & 1), (t >> 1) & 1, abort_flag, p.error, 6);
         if (!ok) break;
         tcgen05_fence_after();
-        const uint32_t p_addr = base + L::P_OFFSET, v_addr = base + L::V_OFFSET + stage * L::KV_BYTES;
+        const uint32_t v_addr = base + L::V_OFFSET + stage * L::KV_BYTES;
 #pragma unroll
-        for (int k = 0; k < BKEYS / 16; ++k)     // 16 keys a step: two groups of 8 rows of V
-          umma_bf16(tmem_base + L::O_COLUMN, k_major_descriptor(p_addr + k * 32),
-                    mn_major_descriptor(v_addr + k * 2048, L::KV_HALF_BYTES), idesc_o, (t > 0 || k > 0) ? 1u : 0u);
-        tcgen05_commit(bar(P_EMPTY));            // P may be written again, and O is at rest until the next P is ready
+        for (int k = 0; k < BKEYS / 16; ++k)     // 16 keys a step: eight columns of P, two groups of 8 rows of V
+          umma_bf16_tmem_a(tmem_base + L::O_COLUMN, tmem_base + (t & 1) * L::S_COLUMNS + k * 8,
+                           mn_major_descriptor(v_addr + k * 2048, L::KV_HALF_BYTES), idesc_o, (t > 0 || k > 0) ? 1u : 0u);
+        tcgen05_commit(bar(O_REST));             // O is at rest until the next P is ready
         tcgen05_commit(bar(V_EMPTY, stage));
       }
       if (ok) tcgen05_commit(bar(O_FULL));       // the output is complete
@@ -881,7 +921,6 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
     bool ok = true;
     for (int t = 0; t < n_tiles; ++t) {
       const int st = t & 1;
-      uint8_t* p_row = generic_base + L::P_OFFSET + r * 128;
       const int key0 = kv_begin + t * BKEYS;
       ok = ok && mbar_wait(bar(S_FULL, st), (t >> 1) & 1, abort_flag, p.error, 8);
       ok = __all_sync(0xffffffffu, ok);
@@ -894,11 +933,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
       const int hi = r < rows ? min(my_pos, kv_end - 1) - key0 : -1;          // relative to the tile
       const int lo = (p.window > 0 ? max(first_key, my_pos - p.window + 1) : first_key) - key0;
       float s[BKEYS];
-      tmem_load32(lane_base + st * L::S_COLUMNS, s);
-      tmem_load32(lane_base + st * L::S_COLUMNS + 32, s + 32);
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(S_EMPTY, st));             // the scores are in registers
+      tmem_load64(lane_base + st * L::S_COLUMNS, s);
       float m4[4] = {-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
       if (unmasked) {
 #pragma unroll
@@ -909,10 +944,6 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
       }
       float tile_max = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
       if (tile_max != -FLT_MAX) tile_max *= p.scale_log2;        // the scale is positive: max(s) scales with it
-      // The second product of the tile before has completed: P may be written, O is at rest.
-      if (t >= 1) ok = mbar_wait(bar(P_EMPTY), (t - 1) & 1, abort_flag, p.error, 7);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
       const bool moves = tile_max > reference + REFERENCE_SLACK || (reference == -FLT_MAX && tile_max != -FLT_MAX);
       if (__any_sync(0xffffffffu, moves)) {
         // Some row of this warp moves its reference: its sum and its row of O are multiplied
@@ -923,14 +954,18 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
           row_sum *= shrink;
         }
         if (t >= 1) {
+          ok = mbar_wait(bar(O_REST), (t - 1) & 1, abort_flag, p.error, 7);      // the product of the tile before has completed
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
           tcgen05_fence_after();
 #pragma unroll
           for (int c = 0; c < D; c += 32) {
             float o[32];
+            uint32_t back[32];
             tmem_load32(lane_base + L::O_COLUMN + c, o);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] *= shrink;
-            tmem_store32(lane_base + L::O_COLUMN + c, o);
+            for (int i = 0; i < 32; ++i) back[i] = __float_as_uint(o[i] * shrink);
+            tmem_store32(lane_base + L::O_COLUMN + c, back);
           }
         }
       }
@@ -938,35 +973,36 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
       // no key yet has no reference and every probability 0.
       const float offset = reference == -FLT_MAX ? 0.f : -reference;
       const float factor = reference == -FLT_MAX ? 0.f : p.scale_log2;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint64_t factor2 = pack2(factor, factor), offset2 = pack2(offset, offset);
+      uint64_t sum01 = 0, sum23 = 0;                            // (0.f, 0.f)
+      uint32_t packed[BKEYS / 2];
+      auto take = [&](int i, auto visible) {
+        float e[4];
+        unpack2(fma2(pack2(s[i], s[i + 1]), factor2, offset2), e[0], e[1]);
+        unpack2(fma2(pack2(s[i + 2], s[i + 3]), factor2, offset2), e[2], e[3]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) e[j] = visible(i + j) ? fast_exp2(e[j]) : 0.f;
+        sum01 = add2(sum01, pack2(e[0], e[1]));
+        sum23 = add2(sum23, pack2(e[2], e[3]));
+        const __nv_bfloat162 h01 = __floats2bfloat162_rn(e[0], e[1]), h23 = __floats2bfloat162_rn(e[2], e[3]);
+        packed[i / 2] = *(const uint32_t*)&h01;
+        packed[i / 2 + 1] = *(const uint32_t*)&h23;
+      };
       if (unmasked) {
 #pragma unroll
-        for (int i = 0; i < BKEYS; ++i) {
-          s[i] = fast_exp2(fmaf(s[i], factor, offset));
-          sum4[i & 3] += s[i];
-        }
+        for (int i = 0; i < BKEYS; i += 4) take(i, [](int) { return true; });
       } else {
 #pragma unroll
-        for (int i = 0; i < BKEYS; ++i) {
-          const float e = fast_exp2(fmaf(s[i], factor, offset));
-          s[i] = (i >= lo && i <= hi && factor != 0.f) ? e : 0.f;
-          sum4[i & 3] += s[i];
-        }
+        for (int i = 0; i < BKEYS; i += 4) take(i, [&](int key) { return key >= lo && key <= hi && factor != 0.f; });
       }
-      row_sum += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      // 64 keys = eight 16-byte chunks of this row, swizzled by the row.
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        uint4 packed;
-        __nv_bfloat162* h2 = (__nv_bfloat162*)&packed;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) h2[e] = __floats2bfloat162_rn(s[j * 8 + 2 * e], s[j * 8 + 2 * e + 1]);
-        *(uint4*)(p_row + ((j ^ (r & 7)) << 4)) = packed;
-      }
+      float sums[4];
+      unpack2(sum01, sums[0], sums[1]);
+      unpack2(sum23, sums[2], sums[3]);
+      row_sum += (sums[0] + sums[1]) + (sums[2] + sums[3]);
+      tmem_store32(lane_base + st * L::S_COLUMNS, packed);      // over the scores, which are in registers
       tcgen05_fence_before();
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // P is for the tensor core's eyes
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(P_READY));
+      if (lane == 0) mbar_arrive(bar(P_READY, st));
     }
     ok = __all_sync(0xffffffffu, ok);
     if (active && ok && n_tiles > 0) {
@@ -1046,8 +1082,26 @@ int sm_count() {
   return count;
 }
 
-// form 0 picks by the size of the launch: the paired kernel when it has at least two blocks per
-// SM; else the wide one, and when its blocks are fewer than half of the SMs (a short portion
+// Whether form 0 takes the paired kernel. Two of its blocks share an SM, so up to two blocks per SM run at once; of the wide
+// kernel one. Times in us from launches of 12 and 28 heads, 1 to 12 requests of 64 to 2,000 tokens over up to 4,000 keys:
+// a wide block 5.5 + 1.95 per tile of 128 keys; a wide block that follows another 4 more; a round of paired blocks 5 + 2.84
+// per tile. With more blocks than SMs and fewer than twice as many, the wide launch's second blocks follow its shortest
+// first ones, so it lasts as long as its longest block or two of middling length: the two estimates are compared (6 requests
+// of 300 tokens, 12 heads: wide 21.5, paired 13.9; 4 portions of 509 tokens after 512: 37.9 and 29.1; but one prompt of 2,000
+// tokens: 36.5 and 46.9). From twice as many on it is the paired kernel (8,192 tokens 346 and 258). With at most half of
+// the SMs busy and three tiles or fewer the paired kernel's shorter set-up shows (64 tokens 8.1 and 5.8, 300 tokens 11.1 and
+// 10.5; at 500 tokens 14.0 and 14.9).
+bool takes_paired(long long blocks, long long blocks_per_tile, int longest, int longest_keys) {
+  const int sms = sm_count();
+  if (blocks >= 2LL * sms) return true;
+  if (blocks <= sms) return longest <= 3 && (blocks * 2 <= sms || longest_keys <= 64);
+  const float middle = fmaxf(0.f, longest - (float)sms / blocks_per_tile);
+  const float wide = fmaxf(5.5f + 1.95f * longest, 15.f + 3.9f * middle), paired = 5.f + 2.84f * longest;
+  return paired < wide;
+}
+
+// form 0 picks by the size of the launch: the paired kernel (above), else the wide one, and when its blocks are fewer than half
+// of the SMs (a short portion
 // of a prompt over a long context) a query tile's keys are shared out over a cluster of 2, 4 or
 // 8 blocks, as long as all blocks still run at once and each has two key tiles or more. A block
 // costs about 10 us around its tiles and only one fits an SM, so a second wave of blocks would
@@ -1062,12 +1116,12 @@ int launch(const Params& p, const void* qkv, const void* keys, const void* value
   // requests of which one brings a portion took 75 us where that portion needs 15).
   dim3 grid(p.heads, (max_q_len + BQ - 1) / BQ, p.work_index != nullptr ? working_seqs : seqs);
   const long long blocks = (long long)grid.x * grid.y * working_seqs;
-  const bool use_paired = form == 2 || (form == 0 && blocks >= 2LL * sm_count());
+  const int seen = p.window > 0 && p.window + BQ < max_kv_len ? p.window + BQ : max_kv_len;
+  const int longest = (seen + BKEYS - 1) / BKEYS;          // key tiles of the longest block
+  const bool use_paired = form == 2 || (form == 0 && takes_paired(blocks, (long long)p.heads * working_seqs, longest, seen));
   unsigned ranks = 1;
   if (form == 4 || form == 8 || form == 16) ranks = form / 2;
   if (form == 0 && !use_paired) {
-    const int seen = p.window > 0 && p.window + BQ < max_kv_len ? p.window + BQ : max_kv_len;
-    const int longest = (seen + BKEYS - 1) / BKEYS;        // key tiles of the longest block
     while (ranks < 8 && blocks * (ranks * 2) <= sm_count() && longest >= (int)(ranks * 2) * 2) ranks *= 2;
   }
   CUtensorMap map_q, map_k, map_v;

@@ -407,3 +407,26 @@ def test_windowed_attention_over_a_table_with_released_pages(ops, heads, kv_head
         ops.use_tensor_cores = True
     assert torch.isfinite(slow).all() and torch.isfinite(slow32).all()
     _close(slow, want, torch.bfloat16, scale=2.0)
+
+
+@pytest.mark.parametrize("d,page", [(128, 16), (64, 64)])
+def test_paired_prefill_attention_gives_the_same_bits_every_time(ops, d, page):
+    """The roles of the paired kernel run ahead of one another by up to a tile: many blocks, many key tiles, and large
+    scores that keep moving the rows' references; no wait gives up and no run differs from another."""
+    heads, kv_heads, n, start = 14, 2, 1500, 3000
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    pages = -(-(start + n) // page)
+    qkv = (torch.randn(n, (heads + 2 * kv_heads) * d, device="cuda", generator=gen) * 4).to(torch.bfloat16)
+    keys, values = ((torch.randn(pages, kv_heads, page, d, device="cuda", generator=gen)).to(torch.bfloat16) for _ in range(2))
+    # Later keys score higher: the maximum grows all along the context.
+    keys *= torch.linspace(0.2, 3.0, pages, device="cuda").view(-1, 1, 1, 1).to(torch.bfloat16)
+    table = torch.randperm(pages, device="cuda", generator=gen).to(torch.int32).view(1, -1)
+    keys[table[0].long()] = keys.clone()
+    i32 = lambda *a: torch.tensor(a, dtype=torch.int32, device="cuda")  # noqa: E731
+    args = (qkv, keys, values, table, i32(0, n), i32(start), i32(start + n), heads, kv_heads, d, page, n, start + n, d**-0.5, 0)
+    first = ops.paged_attention(*args, num_single=0, form=2)
+    for _ in range(30):
+        assert torch.equal(ops.paged_attention(*args, num_single=0, form=2), first)
+    ops.check_device_errors()
+    wide = ops.paged_attention(*args, num_single=0, form=1)
+    _close(first, wide, torch.bfloat16)
