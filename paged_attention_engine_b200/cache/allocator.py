@@ -15,7 +15,6 @@ the table.
 
 from __future__ import annotations
 
-from collections import deque
 from dataclasses import dataclass
 from enum import Enum
 
@@ -49,6 +48,38 @@ class _Table:
         self.kept = 0                 # leading logical blocks that releases pass over
 
 
+_NOTHING_NEW = AllocResult(AllocStatus.OK)
+
+
+class _FreeBlocks:
+    """The free list: a list whose first `_head` ids were handed out. A run of ids leaves and comes back as one slice
+    (a context of 4,096 tokens is 256 of them)."""
+
+    __slots__ = ("_ids", "_head")
+
+    def __init__(self, count: int) -> None:
+        self._ids = list(range(count))
+        self._head = 0
+
+    def __len__(self) -> int:
+        return len(self._ids) - self._head
+
+    def __iter__(self):
+        return iter(self._ids[self._head :])
+
+    def take(self, count: int) -> tuple[int, ...]:
+        end = self._head + count
+        taken = tuple(self._ids[self._head : end])
+        self._head = end
+        if end > 1024 and 2 * end > len(self._ids):
+            del self._ids[:end]
+            self._head = 0
+        return taken
+
+    def extend(self, ids) -> None:
+        self._ids.extend(ids)
+
+
 class BlockAllocator:
     """Every physical block is either in the free list or in exactly one table."""
 
@@ -59,7 +90,7 @@ class BlockAllocator:
             raise ValueError(f"block_size must be at least 1, got {block_size}")
         self.num_blocks = num_blocks
         self.block_size = block_size
-        self._free: deque[int] = deque(range(num_blocks))
+        self._free = _FreeBlocks(num_blocks)
         self._tables: dict[object, _Table] = {}
 
     # -- pool ------------------------------------------------------------- #
@@ -127,7 +158,10 @@ class BlockAllocator:
         if needed > len(self._free):
             return AllocResult(AllocStatus.OUT_OF_BLOCKS)
         t = self._tables[seq_id]
-        taken = tuple(self._free.popleft() for _ in range(needed))
+        if needed <= 0:
+            t.tokens += count
+            return _NOTHING_NEW
+        taken = self._free.take(needed)
         t.blocks.extend(taken)
         t.tokens += count
         return AllocResult(AllocStatus.OK, taken)
@@ -153,7 +187,7 @@ class BlockAllocator:
     def free_sequence(self, seq_id) -> tuple[int, ...]:
         """Drops the table and gives back every block it still held, in table order."""
         t = self._tables.pop(seq_id)
-        freed = tuple(b for b in t.blocks if b != HOLE)
+        freed = tuple(t.blocks) if t.released == 0 else tuple(b for b in t.blocks if b != HOLE)
         self._free.extend(freed)
         return freed
 

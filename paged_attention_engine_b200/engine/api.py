@@ -77,5 +77,5 @@ class LLM:
         for rid, prompt in zip(ids, prompts):
             if not self.add_request(Request(rid, tuple(prompt), max_new_tokens, temperature, seed)):
                 raise ValueError(f"prompt of {len(prompt)} tokens + {max_new_tokens} new ones cannot fit the cache pool")
-        done = self.run_to_completion()
-        return [done[rid] for rid in ids]
+        self.scheduler.run_until_idle()
+        return [tuple(self.scheduler.finished[rid].generated) for rid in ids]

@@ -83,16 +83,17 @@ class _Staging:
         self.pinned = device.type == "cuda"
         self.buffers: list[torch.Tensor | None] = [None] * turns
         self.views: list[np.ndarray | None] = [None] * turns
-        self.events: list[Any] = [None] * turns
+        self.events: list[Any] = [None] * turns     # made once, recorded again at every use
+        self.in_flight = [False] * turns
         self.turn = 0
 
     def acquire(self, size: int) -> tuple[int, np.ndarray]:
         """(turn, int32 host array of at least `size` elements) to be filled, then `commit`ted."""
         i = self.turn
         self.turn = (self.turn + 1) % len(self.buffers)
-        if self.events[i] is not None:
+        if self.in_flight[i]:
             self.events[i].synchronize()
-            self.events[i] = None
+            self.in_flight[i] = False
         buf = self.buffers[i]
         if buf is None or buf.numel() < size:
             buf = torch.empty(max(size, 4096), dtype=torch.int32)
@@ -112,10 +113,11 @@ class _Staging:
             into[:size].copy_(buf[:size])
             return into
         out = into if into is not None else torch.empty(size, dtype=torch.int32, device=self.device)
-        out[:size].copy_(buf[:size], non_blocking=True)
-        event = torch.cuda.Event()
-        event.record()
-        self.events[turn] = event
+        out.narrow(0, 0, size).copy_(buf.narrow(0, 0, size), non_blocking=True)
+        if self.events[turn] is None:
+            self.events[turn] = torch.cuda.Event()
+        self.events[turn].record(torch.cuda.current_stream(self.device))
+        self.in_flight[turn] = True
         return out
 
 
@@ -151,11 +153,11 @@ class BatchBuilder:
         into: torch.Tensor | None = None,
         pad_to: int | None = None,
         max_kv_len: int | None = None,
-    ) -> StepContext:
+    ) -> StepContext | None:
         """Flattens the entries. `sampling` (one row per wanted place: temperature, seed,
         request key, output index) travels in the same copy. `table_width` fixes the width of
         the block tables (a captured graph needs the same layout every step) and `into` is
-        the device buffer that such a graph reads. `pad_to` (a step of single tokens that wants
+        the device buffer that such a graph reads: it is filled and None comes back (the graph's kernels know their parts of it). `pad_to` (a step of single tokens that wants
         all their logits only) adds rows up to that many entries: each is a token at position 0
         of nobody's request, which writes no page (slot -1), reads page 0 and owns the spare
         state slot behind the real ones; its logits and its token are computed and ignored, so
@@ -283,6 +285,8 @@ class BatchBuilder:
             put(f + 4, [_signed32(r.output_index) for r in sampling] + zeros)
         dev = self.staging.commit(turn, size, into)
         self.bytes_uploaded = 4 * size
+        if into is not None:
+            return None
         spans = list(zip(starts, sizes))
 
         def part(i: int) -> torch.Tensor:

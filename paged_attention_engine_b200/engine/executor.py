@@ -21,7 +21,7 @@ class _TokenFuture:
     the tokens are: a step in which a kernel gave up on a wait raises instead of handing out
     tokens."""
 
-    def __init__(self, tokens: torch.Tensor, host: torch.Tensor, ops=None) -> None:
+    def __init__(self, tokens: torch.Tensor, host: torch.Tensor, event: torch.cuda.Event, ops=None) -> None:
         count = tokens.numel()
         self.host = host[: count + 1]
         self.host[:count].copy_(tokens, non_blocking=True)
@@ -29,8 +29,8 @@ class _TokenFuture:
         self.device = tokens.device
         if self.ops is not None:
             self.host[count:].copy_(self.ops.error_flag(self.device), non_blocking=True)
-        self.event = torch.cuda.Event()
-        self.event.record()
+        self.event = event            # the host buffer's, recorded again whenever the buffer is used again
+        self.event.record(torch.cuda.current_stream(self.device))
         self.values: list[int] | None = None
 
     def result(self) -> list[int]:
@@ -55,6 +55,7 @@ class ModelExecutor:
         on_gpu = runner.runtime.device.type == "cuda"
         self.asynchronous = on_gpu if asynchronous is None else (asynchronous and on_gpu)
         self._host_tokens = [torch.empty(1025, dtype=torch.int32).pin_memory() for _ in range(4)] if on_gpu else []
+        self._host_events = [torch.cuda.Event() for _ in self._host_tokens]
         self._turn = 0
 
     def begin(self, key: Hashable) -> bool:
@@ -84,7 +85,7 @@ class ModelExecutor:
         output = self.runner.step(entries, rows if rows else None)
         results = [WorkResult(None) for _ in work]
         if rows and self.asynchronous and not record_logits and len(rows) <= 1024:
-            future = _TokenFuture(output.tokens, self._host_tokens[self._turn], self.runner.runtime.ops)
+            future = _TokenFuture(output.tokens, self._host_tokens[self._turn], self._host_events[self._turn], self.runner.runtime.ops)
             self._turn = (self._turn + 1) % len(self._host_tokens)
             at = 0
             for i, w in enumerate(work):

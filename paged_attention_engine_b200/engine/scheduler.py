@@ -245,6 +245,7 @@ class Scheduler:
         self.waiting: deque[Sequence] = deque()
         self.running: list[Sequence] = []
         self.finished: dict[str, Sequence] = {}
+        self._finished_now: list[str] = []       # in the step that runs
         self.rejected: dict[str, Sequence] = {}
         self.events: list[Event] = []
         self._step = 0
@@ -428,7 +429,7 @@ class Scheduler:
         admitted = self._admit()
 
         preempted: list[str] = []
-        finished_before = set(self.finished)
+        self._finished_now = []
         for seq in decoders:
             if seq.status is not SequenceStatus.RUNNING:
                 continue      # preempted earlier in this step
@@ -446,7 +447,7 @@ class Scheduler:
             step=self._step,
             admitted=tuple(s.request_id for s in admitted),
             decoded=tuple(w.seq.request_id for w in ran if not w.is_prefill),
-            finished=tuple(sorted(set(self.finished) - finished_before)),
+            finished=tuple(sorted(self._finished_now)),
             preempted=tuple(preempted),
             running=len(self.running),
             waiting=len(self.waiting),
@@ -491,12 +492,18 @@ class Scheduler:
         freed = self.executor.release(seq.request_id)
         seq.status = SequenceStatus.FINISHED
         self.finished[seq.request_id] = seq
+        self._finished_now.append(seq.request_id)
         self._log(EventKind.FINISH, seq, f"{len(seq.generated)} tokens, freed {freed} blocks")
 
     def run_to_completion(self, max_steps: int = 100_000) -> dict[str, tuple[int, ...]]:
-        """Steps until nothing waits or runs; {request_id: generated tokens}. `max_steps`
-        is a backstop against a scheduler that makes no progress, not a policy
+        """Steps until nothing waits or runs; {request_id: generated tokens} of every request that ever finished.
+        `max_steps` is a backstop against a scheduler that makes no progress, not a policy
         (engine/scheduler.py:753-770)."""
+        self.run_until_idle(max_steps)
+        return {rid: tuple(seq.generated) for rid, seq in self.finished.items()}
+
+    def run_until_idle(self, max_steps: int = 100_000) -> None:
+        """`run_to_completion` without the answer, which grows with every request that ever finished."""
         steps = 0
         while self.waiting or self.running:
             self.step()
@@ -506,4 +513,3 @@ class Scheduler:
                     f"no progress after {max_steps} steps: {len(self.waiting)} waiting, {len(self.running)} running"
                 )
         self.resolve()
-        return {rid: tuple(seq.generated) for rid, seq in self.finished.items()}
