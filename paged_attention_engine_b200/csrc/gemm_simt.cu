@@ -121,8 +121,8 @@ int launch(void* out, const void* x, const void* w, const float* bias, const voi
 // cores' double-precision instruction adds its four products like four fused multiply-adds in a row; a test of
 // sums that cancel compares them), so a token's result does not depend on its batch.
 //
-// f32_lane_kernel, one or two tokens: a lane owns a weight row, a warp a segment of 32 rows, plain double
-// multiply-adds. f32_few_kernel, 3 to 32 tokens: the same split, with mma.m8n8k4.f64 (eight weight rows x eight
+// f32_lane_kernel, one or two tokens: a lane owns a weight row in a segment, a warp two segments of 16 rows (of 32
+// rows and one segment, N = 1,536 made 48 blocks), plain double multiply-adds. f32_few_kernel, 3 to 32 tokens: the same split, with mma.m8n8k4.f64 (eight weight rows x eight
 // tokens; operands widened from float32, which is exact). Both are bound by the weights' bytes at few tokens and
 // by the chain of a segment's sums; weights pass through a ring of cp.async stages per warp (32 k; rows 144 bytes
 // apart, so that a fragment's reads meet no bank twice).
@@ -130,8 +130,8 @@ int launch(void* out, const void* x, const void* w, const float* bias, const voi
 // the tiles are fewer than half of the SMs the segments are shared out over blocks, each of which leaves its
 // segments' sums in planes of double that f32_planes_kernel adds up.
 //
-// Measured, us, [17,920, 1,536] and [1,536, 8,960] weights: 1 token 24.0 and 26.0 (16.8 and 8.4 at the copy bandwidth;
-// the eight-token kernel 36 and 40), 8 tokens 37 and 43 (63 and 78 with plain multiply-adds, whose operands meet the shared memory's
+// Measured, us, [17,920, 1,536] and [1,536, 8,960] weights: 1 token 22.9 and 15.8 (16.8 and 8.4 at the copy bandwidth;
+// 24.0 and 26.0 with 32 rows a block, the eight-token kernel 36 and 40), 8 tokens 37 and 43 (63 and 78 with plain multiply-adds, whose operands meet the shared memory's
 // bandwidth), 60 tokens 168 and 75 (313 and 171), 256 tokens 450 and 574 (1,232 and 1,496): 31 of 37 TFLOP/s.
 // ---------------------------------------------------------------------------------------
 constexpr int SEGMENT = 128;
@@ -288,18 +288,20 @@ int launch_few(float* out, const float* x, const float* w, const float* bias, co
 
 namespace lane_rows {
 constexpr int WARPS = 16;
-constexpr int ROWS = 32;                    // weight rows of a block: one a lane
+constexpr int ROWS = 16;                    // weight rows of a block
 constexpr int STAGES = 2;
 
 template <int MT>
 struct Layout {
-  static constexpr int STAGE_FLOATS = ROWS * PITCH + MT * CHUNK;
-  static constexpr int WARP_BYTES = STAGES * STAGE_FLOATS * 4 + MT * CHUNK * 8;    // the ring, and a chunk's token values in double
-  static constexpr int PART_BYTES = MT * ROWS * 8;              // a warp's segment sums, [token][row]
+  static constexpr int STAGE_FLOATS = 2 * (ROWS * PITCH + MT * CHUNK);
+  static constexpr int WIDE = MT * CHUNK + 2;                   // doubles of a segment's token values (its neighbour starts on other banks)
+  static constexpr int WARP_BYTES = STAGES * STAGE_FLOATS * 4 + 2 * WIDE * 8;
+  static constexpr int PART_BYTES = 2 * MT * ROWS * 8;          // a warp's two segment sums, [segment][token][row]
   static size_t bytes(int warps) { return (size_t)warps * (WARP_BYTES + PART_BYTES); }
 };
 }  // namespace lane_rows
 
+// A warp takes two neighbouring segments of 16 rows: lane l has row l % 16 of segment l / 16.
 template <int MT>
 __global__ void __launch_bounds__(32 * lane_rows::WARPS) f32_lane_kernel(float* __restrict__ out, const float* __restrict__ x,
                                                                          const float* __restrict__ w, const float* __restrict__ bias,
@@ -308,39 +310,42 @@ __global__ void __launch_bounds__(32 * lane_rows::WARPS) f32_lane_kernel(float* 
   constexpr int STAGES = lane_rows::STAGES, ROWS = lane_rows::ROWS;
   extern __shared__ __align__(16) uint8_t smem[];
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int half = lane >> 4, my_row = lane & 15;
   float* ring = (float*)(smem + (size_t)warp * L::WARP_BYTES);
   double* wide = (double*)(ring + STAGES * L::STAGE_FLOATS);
   double* parts = (double*)(smem + (size_t)warps * L::WARP_BYTES);
   const int n0 = blockIdx.x * ROWS;
-  const int segments = (K + SEGMENT - 1) / SEGMENT;
-  const int mine = warp < segments ? (segments - warp + warps - 1) / warps : 0;
-  const int chunks = mine * CHUNKS_PER_SEGMENT -
-                     (mine > 0 && warp + (mine - 1) * warps == segments - 1 ? (segments * SEGMENT - K) / CHUNK : 0);
-  auto chunk_k = [&](int c) { return (warp + (c / CHUNKS_PER_SEGMENT) * warps) * SEGMENT + (c % CHUNKS_PER_SEGMENT) * CHUNK; };
+  const int segments = (K + SEGMENT - 1) / SEGMENT, pairs = (segments + 1) / 2;
+  // This warp's pairs of segments are warp, warp + warps, ...; its chunks run through all of them in order.
+  const int mine = warp < pairs ? (pairs - warp + warps - 1) / warps : 0;
+  const bool owns_last = mine > 0 && warp + (mine - 1) * warps == pairs - 1;
+  // A lone last segment may be short: its chunks behind K are left out.
+  const int chunks = mine * CHUNKS_PER_SEGMENT - (owns_last && (segments & 1) ? (segments * SEGMENT - K) / CHUNK : 0);
+  auto chunk_k = [&](int c, int h) {
+    return (2 * (warp + (c / CHUNKS_PER_SEGMENT) * warps) + h) * SEGMENT + (c % CHUNKS_PER_SEGMENT) * CHUNK;
+  };
   const uint32_t ring_address = (uint32_t)__cvta_generic_to_shared(ring);
   auto fetch = [&](int c) {
     if (c < chunks) {
-      const int k = chunk_k(c) + (lane & 7) * 4;
+      const int piece = (lane & 7) * 4;       // eight lanes bring a row's 32 k
       const uint32_t stage = ring_address + (c % STAGES) * L::STAGE_FLOATS * 4;
 #pragma unroll
-      for (int i = 0; i < ROWS / 4; ++i) {
-        const int row = i * 4 + (lane >> 3);
-        const bool valid = n0 + row < N && k < K;
-        copy16(stage + (row * PITCH + (lane & 7) * 4) * 4, valid ? w + (size_t)(n0 + row) * K + k : w, valid);
+      for (int i = 0; i < 2 * ROWS / 4; ++i) {
+        const int at = i * 4 + (lane >> 3), n = n0 + at % ROWS, k = chunk_k(c, at / ROWS) + piece;
+        const bool valid = n < N && k < K;
+        copy16(stage + (at * PITCH + piece) * 4, valid ? w + (size_t)n * K + k : w, valid);
       }
-      const int m = lane >> 3;
+      const int at = lane >> 3, m = at % MT, k = chunk_k(c, at / MT) + piece;
       const bool valid = m < M && k < K;
-      if (m < MT) copy16(stage + (ROWS * PITCH + m * CHUNK + (lane & 7) * 4) * 4, valid ? x + (size_t)m * K + k : x, valid);
+      if (at < 2 * MT) copy16(stage + (2 * ROWS * PITCH + at * CHUNK + piece) * 4, valid ? x + (size_t)m * K + k : x, valid);
     }
     copy_commit();
   };
   dependent_launch_prologue();
 #pragma unroll
   for (int c = 0; c < STAGES; ++c) fetch(c);
-  double total[MT];
-#pragma unroll
-  for (int m = 0; m < MT; ++m) total[m] = 0.0;
-  const int rounds = (segments + warps - 1) / warps;
+  double total = 0.0;                         // of this lane's output, in the first warp: row lane % 16 of token lane / 16
+  const int rounds = (pairs + warps - 1) / warps;
   int c = 0;
   for (int round = 0; round < rounds; ++round) {
     if (round < mine) {
@@ -355,49 +360,44 @@ __global__ void __launch_bounds__(32 * lane_rows::WARPS) f32_lane_kernel(float* 
 #pragma unroll
         for (int q = 0; q < CHUNK / 4; ++q) w4[q] = *(const float4*)(stage + lane * PITCH + 4 * q);
 #pragma unroll
-        for (int m = 0; m < MT; ++m) wide[m * CHUNK + lane] = (double)stage[ROWS * PITCH + m * CHUNK + lane];
+        for (int m = 0; m < 2 * MT; ++m) wide[(m / MT) * L::WIDE + (m % MT) * CHUNK + lane] = (double)stage[2 * ROWS * PITCH + m * CHUNK + lane];
         __syncwarp();
         fetch(c + STAGES);
+        const double* mine_wide = wide + half * L::WIDE;
 #pragma unroll
         for (int q = 0; q < CHUNK / 4; ++q) {
           const double w0 = (double)w4[q].x, w1 = (double)w4[q].y, w2 = (double)w4[q].z, w3 = (double)w4[q].w;
 #pragma unroll
           for (int m = 0; m < MT; ++m) {
-            const double2 x01 = *(const double2*)(wide + m * CHUNK + 4 * q), x23 = *(const double2*)(wide + m * CHUNK + 4 * q + 2);
+            const double2 x01 = *(const double2*)(mine_wide + m * CHUNK + 4 * q), x23 = *(const double2*)(mine_wide + m * CHUNK + 4 * q + 2);
             acc[m] = fma(x23.y, w3, fma(x23.x, w2, fma(x01.y, w1, fma(x01.x, w0, acc[m]))));
           }
         }
       }
 #pragma unroll
-      for (int m = 0; m < MT; ++m) parts[(warp * MT + m) * ROWS + lane] = acc[m];
+      for (int m = 0; m < MT; ++m) parts[((2 * warp + half) * MT + m) * ROWS + my_row] = acc[m];
     }
     __syncthreads();
     // The first warp adds a round's segments up in their order.
-    if (warp == 0) {
-      const int present = min(warps, segments - round * warps);
-#pragma unroll
-      for (int m = 0; m < MT; ++m)
-        for (int s = 0; s < present; ++s) total[m] += parts[(s * MT + m) * ROWS + lane];
+    if (warp == 0 && half < MT) {
+      const int present = min(2 * warps, segments - 2 * round * warps);
+#pragma unroll 8
+      for (int s = 0; s < present; ++s) total += parts[(s * MT + half) * ROWS + my_row];
     }
     if (round + 1 < rounds) __syncthreads();
   }
-  const int n = n0 + lane;
-  if (warp != 0 || n >= N) return;
-#pragma unroll
-  for (int m = 0; m < MT; ++m) {
-    if (m >= M) continue;
-    double v = total[m];
-    if (bias != nullptr) v += (double)bias[n];
-    if (residual != nullptr) v += (double)residual[(size_t)m * N + n];
-    out[(size_t)m * N + n] = (float)v;
-  }
+  const int n = n0 + my_row, m = half;
+  if (warp != 0 || n >= N || m >= M || m >= MT) return;
+  if (bias != nullptr) total += (double)bias[n];
+  if (residual != nullptr) total += (double)residual[(size_t)m * N + n];
+  out[(size_t)m * N + n] = (float)total;
 }
 
 template <int MT>
 int launch_lane(float* out, const float* x, const float* w, const float* bias, const float* residual, int M, int N, int K, cudaStream_t s) {
   using L = lane_rows::Layout<MT>;
-  const int segments = (K + SEGMENT - 1) / SEGMENT;
-  const int warps = segments < lane_rows::WARPS ? segments : lane_rows::WARPS;
+  const int pairs = ((K + SEGMENT - 1) / SEGMENT + 1) / 2;
+  const int warps = pairs < lane_rows::WARPS ? pairs : lane_rows::WARPS;
   static const cudaError_t configured =
       cudaFuncSetAttribute(f32_lane_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::bytes(lane_rows::WARPS));
   if (configured != cudaSuccess) return fail(100, "linear_f32: %s", cudaGetErrorString(configured));
