@@ -318,7 +318,9 @@ __global__ void __launch_bounds__(32 * WARPS) paged_attention_f32_kernel(
       sum += merged_sum[w][r] * factor;
       value = fmaf(merged_out[w][r][dim], factor, value);
     }
-    out[((size_t)(first_token + row0 + r) * heads + h) * D + dim] = sum > 0.f ? value * (1.f / sum) : 0.f;
+    // A row without keys is 0; a sum that is no number leaves none in its outputs either.
+    const float inv = sum > 0.f ? 1.f / sum : 0.f;
+    out[((size_t)(first_token + row0 + r) * heads + h) * D + dim] = value * inv;
   }
 }
 

@@ -58,3 +58,28 @@ def test_a_query_has_the_same_bits_however_the_step_is_cut(d):
         part = ops.paged_attention(qkv[at : at + n].contiguous(), keys, values, table, i32(0, n), i32(37 + at), i32(37 + at + n),
                                    **dict(args, max_q_len=n, max_kv_len=37 + at + n))
         assert torch.equal(part, whole[at : at + n])
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("where", ["query", "key", "all keys"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("q_lens,pos0", [([1, 1], [40, 200]), ([6, 30], [40, 0])])
+def test_a_score_that_is_no_number_reaches_the_output(d, where, bad, q_lens, pos0):
+    """As a softmax has it: NaN for every query that sees such a score (infinity less infinity among them), the others untouched."""
+    from paged_attention_engine_b200.kernels import ops
+
+    page = 16
+    tensors, args = _case(q_lens, pos0, 2, 1, d, page, 0, 3)
+    qkv, keys, _, table, _, _, _ = tensors
+    if where == "query":
+        qkv[sum(q_lens) - 1, :d] = bad       # the first head of the last token
+    elif where == "key":
+        keys[table[0, 0], 0, 3] = bad        # key 3 of the first request
+    else:
+        keys[table[0, : -(-(pos0[0] + q_lens[0]) // page)].long()] = bad
+    want = ref.paged_attention(*tensors, **args)
+    got = ops.paged_attention(*[t.cuda() for t in tensors], **args).cpu()
+    assert bool(want.isnan().any()) and bool(want.isfinite().any())
+    assert torch.equal(got.isnan(), want.isnan())
+    there = want.isfinite()
+    assert float((got[there] - want[there]).abs().max()) <= 2e-5 * max(1.0, float(want[there].abs().max()))
