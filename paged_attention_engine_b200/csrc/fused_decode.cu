@@ -117,6 +117,8 @@ __global__ void __launch_bounds__(512) splitk_rms_norm_x4_kernel(T* __restrict__
   // products' weights, so they are read before the wait for the kernel before (the weight is
   // read once a step and comes from DRAM, which takes longer than the sums from L2).
   dependent_launch_trigger();
+  // Another block's shared memory may be used once that block has started: the arrival here, whose wait stands before the swap.
+  if constexpr (PARTS == 2) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   const int quads = width / 4;
   const int row = blockIdx.x / PARTS, part = blockIdx.x % PARTS;
   const int share = (quads + PARTS - 1) / PARTS, begin = part * share, end = min(quads, begin + share);     // this block's columns, in fours
@@ -187,6 +189,7 @@ __global__ void __launch_bounds__(512) splitk_rms_norm_x4_kernel(T* __restrict__
   for (int w = 0; w < warps; ++w) total += reduce[w];
   if constexpr (PARTS == 2) {
     __shared__ float halves[2];
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");      // both blocks have started, long ago as a rule
     if (threadIdx.x < 2) {                      // thread b leaves this block's sum in block b of the cluster
       const uint32_t own = (uint32_t)__cvta_generic_to_shared(&halves[part]);
       uint32_t there;
