@@ -500,18 +500,21 @@ __global__ void __launch_bounds__(128, 3) f32_tile_kernel(float* __restrict__ ou
   }
 }
 
+// out[M, N] (rows ld_out apart) = the planes' sum in their order + bias + residual (rows ld_out apart).
 __global__ void __launch_bounds__(256) f32_planes_kernel(float* __restrict__ out, const double* __restrict__ planes,
                                                          const float* __restrict__ bias, const float* __restrict__ residual,
-                                                         int segments, long long count, int N) {
+                                                         int segments, int M, int N, int ld_out) {
   dependent_launch_prologue();
-  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  const unsigned count = (unsigned)M * (unsigned)N, i = blockIdx.x * 256u + threadIdx.x;      // at most half the SMs' tiles
   if (i >= count) return;
+  const unsigned m = i / (unsigned)N, n = i % (unsigned)N;
+  const size_t at = (size_t)m * ld_out + n;
   double v = 0.0;
 #pragma unroll 8
   for (int s = 0; s < segments; ++s) v += planes[(size_t)s * count + i];
-  if (bias != nullptr) v += (double)bias[i % N];
-  if (residual != nullptr) v += (double)residual[i];
-  out[i] = (float)v;
+  if (bias != nullptr) v += (double)bias[n];
+  if (residual != nullptr) v += (double)residual[at];
+  out[at] = (float)v;
 }
 
 int sm_count() {
@@ -526,18 +529,48 @@ int sm_count() {
 }  // namespace
 
 constexpr int F32_FEW_TOKENS = 32;
+// The planes of a launch hold a double per output and segment, which is as much as the weights are at 64 tokens: they are bounded by cutting
+// the output into slices of whole tiles, one after the other through the same scratch. 64 MB hold 13 tiles of the
+// longest K in use (18,944).
+constexpr long long F32_SCRATCH_BYTES = 64LL << 20;
 
-// How many planes of doubles [M, N] `pae_linear_f32` needs as scratch (0: none): the K segments, when the
-// tiles would leave more than half of the SMs idle.
-PAE_EXPORT int pae_linear_f32_planes(int M, int N, int K) {
+namespace {
+
+struct Slices {
+  int m, n;                  // tokens and weight rows of a slice (whole tiles); 0: K is not shared out over blocks
+};
+
+// K is shared out when the tiles would leave more than half of the SMs idle, and a single tile's segments fit the scratch.
+Slices f32_slices(int M, int N, int K) {
+  constexpr int TILE = tiled::TILE;
   const int segments = (K + SEGMENT - 1) / SEGMENT;
-  if (M <= F32_FEW_TOKENS || segments < 2) return 0;
-  const long long tiles = (long long)((M + tiled::TILE - 1) / tiled::TILE) * ((N + tiled::TILE - 1) / tiled::TILE);
-  return tiles * 2 <= sm_count() ? segments : 0;
+  if (M <= F32_FEW_TOKENS || segments < 2) return {0, 0};
+  const int tiles_m = (M + TILE - 1) / TILE, tiles_n = (N + TILE - 1) / TILE;
+  if ((long long)tiles_m * tiles_n * 2 > sm_count()) return {0, 0};
+  const int most = (int)(F32_SCRATCH_BYTES / ((long long)segments * TILE * TILE * 8));      // tiles of a slice
+  if (most < 1) return {0, 0};
+  auto equal = [](int tiles, int at_most) { const int cuts = (tiles + at_most - 1) / at_most; return (tiles + cuts - 1) / cuts; };
+  const int slice_m = tiles_m <= most ? tiles_m : equal(tiles_m, most);
+  const int slice_n = equal(tiles_n, most / slice_m);
+  return {slice_m * TILE < M ? slice_m * TILE : M, slice_n * TILE < N ? slice_n * TILE : N};
+}
+
+}  // namespace
+
+// How many doubles `pae_linear_f32` needs as scratch (0: none), at most 64 MB of them.
+PAE_EXPORT long long pae_linear_f32_scratch(int M, int N, int K) {
+  const Slices slice = f32_slices(M, N, K);
+  return (long long)((K + SEGMENT - 1) / SEGMENT) * slice.m * slice.n;
+}
+
+// How many kernels it launches.
+PAE_EXPORT int pae_linear_f32_launches(int M, int N, int K) {
+  const Slices slice = f32_slices(M, N, K);
+  return slice.m == 0 ? 1 : 2 * ((M + slice.m - 1) / slice.m) * ((N + slice.n - 1) / slice.n);
 }
 
 // out[M, N] = x[M, K] . w[N, K]^T (+ bias[N]) (+ residual[M, N]), all float32, sums in double; K a multiple of 4,
-// x and w on 16-byte boundaries. planes: double scratch [pae_linear_f32_planes(M, N, K), M, N], or null when that is 0.
+// x and w on 16-byte boundaries. planes: pae_linear_f32_scratch(M, N, K) doubles of scratch, or null when that is 0.
 PAE_EXPORT int pae_linear_f32(float* out, const float* x, const float* w, const float* bias, const float* residual, int M, int N, int K,
                               double* planes, void* stream) {
   if (M == 0 || N == 0) return 0;
@@ -551,20 +584,28 @@ PAE_EXPORT int pae_linear_f32(float* out, const float* x, const float* w, const 
   const int tiles_m = (M + tiled::TILE - 1) / tiled::TILE, tiles_n = (N + tiled::TILE - 1) / tiled::TILE;
   if (tiles_m > 65535) return fail(3, "linear_f32: %d rows are more than one launch takes", M);
   const int segments = (K + SEGMENT - 1) / SEGMENT;
-  const bool split = pae_linear_f32_planes(M, N, K) > 0;
-  if (split && planes == nullptr) return fail(2, "linear_f32: [%d, %d] x [%d, %d] needs scratch planes", M, K, N, K);
+  const Slices slice = f32_slices(M, N, K);
+  if (slice.m > 0 && planes == nullptr) return fail(2, "linear_f32: [%d, %d] x [%d, %d] needs scratch planes", M, K, N, K);
   static const cudaError_t configured =
       cudaFuncSetAttribute(f32_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiled::SMEM_BYTES);
   if (configured != cudaSuccess) return fail(100, "linear_f32: %s", cudaGetErrorString(configured));
-  int blocks_k = split ? (int)(3LL * sm_count() / ((long long)tiles_m * tiles_n)) : 1;
-  blocks_k = blocks_k > segments ? segments : blocks_k;
-  const int per = (segments + blocks_k - 1) / blocks_k;
-  launch_kernel(f32_tile_kernel, dim3(tiles_n, tiles_m, (segments + per - 1) / per), 128, tiled::SMEM_BYTES, s, out, split ? planes : nullptr, x, w, bias,
-                residual, M, N, K, per);
-  if (split) {
-    const long long count = (long long)M * N;
-    launch_kernel(f32_planes_kernel, dim3((unsigned)((count + 255) / 256)), 256, 0, s, out, planes, bias, residual, segments, count, N);
+  if (slice.m == 0) {
+    launch_kernel(f32_tile_kernel, dim3(tiles_n, tiles_m, 1), 128, tiled::SMEM_BYTES, s, out, nullptr, x, w, bias, residual, M, N, K, segments);
+    return check_launch("linear_f32");
   }
+  for (int m0 = 0; m0 < M; m0 += slice.m)
+    for (int n0 = 0; n0 < N; n0 += slice.n) {
+      const int m = slice.m < M - m0 ? slice.m : M - m0, n = slice.n < N - n0 ? slice.n : N - n0;
+      const int grid_m = (m + tiled::TILE - 1) / tiled::TILE, grid_n = (n + tiled::TILE - 1) / tiled::TILE;
+      int blocks_k = (int)(3LL * sm_count() / ((long long)grid_m * grid_n));
+      blocks_k = blocks_k > segments ? segments : blocks_k;
+      const int per = (segments + blocks_k - 1) / blocks_k;
+      const size_t at = (size_t)m0 * N + n0;
+      launch_kernel(f32_tile_kernel, dim3(grid_n, grid_m, (segments + per - 1) / per), 128, tiled::SMEM_BYTES, s, nullptr, planes, x + (size_t)m0 * K,
+                    w + (size_t)n0 * K, nullptr, nullptr, m, n, K, per);
+      launch_kernel(f32_planes_kernel, dim3((unsigned)(((long long)m * n + 255) / 256)), 256, 0, s, out + at, planes, bias != nullptr ? bias + n0 : nullptr,
+                    residual != nullptr ? residual + at : nullptr, segments, m, n, N);
+    }
   return check_launch("linear_f32");
 }
 

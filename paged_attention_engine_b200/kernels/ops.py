@@ -559,10 +559,10 @@ def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str 
     lib = _lib("gemm_simt")
     if (x.dtype == weight.dtype == out_dtype == torch.float32 and k % 4 == 0 and k > 0
             and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0):
-        planes = lib.pae_linear_f32_planes(m, n, k)
-        scratch = torch.empty((planes, m, n), dtype=torch.float64, device=x.device) if planes else None
+        doubles = lib.pae_linear_f32_scratch(m, n, k)
+        scratch = torch.empty(doubles, dtype=torch.float64, device=x.device) if doubles else None
         _check(lib, lib.pae_linear_f32(_ptr(out), _ptr(x), _ptr(weight), _ptr(bias), _ptr(residual), m, n, k, _ptr(scratch), _stream()),
-               2 if planes else 1)
+               lib.pae_linear_f32_launches(m, n, k) if doubles else 1)
         return out
     _check(lib, lib.pae_linear_simt(_ptr(out), _ptr(x), _ptr(weight), _ptr(bias), _ptr(residual), m, n,
                                     k, (_code(x)), (_code(weight)), _DTYPE_CODE[out_dtype],
