@@ -581,8 +581,10 @@ __device__ __forceinline__ void tile_epilogue(const Params& p, uint32_t lane_add
 
 // GATE: the gate's activation of the gated epilogue, known when compiled (a choice at run time in that
 // epilogue cost the SiLU models 1 % of a step). ROTARY: whether the epilogue rotates, likewise: its angles take 168 registers a thread,
-// the others 60, and a block of 60 may start beside the blocks of the kernel before and ask for its first weights there (a
-// 100-token prompt of 8 layers of the 1.5B sizes 628 -> 611 us).
+// the others 60, and a block of 60 may start beside the blocks of the kernel before.
+// Nothing of the operands is read before the wait for the kernel before, the weights neither: a caller may have just written them.
+// (With the first weights asked for before the wait a 100-token prompt of 8 layers of the 1.5B sizes took 573 instead of 583 us, one of 2,048
+// tokens 1,952 instead of 1,930, and products whose weights lie in L2 up to a tenth longer: 512 tokens x 2,048 x 1,024 with SiLU x up 9.2 instead of 8.3.)
 template <int PBN, int GATE, bool ROTARY>
 __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                           const __grid_constant__ CUtensorMap map_b,
@@ -629,25 +631,13 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  dependent_launch_wait();
 
   // A work item is an output tile, or one of the `planes` ranges of K of an output tile when a
   // launch of few tiles and a long K shares each tile out over several blocks.
   const int planes = p.planes > 1 ? p.planes : 1;
   const int total_items = tiles_a * tiles_b * planes;
   const int k_blocks = p.k_blocks;
-  // The weights of the first item's first stages are asked for before the wait for the kernel before, which never writes
-  // them (grouped: which matrix a tile multiplies is that kernel's output, so nothing is): they are a large
-  // part of what a block reads when the tokens are few.
-  int early = 0;
-  if (threadIdx.x == 0 && p.group_tiles == nullptr && (int)blockIdx.x < total_items) {
-    const int item = blockIdx.x, kb_first = (item % planes) * p.kb_per_split;
-    const int count = min(kb_first + p.kb_per_split, k_blocks) - kb_first;
-    for (; early < PSTAGES && early < count; ++early) {
-      mbar_expect_tx(full_bar(early), P_STAGE_BYTES);
-      tma_load_2d(base + early * P_STAGE_BYTES + P_A_BYTES, &map_b, full_bar(early), (kb_first + early) * BK, item / planes / tiles_a * PBN);
-    }
-  }
-  dependent_launch_wait();
   // Grouped: how many of the table's tiles are in use, read once by the thread or warp of each role.
   auto used_tiles = [&]() { return p.group_tiles != nullptr ? min(tiles_a, p.group_tiles[2 * tiles_a]) : tiles_a; };
   // Which tile of the A rows and which of the B rows a tile index means. Plain: neighbouring
@@ -680,9 +670,9 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
             break;
           }
           const uint32_t a_dst = base + s * P_STAGE_BYTES;
-          if (it >= early) mbar_expect_tx(full_bar(s), P_STAGE_BYTES);
+          mbar_expect_tx(full_bar(s), P_STAGE_BYTES);
           tma_load_2d(a_dst, &map_a, full_bar(s), kb * BK, tile_a * BM);
-          if (it >= early) tma_load_2d(a_dst + P_A_BYTES, &map_b, full_bar(s), kb * BK, b_row);
+          tma_load_2d(a_dst + P_A_BYTES, &map_b, full_bar(s), kb * BK, b_row);
         }
       }
       if (*abort_flag) {
@@ -884,16 +874,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PERSISTENT_THREADS)
   const int k_blocks = p.k_blocks;
   if (warp == 0) {
     if (lane == 0) {
-      int it = 0, issued_b = 0;
+      int it = 0;
       bool ok = true;
-      // The weights of the first stages are asked for before the wait for the kernel before: they are not written in a step.
-      if ((int)(blockIdx.x >> 1) < total) {
-        const int b_row = (int)(blockIdx.x >> 1) / tiles_a * PBN + rank * (PBN / 2);
-        for (; issued_b < STAGES && issued_b < k_blocks; ++issued_b) {
-          if (rank == 0) mbar_expect_tx(full_bar(issued_b), 2 * T::STAGE_BYTES);
-          tma_load_2d_pair(base + issued_b * T::STAGE_BYTES + T::A_BYTES, &map_b, in_block(full_bar(issued_b), 0), issued_b * BK, b_row);
-        }
-      }
       dependent_launch_wait();
       for (int tile = blockIdx.x >> 1; tile < total && ok; tile += step) {
         const int a_row = (tile % tiles_a * 2 + rank) * BM, b_row = tile / tiles_a * PBN + rank * (PBN / 2);
@@ -904,9 +886,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PERSISTENT_THREADS)
             break;
           }
           const uint32_t a_dst = base + s * T::STAGE_BYTES, report = in_block(full_bar(s), 0);
-          if (it >= issued_b && rank == 0) mbar_expect_tx(full_bar(s), 2 * T::STAGE_BYTES);
+          if (rank == 0) mbar_expect_tx(full_bar(s), 2 * T::STAGE_BYTES);
           tma_load_2d_pair(a_dst, &map_a, report, kb * BK, a_row);
-          if (it >= issued_b) tma_load_2d_pair(a_dst + T::A_BYTES, &map_b, report, kb * BK, b_row);
+          tma_load_2d_pair(a_dst + T::A_BYTES, &map_b, report, kb * BK, b_row);
         }
       }
       if (*abort_flag && rank == 0) {      // both blocks' loads report here; the other block waits for this one at the end

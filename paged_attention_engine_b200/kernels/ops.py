@@ -513,7 +513,11 @@ def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str 
     """x [M, K] . weight [N, K]^T (+ bias [N], float32) (+ residual [M, N]) -> [M, N]. `activation`
     ("gelu_erf", "gelu_tanh", "relu2": the square of max(z, 0)) is applied to the product (+ bias), rounded to the output's dtype first,
     before the residual: in the tensor-core product's epilogue or in the sum of its splits, else
-    by the activation's own kernel."""
+    by the activation's own kernel.
+
+    The bfloat16 kernels of few tokens (up to 64, or 128 where K is long) or of fewer than 256 columns read `weight` while the kernel
+    before them in the stream may still be running, as they do in `linear_swiglu` and `qkv_projection`: a weight that the call just before
+    wrote needs another launch, or a synchronisation, in between. Larger products read nothing before that kernel has completed."""
     if activation not in ACTIVATIONS:
         raise KernelError(f"linear: activation '{activation}' (known: gelu_erf, gelu_tanh, relu2)")
     if (activation is None and bias is None and out_dtype in (None, torch.bfloat16) and weight.dtype == torch.bfloat16 and weight.dim() == 2

@@ -78,3 +78,19 @@ def test_heads_product_with_rotation_and_page_write(m, heads, kv_heads, d):
     for a, b in zip(*results):
         assert torch.equal(a, b)
     ops.check_device_errors()
+
+
+@pytest.mark.parametrize("m,n,k,pairs", [(8192, 3584, 1536, True), (300, 2048, 1024, False)])
+def test_a_weight_that_the_call_before_wrote(m, n, k, pairs):
+    """The product waits for the kernel before, which starts it early; nothing of the weight is read until then."""
+    from paged_attention_engine_b200.kernels import ops
+
+    assert _by_pairs(m, n, k) == pairs
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x, a, b = _bf(gen, m, k), _bf(gen, n, 512), _bf(gen, k, 512, std=0.002)
+    weight = ops.linear(a, b)
+    torch.cuda.synchronize()
+    want = ops.linear(x, weight)
+    for _ in range(20):
+        assert torch.equal(ops.linear(x, ops.linear(a, b)), want)
+    ops.check_device_errors()

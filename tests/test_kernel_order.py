@@ -41,3 +41,10 @@ def test_no_block_of_a_cluster_reaches_another_before_a_cluster_barrier(kernel):
         if name == kernel and (first := REMOTE.search(body)):
             barrier = BARRIER.search(body)
             assert barrier and barrier.start() < first.start(), f"{name}: {first.group(0)} comes first"
+
+
+@pytest.mark.parametrize("kernel", ["gemm_tcgen05_persistent_kernel", "gemm_tcgen05_pair_kernel"])
+def test_a_many_token_product_loads_nothing_before_the_kernel_before_has_completed(kernel):
+    """Its weights may have been written by the kernel before."""
+    (body,) = [body for _, name, body in _kernels() if name == kernel]
+    assert 0 < body.index("dependent_launch_wait()") < body.index("tma_load_2d")
