@@ -195,12 +195,9 @@ int launch_sized(void* out, const void* q, const void* keys, const void* values,
                  int d, int dv, int vs_row, int page_size, const ScoreRule& rule, cudaStream_t s) {
   const size_t bytes = smem_bytes(d, dv);
   auto kernel = attention_scored_kernel<T, A, MAX_D>;
-  static bool raised = false;
-  if (bytes > 48 * 1024 && !raised) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT);
-    if (err != cudaSuccess) return fail(100, "paged_attention_scored: %s", cudaGetErrorString(err));
-    raised = true;
-  }
+  static DevicesSet raised;
+  if (bytes > 48 * 1024)
+    if (int err = raise_shared_memory(raised, kernel, SMEM_LIMIT, "paged_attention_scored")) return err;
   dim3 grid((max_q_len + BQ - 1) / BQ, heads, seqs);
   launch_kernel(kernel, grid, THREADS, bytes, s, (T*)out, (const T*)q, (const T*)keys, (const T*)values, block_table,
                 table_width, q_start, q_pos0, kv_len, heads, kv_heads, d, dv, vs_row, page_size, rule);

@@ -1131,17 +1131,11 @@ int launch(const Params& p, const void* qkv, const void* keys, const void* value
   const int box_rows = p.page_size < tile_keys ? p.page_size : tile_keys;
   if (int err = tensor_map(&map_k, keys, cache_rows, D, box_rows)) return err;
   if (int err = tensor_map(&map_v, values, cache_rows, D, box_rows)) return err;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(prefill_tcgen05_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Layout<D>::SMEM_BYTES);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(prefill_tcgen05_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Layout<D>::SMEM_BYTES);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(paired::prefill_tcgen05_paired_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)paired::Layout<D>::SMEM_BYTES);
-    if (err != cudaSuccess) return fail(100, "paged_attention_tcgen05: %s", cudaGetErrorString(err));
-    configured = true;
-  }
+  static DevicesSet raised_one, raised_cluster, raised_paired;
+  if (int err = raise_shared_memory(raised_one, prefill_tcgen05_kernel<D, false>, Layout<D>::SMEM_BYTES, "paged_attention_tcgen05")) return err;
+  if (int err = raise_shared_memory(raised_cluster, prefill_tcgen05_kernel<D, true>, Layout<D>::SMEM_BYTES, "paged_attention_tcgen05")) return err;
+  if (int err = raise_shared_memory(raised_paired, paired::prefill_tcgen05_paired_kernel<D>, paired::Layout<D>::SMEM_BYTES, "paged_attention_tcgen05"))
+    return err;
   if (chosen != nullptr) *chosen = use_paired ? 0 : (int)ranks;
   if (use_paired) {
     launch_kernel(paired::prefill_tcgen05_paired_kernel<D>, grid, paired::THREADS, paired::Layout<D>::SMEM_BYTES, stream, map_q, map_k,

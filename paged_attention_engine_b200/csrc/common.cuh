@@ -10,6 +10,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -36,6 +37,23 @@ inline int fail(int code, const char* format, ...) {
 inline int check_launch(const char* what) {
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return fail(100, "%s: %s", what, cudaGetErrorString(err));
+  return 0;
+}
+
+// A kernel's limit of dynamic shared memory is a setting of the kernel on ONE device: `raise_shared_memory` sets it the first time
+// that the kernel is launched on each. One of these per kernel, kept for the life of the process. A failed attempt is not remembered.
+struct DevicesSet {
+  std::atomic<bool> done[64];
+};
+template <typename Kernel>
+inline int raise_shared_memory(DevicesSet& devices, Kernel* kernel, size_t bytes, const char* what) {
+  int device = 0;
+  cudaError_t err = cudaGetDevice(&device);
+  const bool kept = err == cudaSuccess && device >= 0 && device < 64;
+  if (kept && devices.done[device].load(std::memory_order_acquire)) return 0;
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (err != cudaSuccess) return fail(100, "%s: %s", what, cudaGetErrorString(err));
+  if (kept) devices.done[device].store(true, std::memory_order_release);
   return 0;
 }
 

@@ -279,9 +279,8 @@ int launch_few(float* out, const float* x, const float* w, const float* bias, co
   using L = few::Layout<T>;
   const int segments = (K + SEGMENT - 1) / SEGMENT;
   const int warps = segments < few::WARPS ? segments : few::WARPS;
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(f32_few_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::bytes(few::WARPS));
-  if (configured != cudaSuccess) return fail(100, "linear_f32: %s", cudaGetErrorString(configured));
+  static DevicesSet raised;
+  if (int err = raise_shared_memory(raised, f32_few_kernel<T>, L::bytes(few::WARPS), "linear_f32")) return err;
   launch_kernel(f32_few_kernel<T>, dim3((N + few::ROWS - 1) / few::ROWS), 32 * warps, L::bytes(warps), s, out, x, w, bias, residual, M, N, K);
   return check_launch("linear_f32");
 }
@@ -398,9 +397,8 @@ int launch_lane(float* out, const float* x, const float* w, const float* bias, c
   using L = lane_rows::Layout<MT>;
   const int pairs = ((K + SEGMENT - 1) / SEGMENT + 1) / 2;
   const int warps = pairs < lane_rows::WARPS ? pairs : lane_rows::WARPS;
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(f32_lane_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::bytes(lane_rows::WARPS));
-  if (configured != cudaSuccess) return fail(100, "linear_f32: %s", cudaGetErrorString(configured));
+  static DevicesSet raised;
+  if (int err = raise_shared_memory(raised, f32_lane_kernel<MT>, L::bytes(lane_rows::WARPS), "linear_f32")) return err;
   launch_kernel(f32_lane_kernel<MT>, dim3((N + lane_rows::ROWS - 1) / lane_rows::ROWS), 32 * warps, L::bytes(warps), s, out, x, w, bias, residual, M, N, K);
   return check_launch("linear_f32");
 }
@@ -586,9 +584,8 @@ PAE_EXPORT int pae_linear_f32(float* out, const float* x, const float* w, const 
   const int segments = (K + SEGMENT - 1) / SEGMENT;
   const Slices slice = f32_slices(M, N, K);
   if (slice.m > 0 && planes == nullptr) return fail(2, "linear_f32: [%d, %d] x [%d, %d] needs scratch planes", M, K, N, K);
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(f32_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiled::SMEM_BYTES);
-  if (configured != cudaSuccess) return fail(100, "linear_f32: %s", cudaGetErrorString(configured));
+  static DevicesSet raised;
+  if (int err = raise_shared_memory(raised, f32_tile_kernel, tiled::SMEM_BYTES, "linear_f32")) return err;
   if (slice.m == 0) {
     launch_kernel(f32_tile_kernel, dim3(tiles_n, tiles_m, 1), 128, tiled::SMEM_BYTES, s, out, nullptr, x, w, bias, residual, M, N, K, segments);
     return check_launch("linear_f32");

@@ -977,12 +977,8 @@ int launch(const Params& p, const void* a, const void* b, int k, int splits, cud
   if (int err = tensor_map(&map_a, a, p.rows_a, k, BM)) return err;
   if (int err = tensor_map(&map_b, b, p.rows_b, k, BN)) return err;
   auto kernel = gemm_tcgen05_kernel<BN, MODE, SELFTEST>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM_BYTES);
-    if (err != cudaSuccess) return fail(100, "linear_tcgen05: %s", cudaGetErrorString(err));
-    configured = true;
-  }
+  static DevicesSet raised;
+  if (int err = raise_shared_memory(raised, kernel, T::SMEM_BYTES, "linear_tcgen05")) return err;
   dim3 grid((p.rows_a + BM - 1) / BM, (p.rows_b + BN - 1) / BN, splits);
   launch_kernel(kernel, grid, THREADS, T::SMEM_BYTES, stream, map_a, map_b, p);
   return check_launch("linear_tcgen05");
@@ -1003,12 +999,8 @@ int launch_persistent_with(const Params& p, const void* a, const void* b, int k,
   CUtensorMap map_a, map_b;
   if (int err = tensor_map(&map_a, a, p.rows_a, k, BM)) return err;
   if (int err = tensor_map(&map_b, b, p.group_tiles != nullptr ? p.rows_b * p.groups : p.rows_b, k, PBN)) return err;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(gemm_tcgen05_persistent_kernel<PBN, GATE, ROTARY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM_BYTES);
-    if (err != cudaSuccess) return fail(100, "linear_tcgen05: %s", cudaGetErrorString(err));
-    configured = true;
-  }
+  static DevicesSet raised;
+  if (int err = raise_shared_memory(raised, gemm_tcgen05_persistent_kernel<PBN, GATE, ROTARY>, T::SMEM_BYTES, "linear_tcgen05")) return err;
   const int tiles_a = (p.rows_a + BM - 1) / BM, tiles_b = (p.rows_b + PBN - 1) / PBN;
   const int items = tiles_a * tiles_b * (p.planes > 1 ? p.planes : 1);
   const int blocks = items < sm_count() ? items : sm_count();
@@ -1022,9 +1014,8 @@ int launch_pair_with(const Params& p, const void* a, const void* b, int k, cudaS
   CUtensorMap map_a, map_b;
   if (int err = tensor_map(&map_a, a, p.rows_a, k, BM)) return err;
   if (int err = tensor_map(&map_b, b, p.rows_b, k, PBN / 2)) return err;
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<PBN, ROTARY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM_BYTES);
-  if (configured != cudaSuccess) return fail(100, "linear_tcgen05: %s", cudaGetErrorString(configured));
+  static DevicesSet raised;
+  if (int err = raise_shared_memory(raised, gemm_tcgen05_pair_kernel<PBN, ROTARY>, T::SMEM_BYTES, "linear_tcgen05")) return err;
   const int tiles_a = (p.rows_a + 2 * BM - 1) / (2 * BM), tiles_b = (p.rows_b + PBN - 1) / PBN;
   const int pairs = sm_count() / 2;
   const int clusters = tiles_a * tiles_b < pairs ? tiles_a * tiles_b : pairs;

@@ -276,12 +276,9 @@ int launch_columns(Scan p, int seqs, int splits, cudaStream_t s) {
   per_block = per_block > 4 ? 4 : per_block;
   p.cols = WARP_COLS * per_block;
   const size_t smem = 2 * sizeof(float) * ((size_t)TILE * (2 * ROW + p.cols) + 2 * TILE);
-  static bool raised = false;
-  if (smem > 48 * 1024 && !raised) {
-    cudaError_t err = cudaFuncSetAttribute(matrix_memory_scan_columns_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    if (err != cudaSuccess) return fail(100, "matrix_memory: %s", cudaGetErrorString(err));
-    raised = true;
-  }
+  static DevicesSet raised;
+  if (smem > 48 * 1024)
+    if (int err = raise_shared_memory(raised, matrix_memory_scan_columns_kernel<D>, 64 * 1024, "matrix_memory")) return err;
   launch_kernel(matrix_memory_scan_columns_kernel<D>, dim3((warps + per_block - 1) / per_block, p.heads, seqs), 32 * per_block, smem, s, p);
   return check_launch("matrix_memory_scan");
 }
@@ -365,12 +362,9 @@ PAE_EXPORT int pae_matrix_memory_scan(float* o, float* state, float* carry, cons
   }
   const int blocks = (dv + cols - 1) / cols;
   const size_t smem = scan_smem(d, cols);
-  static size_t raised = 48 * 1024;
-  if (smem > raised) {
-    cudaError_t err = cudaFuncSetAttribute(matrix_memory_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (err != cudaSuccess) return fail(100, "matrix_memory: %s", cudaGetErrorString(err));
-    raised = 200 * 1024;
-  }
+  static DevicesSet raised;
+  if (smem > 48 * 1024)
+    if (int err = raise_shared_memory(raised, matrix_memory_scan_kernel, 200 * 1024, "matrix_memory")) return err;
   Scan p{o, state, carry, proj, i_bias, f_bias, q_start, state_slot, ld, q_off, k_off, v_off, i_off, f_off, heads, d, dv, cols, cap, q_scale};
   const int threads = ((cols + 1 + 31) / 32) * 32;
   launch_kernel(matrix_memory_scan_kernel, dim3(blocks, heads, seqs), threads, smem, (cudaStream_t)stream, p);

@@ -363,12 +363,9 @@ bool aligned16(const void* ptr) { return (((uintptr_t)ptr) & 15) == 0; }
 
 template <typename TO, int VEC>
 int launch(const PostNorm& p, int rows, int threads, size_t bytes, cudaStream_t s) {
-  static bool raised = false;
-  if (bytes > 48 * 1024 && !raised) {
-    cudaError_t err = cudaFuncSetAttribute(post_norm_kernel<TO, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MOST);
-    if (err != cudaSuccess) return fail(100, "post_norm: %s", cudaGetErrorString(err));
-    raised = true;
-  }
+  static DevicesSet raised;
+  if (bytes > 48 * 1024)
+    if (int err = raise_shared_memory(raised, post_norm_kernel<TO, VEC>, SMEM_MOST, "post_norm")) return err;
   launch_kernel(post_norm_kernel<TO, VEC>, rows, threads, bytes, s, p);
   return check_launch("post_norm");
 }
