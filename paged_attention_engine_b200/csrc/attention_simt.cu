@@ -169,8 +169,16 @@ int launch(void* out, const void* qkv, const void* keys, const void* values, con
 // one token over 68 keys 56.7 us, over 250 keys 157 (12 heads of 128).
 // ---------------------------------------------------------------------------------------
 namespace wide {
-constexpr int WARPS = 8;
 constexpr int KEYS = 16;                     // keys of a tile
+
+int sm_count() {
+  static const int count = [] {
+    int device = 0, n = 148;
+    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+    return n;
+  }();
+  return count;
+}
 
 template <int DL>
 struct Vec {
@@ -206,15 +214,31 @@ __device__ __forceinline__ float sum_across(float (&s)[KEYS], int lane) {
   return s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);
 }
 
-template <int DL, int ROWS>
-__global__ void __launch_bounds__(32 * WARPS) paged_attention_f32_kernel(
+// This lane's dimensions of the 16 rows of the cache `place` (one per pair of lanes; -1: zeros).
+template <int DL>
+__device__ __forceinline__ void fetch(Vec<DL> (&to)[KEYS], const float* from, int place, int lane) {
+#pragma unroll
+  for (int i = 0; i < KEYS; ++i) {
+    const int at = __shfl_sync(0xffffffffu, place, 2 * i);
+#pragma unroll
+    for (int e = 0; e < DL; ++e) to[i].v[e] = 0.f;
+    if (at >= 0) to[i] = load<DL>(from + (size_t)at * (32 * DL) + lane * DL);
+  }
+}
+
+// PACKED: for launches of more blocks than run at once, in which what counts is how many warps an SM holds (`launch` has the rule and the
+// times). A tile's values are asked for when its scores are there, into the keys' registers (128, 80 and 64 a thread at head
+// sizes 128, 64 and 32 instead of 223, 128 and 101), the four rows go through a tile's steps side by side, and a block has only as many warps W as
+// the longest context has tiles. A row's arithmetic is the same in both, and a warp without a tile adds nothing: the bits are the same.
+template <int DL, int ROWS, int W, bool PACKED>
+__global__ void __launch_bounds__(32 * W, PACKED ? (DL == 1 ? 32 : DL == 2 ? 24 : 16) / W : 0) paged_attention_f32_kernel(
     float* __restrict__ out, const float* __restrict__ qkv, const float* __restrict__ keys, const float* __restrict__ values,
     const int* __restrict__ block_table, int table_width, const int* __restrict__ q_start, const int* __restrict__ q_pos0,
     const int* __restrict__ kv_len, int heads, int kv_heads, int page_size, float scale, int window) {
   constexpr int D = 32 * DL;
   dependent_launch_prologue();
-  __shared__ float merged_max[WARPS][ROWS], merged_sum[WARPS][ROWS];
-  __shared__ __align__(16) float merged_out[WARPS][ROWS][D];
+  __shared__ float merged_max[W][ROWS], merged_sum[W][ROWS];
+  __shared__ __align__(16) float merged_out[W][ROWS][D];
   const int b = blockIdx.z, h = blockIdx.y;
   const int first_token = q_start[b];
   const int q_count = q_start[b + 1] - first_token;
@@ -240,12 +264,67 @@ __global__ void __launch_bounds__(32 * WARPS) paged_attention_f32_kernel(
   }
   const int first_tile = kv_begin / KEYS, end_tile = (kv_end + KEYS - 1) / KEYS;
   const int my_key = lane >> 1;                          // the key of a tile whose score ends in this lane
-  for (int tile = first_tile + (warp - first_tile % WARPS + WARPS) % WARPS; tile < end_tile; tile += WARPS) {
+  for (int tile = first_tile + (warp - first_tile % W + W) % W; tile < end_tile; tile += W) {
     const int j = tile * KEYS + my_key;
     int place = -1;                                      // row of the key in the cache, -1: not seen by any query here
     if (j >= kv_begin && j < kv_end) {
       const int page = checked_page(table[checked_table_index(j / page_size, table_width)]);
       place = (page * kv_heads + g) * page_size + j % page_size;
+    }
+    if constexpr (PACKED) {
+      float p[ROWS], tile_max[ROWS], tile_sum[ROWS], rescale[ROWS];
+      bool seen[ROWS];
+      {
+        Vec<DL> k[KEYS];
+        fetch<DL>(k, keys, place, lane);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          float s[KEYS];
+#pragma unroll
+          for (int i = 0; i < KEYS; ++i) {
+            s[i] = q[r].v[0] * k[i].v[0];
+#pragma unroll
+            for (int e = 1; e < DL; ++e) s[i] = fmaf(q[r].v[e], k[i].v[e], s[i]);
+          }
+          p[r] = sum_across(s, lane);
+        }
+      }
+      Vec<DL> v[KEYS];
+      fetch<DL>(v, values, place, lane);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const int pos = p0 + r;
+        seen[r] = place >= 0 && j <= pos && (window <= 0 || pos - j < window);
+        tile_max[r] = p[r] = seen[r] ? p[r] * scale : -FLT_MAX;
+      }
+#pragma unroll
+      for (int o = 16; o > 1; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) tile_max[r] = fmaxf(tile_max[r], __shfl_xor_sync(0xffffffffu, tile_max[r], o));
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const float new_max = fmaxf(row_max[r], tile_max[r]);
+        rescale[r] = row_max[r] == -FLT_MAX ? 0.f : expf(row_max[r] - new_max);
+        tile_sum[r] = p[r] = seen[r] ? expf(p[r] - new_max) : 0.f;
+        row_max[r] = new_max;
+#pragma unroll
+        for (int e = 0; e < DL; ++e) acc[r][e] *= rescale[r];
+      }
+#pragma unroll
+      for (int o = 16; o > 1; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) tile_sum[r] += __shfl_xor_sync(0xffffffffu, tile_sum[r], o);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) row_sum[r] = row_sum[r] * rescale[r] + tile_sum[r];
+#pragma unroll
+      for (int i = 0; i < KEYS; ++i)
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          const float weight = __shfl_sync(0xffffffffu, p[r], 2 * i);
+#pragma unroll
+          for (int e = 0; e < DL; ++e) acc[r][e] = fmaf(weight, v[i].v[e], acc[r][e]);
+        }
+      continue;
     }
     Vec<DL> k[KEYS], v[KEYS];
 #pragma unroll
@@ -303,14 +382,14 @@ __global__ void __launch_bounds__(32 * WARPS) paged_attention_f32_kernel(
     for (int e = 0; e < DL; ++e) merged_out[warp][r][lane * DL + e] = acc[r][e];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < rows * D; i += 32 * WARPS) {
+  for (int i = threadIdx.x; i < rows * D; i += 32 * W) {
     const int r = i / D, dim = i % D;
     float top = -FLT_MAX;
 #pragma unroll
-    for (int w = 0; w < WARPS; ++w) top = fmaxf(top, merged_max[w][r]);
+    for (int w = 0; w < W; ++w) top = fmaxf(top, merged_max[w][r]);
     float sum = 0.f, value = 0.f;
 #pragma unroll
-    for (int w = 0; w < WARPS; ++w) {
+    for (int w = 0; w < W; ++w) {
       const float factor = merged_max[w][r] == -FLT_MAX ? 0.f : expf(merged_max[w][r] - top);
       sum += merged_sum[w][r] * factor;
       value = fmaf(merged_out[w][r][dim], factor, value);
@@ -323,14 +402,26 @@ __global__ void __launch_bounds__(32 * WARPS) paged_attention_f32_kernel(
 
 template <int DL>
 int launch(float* out, const float* qkv, const float* keys, const float* values, const int* block_table, int table_width,
-           const int* q_start, const int* q_pos0, const int* kv_len, int seqs, int max_q_len, int heads, int kv_heads,
+           const int* q_start, const int* q_pos0, const int* kv_len, int seqs, int max_q_len, int max_kv_len, int heads, int kv_heads,
            int page_size, float scale, int window, cudaStream_t s) {
-  if (max_q_len == 1)
-    launch_kernel(paged_attention_f32_kernel<DL, 1>, dim3(1, heads, seqs), 32 * WARPS, 0, s, out, qkv, keys, values, block_table, table_width,
+  auto run = [&](auto kernel, int rows, int warps) {
+    launch_kernel(kernel, dim3((max_q_len + rows - 1) / rows, heads, seqs), 32 * warps, 0, s, out, qkv, keys, values, block_table, table_width,
                   q_start, q_pos0, kv_len, heads, kv_heads, page_size, scale, window);
-  else
-    launch_kernel(paged_attention_f32_kernel<DL, 4>, dim3((max_q_len + 3) / 4, heads, seqs), 32 * WARPS, 0, s, out, qkv, keys, values,
-                  block_table, table_width, q_start, q_pos0, kv_len, heads, kv_heads, page_size, scale, window);
+  };
+  // Packed when there are more blocks than run at once (one on an SM at head size 128, two at 64 and 32) and most of what a query sees are the
+  // portions' own keys. Below that its second trip to memory per tile shows (head size 128: one prompt of 16 tokens 6.4 us against 6.2), and
+  // few queries after long contexts are the other form's (3 after 4,000 keys 130 against 95 us, 32 requests of 17 after 4,000 at
+  // head size 64 2,541 against 1,835). Many short prompts, general form / not packed / packed: 32 prompts of 64 tokens, 28 heads of 128
+  // 243 / 389 / 157 us, 16 heads of 32 57 / 98 / 38; 32 of 128 tokens 798 / 928 / 615 and 159 / 208 / 131; one of 2,048, 28 heads 5,039 / 2,776 / 2,182.
+  const long long blocks = (long long)((max_q_len + 3) / 4) * heads * seqs, at_once = (DL == 4 ? 1LL : 2LL) * sm_count();
+  const int seen = window > 0 && (long long)window + max_q_len < max_kv_len ? window + max_q_len : max_kv_len;
+  const bool packed = blocks > at_once && seen <= 4LL * max_q_len;
+  if (max_q_len == 1) run(paged_attention_f32_kernel<DL, 1, 8, false>, 1, 8);
+  else if (!packed) run(paged_attention_f32_kernel<DL, 4, 8, false>, 4, 8);
+  else if (max_kv_len <= KEYS) run(paged_attention_f32_kernel<DL, 4, 1, true>, 4, 1);
+  else if (max_kv_len <= 2 * KEYS) run(paged_attention_f32_kernel<DL, 4, 2, true>, 4, 2);
+  else if (max_kv_len <= 4 * KEYS) run(paged_attention_f32_kernel<DL, 4, 4, true>, 4, 4);
+  else run(paged_attention_f32_kernel<DL, 4, 8, true>, 4, 8);
   return check_launch("paged_attention_simt");
 }
 }  // namespace wide
@@ -341,8 +432,8 @@ int launch(float* out, const float* qkv, const float* keys, const float* values,
 // keys, values [pages, kv_heads, page_size, d]; block_table [seqs, table_width].
 PAE_EXPORT int pae_paged_attention_simt(void* out, const void* qkv, const void* keys, const void* values,
                                         const int* block_table, int table_width, const int* q_start,
-                                        const int* q_pos0, const int* kv_len, int seqs, int max_q_len, int heads,
-                                        int kv_heads, int d, int page_size, float scale, int window, int dtype,
+                                        const int* q_pos0, const int* kv_len, int seqs, int max_q_len, int max_kv_len,
+                                        int heads, int kv_heads, int d, int page_size, float scale, int window, int dtype,
                                         void* stream) {
   if (seqs == 0 || max_q_len == 0) return 0;
   if (d % 8 || d > MAX_D || d < 8) return fail(2, "paged_attention_simt: head_dim %d is not a multiple of 8 in [8, %d]", d, MAX_D);
@@ -355,7 +446,7 @@ PAE_EXPORT int pae_paged_attention_simt(void* out, const void* qkv, const void* 
   if (dtype == kF32 && aligned && (d == 32 || d == 64 || d == 128)) {
     const auto launch_wide = d == 32 ? wide::launch<1> : (d == 64 ? wide::launch<2> : wide::launch<4>);
     return launch_wide((float*)out, (const float*)qkv, (const float*)keys, (const float*)values, block_table, table_width, q_start, q_pos0,
-                       kv_len, seqs, max_q_len, heads, kv_heads, page_size, scale, window, s);
+                       kv_len, seqs, max_q_len, max_kv_len, heads, kv_heads, page_size, scale, window, s);
   }
   if (dtype == kF32)
     return launch<float>(out, qkv, keys, values, block_table, table_width, q_start, q_pos0, kv_len, seqs, max_q_len, heads, kv_heads, d, page_size, scale, window, s);

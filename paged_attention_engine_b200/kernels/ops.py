@@ -850,7 +850,7 @@ def paged_attention(qkv, keys, values, block_table, q_start, q_pos0, kv_len, num
     _set_bounds("attention_simt", keys)
     _check(lib, lib.pae_paged_attention_simt(
         _ptr(out), _ptr(qkv), _ptr(keys), _ptr(values), _ptr(block_table), block_table.shape[1], _ptr(q_start),
-        _ptr(q_pos0), _ptr(kv_len), seqs, max_q_len, num_heads, num_kv_heads,
+        _ptr(q_pos0), _ptr(kv_len), seqs, max_q_len, max_kv_len, num_heads, num_kv_heads,
         head_dim, page_size, scale, window, (_code(qkv)), _stream()))
     return out
 

@@ -83,3 +83,25 @@ def test_a_score_that_is_no_number_reaches_the_output(d, where, bad, q_lens, pos
     assert torch.equal(got.isnan(), want.isnan())
     there = want.isfinite()
     assert float((got[there] - want[there]).abs().max()) <= 2e-5 * max(1.0, float(want[there].abs().max()))
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("longest", [3, 16, 17, 32, 33, 64, 65, 130])
+def test_a_prompt_has_the_same_bits_alone_and_in_a_launch_that_fills_the_gpu(d, longest):
+    """Many blocks of short contexts run with fewer warps and fewer registers; windows and lengths off the tiles."""
+    from paged_attention_engine_b200.kernels import ops
+
+    heads, window = 8, 0 if longest % 2 else 20
+    q_lens = [longest] * 40 + [max(1, longest - 5), max(1, longest // 2), 1, longest]
+    pos0 = [0] * 43 + [min(longest, 7)]
+    tensors, args = _case(q_lens, pos0, heads, 2, d, 16, window, 4)
+    want = ref.paged_attention(*tensors, **args)
+    qkv, keys, values, table, q_start, _, kv_len = [t.cuda() for t in tensors]
+    got = ops.paged_attention(*[t.cuda() for t in tensors], **args)
+    assert float((got.cpu() - want).abs().max()) <= 2e-5 * max(1.0, float(want.abs().max()))
+    i32 = lambda *a: torch.tensor(a, dtype=torch.int32, device="cuda")  # noqa: E731
+    for b in (0, 40, 41, 42, 43):
+        at, n = int(q_start[b]), q_lens[b]
+        alone = ops.paged_attention(qkv[at : at + n].contiguous(), keys, values, table[b : b + 1].contiguous(), i32(0, n), i32(pos0[b]), kv_len[b : b + 1],
+                                    **dict(args, max_q_len=n, max_kv_len=pos0[b] + n))
+        assert torch.equal(alone, got[at : at + n])
