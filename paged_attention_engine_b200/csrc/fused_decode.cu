@@ -105,10 +105,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float* v) {
 // last bit of the norm. A thread reads the norm's weight and the bias of its first four
 // columns before anything else, and keeps the values of those columns in registers from the
 // sum to the scaling, so nothing is read after the sum of squares is known.
-// PARTS 2: a row is a cluster of two blocks, half of the columns each, which swap their sums of squares through
-// distributed shared memory (added in the blocks' order): a step of 64 tokens keeps 128 SMs busy with its sums
-// instead of 64. Which form runs depends on the row's width only, so a token's bits do not depend on its batch.
-template <typename T, int PARTS>
+template <typename T>
 __global__ void __launch_bounds__(512) splitk_rms_norm_x4_kernel(T* __restrict__ normed, T* __restrict__ value,
                                                                  const float* __restrict__ partial, int splits,
                                                                  const float* __restrict__ bias, const T* __restrict__ residual,
@@ -117,25 +114,21 @@ __global__ void __launch_bounds__(512) splitk_rms_norm_x4_kernel(T* __restrict__
   // products' weights, so they are read before the wait for the kernel before (the weight is
   // read once a step and comes from DRAM, which takes longer than the sums from L2).
   dependent_launch_trigger();
-  // Another block's shared memory may be used once that block has started: the arrival here, whose wait stands before the swap.
-  if constexpr (PARTS == 2) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   const int quads = width / 4;
-  const int row = blockIdx.x / PARTS, part = blockIdx.x % PARTS;
-  const int share = (quads + PARTS - 1) / PARTS, begin = part * share, end = min(quads, begin + share);     // this block's columns, in fours
-  const int mine = begin + threadIdx.x;
   float w_first[4] = {0.f, 0.f, 0.f, 0.f}, b_first[4] = {0.f, 0.f, 0.f, 0.f};
-  if (mine < end) {
-    load4(weight + 4 * mine, w_first);
-    if (bias != nullptr) load4(bias + 4 * mine, b_first);
+  if ((int)threadIdx.x < quads) {
+    load4(weight + 4 * threadIdx.x, w_first);
+    if (bias != nullptr) load4(bias + 4 * threadIdx.x, b_first);
   }
   dependent_launch_wait();
   extern __shared__ float row_values[];
   __shared__ float reduce[32];
+  const int row = blockIdx.x;
   const size_t plane4 = (size_t)rows * quads;
   const float4* part4 = (const float4*)partial;
   float squares = 0.f;
   float first[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int c = mine; c < end; c += blockDim.x) {
+  for (int c = threadIdx.x; c < quads; c += blockDim.x) {
     const size_t at4 = (size_t)row * quads + c;
     float res[4] = {0.f, 0.f, 0.f, 0.f};
     if (residual != nullptr) load4(residual + (size_t)row * width + 4 * c, res);
@@ -164,7 +157,7 @@ __global__ void __launch_bounds__(512) splitk_rms_norm_x4_kernel(T* __restrict__
       v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
     }
     float e[4] = {v.x, v.y, v.z, v.w};
-    const bool is_first = c == mine;
+    const bool is_first = c == (int)threadIdx.x;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (bias != nullptr) e[j] += is_first ? b_first[j] : bias[4 * c + j];
@@ -178,7 +171,7 @@ __global__ void __launch_bounds__(512) splitk_rms_norm_x4_kernel(T* __restrict__
       for (int j = 0; j < 4; ++j) first[j] = e[j];
     } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) row_values[4 * (c - begin) + j] = e[j];
+      for (int j = 0; j < 4; ++j) row_values[4 * c + j] = e[j];
     }
   }
   squares = warp_sum(squares);
@@ -187,29 +180,136 @@ __global__ void __launch_bounds__(512) splitk_rms_norm_x4_kernel(T* __restrict__
   __syncthreads();
   float total = 0.f;                            // every thread adds the warps' sums in the warps' order
   for (int w = 0; w < warps; ++w) total += reduce[w];
-  if constexpr (PARTS == 2) {
-    __shared__ float halves[2];
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");      // both blocks have started, long ago as a rule
-    if (threadIdx.x < 2) {                      // thread b leaves this block's sum in block b of the cluster
-      const uint32_t own = (uint32_t)__cvta_generic_to_shared(&halves[part]);
-      uint32_t there;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(own), "r"((uint32_t)threadIdx.x));
-      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(there), "f"(total) : "memory");
-    }
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-    total = halves[0] + halves[1];
-  }
   const float scale = rsqrtf(total / (float)width + eps);
-  if (mine < end) {
+  if ((int)threadIdx.x < quads) {
     float o[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) o[j] = first[j] * scale * w_first[j];
-    store4(normed + (size_t)row * width + 4 * mine, o);
+    store4(normed + (size_t)row * width + 4 * threadIdx.x, o);
   }
-  for (int i = 4 * (mine + blockDim.x); i < 4 * end; i += 4 * blockDim.x) {      // more than four columns a thread
+  for (int i = 4 * blockDim.x + threadIdx.x; i < width; i += blockDim.x)      // rows wider than four columns a thread
+    normed[(size_t)row * width + i] = from_float<T>(row_values[i] * scale * weight[i]);
+}
+
+// The same row by a cluster of two blocks, with the bits of the kernel above, for launches whose rows leave SMs idle: a step of 64
+// tokens keeps 128 SMs busy with its sums. Bound by the trips to the L2 that a thread makes one after the other: a block takes half of the
+// threads above, t = 256 rank .. 256 rank + 255, whose columns (fours t, t + 512, ...) two threads share, the first ones and the ones behind
+// them. The second goes on with the first one's sum of squares, so that every thread's, every warp's and the
+// row's sum are added in the order of the kernel above. The blocks swap their warps' sums through distributed shared memory.
+constexpr int CLUSTER_SHARE = 256;
+template <typename T>
+__global__ void __launch_bounds__(2 * CLUSTER_SHARE) splitk_rms_norm_cluster_kernel(T* __restrict__ normed, T* __restrict__ value,
+                                                                                    const float* __restrict__ partial, int splits,
+                                                                                    const float* __restrict__ bias, const T* __restrict__ residual,
+                                                                                    const float* __restrict__ weight, int rows, int width,
+                                                                                    float eps) {
+  constexpr int STEP = 2 * CLUSTER_SHARE;       // fours between a thread's columns: the threads of the kernel above
+  // The norm's weight and the bias are the model's, as above.
+  dependent_launch_trigger();
+  // Another block's shared memory may be used once that block has started: the arrival here, whose wait stands before the swap.
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  const int quads = width / 4, trips = (quads + STEP - 1) / STEP, early = (trips + 1) / 2;
+  const int row = blockIdx.x >> 1, rank = blockIdx.x & 1;
+  const int share = threadIdx.x % CLUSTER_SHARE;
+  const bool second = threadIdx.x >= CLUSTER_SHARE;
+  const int c_begin = rank * CLUSTER_SHARE + share + (second ? early * STEP : 0);                 // this thread's columns, in fours
+  const int c_end = second ? quads : min(quads, early * STEP);
+  float w_first[4] = {0.f, 0.f, 0.f, 0.f}, b_first[4] = {0.f, 0.f, 0.f, 0.f};
+  if (c_begin < c_end) {
+    load4(weight + 4 * c_begin, w_first);
+    if (bias != nullptr) load4(bias + 4 * c_begin, b_first);
+  }
+  dependent_launch_wait();
+  extern __shared__ __align__(16) float row_values[];      // of a thread's columns behind its first four: [trip][thread][4]
+  __shared__ float chain[CLUSTER_SHARE];
+  __shared__ float warp_sums[STEP / 32];                   // of the whole row
+  const size_t plane4 = (size_t)rows * quads;
+  const float4* part4 = (const float4*)partial;
+  float first[4] = {0.f, 0.f, 0.f, 0.f};
+  float squares = 0.f;
+  for (int c = c_begin; c < c_end; c += STEP) {
+    const size_t at4 = (size_t)row * quads + c;
+    float res[4] = {0.f, 0.f, 0.f, 0.f};
+    if (residual != nullptr) load4(residual + (size_t)row * width + 4 * c, res);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    int s = 0;
+    for (; s + 12 <= splits; s += 12) {
+      float4 p[12];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) normed[(size_t)row * width + i + j] = from_float<T>(row_values[i - 4 * begin + j] * scale * weight[i + j]);
+      for (int j = 0; j < 12; ++j) p[j] = part4[(size_t)(s + j) * plane4 + at4];
+#pragma unroll
+      for (int j = 0; j < 12; ++j) {
+        v.x += p[j].x; v.y += p[j].y; v.z += p[j].z; v.w += p[j].w;
+      }
+    }
+    for (; s + 4 <= splits; s += 4) {
+      float4 p[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) p[j] = part4[(size_t)(s + j) * plane4 + at4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v.x += p[j].x; v.y += p[j].y; v.z += p[j].z; v.w += p[j].w;
+      }
+    }
+    for (; s < splits; ++s) {
+      const float4 p = part4[(size_t)s * plane4 + at4];
+      v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+    }
+    float e[4] = {v.x, v.y, v.z, v.w};
+    const bool is_first = c == c_begin;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (bias != nullptr) e[j] += is_first ? b_first[j] : bias[4 * c + j];
+      if (residual != nullptr) e[j] += res[j];
+      e[j] = to_float(from_float<T>(e[j]));
+      squares += e[j] * e[j];                  // of the second thread: made again below, behind the first one's
+    }
+    store4(value + (size_t)row * width + 4 * c, e);
+    if (is_first) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) first[j] = e[j];
+    } else {
+      store4(row_values + 4 * (c / STEP * STEP + threadIdx.x), e);
+    }
+  }
+  if (!second) chain[share] = squares;
+  __syncthreads();
+  if (second) {
+    squares = chain[share];
+    for (int c = c_begin; c < c_end; c += STEP) {
+      float e[4];
+      if (c != c_begin) load4(row_values + 4 * (c / STEP * STEP + threadIdx.x), e);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (c == c_begin) e[j] = first[j];
+        squares += e[j] * e[j];
+      }
+    }
+    squares = warp_sum(squares);
+  }
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");      // both blocks have started, long ago as a rule
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (second && lane < 2) {                    // lane b leaves the warp's sum in block b of the cluster
+    const uint32_t own = (uint32_t)__cvta_generic_to_shared(&warp_sums[(rank - 1) * (CLUSTER_SHARE / 32) + warp]);
+    uint32_t there;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(own), "r"((uint32_t)lane));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(there), "f"(squares) : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  float total = 0.f;                            // every thread adds the warps' sums in the warps' order
+#pragma unroll
+  for (int w = 0; w < STEP / 32; ++w) total += warp_sums[w];
+  const float scale = rsqrtf(total / (float)width + eps);
+  for (int c = c_begin; c < c_end; c += STEP) {
+    float e[4], w[4], o[4];
+    if (c != c_begin) {
+      load4(row_values + 4 * (c / STEP * STEP + threadIdx.x), e);
+      load4(weight + 4 * c, w);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = c == c_begin ? first[j] * scale * w_first[j] : e[j] * scale * w[j];
+    store4(normed + (size_t)row * width + 4 * c, o);
   }
 }
 
@@ -407,6 +507,15 @@ __global__ void splitk_clamped_glu_kernel(TO* __restrict__ out, const float* __r
   out[i] = from_float<TO>(g / (1.f + expf(-alpha * g)) * (u + 1.f));
 }
 
+int sm_count() {
+  static const int count = [] {
+    int device = 0, n = 148;
+    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+    return n;
+  }();
+  return count;
+}
+
 }  // namespace
 
 // value float32 [rows, width]; normed in out_dtype; partial float32 [splits, rows, width]; bias, residual (float32) may be null.
@@ -468,22 +577,22 @@ PAE_EXPORT int pae_splitk_rms_norm(void* normed, void* value, const float* parti
   const int threads = width >= 2048 ? 512 : (width >= 512 ? 384 : (width >= 256 ? 128 : 64));
   const bool by_four = width % 4 == 0 && (((uintptr_t)partial | (uintptr_t)normed | (uintptr_t)value | (uintptr_t)residual |
                                             (uintptr_t)weight | (uintptr_t)bias) & 15) == 0;
-  // A cluster of two shares rows that one block of 512 threads would take in two trips to the L2 (3,584 columns: eight decode steps of
-  // 64 requests at the 7B sizes 11.59 -> 11.41 ms); at 1,536 columns the cluster costs more than it saves (16 steps of 40 requests 9.75
-  // against 9.90 ms).
-  if (by_four && dtype == kBF16 && width > 2048) {
-    const int share = (width / 4 + 1) / 2, block = share >= 512 ? 512 : (share + 31) / 32 * 32;
-    auto kernel = splitk_rms_norm_x4_kernel<__nv_bfloat16, 2>;
-    if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    launch_kernel_cluster(kernel, dim3(2 * rows), dim3(block), bytes, s, 2u, (__nv_bfloat16*)normed, (__nv_bfloat16*)value, partial, splits, bias,
-                          (const __nv_bfloat16*)residual, weight, rows, width, eps);
+  // Clusters of two take rows that one block of 512 threads would take in two trips to the L2 and more, as long as all their blocks run at
+  // once (two on an SM). 3,584 columns, five splits: 25, 64, 128 rows 4.5, 4.6, 4.9 -> 3.3, 3.8, 4.0 us; but 200 and 512 rows 5.2 and 9.5 by
+  // single blocks, 6.3 and 11.7 by clusters. At 1,536 columns a cluster costs more than it saves (16 steps of 40 requests 9.75 against 9.90 ms).
+  if (by_four && dtype == kBF16 && width > 2048 && rows <= sm_count()) {
+    const size_t kept = (size_t)((width / 4 + 511) / 512) * 512 * 4 * sizeof(float);
+    auto kernel = splitk_rms_norm_cluster_kernel<__nv_bfloat16>;
+    if (kept > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 168 * 1024);
+    launch_kernel_cluster(kernel, dim3(2 * rows), dim3(2 * CLUSTER_SHARE), kept, s, 2u, (__nv_bfloat16*)normed, (__nv_bfloat16*)value, partial,
+                          splits, bias, (const __nv_bfloat16*)residual, weight, rows, width, eps);
   } else if (dtype == kBF16) {
-    auto kernel = by_four ? splitk_rms_norm_x4_kernel<__nv_bfloat16, 1> : splitk_rms_norm_kernel<__nv_bfloat16>;
+    auto kernel = by_four ? splitk_rms_norm_x4_kernel<__nv_bfloat16> : splitk_rms_norm_kernel<__nv_bfloat16>;
     if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
     launch_kernel(kernel, rows, threads, bytes, s, (__nv_bfloat16*)normed, (__nv_bfloat16*)value, partial, splits, bias,
                                         (const __nv_bfloat16*)residual, weight, rows, width, eps);
   } else if (dtype == kF32) {
-    auto kernel = by_four ? splitk_rms_norm_x4_kernel<float, 1> : splitk_rms_norm_kernel<float>;
+    auto kernel = by_four ? splitk_rms_norm_x4_kernel<float> : splitk_rms_norm_kernel<float>;
     if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
     launch_kernel(kernel, rows, threads, bytes, s, (float*)normed, (float*)value, partial, splits, bias, (const float*)residual, weight,
                                         rows, width, eps);

@@ -31,7 +31,7 @@ def _kernels():
 
 def test_the_kernels_are_found():
     names = {name for _, name, _ in _kernels()}
-    assert {"splitk_rms_norm_x4_kernel", "gemm_tcgen05_pair_kernel", "prefill_tcgen05_kernel"} <= names
+    assert {"splitk_rms_norm_cluster_kernel", "gemm_tcgen05_pair_kernel", "prefill_tcgen05_kernel"} <= names
 
 
 @pytest.mark.parametrize("kernel", [n for _, n, body in _kernels() if REMOTE.search(body)])

@@ -31,3 +31,21 @@ def test_sum_and_norm(width, splits, extras):
     assert bool(((normed.double() - want).abs() <= want.abs() * (2.0**-8 + 2.0**-18)).all())
     few = ops.PendingSum(partial[:, 2:4].contiguous(), bias, residual[2:4].contiguous() if extras else None, torch.bfloat16)
     assert torch.equal(ops.rms_norm(few, weight, 1e-6), normed[2:4])
+
+
+@pytest.mark.parametrize("width", [2052, 3584, 4100, 5120, 8196])
+@pytest.mark.parametrize("splits", [2, 13])
+def test_a_row_has_the_same_bits_in_launches_of_every_size(width, splits):
+    """Few rows are shared by clusters of two blocks, many are not."""
+    from paged_attention_engine_b200.kernels import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    partial = torch.randn(splits, 400, width, device="cuda", generator=gen)
+    bias = torch.randn(width, device="cuda", generator=gen)
+    residual = torch.randn(400, width, device="cuda", generator=gen).to(torch.bfloat16)
+    weight = torch.rand(width, device="cuda", generator=gen) + 0.5
+    whole = ops.PendingSum(partial, bias, residual, torch.bfloat16)
+    normed = ops.rms_norm(whole, weight, 1e-6)
+    for rows in (1, 64, 148, 149, 300):
+        some = ops.PendingSum(partial[:, -rows:].clone(), bias, residual[-rows:].clone(), torch.bfloat16)      # on 16-byte boundaries
+        assert torch.equal(ops.rms_norm(some, weight, 1e-6), normed[-rows:]) and torch.equal(some.value, whole.value[-rows:])
