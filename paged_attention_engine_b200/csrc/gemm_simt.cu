@@ -503,13 +503,13 @@ __global__ void __launch_bounds__(256) f32_planes_kernel(float* __restrict__ out
                                                          const float* __restrict__ bias, const float* __restrict__ residual,
                                                          int segments, int M, int N, int ld_out) {
   dependent_launch_prologue();
-  const unsigned count = (unsigned)M * (unsigned)N, i = blockIdx.x * 256u + threadIdx.x;      // at most half the SMs' tiles
+  const long long count = (long long)M * N, i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= count) return;
-  const unsigned m = i / (unsigned)N, n = i % (unsigned)N;
-  const size_t at = (size_t)m * ld_out + n;
   double v = 0.0;
 #pragma unroll 8
   for (int s = 0; s < segments; ++s) v += planes[(size_t)s * count + i];
+  const int m = (int)i / N, n = (int)i - m * N;            // a slice has at most half the SMs' tiles
+  const size_t at = (size_t)m * ld_out + n;
   if (bias != nullptr) v += (double)bias[n];
   if (residual != nullptr) v += (double)residual[at];
   out[at] = (float)v;
@@ -528,9 +528,9 @@ int sm_count() {
 
 constexpr int F32_FEW_TOKENS = 32;
 // The planes of a launch hold a double per output and segment, which is as much as the weights are at 64 tokens: they are bounded by cutting
-// the output into slices of whole tiles, one after the other through the same scratch. 64 MB hold 13 tiles of the
+// the output into slices of whole tiles, one after the other through the same scratch. 96 MB hold 19 tiles of the
 // longest K in use (18,944).
-constexpr long long F32_SCRATCH_BYTES = 64LL << 20;
+constexpr long long F32_SCRATCH_BYTES = 96LL << 20;
 
 namespace {
 
@@ -555,7 +555,7 @@ Slices f32_slices(int M, int N, int K) {
 
 }  // namespace
 
-// How many doubles `pae_linear_f32` needs as scratch (0: none), at most 64 MB of them.
+// How many doubles `pae_linear_f32` needs as scratch (0: none), at most 96 MB of them.
 PAE_EXPORT long long pae_linear_f32_scratch(int M, int N, int K) {
   const Slices slice = f32_slices(M, N, K);
   return (long long)((K + SEGMENT - 1) / SEGMENT) * slice.m * slice.n;

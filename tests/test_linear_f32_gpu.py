@@ -70,7 +70,7 @@ def test_misaligned_operands_are_taken():
     assert torch.allclose(ops.linear(shifted, w).double(), want, rtol=1e-6, atol=1e-6)
 
 
-@pytest.mark.parametrize("m,n,k", [(64, 3584, 18944), (300, 100, 65536), (33, 70, 262144)])
+@pytest.mark.parametrize("m,n,k", [(64, 3584, 18944), (300, 100, 65536), (33, 70, 393216)])
 def test_outputs_cut_into_slices_that_share_the_scratch(m, n, k):
     """Sizes whose planes of double do not fit the scratch at once: slices of weight rows, and of tokens too."""
     from paged_attention_engine_b200.kernels import ops
@@ -79,7 +79,7 @@ def test_outputs_cut_into_slices_that_share_the_scratch(m, n, k):
     torch.cuda.reset_peak_memory_stats()
     before = torch.cuda.memory_allocated()
     got = ops.linear(x, w, bias, residual)
-    assert torch.cuda.max_memory_allocated() - before <= (64 << 20) + 4 * m * n + 4096
+    assert torch.cuda.max_memory_allocated() - before <= (96 << 20) + 4 * m * n + 4096
     want = x.double() @ w.double().T + bias.double() + residual.double()
     terms = x.double().abs() @ w.double().abs().T + bias.abs().double() + residual.abs().double()
     assert bool(((got.double() - want).abs() <= want.abs() * 2**-24 + terms * (k + 2) * 2**-52).all())
