@@ -62,6 +62,7 @@ struct Params {
   int table_width, heads, kv_heads, page_size, window, skip_single;
   const int* work_index;  // the requests that this launch works on, one per grid z (null: request z)
   float scale_log2;
+  float slack;            // paired form: a row's reference follows its maximum in steps of more than 2^slack
   int* error;
 };
 
@@ -626,11 +627,14 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
 // working a third of the time, tensor cores half): 8,192 tokens, 12 heads of 128: 277 -> 258 us (800 TFLOP/s), 28 heads:
 // 596 -> 547 us (880); with the probabilities still in shared memory 266 and 568, without the instructions on pairs 268 and 570.
 //
-// The reference of a row is its running maximum, but it only moves when the maximum has grown
+// The reference of a row is its running maximum, but in launches that fill the GPU it only moves when the maximum has grown
 // by more than 2^8 since it was set: probabilities then stay below 256, which float32 sums and
 // the bfloat16 operand hold as well as values below 1, and the output in tensor memory (which
 // must be multiplied by 2^(old - new) whenever the reference moves) is touched on a row's first
-// tiles only. The sum is kept against the same reference, so the quotient is exact softmax.
+// tiles only. The sum is kept against the same reference, so the quotient is exact softmax. A largest probability that is not
+// 1 is rounded, though: 0.2 to 1.5 % further from 64 bits than the wide form (509 tokens after 512: 0.00229 and 0.00232 of the
+// outputs' norm). Smaller launches, which would otherwise take the wide form, move it with every new maximum: a little closer
+// than the wide form (0.00228) for 0.6 us at 100 tokens (7.9 -> 8.5), 1.5 at 6 requests of 300 (14.1 -> 15.6).
 // ---------------------------------------------------------------------------------------
 namespace paired {
 
@@ -638,7 +642,7 @@ constexpr int BKEYS = 64;           // keys per tile
 constexpr int THREADS = 192;        // TMA warp, MMA warp, four softmax warps (one thread per query row)
 constexpr int SOFTMAX_WARPS = 4;
 constexpr int KV_STAGES = 2;
-constexpr float REFERENCE_SLACK = 8.f;   // a row's reference follows its maximum in steps of more than 2^8
+constexpr float REFERENCE_SLACK = 8.f;   // of launches that fill the GPU; 0 below that (`launch`)
 
 // 64 consecutive float32 columns of this thread's lane of tensor memory.
 __device__ __forceinline__ void tmem_load64(uint32_t address, float* v) {
@@ -944,7 +948,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
       }
       float tile_max = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
       if (tile_max != -FLT_MAX) tile_max *= p.scale_log2;        // the scale is positive: max(s) scales with it
-      const bool moves = tile_max > reference + REFERENCE_SLACK || (reference == -FLT_MAX && tile_max != -FLT_MAX);
+      const bool moves = tile_max > reference + p.slack || (reference == -FLT_MAX && tile_max != -FLT_MAX);
       if (__any_sync(0xffffffffu, moves)) {
         // Some row of this warp moves its reference: its sum and its row of O are multiplied
         // by 2^(old - new); the other rows by 1. Reading and writing tensor memory takes the whole warp.
@@ -1084,19 +1088,19 @@ int sm_count() {
 
 // Whether form 0 takes the paired kernel. Two of its blocks share an SM, so up to two blocks per SM run at once; of the wide
 // kernel one. Times in us from launches of 12 and 28 heads, 1 to 12 requests of 64 to 2,000 tokens over up to 4,000 keys:
-// a wide block 5.5 + 1.95 per tile of 128 keys; a wide block that follows another 4 more; a round of paired blocks 5 + 2.84
+// a wide block 5.5 + 1.95 per tile of 128 keys; a wide block that follows another 4 more; a round of paired blocks 6.5 + 3.0
 // per tile. With more blocks than SMs and fewer than twice as many, the wide launch's second blocks follow its shortest
 // first ones, so it lasts as long as its longest block or two of middling length: the two estimates are compared (6 requests
-// of 300 tokens, 12 heads: wide 21.5, paired 13.9; 4 portions of 509 tokens after 512: 37.9 and 29.1; but one prompt of 2,000
-// tokens: 36.5 and 46.9). From twice as many on it is the paired kernel (8,192 tokens 346 and 258). With at most half of
-// the SMs busy and three tiles or fewer the paired kernel's shorter set-up shows (64 tokens 8.1 and 5.8, 300 tokens 11.1 and
-// 10.5; at 500 tokens 14.0 and 14.9).
+// of 300 tokens, 12 heads: wide 22.0, paired 15.6; 4 portions of 509 tokens after 512: 38.2 and 32.5; but one prompt of 2,000
+// tokens: 36.5 and more than 46.9). From twice as many on it is the paired kernel (8,192 tokens 346 and 258). With one of its
+// tiles, and up to three while at most a third of the SMs are busy, the paired kernel's shorter set-up shows (64 tokens 8.3 and 6.3, 100 tokens
+// 8.9 and 8.5, 192 tokens 10.3 and 9.1; but 200 tokens of 28 heads 10.2 and 10.9, 300 of 12 11.3 and 11.7).
 bool takes_paired(long long blocks, long long blocks_per_tile, int longest, int longest_keys) {
   const int sms = sm_count();
   if (blocks >= 2LL * sms) return true;
-  if (blocks <= sms) return longest <= 3 && (blocks * 2 <= sms || longest_keys <= 64);
+  if (blocks <= sms) return longest_keys <= 64 || (longest_keys <= 192 && blocks * 3 <= sms);
   const float middle = fmaxf(0.f, longest - (float)sms / blocks_per_tile);
-  const float wide = fmaxf(5.5f + 1.95f * longest, 15.f + 3.9f * middle), paired = 5.f + 2.84f * longest;
+  const float wide = fmaxf(5.5f + 1.95f * longest, 18.f + 3.9f * middle), paired = 6.5f + 3.f * longest;
   return paired < wide;
 }
 
@@ -1108,7 +1112,7 @@ bool takes_paired(long long blocks, long long blocks_per_tile, int longest, int 
 // cost more than the shorter chains save: 128 tokens after 8,192 take 123 us in 12 blocks.
 // 1: wide, no clusters; 2: paired; 4, 8, 16: wide in clusters of 2, 4, 8.
 template <int D>
-int launch(const Params& p, const void* qkv, const void* keys, const void* values, int tokens, long long pages, int seqs,
+int launch(Params p, const void* qkv, const void* keys, const void* values, int tokens, long long pages, int seqs,
            int working_seqs, int max_q_len, int max_kv_len, int form, int* chosen, cudaStream_t stream) {
   // With a list of the requests to work on, the grid covers those only. Without one it covers
   // all, and the blocks of requests that are left to the decode kernel return at once; they do
@@ -1119,6 +1123,7 @@ int launch(const Params& p, const void* qkv, const void* keys, const void* value
   const int seen = p.window > 0 && p.window + BQ < max_kv_len ? p.window + BQ : max_kv_len;
   const int longest = (seen + BKEYS - 1) / BKEYS;          // key tiles of the longest block
   const bool use_paired = form == 2 || (form == 0 && takes_paired(blocks, (long long)p.heads * working_seqs, longest, seen));
+  p.slack = blocks >= 2LL * sm_count() ? paired::REFERENCE_SLACK : 0.f;
   unsigned ranks = 1;
   if (form == 4 || form == 8 || form == 16) ranks = form / 2;
   if (form == 0 && !use_paired) {

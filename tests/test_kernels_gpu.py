@@ -430,3 +430,31 @@ def test_paired_prefill_attention_gives_the_same_bits_every_time(ops, d, page):
     ops.check_device_errors()
     wide = ops.paged_attention(*args, num_single=0, form=1)
     _close(first, wide, torch.bfloat16)
+
+
+@pytest.mark.parametrize("d,n,start,requests", [(128, 192, 0, 1), (128, 300, 0, 6), (128, 509, 512, 4), (64, 150, 0, 1), (64, 500, 0, 4)])
+def test_prefill_attention_of_few_blocks_is_no_further_from_64_bits_than_the_wide_form(ops, d, n, start, requests):
+    heads, kv_heads, page = 12, 2, 16
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    pages = -(-(start + n) // page)
+    qkv = (torch.randn(requests * n, (heads + 2 * kv_heads) * d, device="cuda", generator=gen) * 0.8).to(torch.bfloat16)
+    keys, values = ((torch.randn(requests * pages, kv_heads, page, d, device="cuda", generator=gen) * 0.8).to(torch.bfloat16) for _ in range(2))
+    table = torch.arange(requests * pages, device="cuda", dtype=torch.int32).view(requests, pages)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")  # noqa: E731
+    args = (qkv, keys, values, table, i32([n * r for r in range(requests + 1)]), i32([start] * requests), i32([start + n] * requests), heads, kv_heads, d, page,
+            n, start + n, d**-0.5, 0)
+    hidden = torch.arange(start + n, device="cuda")[None] > start + torch.arange(n, device="cuda")[:, None]
+    want = []
+    for r in range(requests):
+        q = qkv[r * n : (r + 1) * n].double().view(n, heads + 2 * kv_heads, d)[:, :heads]
+        k, v = (t[r * pages : (r + 1) * pages].double().transpose(1, 2).reshape(-1, kv_heads, d)[: start + n].repeat_interleave(heads // kv_heads, 1)
+                for t in (keys, values))
+        scores = (torch.einsum("qhd,khd->hqk", q, k) * d**-0.5).masked_fill(hidden, float("-inf"))
+        want.append(torch.einsum("hqk,khd->qhd", scores.softmax(-1), v).reshape(n, -1))
+    want = torch.cat(want)
+    info = {}
+    chosen = (ops.paged_attention(*args, num_single=0, info=info).double() - want).norm()
+    wide = (ops.paged_attention(*args, num_single=0, form=1).double() - want).norm()
+    # Both round the probabilities and the result to bfloat16. A rounding of every row's largest probability, too, shows as 0.2 % and more.
+    assert info["cluster"] == 0 and float(chosen) <= 1.001 * float(wide)
+    ops.check_device_errors()
