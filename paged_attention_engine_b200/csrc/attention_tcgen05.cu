@@ -623,8 +623,8 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
 // operand there: no trip through shared memory (sixteen-byte stores into the swizzled layout, a proxy fence, and 16 KB that
 // the tensor core reads back), and the softmax never waits for a product unless a reference moves. The thread that issues the MMAs
 // waits for the product of the tile before last before the next scores are written over the probabilities it reads. Scale
-// and sum take two scores an instruction. The kernel is bound by the chain of a tile's steps (a special-function unit
-// working a third of the time, tensor cores half): 8,192 tokens, 12 heads of 128: 277 -> 258 us (800 TFLOP/s), 28 heads:
+// and sum take two scores an instruction. The kernel is bound by the chain of a tile's steps (the special-function
+// units work 38 % of the time, the tensor cores 50 %, issue slots are 32 % busy): 8,192 tokens, 12 heads of 128: 277 -> 258 us (800 TFLOP/s), 28 heads:
 // 596 -> 547 us (880); with the probabilities still in shared memory 266 and 568, without the instructions on pairs 268 and 570.
 //
 // The reference of a row is its running maximum, but in launches that fill the GPU it only moves when the maximum has grown

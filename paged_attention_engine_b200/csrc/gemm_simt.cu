@@ -1,16 +1,15 @@
-// Matrix products on the CUDA cores: out[M, N] = x[M, K] . w[N, K]^T (+ bias[N]) (+ residual[M, N]).
+// Matrix products out[M, N] = x[M, K] . w[N, K]^T (+ bias[N]) (+ residual[M, N]) of the true 32-bit path, and of whatever the bfloat16
+// path's tensor-core kernels refuse. No TF32 and no bfloat16 staging anywhere.
 //
-// This is the product kernel of the true 32-bit path (FFMA with float32 accumulation:
-// no tensor cores, no TF32, no bfloat16 staging) and the kernel that takes every size
-// and every mix of element types in the bfloat16 path: any M, N, K, no alignment
-// needed, bfloat16 or float32 activations, weights and outputs. The bfloat16 path's
-// tensor-core kernels serve the shapes they are built for; whatever they refuse runs here.
+// The general kernel (CUDA cores) takes every size and every mix of element types: any M, N, K, no alignment
+// needed, bfloat16 or float32 activations, weights and outputs. Float32 products have kernels of their own (second
+// half of this file), from three tokens on with the tensor cores' double-precision instruction.
 //
 // Weights are [out, in] row-major as the checkpoint stores them, which is what
 // x . w^T reads (engine/model.py:303-320 of the reference calls F.linear on the same
 // layout). Every output element sums its K products in the same order whatever M is, so
 // a token's result does not depend on what else is in the batch. When activations, weights
-// and output are all float32 (kernels of their own below, unless K is not a multiple of 4 or an
+// and output are all float32 (in the general kernel if K is not a multiple of 4 or an
 // operand is not 16-byte aligned) the K products are summed in double and rounded once: a
 // sequential float32 sum over a long K loses several bits against what a float32 result
 // can hold, and a model whose layers cancel (a recurrent state read out by a near-orthogonal
@@ -132,7 +131,8 @@ int launch(void* out, const void* x, const void* w, const float* bias, const voi
 //
 // Measured, us, [17,920, 1,536] and [1,536, 8,960] weights: 1 token 22.9 and 15.8 (16.8 and 8.4 at the copy bandwidth;
 // 24.0 and 26.0 with 32 rows a block, the eight-token kernel 36 and 40), 8 tokens 37 and 43 (63 and 78 with plain multiply-adds, whose operands meet the shared memory's
-// bandwidth), 60 tokens 168 and 75 (313 and 171), 256 tokens 450 and 574 (1,232 and 1,496): 31 of 37 TFLOP/s.
+// bandwidth), 60 tokens 153 and 75 (313 and 171), 256 tokens 454 and 475 (1,232 and 1,496): 31 and 15 of 37 TFLOP/s. (The second has 96
+// tiles, more than half of the SMs, so that K is not shared out.)
 // ---------------------------------------------------------------------------------------
 constexpr int SEGMENT = 128;
 constexpr int CHUNK = 32;                   // k of a stage

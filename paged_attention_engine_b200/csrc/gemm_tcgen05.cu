@@ -1,7 +1,8 @@
 // Matrix products of the bfloat16 path on the fifth-generation tensor cores (sm_100a):
 // operands staged in shared memory by TMA (cp.async.bulk.tensor, 128-byte swizzle),
 // tcgen05.mma issued by one thread with the accumulator in tensor memory, tcgen05.ld for
-// the epilogue. No cluster multicast is used anywhere.
+// the epilogue. No load is multicast; the only multicast is the pair kernel's commit, which signals a barrier in both
+// blocks of its cluster.
 //
 // Both operands are K-major ([rows, K] row-major, K contiguous), which is how activations
 // [tokens, K] and checkpoint weights [out, K] lie in memory (the reference calls
@@ -17,12 +18,14 @@
 //            partial[split, token, n], and the kernel that follows sums them in a fixed
 //            order (with bias, residual, or whatever it fuses).
 //
-// One block computes one 128 x BN tile over its K range. Warp 0 issues the TMA loads,
-// warp 1 allocates tensor memory and issues the MMAs, warps 2-5 run the epilogue (each
+// One block computes one 128 x BN tile over its K range; in the persistent kernel one tile after the other, in the pair
+// kernel half of each 256 x PBN tile of its cluster. Warp 0 issues the TMA loads,
+// warp 1 allocates tensor memory and issues the MMAs (of a pair: the first block's, for both), the other warps (four, or eight in the
+// kernels of many tokens) run the epilogue (each
 // reads the 32 lanes of tensor memory that its warp id modulo 4 may touch). Every
 // mbarrier wait is bounded: when one gives up it records a code in `error`, the roles
-// leave their loops, loads in flight are waited for (bounded again), tensor memory is
-// freed and the block returns.
+// leave their loops, loads in flight are waited for (bounded again; of a pair by the first block, where both blocks' loads report, while the
+// second waits for it at the cluster's barrier), tensor memory is freed and the block returns.
 #include "tcgen05.cuh"
 
 using namespace pae;
@@ -1024,7 +1027,7 @@ int launch_pair_with(const Params& p, const void* a, const void* b, int k, cudaS
 }
 
 int launch_pair(const Params& p, int width, const void* a, const void* b, int k, cudaStream_t stream) {
-  if (p.rotary) {                 // a tile holds whole heads: widths that divide 256
+  if (p.rotary) {                 // a tile holds whole heads: the width is a multiple of the head size (`pair_width`)
     if (width == 192) return launch_pair_with<192, true>(p, a, b, k, stream);
     if (width == 160) return launch_pair_with<160, true>(p, a, b, k, stream);
     if (width == 224) return launch_pair_with<224, true>(p, a, b, k, stream);
@@ -1071,8 +1074,8 @@ int persistent_width(const Params& p) {
 // from L2), plus 1 us of a cluster's set-up. Measured, us, single / pair, 1536- and 3584-wide layers: gate|up of 512, 2,048,
 // 8,192 tokens 29.9 / 27.3, 85.6 / 78.2, 316 / 294 and 104 / 93, 367 / 337, 1,481 / 1,369 (1.62 PFLOP/s); down of 8,192
 // 202 / 169 and 935 / 758; but down of 2,048 at K = 8,960 (one round either way, 144 blocks of 176 columns against 64
-// pairs of 192) 50.4 / 52.4, o there 16.8 / 18.0 and q|k|v 23.9 / 24.4. Grouped products, planes of K and
-// gates other than SiLU stay with single blocks.
+// pairs of 192) 50.4 / 52.4, o there 16.8 / 18.0 and q|k|v 23.9 / 24.4. Grouped products and planes of K
+// stay with single blocks, and so do gates other than SiLU, for which no pair kernel is compiled and none was measured.
 int pair_width(const Params& p) {
   if (p.group_tiles != nullptr || p.planes > 1 || (p.swiglu && p.gate_kind != kGateSilu)) return 0;
   auto units = [&](int rows, int w, int at_once) {
