@@ -786,8 +786,8 @@ def paged_attention(qkv, keys, values, block_table, q_start, q_pos0, kv_len, num
     requests that bring more than one token when some do and some do not: the portion kernels
     then launch blocks for those only (a step of 64 decoding requests and one prompt portion
     otherwise launches 65 requests' worth of blocks, 64 of which return at once but not for free). `form` 0 lets the tcgen05 attention pick
-    its kernel by the size of the launch (two blocks of 64-key tiles per SM when there are that
-    many blocks, else one block of 128-key tiles, its keys shared out over a cluster when the
+    its kernel by the size of the launch (64-key tiles, two blocks per SM, when there are that
+    many blocks or an estimate has it the quicker one; else one block of 128-key tiles, its keys shared out over a cluster when the
     blocks are few); 1, 2, 4, 8, 16 name the kernel (tests). `info`, when given, receives which
     kernel ran ("kernel") and, for tcgen05, the blocks per query tile ("cluster": 0 is the
     paired kernel)."""
