@@ -410,10 +410,12 @@ def test_windowed_attention_over_a_table_with_released_pages(ops, heads, kv_head
 
 
 @pytest.mark.parametrize("d,page", [(128, 16), (64, 64)])
-def test_paired_prefill_attention_gives_the_same_bits_every_time(ops, d, page):
+@pytest.mark.parametrize("heads,kv_heads", [(14, 2), (28, 4)])
+def test_paired_prefill_attention_gives_the_same_bits_every_time(ops, d, page, heads, kv_heads):
     """The roles of the paired kernel run ahead of one another by up to a tile: many blocks, many key tiles, and large
-    scores that keep moving the rows' references; no wait gives up and no run differs from another."""
-    heads, kv_heads, n, start = 14, 2, 1500, 3000
+    scores that keep moving the rows' references (with every maximum in the 168 blocks of 14 heads, in steps of 2^8 in the 336 of
+    28); no wait gives up and no run differs from another."""
+    n, start = 1500, 3000
     gen = torch.Generator(device="cuda").manual_seed(5)
     pages = -(-(start + n) // page)
     qkv = (torch.randn(n, (heads + 2 * kv_heads) * d, device="cuda", generator=gen) * 4).to(torch.bfloat16)
