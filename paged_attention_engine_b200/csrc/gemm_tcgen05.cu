@@ -37,8 +37,6 @@ constexpr int BM = 128;          // MMA rows per tile
 constexpr int THREADS = 192;
 constexpr int EPILOGUE_SHARES = 2;           // epilogue warps per quarter of the rows (three were measured slower, one much slower)
 constexpr int PERSISTENT_THREADS = 64 + 128 * EPILOGUE_SHARES;     // TMA warp, MMA warp, the epilogue warps
-constexpr uint32_t WAIT_LIMIT = 1u << 21;
-
 enum Mode : int { NORMAL = 0, SWAPPED = 1 };
 
 struct Params {
@@ -72,21 +70,6 @@ struct Params {
   int* error;
   int skip_kb;       // self-test of the give-up path only: the k-block (of each block's range) that is never loaded
 };
-
-// Waits for a phase of an mbarrier, at most WAIT_LIMIT polls. On giving up it raises the
-// block's abort flag and records `code`; it also returns false as soon as another role
-// has raised the flag.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* error, int code,
-                                          uint32_t limit = WAIT_LIMIT) {
-  for (uint32_t i = 0; i < limit; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (i > 64) __nanosleep(64);
-  }
-  *abort_flag = 1;
-  atomicCAS(error, 0, code);
-  return false;
-}
 
 // The activations a product can apply to its own output. The argument is rounded to the output's
 // element type first, as a stand-alone activation kernel would read it, so both ways give the same bits.
@@ -791,17 +774,8 @@ struct PairTile {
   static_assert(B_BYTES % 1024 == 0, "stages start on 1024 bytes");
 };
 
-__device__ __forceinline__ uint32_t in_block(uint32_t address, uint32_t rank) {
-  uint32_t remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(address), "r"(rank));
-  return remote;
-}
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // A load into this block's shared memory that reports to a barrier of either block of the pair.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {

@@ -206,6 +206,47 @@ class PendingNorm:
         return self.x.device
 
 
+class PendingProduct:
+    """x . weight^T + residual of a step of some tens of tokens that has not run: `linear` returns one, and the
+    `rms_norm` that reads the sum next has the product's own epilogue prepare the norm (`ScaledNorm`), which saves the
+    norm's launch; anything else calls `materialized`, which runs the product alone and keeps its result in `value`."""
+
+    def __init__(self, operand, weight, residual) -> None:
+        self.operand, self.weight, self.residual = operand, weight, residual
+        self.dtype = torch.bfloat16
+        self.value = None
+
+    @property
+    def shape(self):
+        return self.residual.shape
+
+    @property
+    def device(self):
+        return self.residual.device
+
+
+class ScaledNorm:
+    """RMSNorm(x) * weight as the product that made x left it: `scaled` = x * weight, and `squares` [parts, tokens], whose
+    sum over the parts is a row's sum of squares. The products that follow take `scaled` and apply rsqrt(mean + eps) to
+    their sums; anything else calls `materialized`, which runs the norm's kernel and keeps its result in `value`."""
+
+    def __init__(self, x, weight, eps: float, scaled, squares) -> None:
+        self.x, self.weight, self.eps, self.scaled, self.squares = x, weight, float(eps), scaled, squares
+        self.value = None
+
+    @property
+    def shape(self):
+        return self.x.shape
+
+    @property
+    def dtype(self):
+        return self.x.dtype
+
+    @property
+    def device(self):
+        return self.x.device
+
+
 class PendingStreams:
     """Residual streams [tokens, streams * width] whose write x'_t = sum_s mix[s, t] x_s + out[t] y has
     not run: `streams_write` returns one, and the `streams_read_norm` of the next sublayer does
@@ -296,7 +337,11 @@ def materialized(x):
         if x.value is None:
             _dyt_step(x, None, None)
         return x.value
-    if isinstance(x, PendingNorm):
+    if isinstance(x, PendingProduct):
+        if x.value is None:
+            _cluster_product(x, None)
+        return x.value
+    if isinstance(x, (PendingNorm, ScaledNorm)):
         if x.value is None:
             x.value = _rms_norm_now(x.x, x.weight, x.eps)
         return x.value
@@ -370,6 +415,9 @@ def rms_norm(x, weight: torch.Tensor, eps: float) -> torch.Tensor:
                                             _DTYPE_CODE[x.dtype], _stream()))
         x.value = value
         return normed
+    if isinstance(x, PendingProduct) and x.value is None and weight.is_contiguous() and weight.data_ptr() % 16 == 0:
+        scaled, squares = _cluster_product(x, weight)
+        return ScaledNorm(x.value, weight, eps, scaled, squares)
     x = materialized(x)
     _need(x, "rms_norm: x")
     if x.dim() == 2 and _few_tokens(x, x.shape[-1], normed=True):
@@ -421,6 +469,70 @@ def _few_tokens(x: torch.Tensor, k: int, normed: bool = False, kind: int = GATE_
     most = (FEW_TOKENS_MAX_QKV if kind == QKV_KIND else FEW_TOKENS_MAX_GATE_UP if kind == GATE_UP_KIND
             else FEW_TOKENS_MAX_RESIDUAL if k < SWAPPED_LONG_K else FEW_TOKENS_MAX_RESIDUAL_LONG_K)
     return answer == 2 and x.shape[0] <= most
+
+
+# A step of some tens of tokens runs a product as one kernel too (csrc/gemm_cluster.cu: a cluster of blocks shares the K of
+# 128 weight rows and finishes its tokens itself), with the RMSNorm before it and what follows it inside.
+# False sends such products to the other kernels and their sums (tests compare the two).
+use_cluster_products = True
+# From how many tokens on, by the width of the rows that the norms read. Measured, us, the four products of a layer with
+# their norms in a row, other kernels / these. Width 896: 16 tokens 19.8 / 22.1, 24 24.1 / 23.0, 64 36.6 / 26.5, 128 42.6 / 32.5; 1,536:
+# 16 tokens 29.9 / 33.0, 20 34.3 / 32.7, 40 44.2 / 34.0, 64 46.1 / 36.0, 128 51.8 / 50.2. From 2,048 on the few-token
+# kernels' blocks no longer all run at once, and these are ahead from one token on: 2,048 1 token 44.7 / 37.6, 8 46.2 / 40.4,
+# 64 58.8 / 49.9; 3,584 83.9 / 79.7, 87.0 / 82.6 and 106.7 / 91.8; 5,120 109.4 / 93.5, 105.6 / 95.9 and 121.5 / 106.8.
+CLUSTER_MIN_TOKENS = 17
+CLUSTER_WIDE = 2048
+CLUSTER_MAX_TOKENS = 128
+
+
+def _cluster_takes(tokens: int, n: int, k: int, weight, width: int) -> bool:
+    """Whether the cluster kernels run a bfloat16 product of these sizes; `width`: of the rows that the norm before or behind it reads."""
+    return (use_cluster_products and use_tensor_cores and not few_token_products_everywhere
+            and (CLUSTER_MIN_TOKENS if width < CLUSTER_WIDE else 1) <= tokens <= CLUSTER_MAX_TOKENS
+            and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.shape[1] == k and n % 8 == 0 and k % 64 == 0
+            and weight.is_contiguous() and weight.data_ptr() % 16 == 0)
+
+
+def _uneven_gate(tokens: int, n: int, device) -> bool:
+    """gate|up of more than 64 tokens whose tiles are some more than the SMs: the SMs that get two draw twice the operands (width 2,048, 172
+    tiles, 128 tokens: the layer's products 75.0 us against 70.1 with the many-token kernel throughout)."""
+    tiles, sms = -(-n // 128), _sm_count(device)
+    return tokens > 64 and sms < tiles <= sms * 8 // 5
+
+
+def _cluster_operand(x):
+    """(tensor, squares or None, width, eps) of a cluster product's operand, which may be a ScaledNorm; None when it is not one
+    that they take."""
+    if isinstance(x, ScaledNorm) and x.value is None:
+        return x.scaled, x.squares, x.shape[1], x.eps
+    x = materialized(x)
+    if x.dtype != torch.bfloat16 or x.dim() != 2 or not x.is_contiguous() or x.data_ptr() % 16:
+        return None
+    return x, None, 0, 0.0
+
+
+def _early_weights(tokens: int, k: int) -> int:
+    """Whether a product may read its weight before the kernel before it has completed (see `linear`)."""
+    return 1 if _swapped(tokens, k) else 0
+
+
+def _cluster_product(pending: PendingProduct, gamma):
+    """Runs a pending product; with `gamma`, the weight of the norm that reads the sum, returns (sum * gamma, squares)."""
+    source, squares_in, width, eps = pending.operand
+    weight = pending.weight
+    m, k = source.shape
+    n = weight.shape[0]
+    lib = _lib("gemm_cluster")
+    out = torch.empty((m, n), dtype=torch.bfloat16, device=source.device)
+    scaled = squares = None
+    if gamma is not None:
+        scaled = torch.empty_like(out)
+        squares = torch.empty((lib.pae_linear_cluster_parts(m, n, k), m), dtype=torch.float32, device=source.device)
+    _check(lib, lib.pae_linear_cluster(_ptr(out), _ptr(source), _ptr(weight), _ptr(pending.residual), _ptr(gamma), _ptr(scaled), _ptr(squares),
+                                       _ptr(squares_in), 0 if squares_in is None else squares_in.shape[0], width, eps, m, n, k,
+                                       _early_weights(m, k), 0, 0, 0, _ptr(_error_flag(source.device)), _stream()))
+    pending.value = out
+    return scaled, squares
 
 
 def _norm_of(x):
@@ -515,6 +627,7 @@ def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str 
     before the residual: in the tensor-core product's epilogue or in the sum of its splits, else
     by the activation's own kernel.
 
+    The product of some tens of tokens with a residual is not run before its value or the norm that reads it is asked for (`PendingProduct`).
     The bfloat16 kernels of few tokens (up to 64, or 128 where K is long) or of fewer than 256 columns read `weight` while the kernel
     before them in the stream may still be running, as they do in `linear_swiglu` and `qkv_projection`: a weight that the call just before
     wrote needs another launch, or a synchronisation, in between. Larger products read nothing before that kernel has completed."""
@@ -522,6 +635,15 @@ def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str 
         raise KernelError(f"linear: activation '{activation}' (known: gelu_erf, gelu_tanh, relu2)")
     if (activation is None and bias is None and out_dtype in (None, torch.bfloat16) and weight.dtype == torch.bfloat16 and weight.dim() == 2
             and weight.data_ptr() % 16 == 0 and weight.shape[0] <= 65536):
+        if residual is not None and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0]):
+            operand, residual = _cluster_operand(x), materialized(residual)
+            if operand is not None and residual.dtype == torch.bfloat16 and residual.data_ptr() % 16 == 0:
+                _need(operand[0], "linear: x")
+                _need(weight, "linear: weight")
+                _need(residual, "linear: residual", torch.bfloat16)
+                if tuple(residual.shape) != (x.shape[0], weight.shape[0]):
+                    raise KernelError(f"linear: residual is {tuple(residual.shape)}, the product is [{x.shape[0]}, {weight.shape[0]}]")
+                return PendingProduct(operand, weight, residual)
         source, norm_weight, eps = _norm_of(x)
         if (_few_tokens(source, weight.shape[1], norm_weight is not None, RESIDUAL_KIND, weight.shape[0]) and source.dim() == 2 and source.shape[1] == weight.shape[1]
                 and source.is_contiguous() and weight.is_contiguous()):
@@ -659,6 +781,26 @@ def rotary_qk_cache_write(qkv, table, slots, keys, values, num_heads, num_kv_hea
     return qkv
 
 
+def _aligned(*tensors) -> bool:
+    return all(t is None or t.data_ptr() % 16 == 0 for t in tensors)
+
+
+def _need_qkv(bias, table, slots, keys, values, m: int, n: int, head_dim: int) -> None:
+    """What a kernel that rotates and writes pages needs of its bfloat16 operands."""
+    if bias is not None:
+        _need(bias, "qkv_projection: bias", torch.float32)
+        if bias.numel() != n:
+            raise KernelError(f"qkv_projection: bias of {bias.numel()} for {n} columns")
+    if table is not None:
+        _need(table, "qkv_projection: table", torch.float32)
+        if tuple(table.shape) != (m, head_dim):
+            raise KernelError(f"qkv_projection: table is {tuple(table.shape)}, [{m}, {head_dim}] is needed")
+    if slots is not None:
+        _need(slots, "qkv_projection: slots", torch.int32)
+        _need(keys, "qkv_projection: keys", torch.bfloat16)
+        _need(values, "qkv_projection: values", torch.bfloat16)
+
+
 # Whether q|k|v of a prompt's portion is finished (bias, rotation, page write) by the product's own epilogue.
 fuse_qkv_epilogue = True
 
@@ -670,6 +812,25 @@ def qkv_projection(x, weight, bias, table, slots, keys, values, num_heads, num_k
     for few tokens fuse the other way round (the split sum runs inside the rotation kernel)."""
     m, k = x.shape
     n = weight.shape[0]
+    # A plain operand of more than 64 tokens keeps the bits of `linear` followed by the rotation (a prompt's first layer only: in
+    # the others the product before has prepared the norm).
+    if ((m <= SWAPPED_MAX_TOKENS or isinstance(x, ScaledNorm)) and _cluster_takes(m, n, k, weight, k) and n == (num_heads + 2 * num_kv_heads) * head_dim
+            and (slots is None or (keys.dtype == torch.bfloat16 and values.dtype == torch.bfloat16))):
+        operand = _cluster_operand(x)
+        lib = _lib("gemm_cluster")
+        if (operand is not None and lib.pae_qkv_cluster_supports(head_dim) and _aligned(bias, table)
+                and (slots is None or _aligned(keys, values))):
+            source, squares, width, eps = operand
+            _need(source, "qkv_projection: x")
+            _need(weight, "qkv_projection: weight")
+            _need_qkv(bias, table, slots, keys, values, m, n, head_dim)
+            out = torch.empty((m, n), dtype=torch.bfloat16, device=source.device)
+            _set_bounds("gemm_cluster", keys if slots is not None else None)
+            _check(lib, lib.pae_qkv_cluster(
+                _ptr(out), _ptr(source), _ptr(weight), _ptr(bias), _ptr(squares), 0 if squares is None else squares.shape[0], width, eps,
+                _ptr(table), _ptr(slots), _ptr(keys if slots is not None else None), _ptr(values if slots is not None else None), m,
+                num_heads, num_kv_heads, head_dim, page_size, k, _early_weights(m, k), 0, 0, 0, _ptr(_error_flag(source.device)), _stream()))
+            return out
     source, norm_weight, eps = _norm_of(x)
     if (_few_tokens(source, k, norm_weight is not None, QKV_KIND, n) and weight.dtype == torch.bfloat16 and weight.is_contiguous() and weight.data_ptr() % 16 == 0
             and n == (num_heads + 2 * num_kv_heads) * head_dim and weight.shape[1] == k and head_dim % 16 == 0
@@ -702,18 +863,7 @@ def qkv_projection(x, weight, bias, table, slots, keys, values, num_heads, num_k
         if lib.pae_linear_rotary_tcgen05_supports(head_dim) and lib.pae_linear_tcgen05_plane_count(m, n, k) == 1:
             _need(x, "qkv_projection: x")
             _need(weight, "qkv_projection: weight")
-            if bias is not None:
-                _need(bias, "qkv_projection: bias", torch.float32)
-                if bias.numel() != n:
-                    raise KernelError(f"qkv_projection: bias of {bias.numel()} for {n} columns")
-            if table is not None:
-                _need(table, "qkv_projection: table", torch.float32)
-                if tuple(table.shape) != (m, head_dim):
-                    raise KernelError(f"qkv_projection: table is {tuple(table.shape)}, [{m}, {head_dim}] is needed")
-            if slots is not None:
-                _need(slots, "qkv_projection: slots", torch.int32)
-                _need(keys, "qkv_projection: keys", torch.bfloat16)
-                _need(values, "qkv_projection: values", torch.bfloat16)
+            _need_qkv(bias, table, slots, keys, values, m, n, head_dim)
             out = torch.empty((m, n), dtype=x.dtype, device=x.device)
             _set_bounds("gemm_tcgen05", keys if slots is not None else None)
             _check(lib, lib.pae_linear_rotary_tcgen05(
@@ -901,6 +1051,20 @@ def linear_swiglu(x, weight, gate: str = "silu") -> torch.Tensor:
     tokens the activation runs in the product's epilogue; with few, in the kernel that sums the
     splits; otherwise as a kernel of its own. Gate and up are rounded to the engine dtype first in
     every one of them, so all give the same bits."""
+    if (x.dtype == torch.bfloat16 and weight.shape[0] % 32 == 0 and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[1])
+            and not _uneven_gate(x.shape[0], weight.shape[0], x.device)):
+        operand = _cluster_operand(x)
+        if operand is not None:
+            source, squares, width, eps = operand
+            m, n, k = source.shape[0], weight.shape[0], weight.shape[1]
+            _need(source, "linear_swiglu: x")
+            _need(weight, "linear_swiglu: weight")
+            out = torch.empty((m, n // 2), dtype=torch.bfloat16, device=source.device)
+            lib = _lib("gemm_cluster")
+            _check(lib, lib.pae_linear_swiglu_cluster(
+                _ptr(out), _ptr(source), _ptr(weight), _ptr(squares), 0 if squares is None else squares.shape[0], width, eps, m, n, k,
+                GATE_KINDS[gate], _early_weights(m, k), 0, 0, 0, _ptr(_error_flag(source.device)), _stream()))
+            return out
     source, norm_weight, eps = _norm_of(x)
     if (_few_tokens(source, weight.shape[1], norm_weight is not None, GATE_UP_KIND, weight.shape[0]) and weight.dtype == torch.bfloat16 and weight.is_contiguous()
             and weight.data_ptr() % 16 == 0 and weight.shape[0] % 32 == 0 and source.shape[1] == weight.shape[1]):
