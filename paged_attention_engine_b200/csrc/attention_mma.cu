@@ -56,6 +56,68 @@ PAE_EXPORT int pae_paged_attention_decode(void* out, const void* qkv, const void
                              page_size, scale, window, slice_keys, max_slices, scratch, (cudaStream_t)stream);
 }
 
+// int32 elements of a plan of `items` slices.
+PAE_EXPORT long long pae_decode_plan_ints(int seqs, int kv_heads, int items) { return 4ll * items + 2ll * seqs * kv_heads; }
+
+// The slices of a step's requests of one token (plan, 16-byte aligned): at most `items`, which is at least seqs * kv_heads, of one length, at least `least`
+// tiles of 16 keys. Up to 2,048 requests.
+PAE_EXPORT int pae_plan_decode(int* plan, const int* q_start, const int* kv_len, int seqs, int kv_heads, int window, int items, int least, void* stream) {
+  if (seqs == 0) return 0;
+  if (seqs > MAX_PLANNED_REQUESTS) return fail(2, "plan_decode: %d requests are more than %d", seqs, MAX_PLANNED_REQUESTS);
+  if (kv_heads < 1 || (long long)items < (long long)seqs * kv_heads || least < 1) return fail(2, "plan_decode: %d slices for %d requests x %d heads", items, seqs, kv_heads);
+  if ((uintptr_t)plan & 15) return fail(2, "plan_decode: the plan does not start on a 16-byte boundary");
+  launch_kernel(plan_decode_kernel, dim3(1), dim3(PLAN_THREADS), 0, (cudaStream_t)stream, (DecodeSlice*)plan, (PairSlices*)(plan + 4ll * items), q_start,
+                kv_len, seqs, kv_heads, window, items, least);
+  return check_launch("plan_decode");
+}
+
+// Floats of scratch that `pae_paged_attention_decode_planned` needs.
+PAE_EXPORT long long pae_decode_planned_floats(int heads, int kv_heads, int d, int items) { return (long long)items * (heads / kv_heads) * (d + 2); }
+
+// As pae_paged_attention_decode, over the slices of a plan that pae_plan_decode made of the same q_start, kv_len, kv_heads, window, items and
+// `least`. max_kv_len: the longest request's keys at most (a longer one's result means nothing).
+PAE_EXPORT int pae_paged_attention_decode_planned(void* out, const void* qkv, const void* keys, const void* values, const int* block_table,
+                                                  int table_width, const int* q_start, const int* kv_len, const int* plan, int seqs, int heads,
+                                                  int kv_heads, int d, int page_size, float scale, int window, int max_kv_len, int items, int least,
+                                                  float* scratch, void* stream) {
+  if (seqs == 0) return 0;
+  if (int err = check_sizes("paged_attention_decode", heads, kv_heads, d, page_size, seqs)) return err;
+  if (heads / kv_heads > 16) return fail(2, "paged_attention_decode: %d query heads per kv head are more than 16", heads / kv_heads);
+  if (items < 1 || least < 1 || max_kv_len < 1) return fail(2, "paged_attention_decode: %d slices of %d tiles, %d keys", items, least, max_kv_len);
+  if (plan == nullptr || scratch == nullptr) return fail(2, "paged_attention_decode: no plan, or no scratch for the slices' results");
+  const int max_slices = (max_kv_len / TILE_KEYS + 2 + least - 1) / least;
+  if ((size_t)(max_slices + MERGE_WARPS * d) * sizeof(float) > 40 * 1024)
+    return fail(2, "paged_attention_decode: %d slices are more than the merge takes (%d at head size %d)", max_slices,
+                (int)(40 * 1024 / sizeof(float)) - MERGE_WARPS * d, d);
+  PlannedParams a{};
+  a.out = (__nv_bfloat16*)out;
+  a.slices = (const DecodeSlice*)plan;
+  a.pairs = (const PairSlices*)(plan + 4ll * items);
+  a.items = items;
+  DecodeParams& p = a.d;
+  p.qkv = (const __nv_bfloat16*)qkv;
+  p.keys = (const __nv_bfloat16*)keys;
+  p.values = (const __nv_bfloat16*)values;
+  p.block_table = block_table;
+  p.q_start = q_start;
+  p.kv_len = kv_len;
+  const size_t rows = (size_t)items * (heads / kv_heads);
+  p.part_out = scratch;
+  p.part_max = scratch + rows * d;
+  p.part_sum = p.part_max + rows;
+  p.table_width = table_width;
+  p.heads = heads;
+  p.kv_heads = kv_heads;
+  p.page_size = page_size;
+  p.window = window;
+  p.max_slices = max_slices;
+  p.scale_log2 = scale * LOG2E;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (d == 32) return launch_planned<32>(a, seqs, s);
+  if (d == 64) return launch_planned<64>(a, seqs, s);
+  return launch_planned<128>(a, seqs, s);
+}
+
 // Requests that bring several tokens (and, unless skip_single, those that bring one); with
 // `work_index` (device, `work_count` entries) only the requests it lists get blocks.
 PAE_EXPORT int pae_paged_attention_prefill(void* out, const void* qkv, const void* keys, const void* values,

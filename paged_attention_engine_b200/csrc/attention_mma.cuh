@@ -251,32 +251,14 @@ struct DecodeParams {
   float scale_log2;
 };
 
-template <int D>
-__global__ void __launch_bounds__(SLICE_WARPS * 32) decode_slices_kernel(const DecodeParams p) {
-  // The step's integers (starts, lengths, block tables) were copied in before the step began
-  // and the keys and values of EARLIER tokens are not written by any kernel of this step, so
-  // a slice's first tiles are fetched before the wait for the kernel that precedes this one
-  // (which writes this step's queries, keys and values). Every block waits before it leaves.
-  dependent_launch_trigger();
-  extern __shared__ __align__(128) uint8_t smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int slice = blockIdx.x * SLICE_WARPS + warp;
-  const int g = blockIdx.y, b = blockIdx.z;
-  const int token = p.q_start[b];
-  const int kv_len = p.kv_len[b];
-  const int first_key = p.window > 0 ? max(0, kv_len - p.window) : 0;     // the query stands at kv_len - 1
-  const int base = (first_key / TILE_KEYS) * TILE_KEYS;
-  const int begin = base + slice * p.slice_keys;
-  const int end = min(kv_len, begin + p.slice_keys);
-  if (p.q_start[b + 1] - token != 1 || slice >= p.max_slices || begin >= kv_len) {   // nothing for this warp
-    dependent_launch_wait();
-    return;
-  }
-
+// One warp's slice, keys begin .. end - 1 of request b and kv head g, in `mine`, its stages of (K tile, V tile); `leave` gets the
+// unnormalised output with the rows' maxima and sums.
+template <int D, typename Leave>
+__device__ __forceinline__ void decode_slice(const DecodeParams& p, uint8_t* mine, int lane, int b, int g, int token, int kv_len, int first_key,
+                                             int begin, int end, Leave leave) {
   const int groups = p.heads / p.kv_heads;
   const int row_elems = (p.heads + 2 * p.kv_heads) * D;
   constexpr int TILE_BYTES = TILE_KEYS * D * 2;
-  uint8_t* mine = smem + warp * SLICE_STAGES * 2 * TILE_BYTES;      // stages of (K tile, V tile)
   const uint32_t mine_u32 = smem_u32(mine);
   const int* table = p.block_table + (size_t)b * p.table_width;
 
@@ -339,21 +321,50 @@ __global__ void __launch_bounds__(SLICE_WARPS * 32) decode_slices_kernel(const D
   }
   cp_async_wait<0>();
 
-  // Rows 0..groups-1 are real heads. Row lane/4 (half 0) and lane/4 + 8 (half 1).
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int r = (lane >> 2) + half * 8;
-    if (r >= groups) continue;
-    const size_t at = ((size_t)b * p.heads + g * groups + r) * p.max_slices + slice;
-    float* out = p.part_out + at * D;
-#pragma unroll
-    for (int n = 0; n < D / 8; ++n)
-      *(float2*)(out + n * 8 + (lane & 3) * 2) = make_float2(o[n][half * 2], o[n][half * 2 + 1]);
-    if ((lane & 3) == 0) {
-      p.part_max[at] = row_max[half];
-      p.part_sum[at] = row_sum[half];
-    }
+  leave(o, row_max, row_sum);
+}
+
+template <int D>
+__global__ void __launch_bounds__(SLICE_WARPS * 32) decode_slices_kernel(const DecodeParams p) {
+  // The step's integers (starts, lengths, block tables) were copied in before the step began
+  // and the keys and values of EARLIER tokens are not written by any kernel of this step, so
+  // a slice's first tiles are fetched before the wait for the kernel that precedes this one
+  // (which writes this step's queries, keys and values). Every block waits before it leaves.
+  dependent_launch_trigger();
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slice = blockIdx.x * SLICE_WARPS + warp;
+  const int g = blockIdx.y, b = blockIdx.z;
+  const int token = p.q_start[b];
+  const int kv_len = p.kv_len[b];
+  const int first_key = p.window > 0 ? max(0, kv_len - p.window) : 0;     // the query stands at kv_len - 1
+  const int base = (first_key / TILE_KEYS) * TILE_KEYS;
+  const int begin = base + slice * p.slice_keys;
+  const int end = min(kv_len, begin + p.slice_keys);
+  if (p.q_start[b + 1] - token != 1 || slice >= p.max_slices || begin >= kv_len) {   // nothing for this warp
+    dependent_launch_wait();
+    return;
   }
+
+  decode_slice<D>(p, smem + warp * SLICE_STAGES * 2 * TILE_KEYS * D * 2, lane, b, g, token, kv_len, first_key, begin, end,
+                  [&](float (&o)[D / 8][4], float (&row_max)[2], float (&row_sum)[2]) {
+    const int groups = p.heads / p.kv_heads;
+    // Rows 0..groups-1 are real heads. Row lane/4 (half 0) and lane/4 + 8 (half 1).
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int r = (lane >> 2) + half * 8;
+      if (r >= groups) continue;
+      const size_t at = ((size_t)b * p.heads + g * groups + r) * p.max_slices + slice;
+      float* out = p.part_out + at * D;
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n)
+        *(float2*)(out + n * 8 + (lane & 3) * 2) = make_float2(o[n][half * 2], o[n][half * 2 + 1]);
+      if ((lane & 3) == 0) {
+        p.part_max[at] = row_max[half];
+        p.part_sum[at] = row_sum[half];
+      }
+    }
+  });
 }
 
 // out[token, head, :] = sum_s w_s part_out[s] / sum_s w_s part_sum[s], w_s = 2^(max_s - max).
@@ -368,7 +379,7 @@ __global__ void __launch_bounds__(SLICE_WARPS * 32) decode_slices_kernel(const D
 constexpr int MERGE_WARPS = 4;
 constexpr int MERGE_DEPTH = 24;      // slices per warp whose partial outputs are in registers at one time
 
-template <int D>
+template <int D, int DEPTH>
 __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
     __nv_bfloat16* __restrict__ out, const float* __restrict__ part_out, const float* __restrict__ part_max,
     const float* __restrict__ part_sum, const int* __restrict__ q_start, const int* __restrict__ kv_len, int heads, int window,
@@ -391,10 +402,10 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int PER_LANE = D / 32;
 
-  // ---- requests: this warp's first MERGE_DEPTH partial outputs, then the maxima and sums
-  float part[MERGE_DEPTH][PER_LANE];
+  // ---- requests: this warp's first DEPTH partial outputs, then the maxima and sums
+  float part[DEPTH][PER_LANE];
 #pragma unroll
-  for (int i = 0; i < MERGE_DEPTH; ++i) {
+  for (int i = 0; i < DEPTH; ++i) {
     const int s = warp + i * MERGE_WARPS;
 #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) part[i][j] = 0.f;
@@ -442,7 +453,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
 #pragma unroll
   for (int j = 0; j < PER_LANE; ++j) acc[j] = 0.f;
 #pragma unroll
-  for (int i = 0; i < MERGE_DEPTH; ++i) {
+  for (int i = 0; i < DEPTH; ++i) {
     const int s = warp + i * MERGE_WARPS;
     if (s < slices) {
       const float w = weights[s];
@@ -450,7 +461,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
       for (int j = 0; j < PER_LANE; ++j) acc[j] += part[i][j] * w;
     }
   }
-  for (int s = warp + MERGE_DEPTH * MERGE_WARPS; s < slices; s += MERGE_WARPS) {     // more than 96 slices
+  for (int s = warp + DEPTH * MERGE_WARPS; s < slices; s += MERGE_WARPS) {     // more than 96 slices
     const float w = weights[s];
     const float* from = part_out + (at + s) * D + lane * PER_LANE;
 #pragma unroll
@@ -465,6 +476,267 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
 #pragma unroll
     for (int w = 0; w < MERGE_WARPS; ++w) v += across[w * D + d];
     out[((size_t)token * heads + h) * D + d] = __float2bfloat16_rn(v * inv);
+  }
+}
+
+// ---------------------------------------------------------------------------------------
+// decode, planned
+// ---------------------------------------------------------------------------------------
+// The sliced kernel cuts every request into slices of one length that the launch fixes by the longest, so of requests of unequal
+// lengths many slices are empty while the warps of the longest walk theirs, one trip to memory after the other (64 requests of
+// 16 to 2,048 keys at the 3584-wide sizes: half of the slices; 36 us where the bytes need 20). Here the slices are planned
+// once a step, by a kernel that reads the step's lengths: the shortest slice with which all requests' slices number no more than
+// the warps that run at one time. A warp finds its slice in the plan, the merge its (request, kv head)'s slices; every
+// layer of the step uses the plan, and a recorded step plans anew in each replay.
+struct DecodeSlice {
+  int request, kv_head, begin, end;            // keys; begin == end: nothing
+};
+struct PairSlices {
+  int first, count;
+};
+
+// Keys that request b's one token sees, from the tile that holds the first of them on; 0: it brings another number of tokens.
+struct DecodeKeys {
+  int base, end;
+};
+__device__ __forceinline__ DecodeKeys decode_keys(const int* q_start, const int* kv_len, int window, int b) {
+  if (q_start[b + 1] - q_start[b] != 1) return {0, 0};
+  const int n = kv_len[b], first = window > 0 ? max(0, n - window) : 0;
+  return {first / TILE_KEYS * TILE_KEYS, n};
+}
+
+constexpr int PLAN_THREADS = 1024;
+constexpr int MAX_PLANNED_REQUESTS = 2048;
+
+// slices [items], pairs [seqs, kv_heads]. `least`: tiles of 16 keys that a slice has at least. items >= seqs * kv_heads, so that the
+// search ends with a slice a pair at the latest.
+__global__ void __launch_bounds__(PLAN_THREADS) plan_decode_kernel(DecodeSlice* __restrict__ slices, PairSlices* __restrict__ pairs,
+                                                                   const int* __restrict__ q_start, const int* __restrict__ kv_len, int seqs,
+                                                                   int kv_heads, int window, int items, int least) {
+  // The layers' kernels read the plan before their waits: the kernel behind this one is not let go before this one has ended.
+  dependent_launch_wait();
+  __shared__ int before[MAX_PLANNED_REQUESTS + 1];         // slices of the requests before, for one kv head
+  __shared__ int warp_sums[PLAN_THREADS / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto tiles_of = [&](int b) {
+    const DecodeKeys keys = decode_keys(q_start, kv_len, window, b);
+    return (keys.end - keys.base + TILE_KEYS - 1) / TILE_KEYS;
+  };
+  // the sum over the block, for every thread
+  auto block_sum = [&](int v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if (lane == 0) warp_sums[warp] = v;
+    __syncthreads();
+    v = 0;
+#pragma unroll
+    for (int w = 0; w < PLAN_THREADS / 32; ++w) v += warp_sums[w];
+    return v;
+  };
+  int tiles = 0;
+  for (int b = threadIdx.x; b < seqs; b += PLAN_THREADS) tiles += tiles_of(b);
+  int length = max(least, (block_sum(tiles) * kv_heads + items - 1) / items);      // of a slice, in tiles
+  for (;;) {
+    int count = 0, longest = 0;
+    for (int b = threadIdx.x; b < seqs; b += PLAN_THREADS) {
+      const int n = tiles_of(b);
+      count += (n + length - 1) / length;
+      longest |= n > length;
+    }
+    if (block_sum(count) * kv_heads <= items || !__syncthreads_or(longest)) break;
+    length += max(1, length / 32);
+  }
+  int carry = 0;
+  for (int first = 0; first < seqs; first += PLAN_THREADS) {
+    const int b = first + threadIdx.x;
+    const int mine = b < seqs ? (tiles_of(b) + length - 1) / length : 0;
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int other = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += other;
+    }
+    __syncthreads();
+    if (lane == 31) warp_sums[warp] = upto;
+    __syncthreads();
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < PLAN_THREADS / 32; ++w) {
+      if (w < warp) upto += warp_sums[w];
+      total += warp_sums[w];
+    }
+    if (b < seqs) {
+      before[b] = carry + upto - mine;
+      for (int g = 0; g < kv_heads; ++g) pairs[(size_t)b * kv_heads + g] = {(carry + upto - mine) * kv_heads + g * mine, mine};
+    }
+    carry += total;
+  }
+  if (threadIdx.x == 0) before[seqs] = carry;
+  __syncthreads();
+  for (int i = threadIdx.x; i < items; i += PLAN_THREADS) {
+    if (i >= carry * kv_heads) {
+      slices[i] = {0, 0, 0, 0};
+      continue;
+    }
+    int low = 0, high = seqs;                              // the last request whose slices begin at or before i
+    while (high - low > 1) {
+      const int middle = (low + high) >> 1;
+      if (before[middle] * kv_heads <= i) low = middle;
+      else high = middle;
+    }
+    const int inside = i - before[low] * kv_heads, count = before[low + 1] - before[low];
+    const int g = inside / count;
+    const DecodeKeys keys = decode_keys(q_start, kv_len, window, low);
+    const int begin = keys.base + (inside - g * count) * length * TILE_KEYS;
+    slices[i] = {low, g, begin, min(keys.end, begin + length * TILE_KEYS)};
+  }
+  __threadfence();
+}
+
+struct PlannedParams {
+  DecodeParams d;               // part_out [query head of the pair, slice, D], part_max and part_sum [query head, slice]
+  __nv_bfloat16* out;
+  const DecodeSlice* slices;
+  const PairSlices* pairs;
+  int items;
+};
+
+template <int D>
+__global__ void __launch_bounds__(SLICE_WARPS * 32) decode_planned_kernel(const PlannedParams a) {
+  // What is read before the wait: as in the sliced kernel above, and the plan, whose kernel has ended before any kernel behind it began.
+  dependent_launch_trigger();
+  const DecodeParams& p = a.d;
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int item = blockIdx.x * SLICE_WARPS + warp;
+  const int4 slice = item < a.items ? *(const int4*)(a.slices + item) : make_int4(0, 0, 0, 0);
+  const int b = slice.x, g = slice.y, begin = slice.z, end = slice.w;
+  if (begin >= end) {           // nothing for this warp
+    dependent_launch_wait();
+    return;
+  }
+  const int token = p.q_start[b], kv_len = p.kv_len[b];
+  const int first_key = p.window > 0 ? max(0, kv_len - p.window) : 0;     // the query stands at kv_len - 1
+  decode_slice<D>(p, smem + warp * SLICE_STAGES * 2 * TILE_KEYS * D * 2, lane, b, g, token, kv_len, first_key, begin, end,
+                  [&](float (&o)[D / 8][4], float (&row_max)[2], float (&row_sum)[2]) {
+    const int groups = p.heads / p.kv_heads;
+    const bool whole = begin <= first_key && end == kv_len;                // the pair's one slice: finished here
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int r = (lane >> 2) + half * 8;
+      if (r >= groups) continue;
+      if (whole) {
+        const float inv = row_sum[half] > 0.f ? 1.f / row_sum[half] : 0.f;
+        __nv_bfloat16* to = a.out + ((size_t)token * p.heads + (size_t)g * groups + r) * D;
+#pragma unroll
+        for (int n = 0; n < D / 8; ++n)
+          *(uint32_t*)(to + n * 8 + (lane & 3) * 2) = pack_bf16(o[n][half * 2] * inv, o[n][half * 2 + 1] * inv);
+        continue;
+      }
+      const size_t row = (size_t)r * a.items + item;
+      float* to = p.part_out + row * D;
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n) *(float2*)(to + n * 8 + (lane & 3) * 2) = make_float2(o[n][half * 2], o[n][half * 2 + 1]);
+      if ((lane & 3) == 0) {
+        p.part_max[row] = row_max[half];
+        p.part_sum[row] = row_sum[half];
+      }
+    }
+  });
+}
+
+// The merge of the planned slices: as above, DEPTH parts per warp at one time in registers.
+template <int D, int DEPTH>
+__global__ void __launch_bounds__(MERGE_WARPS * 32) merge_planned_kernel(const PlannedParams a) {
+  dependent_launch_trigger();
+  const DecodeParams& p = a.d;
+  extern __shared__ float weights[];          // [max_slices], then [MERGE_WARPS][D]
+  __shared__ float reduce[2 * MERGE_WARPS];
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int groups = p.heads / p.kv_heads, g = h / groups;
+  const int token = p.q_start[b];
+  const PairSlices pair = a.pairs[(size_t)b * p.kv_heads + g];
+  dependent_launch_wait();
+  if (pair.count < 2) return;                 // not a request of one token; or finished by its one warp
+  const int slices = min(p.max_slices, pair.count);
+  const size_t at = (size_t)(h - g * groups) * a.items + pair.first;
+  constexpr int PER_LANE = D / 32;
+
+  // ---- requests: this warp's first DEPTH partial outputs, then the maxima and sums
+  auto load_part = [&](int s, float* v) {
+    const float* from = p.part_out + (at + s) * D + lane * PER_LANE;
+    if (PER_LANE == 4) {
+      const float4 t = *(const float4*)from;
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < PER_LANE; ++j) v[j] = from[j];
+    }
+  };
+  float part[DEPTH][4];
+#pragma unroll
+  for (int i = 0; i < DEPTH; ++i) {
+    const int s = warp + i * MERGE_WARPS;
+    part[i][0] = part[i][1] = part[i][2] = part[i][3] = 0.f;
+    if (s < slices) load_part(s, part[i]);
+  }
+  float top = -FLT_MAX;
+  for (int s = threadIdx.x; s < slices; s += blockDim.x) {
+    const float m = p.part_max[at + s];
+    weights[s] = m;
+    top = fmaxf(top, m);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+  if (lane == 0) reduce[warp] = top;
+  __syncthreads();
+  top = reduce[0];
+#pragma unroll
+  for (int w = 1; w < MERGE_WARPS; ++w) top = fmaxf(top, reduce[w]);
+
+  float total = 0.f;
+  for (int s = threadIdx.x; s < slices; s += blockDim.x) {
+    const float w = exp2f(weights[s] - top);    // this thread wrote weights[s] itself
+    weights[s] = w;
+    total += p.part_sum[at + s] * w;
+  }
+  total = warp_sum(total);
+  if (lane == 0) reduce[MERGE_WARPS + warp] = total;
+  __syncthreads();                              // the weights of all slices and the warps' sums are in place
+  total = 0.f;
+#pragma unroll
+  for (int w = 0; w < MERGE_WARPS; ++w) total += reduce[MERGE_WARPS + w];
+  const float inv = total > 0.f ? 1.f / total : 0.f;
+
+  // ---- this warp's slices in their order
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < DEPTH; ++i) {
+    const int s = warp + i * MERGE_WARPS;
+    if (s < slices) {
+      const float w = weights[s];
+#pragma unroll
+      for (int j = 0; j < PER_LANE; ++j) acc[j] += part[i][j] * w;
+    }
+  }
+  for (int s = warp + DEPTH * MERGE_WARPS; s < slices; s += MERGE_WARPS) {
+    float v[4];
+    load_part(s, v);
+    const float w = weights[s];
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) acc[j] += v[j] * w;
+  }
+  float* across = weights + p.max_slices;          // [MERGE_WARPS][D]
+#pragma unroll
+  for (int j = 0; j < PER_LANE; ++j) across[warp * D + lane * PER_LANE + j] = acc[j];
+  __syncthreads();
+  for (int d = threadIdx.x; d < D; d += blockDim.x) {
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < MERGE_WARPS; ++w) v += across[w * D + d];
+    a.out[((size_t)token * p.heads + h) * D + d] = __float2bfloat16_rn(v * inv);
   }
 }
 
@@ -635,6 +907,10 @@ int allow_smem(Kernel kernel, size_t bytes, const char* what) {
 
 inline size_t slices_smem_bytes(int d) { return (size_t)SLICE_WARPS * SLICE_STAGES * 2 * TILE_KEYS * d * 2; }
 
+// Which merge: many blocks hold eight slices a warp in registers (64 of them instead of 128), so that more blocks run at once (12 heads of 64
+// requests, 8 slices: 3.0 us instead of 5.2); few blocks with many slices take up to 96 in one trip.
+inline bool merge_in_few_registers(int heads, int seqs, int max_slices) { return (long long)heads * seqs > 4 * 148 || max_slices <= 8 * MERGE_WARPS; }
+
 template <int D>
 int launch_decode(const DecodeParams& p, __nv_bfloat16* out, int seqs, cudaStream_t s) {
   const size_t bytes = slices_smem_bytes(D);
@@ -642,8 +918,21 @@ int launch_decode(const DecodeParams& p, __nv_bfloat16* out, int seqs, cudaStrea
   dim3 grid((p.max_slices + SLICE_WARPS - 1) / SLICE_WARPS, p.kv_heads, seqs);
   launch_kernel(decode_slices_kernel<D>, grid, SLICE_WARPS * 32, bytes, s, p);
   if (int err = check_launch("paged_attention_decode")) return err;
-  launch_kernel(merge_slices_kernel<D>, dim3(p.heads, seqs), MERGE_WARPS * 32, (p.max_slices + MERGE_WARPS * D) * sizeof(float), s, out, p.part_out, p.part_max, p.part_sum, p.q_start,
-                                                                     p.kv_len, p.heads, p.window, p.slice_keys, p.max_slices);
+  const auto merge = merge_in_few_registers(p.heads, seqs, p.max_slices) ? merge_slices_kernel<D, 8> : merge_slices_kernel<D, MERGE_DEPTH>;
+  launch_kernel(merge, dim3(p.heads, seqs), dim3(MERGE_WARPS * 32), (p.max_slices + MERGE_WARPS * D) * sizeof(float), s, out, p.part_out, p.part_max,
+                p.part_sum, p.q_start, p.kv_len, p.heads, p.window, p.slice_keys, p.max_slices);
+  return check_launch("paged_attention_merge");
+}
+
+template <int D>
+int launch_planned(const PlannedParams& a, int seqs, cudaStream_t s) {
+  const size_t bytes = slices_smem_bytes(D);
+  if (int err = allow_smem(decode_planned_kernel<D>, bytes, "paged_attention_decode")) return err;
+  launch_kernel(decode_planned_kernel<D>, dim3((a.items + SLICE_WARPS - 1) / SLICE_WARPS), dim3(SLICE_WARPS * 32), bytes, s, a);
+  if (int err = check_launch("paged_attention_decode")) return err;
+  const size_t merge_bytes = (a.d.max_slices + MERGE_WARPS * D) * sizeof(float);
+  const auto merge = merge_in_few_registers(a.d.heads, seqs, a.d.max_slices) ? merge_planned_kernel<D, 8> : merge_planned_kernel<D, MERGE_DEPTH>;
+  launch_kernel(merge, dim3(a.d.heads, seqs), dim3(MERGE_WARPS * 32), merge_bytes, s, a);
   return check_launch("paged_attention_merge");
 }
 

@@ -59,6 +59,7 @@ class StepContext:
     # int32 [entries - num_single]: the entries that bring more than one token, in their order; None
     # when all or none do. Attention's portion kernels then launch blocks for these entries only.
     multi_index: torch.Tensor | None
+    ragged: bool                  # a step of single tokens whose contexts are much shorter than the longest one planned for (`ragged_contexts`)
     wants_every_token: bool       # logit_rows is 0, 1, ..., tokens - 1: no gather is needed
     groups: list[GroupStep]
     # Host copies, for parts (and tests) that plan on the host.
@@ -71,6 +72,12 @@ class StepContext:
     # (last_token [slots], state_slot, seq_index): where a token id of -1 is looked up on the device
     feedback: tuple | None = None
     memo: dict = field(default_factory=dict)
+
+
+def ragged_contexts(keys: int, requests: int, planned_kv: int) -> bool:
+    """Whether `requests` contexts of `keys` keys in all fill at most three quarters of as many of `planned_kv` keys: then decode
+    attention plans the step's slices (`ops.plan_decode`) instead of cutting every request as the longest."""
+    return requests > 1 and 4 * keys <= 3 * requests * planned_kv
 
 
 class _Staging:
@@ -153,6 +160,7 @@ class BatchBuilder:
         into: torch.Tensor | None = None,
         pad_to: int | None = None,
         max_kv_len: int | None = None,
+        ragged: bool | None = None,
     ) -> StepContext | None:
         """Flattens the entries. `sampling` (one row per wanted place: temperature, seed,
         request key, output index) travels in the same copy. `table_width` fixes the width of
@@ -163,7 +171,8 @@ class BatchBuilder:
         state slot behind the real ones; its logits and its token are computed and ignored, so
         that steps of neighbouring batch sizes can share one captured graph. `max_kv_len` is the
         longest context that the step's kernels are to plan for (at least the true one; a captured
-        graph fixes it); without it, the table's width when that is fixed, else the true one."""
+        graph fixes it); without it, the table's width when that is fixed, else the true one. `ragged`: whether the contexts are of
+        unequal lengths (a captured graph fixes it); without it, what they are."""
         if not entries:
             raise ValueError("a step needs at least one entry")
         manager = self.manager
@@ -232,6 +241,8 @@ class BatchBuilder:
         planned_kv = max_kv_len if max_kv_len is not None else (width * page if table_width is not None else max_kv)
         if planned_kv < max_kv:
             raise ValueError(f"a context of {max_kv} keys does not fit the {planned_kv} that the step plans for")
+        if ragged is None:
+            ragged = decode_only and ragged_contexts(int(kv_len[:real].sum()), real, planned_kv)
         num_groups = len(manager.groups)
         if sampling is not None and len(sampling) != len(rows) - pads:
             raise ValueError(f"{len(sampling)} sampling rows for {len(rows) - pads} wanted places")
@@ -305,7 +316,7 @@ class BatchBuilder:
             token_ids=part(0), positions=part(1), seq_index=part(2), q_start=part(3), q_pos0=part(4),
             kv_len=part(5), state_slot=part(6), logit_rows=part(7),
             max_q_len=max(q_lens), max_kv_len=planned_kv,
-            num_single=sum(1 for n in q_lens if n == 1), multi_index=part(multi_at) if multi else None, wants_every_token=len(rows) == total and rows == list(range(total)), groups=groups,
+            num_single=sum(1 for n in q_lens if n == 1), multi_index=part(multi_at) if multi else None, ragged=ragged, wants_every_token=len(rows) == total and rows == list(range(total)), groups=groups,
             host_q_lens=list(q_lens), host_q_pos0=list(pos0), host_state_slots=list(slots_of),
             sampling=sampling_parts, buffer=dev,
         )

@@ -34,7 +34,7 @@ from typing import Any, Hashable, Sequence
 import torch
 
 from ..cache.storage import PagedKVCache
-from .batch import BatchBuilder, StepEntry
+from .batch import BatchBuilder, StepEntry, ragged_contexts
 from .model import DecoderModel
 
 
@@ -61,7 +61,7 @@ class _DecodeGraph:
 
 
 class ModelRunner:
-    # A graph per (batch size, block-table width, longest context rounded up, sampling). They share
+    # A graph per (batch size, block-table width, longest context rounded up, sampling, contexts of unequal lengths). They share
     # one memory pool (they never run at the same time), so a graph costs its launches and little else.
     MAX_GRAPHS = 512
     # A recorded step plans its attention (how the keys are sliced) for a longest context that is
@@ -88,7 +88,7 @@ class ModelRunner:
         # The checked build hands its limits to the libraries between launches: it records no graphs.
         self.use_graphs = (use_graphs and self.runtime.device.type == "cuda" and model.graph_safe
                            and not getattr(self.runtime.ops, "bounds_checked", False))
-        self.graphs: dict[tuple[int, int, int, bool], _DecodeGraph] = {}
+        self.graphs: dict[tuple[int, int, int, bool, bool], _DecodeGraph] = {}
         self.graph_pool = None
         self.capture_stream = None
         self.graph_replays = 0
@@ -125,19 +125,24 @@ class ModelRunner:
             tokens = ops.sample(logits, *ctx.sampling, keep=(self.last_token, ctx.logit_rows, ctx.seq_index, ctx.state_slot))
         return logits, tokens
 
-    def _graph_key(self, entries, sampling) -> tuple[int, int, int, bool] | None:
+    def _graph_key(self, entries, sampling) -> tuple[int, int, int, bool, bool] | None:
         if not self.use_graphs or len(entries) > 256:
             return None
+        longest, keys, computed = 0, len(entries), self.manager.num_computed
         for e in entries:
             if len(e.tokens) != 1 or tuple(e.want) != (0,):
                 return None
+            context = computed(e.key)
+            keys += context
+            if context > longest:
+                longest = context
+        longest += 1
         page = self.manager.block_size
-        longest = max(self.manager.num_computed(e.key) + 1 for e in entries)
         width = 16
         while width * page < longest:
             width *= 2
         bucket = min(width * page, -(-longest // self.KV_BUCKET) * self.KV_BUCKET)
-        return (self.graph_batch(len(entries)), width, bucket, sampling is not None)
+        return (self.graph_batch(len(entries)), width, bucket, sampling is not None, ragged_contexts(keys, len(entries), bucket))
 
     def _shape_key(self, entries, sampling) -> tuple | None:
         """The exact shape of a step that is not decode-only (per entry: tokens, start, wanted places,
@@ -164,7 +169,7 @@ class ModelRunner:
         key = self._graph_key(entries, sampling)
         slot = self.graphs.get(key) if key is not None else None
         if slot is not None and slot.graph is not None:
-            self.builder.build(entries, sampling, table_width=key[1], into=slot.buffer, pad_to=key[0], max_kv_len=key[2])
+            self.builder.build(entries, sampling, table_width=key[1], into=slot.buffer, pad_to=key[0], max_kv_len=key[2], ragged=key[4])
             slot.graph.replay()
             self.model.forward_pass_count += 1
             self.graph_replays += 1
@@ -176,7 +181,7 @@ class ModelRunner:
         elif key is not None and len(self.graphs) < self.MAX_GRAPHS:
             # First time for this shape: its launches are recorded (nothing runs), then the
             # recording is replayed, which is this step's real work.
-            ctx = self.builder.build(entries, sampling, table_width=key[1], pad_to=key[0], max_kv_len=key[2])
+            ctx = self.builder.build(entries, sampling, table_width=key[1], pad_to=key[0], max_kv_len=key[2], ragged=key[4])
             slot = _DecodeGraph(ctx.buffer)
             self._capture(slot, ctx)
             self.graphs[key] = slot

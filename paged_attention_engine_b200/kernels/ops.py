@@ -487,10 +487,10 @@ CLUSTER_MAX_TOKENS = 128
 
 def _cluster_takes(tokens: int, n: int, k: int, weight, width: int) -> bool:
     """Whether the cluster kernels run a bfloat16 product of these sizes; `width`: of the rows that the norm before or behind it reads."""
-    return (use_cluster_products and use_tensor_cores and not few_token_products_everywhere
+    return (weight.dtype == torch.bfloat16 and use_cluster_products and use_tensor_cores and not few_token_products_everywhere
             and (CLUSTER_MIN_TOKENS if width < CLUSTER_WIDE else 1) <= tokens <= CLUSTER_MAX_TOKENS
-            and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.shape[1] == k and n % 8 == 0 and k % 64 == 0
-            and weight.is_contiguous() and weight.data_ptr() % 16 == 0)
+            and weight.dim() == 2 and weight.shape[1] == k and n % 8 == 0 and k % 64 == 0 and weight.is_contiguous()
+            and weight.data_ptr() % 16 == 0)
 
 
 def _uneven_gate(tokens: int, n: int, device) -> bool:
@@ -899,6 +899,40 @@ def decode_slicing(seqs: int, kv_heads: int, max_kv_len: int, most: int | None =
     return slice_keys, -(-(max_kv_len + 15) // slice_keys)
 
 
+# Whether the decode attention of requests of unequal lengths is planned (tests compare both), and from how many tiles of 16 keys on that the
+# slices of the longest request's length would have room for. The plan takes 5 us a step. Measured, us for eight steps of eight
+# layers, contexts drawn evenly, cut as the longest / planned: 16 requests of 16 to 1,000 keys (2,080 tiles) 3,216 / 3,301, 24 (3,120) 3,497 /
+# 3,525, 32 (4,160) 3,676 / 3,647, 64 (8,320) 4,426 / 4,145; of 16 to 4,080 keys 12 (6,168) 3,513 / 3,497, 24 (12,336) 4,069 / 3,831, 64 (32,896) 5,981 / 5,035. Of requests of one length nothing
+# is gained (48 of 4,080: 5,773 / 5,907): see `ragged_contexts` of engine/batch.py.
+use_decode_plans = True
+PLANNED_MIN_TILES = 4000
+
+
+def plan_decode(q_start, kv_len, max_kv_len: int, num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, window: int,
+                dtype) -> None:
+    """Plans the slices of a step of single tokens, once a step for all layers of the same kv heads and window: the
+    plan stays with the step's `kv_len`, where `paged_attention` finds it. q_start and kv_len are not written after this call."""
+    seqs = kv_len.numel()
+    key = (num_kv_heads, head_dim, window)
+    tiles = (max_kv_len + 15) // 16 + 1
+    if (not use_decode_plans or seqs * num_kv_heads * tiles < PLANNED_MIN_TILES or seqs > 2048 or key in getattr(kv_len, "decode_plans", {})
+            or not plain_attention_takes(num_heads, num_kv_heads, head_dim, page_size, dtype)):
+        return
+    lib = _lib("attention_mma")
+    for name, t in (("q_start", q_start), ("kv_len", kv_len)):
+        _need(t, f"plan_decode: {name}", torch.int32)
+    # No more slices of a request than `decode_slicing` cuts, of 32 keys at least, and as many of all requests as warps run at one time.
+    most = 96 if max_kv_len <= 96 * 64 else min(192, max_kv_len // 64)
+    least = max(2, -(-tiles // most))
+    items = lib.pae_decode_blocks_per_wave(head_dim) * lib.pae_decode_slices_per_block()
+    items = max(seqs * num_kv_heads, min(items, seqs * num_kv_heads * -(-tiles // least)))
+    plan = torch.empty(lib.pae_decode_plan_ints(seqs, num_kv_heads, items), dtype=torch.int32, device=kv_len.device)
+    _check(lib, lib.pae_plan_decode(_ptr(plan), _ptr(q_start), _ptr(kv_len), seqs, num_kv_heads, window, items, least, _stream()))
+    if not hasattr(kv_len, "decode_plans"):
+        kv_len.decode_plans = {}
+    kv_len.decode_plans[key] = (plan, items, least)
+
+
 use_tcgen05_attention = True
 TCGEN05_ATTENTION_MIN_TOKENS = 64
 
@@ -908,12 +942,20 @@ def _decode_attention(lib, out, qkv, keys, values, block_table, q_start, kv_len,
     """The requests that bring one token: sliced over their keys, then merged."""
     count = seqs if singles < 0 else singles
     wave = lib.pae_decode_blocks_per_wave(head_dim)
-    slice_keys, max_slices = decode_slicing(count, num_kv_heads, max_kv_len, wave_blocks=wave,
-                                            slices_per_block=lib.pae_decode_slices_per_block())
+    per_block = lib.pae_decode_slices_per_block()
+    _set_bounds("attention_mma", keys)
+    plan = getattr(kv_len, "decode_plans", {}).get((num_kv_heads, head_dim, window))
+    if plan is not None:
+        slices, items, least = plan
+        scratch = torch.empty(lib.pae_decode_planned_floats(num_heads, num_kv_heads, head_dim, items), dtype=torch.float32, device=qkv.device)
+        _check(lib, lib.pae_paged_attention_decode_planned(
+            _ptr(out), _ptr(qkv), _ptr(keys), _ptr(values), _ptr(block_table), block_table.shape[1], _ptr(q_start), _ptr(kv_len), _ptr(slices), seqs,
+            num_heads, num_kv_heads, head_dim, page_size, scale, window, max_kv_len, items, least, _ptr(scratch), _stream()), 2)
+        return
+    slice_keys, max_slices = decode_slicing(count, num_kv_heads, max_kv_len, wave_blocks=wave, slices_per_block=per_block)
     floats = lib.pae_decode_scratch_floats(seqs, num_heads, head_dim, max_slices)
     scratch = torch.empty(floats, dtype=torch.float32, device=qkv.device)
     launches = 2
-    _set_bounds("attention_mma", keys)
     _check(lib, lib.pae_paged_attention_decode(
         _ptr(out), _ptr(qkv), _ptr(keys), _ptr(values), _ptr(block_table), block_table.shape[1],
         _ptr(q_start), _ptr(kv_len), seqs, num_heads, num_kv_heads, head_dim,

@@ -72,6 +72,10 @@ class GQAAttention(Part):
         group = ctx.groups[cache.group]
         table = self.position_encoding.table(ctx) if self.position_encoding is not None else None
         slots = group.slots if cache.writes else None
+        plan = getattr(ops, "plan_decode", None)
+        if plan is not None and getattr(ctx, "ragged", False):       # once a step: the layers share the plan
+            plan(ctx.q_start, ctx.kv_len, ctx.max_kv_len, self.num_heads, self.num_kv_heads, self.head_dim, cache.page_size,
+                 self.window, x.dtype)
         project = getattr(ops, "qkv_projection", None)
         if project is not None:          # the product, the rotation and the page write as one call
             qkv = project(x, self.qkv_weight, self.qkv_bias, table, slots, cache.keys, cache.values,
