@@ -99,6 +99,25 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   atomicCAS(error, 0, code);
   return false;
 }
+// The same by a whole warp, which goes on together.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* error, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, error, code));
+}
+// True in one lane of a converged warp. The warp that issues MMAs runs its role together and lets this lane issue them: what all lanes
+// hold alike lies in uniform registers, which the instruction takes; issued from a branch of one lane (`if (lane == 0)`) each MMA cost some
+// 110 cycles, more than its work.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t chosen;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(chosen));
+  return chosen != 0;
+}
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -194,6 +213,11 @@ __device__ __forceinline__ uint64_t mn_major_descriptor(uint32_t address, uint32
   d |= (uint64_t)1 << 46;
   d |= (uint64_t)2 << 61;
   return d;
+}
+// The descriptor of the place `bytes` (a multiple of 16) further: shared memory ends below 256 KB, so nothing carries out of the address
+// field.
+__device__ __forceinline__ uint64_t further(uint64_t descriptor, uint32_t bytes) {
+  return (descriptor & 0xFFFFFFFF00000000ull) | (uint32_t)((uint32_t)descriptor + (bytes >> 4));
 }
 // float32 accumulator, bfloat16 operands, A K-major; B K-major or MN-major (bit 16).
 __host__ __device__ constexpr uint32_t instruction_descriptor(int m, int n, bool b_mn_major) {
@@ -383,6 +407,8 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
     if (lane == 0 && working) {
       constexpr uint32_t idesc_s = instruction_descriptor(BQ, BKEYS, false);
       constexpr uint32_t idesc_o = instruction_descriptor(BQ, D, true);
+      const uint64_t q_first = k_major_descriptor(base + L::Q_OFFSET), k_first = k_major_descriptor(base + L::K_OFFSET);
+      const uint64_t p_first = k_major_descriptor(base + L::P_OFFSET), v_first = mn_major_descriptor(base + L::V_OFFSET, L::HALF_TILE_BYTES);
       bool ok = mbar_wait(bar(Q_FULL), 0, abort_flag, p.error, 2);
       auto issue_scores = [&](int t) {
         const int st = t & 1;
@@ -390,13 +416,13 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
         if (t >= 2) ok = ok && mbar_wait(bar(S_EMPTY, st), ((t >> 1) - 1) & 1, abort_flag, p.error, 4);
         if (!ok) return;
         tcgen05_fence_after();
-        const uint32_t q_addr = base + L::Q_OFFSET, k_addr = base + L::K_OFFSET + st * L::KV_BYTES;
+        const uint64_t keys = further(k_first, st * L::KV_BYTES);
 #pragma unroll
         for (int half = 0; half < L::HALVES; ++half)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_bf16(tmem_base + st * L::S_COLUMNS, k_major_descriptor(q_addr + half * L::HALF_TILE_BYTES + k * 32),
-                      k_major_descriptor(k_addr + half * L::HALF_TILE_BYTES + k * 32), idesc_s, (half > 0 || k > 0) ? 1u : 0u);
+            umma_bf16(tmem_base + st * L::S_COLUMNS, further(q_first, half * L::HALF_TILE_BYTES + k * 32),
+                      further(keys, half * L::HALF_TILE_BYTES + k * 32), idesc_s, (half > 0 || k > 0) ? 1u : 0u);
         tcgen05_commit(bar(S_FULL, st));
         tcgen05_commit(bar(K_EMPTY, st));       // the K stage is free once these MMAs have read it
       };
@@ -409,11 +435,11 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
         if (t >= 2) ok = ok && mbar_wait(bar(O_EMPTY, st), ((t >> 1) - 1) & 1, abort_flag, p.error, 7);
         if (!ok) break;
         tcgen05_fence_after();
-        const uint32_t p_addr = base + L::P_OFFSET + st * L::P_BYTES, v_addr = base + L::V_OFFSET + st * L::KV_BYTES;
+        const uint64_t probabilities = further(p_first, st * L::P_BYTES), values = further(v_first, st * L::KV_BYTES);
 #pragma unroll
         for (int k = 0; k < BKEYS / 16; ++k)     // 16 keys a step: two groups of 8 rows of V
-          umma_bf16(tmem_base + L::O_COLUMN + st * D, k_major_descriptor(p_addr + (k >> 2) * L::HALF_TILE_BYTES + (k & 3) * 32),
-                    mn_major_descriptor(v_addr + k * 2048, L::HALF_TILE_BYTES), idesc_o, k > 0 ? 1u : 0u);
+          umma_bf16(tmem_base + L::O_COLUMN + st * D, further(probabilities, (k >> 2) * L::HALF_TILE_BYTES + (k & 3) * 32), further(values, k * 2048),
+                    idesc_o, k > 0 ? 1u : 0u);
         tcgen05_commit(bar(O_FULL, st));
         tcgen05_commit(bar(V_EMPTY, st));
       }
@@ -622,7 +648,8 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
 // The probabilities of a tile go into tensor memory, over the scores they came from, and are the second product's A
 // operand there: no trip through shared memory (sixteen-byte stores into the swizzled layout, a proxy fence, and 16 KB that
 // the tensor core reads back), and the softmax never waits for a product unless a reference moves. The thread that issues the MMAs
-// waits for the product of the tile before last before the next scores are written over the probabilities it reads. Scale
+// waits for the product of the tile before last before the next scores are written over the probabilities it reads; its warp runs the
+// role together and an elected lane issues, and K is asked for two tiles ahead of its scores (8,192 tokens, 12 heads: 261 -> 235 us). Scale
 // and sum take two scores an instruction. The kernel is bound by the chain of a tile's steps (the special-function
 // units work 38 % of the time, the tensor cores 50 %, issue slots are 32 % busy): 8,192 tokens, 12 heads of 128: 277 -> 258 us (800 TFLOP/s), 28 heads:
 // 596 -> 547 us (880); with the probabilities still in shared memory 266 and 568, without the instructions on pairs 268 and 570.
@@ -643,6 +670,7 @@ constexpr int THREADS = 192;        // TMA warp, MMA warp, four softmax warps (o
 constexpr int SOFTMAX_WARPS = 4;
 constexpr int KV_STAGES = 2;
 constexpr float REFERENCE_SLACK = 8.f;   // of launches that fill the GPU; 0 below that (`launch`)
+constexpr float REFERENCE_LIMIT = 1099511627776.f;      // 2^40: a tile's sum beyond it moves the reference
 
 // 64 consecutive float32 columns of this thread's lane of tensor memory.
 __device__ __forceinline__ void tmem_load64(uint32_t address, float* v) {
@@ -656,6 +684,19 @@ __device__ __forceinline__ void tmem_load64(uint32_t address, float* v) {
       : "memory");
 #pragma unroll
   for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
+}
+// 32 columns that are there after `tmem_arrived` of the same variables.
+__device__ __forceinline__ void tmem_ask32(uint32_t address, float (&v)[32]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+               : "r"(address)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_arrived(float (&v)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]), "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]), "+f"(v[29]), "+f"(v[30]), "+f"(v[31])
+               :
+               : "memory");
 }
 // 32 columns written (the whole warp calls it).
 __device__ __forceinline__ void tmem_store32(uint32_t address, const uint32_t* v) {
@@ -738,7 +779,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
   volatile uint32_t* tmem_holder = (volatile uint32_t*)(generic_base + L::BAR_OFFSET + 8 * NUM_BARS);
   volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
   auto bar = [&](int which, int i = 0) { return bars + 8u * (which + i); };
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const bool fits = (base - raw) + (uint32_t)L::USED_BYTES <= (uint32_t)L::SMEM_BYTES;
   if (!fits) {                     // the alignment took more than the slack: nothing is touched
     if (threadIdx.x == 0) atomicCAS(p.error, 0, 20);
@@ -830,90 +871,101 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
         const int page = checked_page(table[checked_table_index(max(min(key / p.page_size, last_page), window_page), p.table_width)]);
         return (page * p.kv_heads + g) * p.page_size + key % p.page_size;
       };
-      int row = mine ? (first_page * p.kv_heads + g) * p.page_size + (kv_begin + lane * box_rows) % p.page_size : 0;
-      int issued = 0;
-      bool ok = true;
-      for (int t = 0; t < n_tiles; ++t) {
+      // One tile of K or of V into its stage. In this order: V of tile t may follow when the product of tile t - 2 has completed, and the
+      // scores of tile t, which free the stage of K for tile t + 2, follow that product. So K is asked for two tiles ahead of its
+      // scores (K and V of a tile together, K waited for V's stage, one tile: the scores then came 820 cycles late).
+      auto load = [&](bool values, int t, int row) {
         const int stage = t % KV_STAGES;
-        const uint32_t round = (uint32_t)(t / KV_STAGES);
-        int next_row = 0;
-        if (mine && t + 1 < n_tiles) next_row = box_row(t + 1);
-        if (t >= KV_STAGES) {
-          if (lane == 0) ok = mbar_wait(bar(K_EMPTY, stage), (round - 1) & 1, abort_flag, p.error, 1);
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-          if (!ok) break;
-        }
-        if (lane == 0) mbar_expect_tx(bar(K_FULL, stage), L::KV_BYTES);
-        __syncwarp();
-        const uint32_t dst = stage * L::KV_BYTES + lane * box_rows * 128;
-        if (mine) {
-#pragma unroll
-          for (int half = 0; half < L::HALVES; ++half)
-            tma_load_2d(base + L::K_OFFSET + dst + half * L::KV_HALF_BYTES, &map_k, bar(K_FULL, stage), half * 64, row);
-        }
-        if (t >= KV_STAGES) {
-          if (lane == 0) ok = mbar_wait(bar(V_EMPTY, stage), (round - 1) & 1, abort_flag, p.error, 10);
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-          if (!ok) break;
-        }
-        if (lane == 0) mbar_expect_tx(bar(V_FULL, stage), L::KV_BYTES);
+        const uint32_t full = bar(values ? V_FULL : K_FULL, stage);
+        if (t >= KV_STAGES && !mbar_wait_warp(bar(values ? V_EMPTY : K_EMPTY, stage), (t / KV_STAGES - 1) & 1, abort_flag, p.error, values ? 10 : 1))
+          return false;
+        if (lane == 0) mbar_expect_tx(full, L::KV_BYTES);
         __syncwarp();
         if (mine) {
+          const uint32_t dst = base + (values ? L::V_OFFSET : L::K_OFFSET) + stage * L::KV_BYTES + lane * box_rows * 128;
 #pragma unroll
           for (int half = 0; half < L::HALVES; ++half)
-            tma_load_2d(base + L::V_OFFSET + dst + half * L::KV_HALF_BYTES, &map_v, bar(V_FULL, stage), half * 64, row);
+            tma_load_2d(dst + half * L::KV_HALF_BYTES, values ? &map_v : &map_k, full, half * 64, row);
         }
-        row = next_row;
-        issued = t + 1;
+        return true;
+      };
+      auto row_of = [&](int t) { return mine && t < n_tiles ? box_row(t) : 0; };
+      int row0 = mine ? (first_page * p.kv_heads + g) * p.page_size + (kv_begin + lane * box_rows) % p.page_size : 0;
+      bool ok = load(false, 0, row0);
+      int row1 = row_of(1), row2 = row_of(2);                   // of tiles t, t + 1, t + 2
+      int keys_issued = 1, values_issued = 0;
+      if (n_tiles > 1) {
+        ok = ok && load(false, 1, row1);
+        keys_issued = 2;
+      }
+      for (int t = 0; t < n_tiles && ok; ++t) {
+        const int row3 = row_of(t + 3);
+        if (!(ok = load(true, t, row0))) break;
+        values_issued = t + 1;
+        if (t + 2 < n_tiles) {
+          if (!(ok = load(false, t + 2, row2))) break;
+          keys_issued = t + 3;
+        }
+        row0 = row1;
+        row1 = row2;
+        row2 = row3;
       }
       if (lane == 0 && *abort_flag) {      // copies that were issued still write into this block's shared memory
-        for (int t = max(0, issued - KV_STAGES); t < issued; ++t) {
+        for (int t = max(0, keys_issued - KV_STAGES); t < keys_issued; ++t)
           for (uint32_t w = 0; w < WAIT_LIMIT && !mbar_try_wait(bar(K_FULL, t % KV_STAGES), (t / KV_STAGES) & 1); ++w) __nanosleep(64);
+        for (int t = max(0, values_issued - KV_STAGES); t < values_issued; ++t)
           for (uint32_t w = 0; w < WAIT_LIMIT && !mbar_try_wait(bar(V_FULL, t % KV_STAGES), (t / KV_STAGES) & 1); ++w) __nanosleep(64);
-        }
         for (uint32_t w = 0; w < WAIT_LIMIT && !mbar_try_wait(bar(Q_FULL), 0); ++w) __nanosleep(64);
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && active) {
+    if (active) {
+      const bool leader = elect_one();
       constexpr uint32_t idesc_s = instruction_descriptor(BQ, BKEYS, false);
       constexpr uint32_t idesc_o = instruction_descriptor(BQ, D, true);
-      bool ok = mbar_wait(bar(Q_FULL), 0, abort_flag, p.error, 2);
+      const uint64_t q_first = k_major_descriptor(base + L::Q_OFFSET), k_first = k_major_descriptor(base + L::K_OFFSET);
+      const uint64_t v_first = mn_major_descriptor(base + L::V_OFFSET, L::KV_HALF_BYTES);
+      bool ok = mbar_wait_warp(bar(Q_FULL), 0, abort_flag, p.error, 2);
       auto issue_scores = [&](int t) {
         const int st = t & 1, stage = t % KV_STAGES;
-        ok = ok && mbar_wait(bar(K_FULL, stage), (t / KV_STAGES) & 1, abort_flag, p.error, 3);
+        ok = ok && mbar_wait_warp(bar(K_FULL, stage), (t / KV_STAGES) & 1, abort_flag, p.error, 3);
         // These scores go where the probabilities of tile t - 2 lay.
-        if (t >= 2) ok = ok && mbar_wait(bar(O_REST), (t - 2) & 1, abort_flag, p.error, 4);
+        if (t >= 2) ok = ok && mbar_wait_warp(bar(O_REST), (t - 2) & 1, abort_flag, p.error, 4);
         if (!ok) return;
         tcgen05_fence_after();
-        const uint32_t q_addr = base + L::Q_OFFSET, k_addr = base + L::K_OFFSET + stage * L::KV_BYTES;
+        const uint64_t keys = further(k_first, stage * L::KV_BYTES);
+        if (leader) {
 #pragma unroll
-        for (int half = 0; half < L::HALVES; ++half)
+          for (int half = 0; half < L::HALVES; ++half)
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_bf16(tmem_base + st * L::S_COLUMNS, k_major_descriptor(q_addr + half * L::Q_HALF_BYTES + k * 32),
-                      k_major_descriptor(k_addr + half * L::KV_HALF_BYTES + k * 32), idesc_s, (half > 0 || k > 0) ? 1u : 0u);
-        tcgen05_commit(bar(S_FULL, st));
-        tcgen05_commit(bar(K_EMPTY, stage));    // the K stage is free once these MMAs have read it
+            for (int k = 0; k < 4; ++k)
+              umma_bf16(tmem_base + st * L::S_COLUMNS, further(q_first, half * L::Q_HALF_BYTES + k * 32),
+                        further(keys, half * L::KV_HALF_BYTES + k * 32), idesc_s, (half > 0 || k > 0) ? 1u : 0u);
+          tcgen05_commit(bar(S_FULL, st));
+          tcgen05_commit(bar(K_EMPTY, stage));    // the K stage is free once these MMAs have read it
+        }
+        __syncwarp();
       };
       if (n_tiles > 0) issue_scores(0);
       for (int t = 0; t < n_tiles && ok; ++t) {
         if (t + 1 < n_tiles) issue_scores(t + 1);
         const int stage = t % KV_STAGES;
-        ok = ok && mbar_wait(bar(V_FULL, stage), (t / KV_STAGES) & 1, abort_flag, p.error, 5);
-        ok = ok && mbar_wait(bar(P_READY, t & 1), (t >> 1) & 1, abort_flag, p.error, 6);
+        ok = ok && mbar_wait_warp(bar(V_FULL, stage), (t / KV_STAGES) & 1, abort_flag, p.error, 5);
+        ok = ok && mbar_wait_warp(bar(P_READY, t & 1), (t >> 1) & 1, abort_flag, p.error, 6);
         if (!ok) break;
         tcgen05_fence_after();
-        const uint32_t v_addr = base + L::V_OFFSET + stage * L::KV_BYTES;
+        const uint64_t values = further(v_first, stage * L::KV_BYTES);
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < BKEYS / 16; ++k)     // 16 keys a step: eight columns of P, two groups of 8 rows of V
-          umma_bf16_tmem_a(tmem_base + L::O_COLUMN, tmem_base + (t & 1) * L::S_COLUMNS + k * 8,
-                           mn_major_descriptor(v_addr + k * 2048, L::KV_HALF_BYTES), idesc_o, (t > 0 || k > 0) ? 1u : 0u);
-        tcgen05_commit(bar(O_REST));             // O is at rest until the next P is ready
-        tcgen05_commit(bar(V_EMPTY, stage));
+          for (int k = 0; k < BKEYS / 16; ++k)     // 16 keys a step: eight columns of P, two groups of 8 rows of V
+            umma_bf16_tmem_a(tmem_base + L::O_COLUMN, tmem_base + (t & 1) * L::S_COLUMNS + k * 8, further(values, k * 2048), idesc_o, (t > 0 || k > 0) ? 1u : 0u);
+          tcgen05_commit(bar(O_REST));             // O is at rest until the next P is ready
+          tcgen05_commit(bar(V_EMPTY, stage));
+          if (t + 1 == n_tiles) tcgen05_commit(bar(O_FULL));       // the output is complete
+        }
+        __syncwarp();
       }
-      if (ok) tcgen05_commit(bar(O_FULL));       // the output is complete
     }
   } else {
     // ------------------------------------------------------------------ softmax, one thread per row
@@ -936,54 +988,23 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
                             (p.window <= 0 || pos0 + rows - 1 - key0 < p.window);
       const int hi = r < rows ? min(my_pos, kv_end - 1) - key0 : -1;          // relative to the tile
       const int lo = (p.window > 0 ? max(first_key, my_pos - p.window + 1) : first_key) - key0;
-      float s[BKEYS];
-      tmem_load64(lane_base + st * L::S_COLUMNS, s);
-      float m4[4] = {-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
-      if (unmasked) {
-#pragma unroll
-        for (int i = 0; i < BKEYS; ++i) m4[i & 3] = fmaxf(m4[i & 3], s[i]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < BKEYS; ++i) m4[i & 3] = fmaxf(m4[i & 3], (i >= lo && i <= hi) ? s[i] : -FLT_MAX);
-      }
-      float tile_max = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-      if (tile_max != -FLT_MAX) tile_max *= p.scale_log2;        // the scale is positive: max(s) scales with it
-      const bool moves = tile_max > reference + p.slack || (reference == -FLT_MAX && tile_max != -FLT_MAX);
-      if (__any_sync(0xffffffffu, moves)) {
-        // Some row of this warp moves its reference: its sum and its row of O are multiplied
-        // by 2^(old - new); the other rows by 1. Reading and writing tensor memory takes the whole warp.
-        const float shrink = !moves ? 1.f : (reference == -FLT_MAX ? 0.f : fast_exp2(reference - tile_max));
-        if (moves) {
-          reference = tile_max;
-          row_sum *= shrink;
-        }
-        if (t >= 1) {
-          ok = mbar_wait(bar(O_REST), (t - 1) & 1, abort_flag, p.error, 7);      // the product of the tile before has completed
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tcgen05_fence_after();
-#pragma unroll
-          for (int c = 0; c < D; c += 32) {
-            float o[32];
-            uint32_t back[32];
-            tmem_load32(lane_base + L::O_COLUMN + c, o);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) back[i] = __float_as_uint(o[i] * shrink);
-            tmem_store32(lane_base + L::O_COLUMN + c, back);
-          }
-        }
-      }
+      uint32_t packed[BKEYS / 2];
+      uint64_t sum01, sum23;
+      uint64_t factor2, offset2;
+      bool has_reference;
       // exp2(s * scale - reference) as one fused multiply-add and one ex2; a row that has seen
       // no key yet has no reference and every probability 0.
-      const float offset = reference == -FLT_MAX ? 0.f : -reference;
-      const float factor = reference == -FLT_MAX ? 0.f : p.scale_log2;
-      const uint64_t factor2 = pack2(factor, factor), offset2 = pack2(offset, offset);
-      uint64_t sum01 = 0, sum23 = 0;                            // (0.f, 0.f)
-      uint32_t packed[BKEYS / 2];
-      auto take = [&](int i, auto visible) {
+      auto begin = [&] {
+        has_reference = reference != -FLT_MAX;
+        const float offset = has_reference ? -reference : 0.f, factor = has_reference ? p.scale_log2 : 0.f;
+        factor2 = pack2(factor, factor);
+        offset2 = pack2(offset, offset);
+        sum01 = sum23 = 0;                                      // (0.f, 0.f)
+      };
+      auto take = [&](const float* s, int i, auto visible) {    // s: the scores of keys i .. i + 3
         float e[4];
-        unpack2(fma2(pack2(s[i], s[i + 1]), factor2, offset2), e[0], e[1]);
-        unpack2(fma2(pack2(s[i + 2], s[i + 3]), factor2, offset2), e[2], e[3]);
+        unpack2(fma2(pack2(s[0], s[1]), factor2, offset2), e[0], e[1]);
+        unpack2(fma2(pack2(s[2], s[3]), factor2, offset2), e[2], e[3]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) e[j] = visible(i + j) ? fast_exp2(e[j]) : 0.f;
         sum01 = add2(sum01, pack2(e[0], e[1]));
@@ -992,18 +1013,82 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
         packed[i / 2] = *(const uint32_t*)&h01;
         packed[i / 2 + 1] = *(const uint32_t*)&h23;
       };
-      if (unmasked) {
+      auto take32 = [&](const float* s, int first) {
+        if (unmasked) {
 #pragma unroll
-        for (int i = 0; i < BKEYS; i += 4) take(i, [](int) { return true; });
-      } else {
+          for (int i = 0; i < 32; i += 4) take(s + i, first + i, [](int) { return true; });
+        } else {
 #pragma unroll
-        for (int i = 0; i < BKEYS; i += 4) take(i, [&](int key) { return key >= lo && key <= hi && factor != 0.f; });
+          for (int i = 0; i < 32; i += 4) take(s + i, first + i, [&](int key) { return key >= lo && key <= hi && has_reference; });
+        }
+      };
+      auto tile_sum = [&] {
+        float sums[4];
+        unpack2(sum01, sums[0], sums[1]);
+        unpack2(sum23, sums[2], sums[3]);
+        return (sums[0] + sums[1]) + (sums[2] + sums[3]);
+      };
+      const uint32_t scores = lane_base + st * L::S_COLUMNS;
+      bool taken = false;
+      if (p.slack > 0.f && !__any_sync(0xffffffffu, reference == -FLT_MAX)) {
+        // Every row has a reference: the probabilities are taken against it without a look at the tile's maximum, the second half
+        // of the scores on its way meanwhile. Should a sum come out beyond REFERENCE_LIMIT (or not a number), the tile is taken again below.
+        float s[32], behind[32];
+        tmem_ask32(scores, s);
+        tmem_arrived(s);
+        tmem_ask32(scores + 32, behind);
+        begin();
+        take32(s, 0);
+        tmem_arrived(behind);
+        take32(behind, 32);
+        const float sum = tile_sum();
+        taken = __all_sync(0xffffffffu, sum <= REFERENCE_LIMIT);
+        if (taken) row_sum += sum;
       }
-      float sums[4];
-      unpack2(sum01, sums[0], sums[1]);
-      unpack2(sum23, sums[2], sums[3]);
-      row_sum += (sums[0] + sums[1]) + (sums[2] + sums[3]);
-      tmem_store32(lane_base + st * L::S_COLUMNS, packed);      // over the scores, which are in registers
+      if (!taken) {
+        float s[BKEYS];
+        tmem_load64(scores, s);
+        float m4[4] = {-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
+        if (unmasked) {
+#pragma unroll
+          for (int i = 0; i < BKEYS; ++i) m4[i & 3] = fmaxf(m4[i & 3], s[i]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < BKEYS; ++i) m4[i & 3] = fmaxf(m4[i & 3], (i >= lo && i <= hi) ? s[i] : -FLT_MAX);
+        }
+        float tile_max = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+        if (tile_max != -FLT_MAX) tile_max *= p.scale_log2;        // the scale is positive: max(s) scales with it
+        const bool moves = tile_max > reference + p.slack || (reference == -FLT_MAX && tile_max != -FLT_MAX);
+        if (__any_sync(0xffffffffu, moves)) {
+          // Some row of this warp moves its reference: its sum and its row of O are multiplied
+          // by 2^(old - new); the other rows by 1. Reading and writing tensor memory takes the whole warp.
+          const float shrink = !moves ? 1.f : (reference == -FLT_MAX ? 0.f : fast_exp2(reference - tile_max));
+          if (moves) {
+            reference = tile_max;
+            row_sum *= shrink;
+          }
+          if (t >= 1) {
+            ok = mbar_wait(bar(O_REST), (t - 1) & 1, abort_flag, p.error, 7);      // the product of the tile before has completed
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tcgen05_fence_after();
+#pragma unroll
+            for (int c = 0; c < D; c += 32) {
+              float o[32];
+              uint32_t back[32];
+              tmem_load32(lane_base + L::O_COLUMN + c, o);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) back[i] = __float_as_uint(o[i] * shrink);
+              tmem_store32(lane_base + L::O_COLUMN + c, back);
+            }
+          }
+        }
+        begin();
+        take32(s, 0);
+        take32(s + 32, 32);
+        row_sum += tile_sum();
+      }
+      tmem_store32(scores, packed);      // over the scores, which are in registers
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(P_READY, st));

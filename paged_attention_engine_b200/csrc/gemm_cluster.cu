@@ -346,6 +346,8 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
     // ---------------------------------------------------------------- MMA issuer
     if (lane == 0) {
       const uint32_t idesc = instruction_descriptor(BM, p.columns);
+      // A stage's descriptors are the first stage's plus an offset in the address field (units of 16 bytes, below 256 KB: no carry).
+      const uint64_t w_first = smem_descriptor(base), x_first = smem_descriptor(base + a_bytes);
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -353,10 +355,10 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
         ok = mbar_wait(full_bar(s), phase, abort_flag, p.error, 2);
         if (!ok) break;
         tcgen05_fence_after();
-        const uint32_t a = base + s * stage_bytes, b = a + a_bytes;
+        const uint64_t offset = (uint64_t)(uint32_t)(s * (stage_bytes >> 4)), a = w_first + offset, b = x_first + offset;
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; ++k)
-          umma_bf16(tmem_base, smem_descriptor(a + k * UMMA_K * 2), smem_descriptor(b + k * UMMA_K * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+          umma_bf16(tmem_base, a + (uint64_t)(k * UMMA_K * 2 >> 4), b + (uint64_t)(k * UMMA_K * 2 >> 4), idesc, (i > 0 || k > 0) ? 1u : 0u);
         tcgen05_commit(empty_bar(s));
         if (++s == stages) {
           s = 0;
