@@ -124,6 +124,53 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
+// A box of keys or values: coordinates in a pool seen as [pages][kv heads][D / 64][rows of a page][64].
+__device__ __forceinline__ void tma_load_pages(uint32_t dst, const CUtensorMap* map, uint32_t bar, int row, int half, int head, int page) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(row), "r"(half), "r"(head), "r"(page)
+      : "memory");
+}
+// How keys and values come into shared memory. What the TMA unit takes is time per box, not bytes: with a box a page and half of
+// a row, 16 boxes of 2 KB for 64 keys of a page size of 16, it set the pace of the paired kernel (8,192 tokens, 12 heads of 128: 235 us against
+// 177 with pages of 64; now 173 with either, 1,190 TFLOP/s, and a tenth more where no two pages follow one another). So the pages of a tile that follow one another in the pool, as a prompt's pages mostly do, come as ONE box per half
+// of the keys and one of the values; others come a box each (and half, of the keys). The values lie [page][half][row][64] (the
+// halves' distance is the descriptor's leading byte offset), the keys [half][page][row][64].
+struct PageMaps {
+  CUtensorMap key, value;                // a page (or the rows of it that a tile covers)
+  CUtensorMap key_run, value_run;        // the pages of a tile
+};
+// Tile of `rows` keys, `rows_a_box` of them a box, by a converged warp: lane i brings the box at `row` of `page`, or lane 0 all of them.
+template <int D>
+__device__ __forceinline__ void load_pages(const PageMaps& maps, bool values, uint32_t dst, uint32_t full, int rows, int rows_a_box, int lane, int head,
+                                           int page, int row) {
+  constexpr int HALVES = D / 64;
+  const int boxes = rows / rows_a_box;
+  const int first = __shfl_sync(0xffffffffu, page, 0);
+  if (boxes > 1 && __all_sync(0xffffffffu, lane >= boxes || page == first + lane)) {
+    if (lane == 0) {
+      if (values) {
+        tma_load_pages(dst, &maps.value_run, full, 0, 0, head, page);
+      } else {
+#pragma unroll
+        for (int half = 0; half < HALVES; ++half) tma_load_pages(dst + half * rows * 128, &maps.key_run, full, 0, half, head, page);
+      }
+    }
+  } else if (lane < boxes) {
+    if (values) {
+      tma_load_pages(dst + lane * rows_a_box * 128 * HALVES, &maps.value, full, row, 0, head, page);
+    } else {
+#pragma unroll
+      for (int half = 0; half < HALVES; ++half) tma_load_pages(dst + half * rows * 128 + lane * rows_a_box * 128, &maps.key, full, row, half, head, page);
+    }
+  }
+}
+// Where the 16 keys of step k of the second product lie among a tile's values (a box has 16, 32, 64 or 128 rows).
+template <int D>
+__device__ __forceinline__ uint32_t value_step(int k, int rows_a_box) {
+  const int row = k * 16;
+  return (uint32_t)(row + (D / 64 - 1) * (row & -rows_a_box)) * 128;
+}
 __device__ __forceinline__ void tmem_alloc(uint32_t holder, uint32_t columns) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(holder), "r"(columns) : "memory");
 }
@@ -250,14 +297,13 @@ enum Bar : int { Q_FULL = 0, K_FULL = 1, V_FULL = 3, K_EMPTY = 5, V_EMPTY = 7, S
 
 template <int D, bool SPLIT>
 __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q,
-                                                                  const __grid_constant__ CUtensorMap map_k,
-                                                                  const __grid_constant__ CUtensorMap map_v, const Params p) {
+                                                                  const __grid_constant__ PageMaps maps, const Params p) {
   using L = Layout<D>;
   dependent_launch_trigger();
   if (threadIdx.x == 0) {         // the descriptors do not depend on the kernel before: fetch them early
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.key_run) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.value_run) : "memory");
   }
   extern __shared__ uint8_t raw_smem[];
   const uint32_t raw = smem_u32(raw_smem);
@@ -267,7 +313,7 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
   volatile uint32_t* tmem_holder = (volatile uint32_t*)(generic_base + L::BAR_OFFSET + 8 * NUM_BARS);
   volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
   auto bar = [&](int which, int i = 0) { return bars + 8u * (which + i); };
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     mbar_init(bar(Q_FULL), 1);
@@ -352,96 +398,108 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
                       first_token + tile * BQ);
       }
       const int* table = p.block_table + (size_t)b * p.table_width;
-      const int pages_per_tile = BKEYS / p.page_size;
-      const int page_rows_bytes = p.page_size * 128;
-      const bool mine = lane < pages_per_tile;
+      const bool mine = lane < BKEYS / p.page_size;
       // A page past the last visible key may not exist: its rows are masked, so any page of
       // the request will do; the last visible one is taken.
-      int page = first_page;
-      int issued = 0;
-      bool ok = true;
-      for (int t = 0; t < n_tiles; ++t) {
+      auto page_of = [&](int t) {
+        return mine && t < n_tiles ? checked_page(table[checked_table_index(min((kv_begin + t * BKEYS) / p.page_size + lane, last_page), p.table_width)]) : 0;
+      };
+      // Two tiles of K ahead of V, whose stage is free later: the scores of tile t free the stage of K for tile t + 2 while the softmax of
+      // tile t - 2 or t - 1 runs, and V of tile t follows the product of tile t - 2.
+      auto load = [&](bool values, int t, int page) {
         const int st = t & 1;
-        int next_page = 0;
-        if (mine && t + 1 < n_tiles)
-          next_page = checked_page(table[checked_table_index(min((kv_begin + (t + 1) * BKEYS) / p.page_size + lane, last_page), p.table_width)]);
-        if (t >= 2) {
-          if (lane == 0) ok = mbar_wait(bar(K_EMPTY, st), ((t >> 1) - 1) & 1, abort_flag, p.error, 1);
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-          if (!ok) break;
-        }
-        if (lane == 0) mbar_expect_tx(bar(K_FULL, st), L::KV_BYTES);
+        const uint32_t full = bar(values ? V_FULL : K_FULL, st);
+        if (t >= 2 && !mbar_wait_warp(bar(values ? V_EMPTY : K_EMPTY, st), ((t >> 1) - 1) & 1, abort_flag, p.error, values ? 10 : 1)) return false;
+        if (lane == 0) mbar_expect_tx(full, L::KV_BYTES);
         __syncwarp();
-        const int row = (page * p.kv_heads + g) * p.page_size;
-        const uint32_t dst = st * L::KV_BYTES + lane * page_rows_bytes;
-        if (mine) {
-#pragma unroll
-          for (int half = 0; half < L::HALVES; ++half)
-            tma_load_2d(base + L::K_OFFSET + dst + half * L::HALF_TILE_BYTES, &map_k, bar(K_FULL, st), half * 64, row);
+        load_pages<D>(maps, values, base + (values ? L::V_OFFSET : L::K_OFFSET) + st * L::KV_BYTES, full, BKEYS, p.page_size, lane, g, page, 0);
+        return true;
+      };
+      int page0 = first_page;
+      bool ok = true;
+      int keys_issued = 0, values_issued = 0;
+      if (n_tiles > 0) {
+        ok = load(false, 0, page0);
+        keys_issued = 1;
+      }
+      int page1 = page_of(1), page2 = page_of(2);               // of tiles t, t + 1, t + 2
+      if (n_tiles > 1 && ok) {
+        ok = load(false, 1, page1);
+        keys_issued = 2;
+      }
+      for (int t = 0; t < n_tiles && ok; ++t) {
+        const int page3 = page_of(t + 3);
+        if (t == 0) {                                           // nothing has to be waited for: V before K of a later tile
+          load(true, 0, page0);
+          values_issued = 1;
         }
-        if (t >= 2) {
-          if (lane == 0) ok = mbar_wait(bar(V_EMPTY, st), ((t >> 1) - 1) & 1, abort_flag, p.error, 10);
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-          if (!ok) break;
+        if (t + 2 < n_tiles) {
+          if (!(ok = load(false, t + 2, page2))) break;
+          keys_issued = t + 3;
         }
-        if (lane == 0) mbar_expect_tx(bar(V_FULL, st), L::KV_BYTES);
-        __syncwarp();
-        if (mine) {
-#pragma unroll
-          for (int half = 0; half < L::HALVES; ++half)
-            tma_load_2d(base + L::V_OFFSET + dst + half * L::HALF_TILE_BYTES, &map_v, bar(V_FULL, st), half * 64, row);
+        if (t > 0) {
+          if (!(ok = load(true, t, page0))) break;
+          values_issued = t + 1;
         }
-        page = next_page;
-        issued = t + 1;
+        page0 = page1;
+        page1 = page2;
+        page2 = page3;
       }
       if (lane == 0 && *abort_flag) {
-        for (int t = max(0, issued - 2); t < issued; ++t) {
+        for (int t = max(0, keys_issued - 2); t < keys_issued; ++t)
           for (uint32_t w = 0; w < WAIT_LIMIT && !mbar_try_wait(bar(K_FULL, t & 1), (t >> 1) & 1); ++w) __nanosleep(64);
+        for (int t = max(0, values_issued - 2); t < values_issued; ++t)
           for (uint32_t w = 0; w < WAIT_LIMIT && !mbar_try_wait(bar(V_FULL, t & 1), (t >> 1) & 1); ++w) __nanosleep(64);
-        }
         for (uint32_t w = 0; w < WAIT_LIMIT && !mbar_try_wait(bar(Q_FULL), 0); ++w) __nanosleep(64);
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && working) {
+    if (working) {
+      const bool leader = elect_one();
       constexpr uint32_t idesc_s = instruction_descriptor(BQ, BKEYS, false);
       constexpr uint32_t idesc_o = instruction_descriptor(BQ, D, true);
       const uint64_t q_first = k_major_descriptor(base + L::Q_OFFSET), k_first = k_major_descriptor(base + L::K_OFFSET);
-      const uint64_t p_first = k_major_descriptor(base + L::P_OFFSET), v_first = mn_major_descriptor(base + L::V_OFFSET, L::HALF_TILE_BYTES);
-      bool ok = mbar_wait(bar(Q_FULL), 0, abort_flag, p.error, 2);
+      const uint64_t p_first = k_major_descriptor(base + L::P_OFFSET), v_first = mn_major_descriptor(base + L::V_OFFSET, p.page_size * 128);
+      bool ok = mbar_wait_warp(bar(Q_FULL), 0, abort_flag, p.error, 2);
       auto issue_scores = [&](int t) {
         const int st = t & 1;
-        ok = ok && mbar_wait(bar(K_FULL, st), (t >> 1) & 1, abort_flag, p.error, 3);
-        if (t >= 2) ok = ok && mbar_wait(bar(S_EMPTY, st), ((t >> 1) - 1) & 1, abort_flag, p.error, 4);
+        ok = ok && mbar_wait_warp(bar(K_FULL, st), (t >> 1) & 1, abort_flag, p.error, 3);
+        if (t >= 2) ok = ok && mbar_wait_warp(bar(S_EMPTY, st), ((t >> 1) - 1) & 1, abort_flag, p.error, 4);
         if (!ok) return;
         tcgen05_fence_after();
         const uint64_t keys = further(k_first, st * L::KV_BYTES);
+        if (leader) {
 #pragma unroll
-        for (int half = 0; half < L::HALVES; ++half)
+          for (int half = 0; half < L::HALVES; ++half)
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_bf16(tmem_base + st * L::S_COLUMNS, further(q_first, half * L::HALF_TILE_BYTES + k * 32),
-                      further(keys, half * L::HALF_TILE_BYTES + k * 32), idesc_s, (half > 0 || k > 0) ? 1u : 0u);
-        tcgen05_commit(bar(S_FULL, st));
-        tcgen05_commit(bar(K_EMPTY, st));       // the K stage is free once these MMAs have read it
+            for (int k = 0; k < 4; ++k)
+              umma_bf16(tmem_base + st * L::S_COLUMNS, further(q_first, half * L::HALF_TILE_BYTES + k * 32),
+                        further(keys, half * L::HALF_TILE_BYTES + k * 32), idesc_s, (half > 0 || k > 0) ? 1u : 0u);
+          tcgen05_commit(bar(S_FULL, st));
+          tcgen05_commit(bar(K_EMPTY, st));       // the K stage is free once these MMAs have read it
+        }
+        __syncwarp();
       };
       if (n_tiles > 0) issue_scores(0);
       for (int t = 0; t < n_tiles && ok; ++t) {
         if (t + 1 < n_tiles) issue_scores(t + 1);
         const int st = t & 1;
-        ok = ok && mbar_wait(bar(V_FULL, st), (t >> 1) & 1, abort_flag, p.error, 5);
-        ok = ok && mbar_wait(bar(P_READY, st), (t >> 1) & 1, abort_flag, p.error, 6);
-        if (t >= 2) ok = ok && mbar_wait(bar(O_EMPTY, st), ((t >> 1) - 1) & 1, abort_flag, p.error, 7);
+        ok = ok && mbar_wait_warp(bar(V_FULL, st), (t >> 1) & 1, abort_flag, p.error, 5);
+        ok = ok && mbar_wait_warp(bar(P_READY, st), (t >> 1) & 1, abort_flag, p.error, 6);
+        if (t >= 2) ok = ok && mbar_wait_warp(bar(O_EMPTY, st), ((t >> 1) - 1) & 1, abort_flag, p.error, 7);
         if (!ok) break;
         tcgen05_fence_after();
         const uint64_t probabilities = further(p_first, st * L::P_BYTES), values = further(v_first, st * L::KV_BYTES);
+        if (leader) {
 #pragma unroll
         for (int k = 0; k < BKEYS / 16; ++k)     // 16 keys a step: two groups of 8 rows of V
-          umma_bf16(tmem_base + L::O_COLUMN + st * D, further(probabilities, (k >> 2) * L::HALF_TILE_BYTES + (k & 3) * 32), further(values, k * 2048),
+          umma_bf16(tmem_base + L::O_COLUMN + st * D, further(probabilities, (k >> 2) * L::HALF_TILE_BYTES + (k & 3) * 32), further(values, value_step<D>(k, p.page_size)),
                     idesc_o, k > 0 ? 1u : 0u);
         tcgen05_commit(bar(O_FULL, st));
         tcgen05_commit(bar(V_EMPTY, st));
+        }
+        __syncwarp();
       }
     }
   } else {
@@ -762,14 +820,13 @@ enum Bar : int {
 
 template <int D>
 __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(const __grid_constant__ CUtensorMap map_q,
-                                                                     const __grid_constant__ CUtensorMap map_k,
-                                                                     const __grid_constant__ CUtensorMap map_v, const Params p) {
+                                                                     const __grid_constant__ PageMaps maps, const Params p) {
   using L = Layout<D>;
   dependent_launch_trigger();
   if (threadIdx.x == 0) {         // the descriptors do not depend on the kernel before: fetch them early
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.key_run) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.value_run) : "memory");
   }
   extern __shared__ __align__(1024) uint8_t raw_smem[];
   const uint32_t raw = smem_u32(raw_smem);
@@ -866,49 +923,44 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
       const bool mine = lane < boxes;
       // A page past the last visible key may not exist: its rows are masked, so any page of
       // the request will do; the last visible one is taken.
-      auto box_row = [&](int t) {
+      const int page_shift = 31 - __clz(p.page_size);          // page sizes are powers of two
+      auto page_of = [&](int t) {
         const int key = kv_begin + t * BKEYS + lane * box_rows;
-        const int page = checked_page(table[checked_table_index(max(min(key / p.page_size, last_page), window_page), p.table_width)]);
-        return (page * p.kv_heads + g) * p.page_size + key % p.page_size;
+        return mine && t < n_tiles ? checked_page(table[checked_table_index(max(min(key >> page_shift, last_page), window_page), p.table_width)]) : 0;
       };
       // One tile of K or of V into its stage. In this order: V of tile t may follow when the product of tile t - 2 has completed, and the
       // scores of tile t, which free the stage of K for tile t + 2, follow that product. So K is asked for two tiles ahead of its
       // scores (K and V of a tile together, K waited for V's stage, one tile: the scores then came 820 cycles late).
-      auto load = [&](bool values, int t, int row) {
+      auto load = [&](bool values, int t, int page) {
         const int stage = t % KV_STAGES;
         const uint32_t full = bar(values ? V_FULL : K_FULL, stage);
         if (t >= KV_STAGES && !mbar_wait_warp(bar(values ? V_EMPTY : K_EMPTY, stage), (t / KV_STAGES - 1) & 1, abort_flag, p.error, values ? 10 : 1))
           return false;
         if (lane == 0) mbar_expect_tx(full, L::KV_BYTES);
         __syncwarp();
-        if (mine) {
-          const uint32_t dst = base + (values ? L::V_OFFSET : L::K_OFFSET) + stage * L::KV_BYTES + lane * box_rows * 128;
-#pragma unroll
-          for (int half = 0; half < L::HALVES; ++half)
-            tma_load_2d(dst + half * L::KV_HALF_BYTES, values ? &map_v : &map_k, full, half * 64, row);
-        }
+        load_pages<D>(maps, values, base + (values ? L::V_OFFSET : L::K_OFFSET) + stage * L::KV_BYTES, full, BKEYS, box_rows, lane, g, page,
+                      (kv_begin + t * BKEYS + lane * box_rows) & (p.page_size - 1));
         return true;
       };
-      auto row_of = [&](int t) { return mine && t < n_tiles ? box_row(t) : 0; };
-      int row0 = mine ? (first_page * p.kv_heads + g) * p.page_size + (kv_begin + lane * box_rows) % p.page_size : 0;
-      bool ok = load(false, 0, row0);
-      int row1 = row_of(1), row2 = row_of(2);                   // of tiles t, t + 1, t + 2
+      int page0 = first_page;
+      bool ok = load(false, 0, page0);
+      int page1 = page_of(1), page2 = page_of(2);               // of tiles t, t + 1, t + 2
       int keys_issued = 1, values_issued = 0;
       if (n_tiles > 1) {
-        ok = ok && load(false, 1, row1);
+        ok = ok && load(false, 1, page1);
         keys_issued = 2;
       }
       for (int t = 0; t < n_tiles && ok; ++t) {
-        const int row3 = row_of(t + 3);
-        if (!(ok = load(true, t, row0))) break;
+        const int page3 = page_of(t + 3);
+        if (!(ok = load(true, t, page0))) break;
         values_issued = t + 1;
         if (t + 2 < n_tiles) {
-          if (!(ok = load(false, t + 2, row2))) break;
+          if (!(ok = load(false, t + 2, page2))) break;
           keys_issued = t + 3;
         }
-        row0 = row1;
-        row1 = row2;
-        row2 = row3;
+        page0 = page1;
+        page1 = page2;
+        page2 = page3;
       }
       if (lane == 0 && *abort_flag) {      // copies that were issued still write into this block's shared memory
         for (int t = max(0, keys_issued - KV_STAGES); t < keys_issued; ++t)
@@ -925,7 +977,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
       constexpr uint32_t idesc_s = instruction_descriptor(BQ, BKEYS, false);
       constexpr uint32_t idesc_o = instruction_descriptor(BQ, D, true);
       const uint64_t q_first = k_major_descriptor(base + L::Q_OFFSET), k_first = k_major_descriptor(base + L::K_OFFSET);
-      const uint64_t v_first = mn_major_descriptor(base + L::V_OFFSET, L::KV_HALF_BYTES);
+      const uint64_t v_first = mn_major_descriptor(base + L::V_OFFSET, box_rows * 128);
       bool ok = mbar_wait_warp(bar(Q_FULL), 0, abort_flag, p.error, 2);
       auto issue_scores = [&](int t) {
         const int st = t & 1, stage = t % KV_STAGES;
@@ -959,7 +1011,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
         if (leader) {
 #pragma unroll
           for (int k = 0; k < BKEYS / 16; ++k)     // 16 keys a step: eight columns of P, two groups of 8 rows of V
-            umma_bf16_tmem_a(tmem_base + L::O_COLUMN, tmem_base + (t & 1) * L::S_COLUMNS + k * 8, further(values, k * 2048), idesc_o, (t > 0 || k > 0) ? 1u : 0u);
+            umma_bf16_tmem_a(tmem_base + L::O_COLUMN, tmem_base + (t & 1) * L::S_COLUMNS + k * 8, further(values, value_step<D>(k, box_rows)), idesc_o, (t > 0 || k > 0) ? 1u : 0u);
           tcgen05_commit(bar(O_REST));             // O is at rest until the next P is ready
           tcgen05_commit(bar(V_EMPTY, stage));
           if (t + 1 == n_tiles) tcgen05_commit(bar(O_FULL));       // the output is complete
@@ -1147,6 +1199,59 @@ EncodeTiled encode_tiled() {
   return fn;
 }
 
+// A pool [pages, kv_heads, page_size, d] as boxes of `rows` rows of `halves` halves of `run` pages, 128-byte swizzle.
+int page_map(CUtensorMap* out, const void* ptr, long long pages, int kv_heads, int page_size, int d, int rows, int halves, int run) {
+  EncodeTiled encode = encode_tiled();
+  if (encode == nullptr) return fail(101, "paged_attention_tcgen05: the driver does not export cuTensorMapEncodeTiled");
+  const cuuint64_t dims[5] = {64, (cuuint64_t)page_size, (cuuint64_t)(d / 64), (cuuint64_t)kv_heads, (cuuint64_t)pages};
+  const cuuint64_t strides[4] = {(cuuint64_t)d * 2, 128, (cuuint64_t)page_size * d * 2, (cuuint64_t)kv_heads * page_size * d * 2};
+  const cuuint32_t box[5] = {64, (cuuint32_t)rows, (cuuint32_t)halves, 1, (cuuint32_t)run};
+  const cuuint32_t element_strides[5] = {1, 1, 1, 1, 1};
+  CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(ptr), dims, strides, box, element_strides,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(102, "paged_attention_tcgen05: cuTensorMapEncodeTiled failed with %d for pages of %d", (int)r, page_size);
+  return 0;
+}
+// What brings tiles of `tile_keys` keys. A pool's maps say where it lies and how it is laid out, nothing of what it holds; they are kept
+// (encoding four takes a microsecond and more of every launch).
+struct PageMapsKey {
+  const void *keys, *values;
+  long long pages;
+  int kv_heads, page_size, d, tile_keys;
+  bool operator==(const PageMapsKey& o) const {
+    return keys == o.keys && values == o.values && pages == o.pages && kv_heads == o.kv_heads && page_size == o.page_size && d == o.d && tile_keys == o.tile_keys;
+  }
+};
+struct PageMapsKeyHash {
+  size_t operator()(const PageMapsKey& key) const {
+    size_t h = (size_t)key.keys;
+    h = h * 1000003u ^ (size_t)key.values;
+    h = h * 1000003u ^ (size_t)key.pages;
+    h = h * 1000003u ^ (size_t)(key.kv_heads * 4096 + key.page_size);
+    return h * 1000003u ^ (size_t)(key.d * 4096 + key.tile_keys);
+  }
+};
+int page_maps(PageMaps* out, const void* keys, const void* values, long long pages, int kv_heads, int page_size, int d, int tile_keys) {
+  static std::mutex mutex;
+  static std::unordered_map<PageMapsKey, PageMaps, PageMapsKeyHash> cache;
+  const PageMapsKey key{keys, values, pages, kv_heads, page_size, d, tile_keys};
+  std::lock_guard<std::mutex> guard(mutex);
+  auto found = cache.find(key);
+  if (found != cache.end()) {
+    *out = found->second;
+    return 0;
+  }
+  const int rows = page_size < tile_keys ? page_size : tile_keys, run = tile_keys / rows, halves = d / 64;
+  if (int err = page_map(&out->key, keys, pages, kv_heads, page_size, d, rows, 1, 1)) return err;
+  if (int err = page_map(&out->value, values, pages, kv_heads, page_size, d, rows, halves, 1)) return err;
+  if (int err = page_map(&out->key_run, keys, pages, kv_heads, page_size, d, rows, 1, run)) return err;
+  if (int err = page_map(&out->value_run, values, pages, kv_heads, page_size, d, rows, halves, run)) return err;
+  if (cache.size() > 1024) cache.clear();
+  cache.emplace(key, *out);
+  return 0;
+}
+
 // [rows, cols] bfloat16 row-major as boxes of 64 columns x box_rows rows, 128-byte swizzle.
 int tensor_map(CUtensorMap* out, const void* ptr, long long rows, int cols, int box_rows) {
   EncodeTiled encode = encode_tiled();
@@ -1176,8 +1281,8 @@ int sm_count() {
 // a wide block 5.5 + 1.95 per tile of 128 keys; a wide block that follows another 4 more; a round of paired blocks 6.5 + 3.0
 // per tile. With more blocks than SMs and fewer than twice as many, the wide launch's second blocks follow its shortest
 // first ones, so it lasts as long as its longest block or two of middling length: the two estimates are compared (6 requests
-// of 300 tokens, 12 heads: wide 22.0, paired 15.6; 4 portions of 509 tokens after 512: 38.2 and 32.5; but one prompt of 2,000
-// tokens: 36.5 and more than 46.9). From twice as many on it is the paired kernel (8,192 tokens 346 and 258). With one of its
+// of 300 tokens, 12 heads: wide 21.3, paired 15.8; 4 portions of 509 tokens after 512: 34.3 and 29.7; but one prompt of 2,048
+// tokens: 31.9 and 43.2). From twice as many on it is the paired kernel (4,096 tokens 87.5 and 63.0). With one of its
 // tiles, and up to three while at most a third of the SMs are busy, the paired kernel's shorter set-up shows (64 tokens 8.3 and 6.3, 100 tokens
 // 8.9 and 8.5, 192 tokens 10.3 and 9.1; but 200 tokens of 28 heads 10.2 and 10.9, 300 of 12 11.3 and 11.7).
 bool takes_paired(long long blocks, long long blocks_per_tile, int longest, int longest_keys) {
@@ -1214,13 +1319,10 @@ int launch(Params p, const void* qkv, const void* keys, const void* values, int 
   if (form == 0 && !use_paired) {
     while (ranks < 8 && blocks * (ranks * 2) <= sm_count() && longest >= (int)(ranks * 2) * 2) ranks *= 2;
   }
-  CUtensorMap map_q, map_k, map_v;
+  CUtensorMap map_q;
   if (int err = tensor_map(&map_q, qkv, tokens, (p.heads + 2 * p.kv_heads) * D, BQ)) return err;
-  const long long cache_rows = pages * p.kv_heads * p.page_size;
-  const int tile_keys = use_paired ? paired::BKEYS : BKEYS;
-  const int box_rows = p.page_size < tile_keys ? p.page_size : tile_keys;
-  if (int err = tensor_map(&map_k, keys, cache_rows, D, box_rows)) return err;
-  if (int err = tensor_map(&map_v, values, cache_rows, D, box_rows)) return err;
+  PageMaps maps;
+  if (int err = page_maps(&maps, keys, values, pages, p.kv_heads, p.page_size, D, use_paired ? paired::BKEYS : BKEYS)) return err;
   static DevicesSet raised_one, raised_cluster, raised_paired;
   if (int err = raise_shared_memory(raised_one, prefill_tcgen05_kernel<D, false>, Layout<D>::SMEM_BYTES, "paged_attention_tcgen05")) return err;
   if (int err = raise_shared_memory(raised_cluster, prefill_tcgen05_kernel<D, true>, Layout<D>::SMEM_BYTES, "paged_attention_tcgen05")) return err;
@@ -1228,14 +1330,14 @@ int launch(Params p, const void* qkv, const void* keys, const void* values, int 
     return err;
   if (chosen != nullptr) *chosen = use_paired ? 0 : (int)ranks;
   if (use_paired) {
-    launch_kernel(paired::prefill_tcgen05_paired_kernel<D>, grid, paired::THREADS, paired::Layout<D>::SMEM_BYTES, stream, map_q, map_k,
-                  map_v, p);
+    launch_kernel(paired::prefill_tcgen05_paired_kernel<D>, grid, paired::THREADS, paired::Layout<D>::SMEM_BYTES, stream, map_q, maps,
+                  p);
   } else {
     grid.x *= ranks;
     if (ranks > 1)
-      launch_kernel_cluster(prefill_tcgen05_kernel<D, true>, grid, dim3(THREADS), Layout<D>::SMEM_BYTES, stream, ranks, map_q, map_k, map_v, p);
+      launch_kernel_cluster(prefill_tcgen05_kernel<D, true>, grid, dim3(THREADS), Layout<D>::SMEM_BYTES, stream, ranks, map_q, maps, p);
     else
-      launch_kernel(prefill_tcgen05_kernel<D, false>, grid, THREADS, Layout<D>::SMEM_BYTES, stream, map_q, map_k, map_v, p);
+      launch_kernel(prefill_tcgen05_kernel<D, false>, grid, THREADS, Layout<D>::SMEM_BYTES, stream, map_q, maps, p);
   }
   return check_launch("paged_attention_tcgen05");
 }

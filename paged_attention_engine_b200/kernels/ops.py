@@ -329,6 +329,8 @@ class PendingPostNorm:
 
 def materialized(x):
     """The tensor that `x` stands for (x itself unless it is one of the Pending classes above)."""
+    if type(x) is torch.Tensor:
+        return x
     if isinstance(x, (PendingPostNorm, PendingBranches)):
         if x.value is None:
             _post_norm_step(x)
@@ -420,7 +422,7 @@ def rms_norm(x, weight: torch.Tensor, eps: float) -> torch.Tensor:
         return ScaledNorm(x.value, weight, eps, scaled, squares)
     x = materialized(x)
     _need(x, "rms_norm: x")
-    if x.dim() == 2 and _few_tokens(x, x.shape[-1], normed=True):
+    if x.dim() == 2 and x.shape[0] <= FEW_TOKENS_MAX and _few_tokens(x, x.shape[-1], normed=True):
         return PendingNorm(x, weight, eps)       # the product that follows applies it
     return _rms_norm_now(x, weight, eps)
 
@@ -458,8 +460,8 @@ FEW_TOKENS_MAX_GATE_UP = 24
 def _few_tokens(x: torch.Tensor, k: int, normed: bool = False, kind: int = GATE_UP_KIND, n: int = 16) -> bool:
     """Whether a product of `kind` over x [tokens, K] with `n` weight rows runs as a few-token
     kernel; `normed`: with the RMSNorm of x folded in (the normed operand has to fit shared memory)."""
-    if not (use_few_token_products and use_tensor_cores and x.dtype == torch.bfloat16 and x.dim() == 2
-            and 0 < x.shape[0] <= FEW_TOKENS_MAX and x.data_ptr() % 16 == 0):
+    if not (0 < x.shape[0] <= FEW_TOKENS_MAX and use_few_token_products and use_tensor_cores and x.dtype == torch.bfloat16 and x.dim() == 2
+            and x.data_ptr() % 16 == 0):
         return False
     if k < 64 or k % 64:        # not for these kernels: their library is not even built for such a model
         return False
@@ -633,8 +635,8 @@ def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str 
     wrote needs another launch, or a synchronisation, in between. Larger products read nothing before that kernel has completed."""
     if activation not in ACTIVATIONS:
         raise KernelError(f"linear: activation '{activation}' (known: gelu_erf, gelu_tanh, relu2)")
-    if (activation is None and bias is None and out_dtype in (None, torch.bfloat16) and weight.dtype == torch.bfloat16 and weight.dim() == 2
-            and weight.data_ptr() % 16 == 0 and weight.shape[0] <= 65536):
+    if (x.shape[0] <= CLUSTER_MAX_TOKENS and activation is None and bias is None and out_dtype in (None, torch.bfloat16)
+            and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.data_ptr() % 16 == 0 and weight.shape[0] <= 65536):
         if residual is not None and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0]):
             operand, residual = _cluster_operand(x), materialized(residual)
             if operand is not None and residual.dtype == torch.bfloat16 and residual.data_ptr() % 16 == 0:
@@ -814,7 +816,7 @@ def qkv_projection(x, weight, bias, table, slots, keys, values, num_heads, num_k
     n = weight.shape[0]
     # A plain operand of more than 64 tokens keeps the bits of `linear` followed by the rotation (a prompt's first layer only: in
     # the others the product before has prepared the norm).
-    if ((m <= SWAPPED_MAX_TOKENS or isinstance(x, ScaledNorm)) and _cluster_takes(m, n, k, weight, k) and n == (num_heads + 2 * num_kv_heads) * head_dim
+    if (m <= CLUSTER_MAX_TOKENS and (m <= SWAPPED_MAX_TOKENS or isinstance(x, ScaledNorm)) and _cluster_takes(m, n, k, weight, k) and n == (num_heads + 2 * num_kv_heads) * head_dim
             and (slots is None or (keys.dtype == torch.bfloat16 and values.dtype == torch.bfloat16))):
         operand = _cluster_operand(x)
         lib = _lib("gemm_cluster")
@@ -1093,7 +1095,7 @@ def linear_swiglu(x, weight, gate: str = "silu") -> torch.Tensor:
     tokens the activation runs in the product's epilogue; with few, in the kernel that sums the
     splits; otherwise as a kernel of its own. Gate and up are rounded to the engine dtype first in
     every one of them, so all give the same bits."""
-    if (x.dtype == torch.bfloat16 and weight.shape[0] % 32 == 0 and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[1])
+    if (x.shape[0] <= CLUSTER_MAX_TOKENS and x.dtype == torch.bfloat16 and weight.shape[0] % 32 == 0 and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[1])
             and not _uneven_gate(x.shape[0], weight.shape[0], x.device)):
         operand = _cluster_operand(x)
         if operand is not None:
