@@ -23,8 +23,8 @@
 // two fit an SM and the next product's blocks fill their rings while this one's finish.
 //
 // What bounds it: the chain, then memory. The four products with their norms in a row, before and now: 1,536-wide layers (93.5 MB of
-// weights, 14.3 us at the copy rate) 44.2 -> 34.0 us at 40 tokens, 46.1 -> 36.0 at 64; 3,584-wide (466 MB, 71 us) 106.7 -> 91.8 at
-// 64. Of q|k|v's 6 us at 40 tokens 0.8 pass before the kernel before releases this one, 1.0 until its tokens' first stage is there, 1.0 in
+// weights, 14.3 us at the copy rate) 43.0 -> 30.4 us at 40 tokens, 44.4 -> 32.8 at 64; 3,584-wide (466 MB, 71 us) 104.9 -> 90.4 at
+// 64; of these 3.5 us by issuing the MMAs from uniform registers. Without that, of q|k|v's 6 us at 40 tokens 0.8 pass before the kernel before releases this one, 1.0 until its tokens' first stage is there, 1.0 in
 // the MMAs, 2 between the accumulator and the barrier, 1 in the epilogue; gate|up and down run at 5.2 TB/s between. Sums read from
 // the other blocks' shared memory instead of stored there: a trip there and back behind the barrier, 0.6 us a kernel more (35.4 and 38.1 us);
 // norm weight, bias and residual asked for behind the barrier 1.2 us a kernel more.
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
   }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int tile = CLUSTER ? blockIdx.x / cluster : blockIdx.x, rank = CLUSTER ? blockIdx.x - tile * cluster : 0;
   const int column0 = tile * p.rows;
   const int kb_begin = CLUSTER ? rank * p.k_blocks / cluster : 0;
@@ -344,7 +344,8 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
     if (CLUSTER) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       const uint32_t idesc = instruction_descriptor(BM, p.columns);
       // A stage's descriptors are the first stage's plus an offset in the address field (units of 16 bytes, below 256 KB: no carry).
       const uint64_t w_first = smem_descriptor(base), x_first = smem_descriptor(base + a_bytes);
@@ -352,20 +353,23 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
       uint32_t phase = 0;
       bool ok = true;
       for (int i = 0; i < kb_count; ++i) {
-        ok = mbar_wait(full_bar(s), phase, abort_flag, p.error, 2);
+        ok = mbar_wait_warp(full_bar(s), phase, abort_flag, p.error, 2);
         if (!ok) break;
         tcgen05_fence_after();
         const uint64_t offset = (uint64_t)(uint32_t)(s * (stage_bytes >> 4)), a = w_first + offset, b = x_first + offset;
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < BK / UMMA_K; ++k)
-          umma_bf16(tmem_base, a + (uint64_t)(k * UMMA_K * 2 >> 4), b + (uint64_t)(k * UMMA_K * 2 >> 4), idesc, (i > 0 || k > 0) ? 1u : 0u);
-        tcgen05_commit(empty_bar(s));
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_bf16(tmem_base, a + (uint64_t)(k * UMMA_K * 2 >> 4), b + (uint64_t)(k * UMMA_K * 2 >> 4), idesc, (i > 0 || k > 0) ? 1u : 0u);
+          tcgen05_commit(empty_bar(s));
+        }
+        __syncwarp();
         if (++s == stages) {
           s = 0;
           phase ^= 1u;
         }
       }
-      if (ok) tcgen05_commit(done_bar);
+      if (ok && leader) tcgen05_commit(done_bar);
     }
     __syncwarp();
     if (CLUSTER) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");

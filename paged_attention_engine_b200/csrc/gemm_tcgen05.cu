@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
   }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int tile_a = blockIdx.x, tile_b = blockIdx.y;
   const int kb_begin = blockIdx.z * p.kb_per_split;
   const int kb_end = min(p.k_blocks, kb_begin + p.kb_per_split);
@@ -424,25 +424,27 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = instruction_descriptor(BM, BN);
-      bool ok = true;
-      for (int i = 0; i < kb_count && ok; ++i) {
-        const int s = i % T::STAGES;
-        ok = mbar_wait(full_bar(s), (i / T::STAGES) & 1, abort_flag, p.error, 2, limit);
-        if (!ok) break;
-        tcgen05_fence_after();
-        const uint32_t a_addr = base + s * T::STAGE_BYTES;
-        const uint32_t b_addr = a_addr + T::A_BYTES;
+    constexpr uint32_t idesc = instruction_descriptor(BM, BN);
+    const bool leader = elect_one();
+    const uint64_t a_desc0 = smem_descriptor(base), b_desc0 = smem_descriptor(base + T::A_BYTES);      // of the first stage: see the persistent kernel
+    bool ok = true;
+    for (int i = 0; i < kb_count; ++i) {
+      const int s = i % T::STAGES;
+      ok = mbar_wait_warp(full_bar(s), (i / T::STAGES) & 1, abort_flag, p.error, 2, limit);
+      if (!ok) break;
+      tcgen05_fence_after();
+      const uint64_t stage_offset = (uint64_t)(uint32_t)(s * (T::STAGE_BYTES >> 4));
+      const uint64_t a_desc = a_desc0 + stage_offset, b_desc = b_desc0 + stage_offset;
+      if (leader) {
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; ++k) {
           // Inside the 128-byte swizzle row a step of 16 elements is 32 bytes.
-          umma_bf16(tmem_base, smem_descriptor(a_addr + k * UMMA_K * 2), smem_descriptor(b_addr + k * UMMA_K * 2), idesc,
-                    (i > 0 || k > 0) ? 1u : 0u);
+          umma_bf16(tmem_base, a_desc + (uint64_t)(k * UMMA_K * 2 >> 4), b_desc + (uint64_t)(k * UMMA_K * 2 >> 4), idesc, (i > 0 || k > 0) ? 1u : 0u);
         }
         tcgen05_commit(empty_bar(s));      // the stage is free once these MMAs have read it
+        if (i + 1 == kb_count) tcgen05_commit(tmem_full_bar);  // the accumulator is complete once all MMAs are done
       }
-      if (ok) tcgen05_commit(tmem_full_bar);  // the accumulator is complete once all MMAs are done
+      __syncwarp();
     }
   } else {
     // ---------------------------------------------------------------- epilogue (warps 2..5)
@@ -591,7 +593,7 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
   const uint32_t bars = base + PSTAGES * P_STAGE_BYTES;   // full[S], empty[S], tmem_full[2], tmem_empty[2]
   volatile uint32_t* tmem_holder = (volatile uint32_t*)(generic_base + PSTAGES * P_STAGE_BYTES + 8 * (2 * PSTAGES + 4));
   volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (PSTAGES + s); };
   auto tmem_full_bar = [&](int a) { return bars + 8u * (2 * PSTAGES + a); };
@@ -667,10 +669,11 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       constexpr uint32_t idesc = instruction_descriptor(BM, PBN);
-      // This one thread's instruction stream paces the tensor core (four MMAs of a k-block run
-      // about as long as issuing them takes), so it is kept short: the stage index and its
+      // This warp's instruction stream paces the tensor core, so it is kept short: an elected lane issues from uniform registers (from a
+      // branch of one lane, us: o of 1,024 tokens 12.7 -> 10.7, q|k|v 17.7 -> 15.2, down of 1,500 45.7 -> 36.7); the stage index and its
       // phase are counted, not divided out, and the operand descriptors of a stage are the
       // first stage's plus a multiple of the stage size in the address field (bits 0-13, in
       // units of 16 bytes; the stages lie below 256 KB, so nothing carries out of the field).
@@ -684,29 +687,33 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
         if (a_of(item / planes) >= used) continue;
         const int acc = local & 1, use = local >> 1;
         ++local;
-        if (local > 2) ok = mbar_wait(tmem_empty_bar(acc), (use - 1) & 1, abort_flag, p.error, 4);
+        if (local > 2) ok = mbar_wait_warp(tmem_empty_bar(acc), (use - 1) & 1, abort_flag, p.error, 4);
         if (!ok) break;
         tcgen05_fence_after();
         const uint32_t tmem_acc = tmem_base + acc * ACC;
         const int kb_first = (item % planes) * p.kb_per_split;
         const int kb_count = min(kb_first + p.kb_per_split, k_blocks) - kb_first;
         for (int kb = 0; kb < kb_count; ++kb) {
-          if (!mbar_try_wait(full_bar(s), phase)) ok = mbar_wait(full_bar(s), phase, abort_flag, p.error, 2);
+          ok = mbar_wait_warp(full_bar(s), phase, abort_flag, p.error, 2);
           if (!ok) break;
           tcgen05_fence_after();
           const uint64_t stage_offset = (uint64_t)(uint32_t)(s * (P_STAGE_BYTES >> 4));
           const uint64_t a_desc = a_desc0 + stage_offset, b_desc = b_desc0 + stage_offset;
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_bf16(tmem_acc, a_desc + (uint64_t)(k * UMMA_K * 2 >> 4), b_desc + (uint64_t)(k * UMMA_K * 2 >> 4), idesc,
-                      (kb > 0 || k > 0) ? 1u : 0u);
-          tcgen05_commit(empty_bar(s));
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_bf16(tmem_acc, a_desc + (uint64_t)(k * UMMA_K * 2 >> 4), b_desc + (uint64_t)(k * UMMA_K * 2 >> 4), idesc,
+                        (kb > 0 || k > 0) ? 1u : 0u);
+            tcgen05_commit(empty_bar(s));
+          }
+          __syncwarp();
           if (++s == PSTAGES) {
             s = 0;
             phase ^= 1u;
           }
         }
-        if (ok) tcgen05_commit(tmem_full_bar(acc));
+        if (ok && leader) tcgen05_commit(tmem_full_bar(acc));
+        __syncwarp();
       }
     }
   } else {
@@ -818,7 +825,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PERSISTENT_THREADS)
   const uint32_t bars = base + STAGES * T::STAGE_BYTES;       // full[S], empty[S], tmem_full[2], tmem_empty[2]
   volatile uint32_t* tmem_holder = (volatile uint32_t*)(generic_base + STAGES * T::STAGE_BYTES + 8 * (2 * STAGES + 4));
   volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int rank = blockIdx.x & 1;                            // the first block of the pair issues the MMAs
   auto full_bar = [&](int s) { return bars + 8u * s; };       // the first block's count for both blocks' loads
   auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
@@ -874,7 +881,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PERSISTENT_THREADS)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
+      const bool leader = elect_one();
       constexpr uint32_t idesc = instruction_descriptor(2 * BM, PBN);
       const uint64_t a_desc0 = smem_descriptor(base);
       const uint64_t b_desc0 = smem_descriptor(base + T::A_BYTES);
@@ -884,27 +892,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PERSISTENT_THREADS)
       for (int tile = blockIdx.x >> 1; tile < total && ok; tile += step) {
         const int acc = local & 1, use = local >> 1;
         ++local;
-        if (local > 2) ok = mbar_wait(tmem_empty_bar(acc), (use - 1) & 1, abort_flag, p.error, 4);
+        if (local > 2) ok = mbar_wait_warp(tmem_empty_bar(acc), (use - 1) & 1, abort_flag, p.error, 4);
         if (!ok) break;
         tcgen05_fence_after();
         const uint32_t tmem_acc = tmem_base + acc * ACC;
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_try_wait(full_bar(s), phase)) ok = mbar_wait(full_bar(s), phase, abort_flag, p.error, 2);
+          ok = mbar_wait_warp(full_bar(s), phase, abort_flag, p.error, 2);
           if (!ok) break;
           tcgen05_fence_after();
           const uint64_t stage_offset = (uint64_t)(uint32_t)(s * (T::STAGE_BYTES >> 4));
           const uint64_t a_desc = a_desc0 + stage_offset, b_desc = b_desc0 + stage_offset;
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_bf16_pair(tmem_acc, a_desc + (uint64_t)(k * UMMA_K * 2 >> 4), b_desc + (uint64_t)(k * UMMA_K * 2 >> 4), idesc,
-                           (kb > 0 || k > 0) ? 1u : 0u);
-          tcgen05_commit_pair(empty_bar(s));
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_bf16_pair(tmem_acc, a_desc + (uint64_t)(k * UMMA_K * 2 >> 4), b_desc + (uint64_t)(k * UMMA_K * 2 >> 4), idesc,
+                             (kb > 0 || k > 0) ? 1u : 0u);
+            tcgen05_commit_pair(empty_bar(s));
+          }
+          __syncwarp();
           if (++s == STAGES) {
             s = 0;
             phase ^= 1u;
           }
         }
-        if (ok) tcgen05_commit_pair(tmem_full_bar(acc));
+        if (ok && leader) tcgen05_commit_pair(tmem_full_bar(acc));
+        __syncwarp();
       }
     }
   } else {

@@ -59,6 +59,28 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
+// The same by a whole warp, which goes on together.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* error, int code,
+                                               uint32_t limit = WAIT_LIMIT) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, error, code, limit));
+}
+// True in one lane of a converged warp. The warp that issues MMAs runs its role together and lets this lane issue them: what all lanes
+// hold alike lies in uniform registers, which the instruction takes; from a branch of one lane (`if (lane == 0)`) an MMA took some 110
+// cycles to issue, more than many of them run.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t chosen;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(chosen));
+  return chosen != 0;
+}
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
