@@ -1,4 +1,4 @@
-// The products of a step of some tens of tokens (a decode batch of 17 to 128 requests, a short prompt portion; of wide models
+// The products of a step of some tens of tokens (a decode batch of 9 to 128 requests, a short prompt portion; of wide models
 // any step of up to 128), each as ONE kernel that leaves finished output.
 //
 // Such a step streams every weight once, and what it costs beside that is the chain: with K split over blocks

@@ -478,19 +478,22 @@ def _few_tokens(x: torch.Tensor, k: int, normed: bool = False, kind: int = GATE_
 # False sends such products to the other kernels and their sums (tests compare the two).
 use_cluster_products = True
 # From how many tokens on, by the width of the rows that the norms read. Measured, us, the four products of a layer with
-# their norms in a row, other kernels / these. Width 896: 16 tokens 19.8 / 22.1, 24 24.1 / 23.0, 64 36.6 / 26.5, 128 42.6 / 32.5; 1,536:
-# 16 tokens 29.9 / 33.0, 20 34.3 / 32.7, 40 44.2 / 34.0, 64 46.1 / 36.0, 128 51.8 / 50.2. From 2,048 on the few-token
+# their norms in a row, other kernels / these. Width 896: 8 tokens 14.8 / 19.0, 16 19.7 / 19.9, 18 23.6 / 19.8, 64 36.6 / 26.5; 1,536:
+# 8 tokens 23.0 / 27.6, 9 29.0 / 27.5, 16 29.8 / 28.5, 40 43.0 / 30.6, 64 44.4 / 32.9, 100 48.2 / 43.0. From 2,048 on the few-token
 # kernels' blocks no longer all run at once, and these are ahead from one token on: 2,048 1 token 44.7 / 37.6, 8 46.2 / 40.4,
-# 64 58.8 / 49.9; 3,584 83.9 / 79.7, 87.0 / 82.6 and 106.7 / 91.8; 5,120 109.4 / 93.5, 105.6 / 95.9 and 121.5 / 106.8.
-CLUSTER_MIN_TOKENS = 17
-CLUSTER_WIDE = 2048
+# 64 58.8 / 49.9; 3,584 83.9 / 79.7, 85.6 / 80.1 and 104.9 / 90.5; 5,120 109.4 / 93.5, 105.6 / 95.9 and 121.5 / 106.8.
+CLUSTER_MIN_TOKENS = 9
+CLUSTER_MIN_TOKENS_NARROW = 17        # rows narrower than this:
+CLUSTER_NARROW = 1024
+CLUSTER_WIDE = 2048                   # ... and of rows from this width on, every number of tokens
 CLUSTER_MAX_TOKENS = 128
 
 
 def _cluster_takes(tokens: int, n: int, k: int, weight, width: int) -> bool:
     """Whether the cluster kernels run a bfloat16 product of these sizes; `width`: of the rows that the norm before or behind it reads."""
     return (weight.dtype == torch.bfloat16 and use_cluster_products and use_tensor_cores and not few_token_products_everywhere
-            and (CLUSTER_MIN_TOKENS if width < CLUSTER_WIDE else 1) <= tokens <= CLUSTER_MAX_TOKENS
+            and tokens <= CLUSTER_MAX_TOKENS
+            and tokens >= (1 if width >= CLUSTER_WIDE else CLUSTER_MIN_TOKENS if width >= CLUSTER_NARROW else CLUSTER_MIN_TOKENS_NARROW)
             and weight.dim() == 2 and weight.shape[1] == k and n % 8 == 0 and k % 64 == 0 and weight.is_contiguous()
             and weight.data_ptr() % 16 == 0)
 
