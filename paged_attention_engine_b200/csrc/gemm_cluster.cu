@@ -295,11 +295,14 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
   const int first = min(kb_count, stages);
   auto load_weights = [&](int i, int s) { tma_load_2d(base + s * stage_bytes, &map_w, full_bar(s), (kb_begin + i) * BK, column0); };
   auto load_tokens = [&](int i, int s) { tma_load_2d(base + s * stage_bytes + a_bytes, &map_x, full_bar(s), (kb_begin + i) * BK, 0); };
-  if (warp == 0 && lane == 0 && p.early) {
-    for (int i = 0; i < first; ++i) {
-      mbar_expect_tx(full_bar(i), stage_bytes);
-      load_weights(i, i);
+  if (warp == 0 && p.early) {
+    if (elect_one()) {
+      for (int i = 0; i < first; ++i) {
+        mbar_expect_tx(full_bar(i), stage_bytes);
+        load_weights(i, i);
+      }
     }
+    __syncwarp();
   }
   dependent_launch_wait();
 
@@ -312,8 +315,8 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      int issued = first;
+    const bool leader = elect_one();
+    if (leader) {
       for (int i = 0; i < first; ++i) {
         if (!p.early) {
           mbar_expect_tx(full_bar(i), stage_bytes);
@@ -321,24 +324,28 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
         }
         load_tokens(i, i);
       }
-      int s = 0;
-      uint32_t phase = 0;
-      for (int i = first; i < kb_count; ++i) {
-        if (!mbar_wait(empty_bar(s), phase, abort_flag, p.error, 1)) break;
+    }
+    __syncwarp();
+    int issued = first, s = 0;
+    uint32_t phase = 0;
+    for (int i = first; i < kb_count; ++i) {
+      if (!mbar_wait_warp(empty_bar(s), phase, abort_flag, p.error, 1)) break;
+      if (leader) {
         mbar_expect_tx(full_bar(s), stage_bytes);
         load_weights(i, s);
         load_tokens(i, s);
-        issued = i + 1;
-        if (++s == stages) {
-          s = 0;
-          phase ^= 1u;
-        }
       }
-      if (*abort_flag) {
-        // Loads that were issued still write into this block's shared memory: wait for them.
-        for (int i = max(0, issued - stages); i < issued; ++i)
-          for (uint32_t t = 0; t < WAIT_LIMIT && !mbar_try_wait(full_bar(i % stages), (i / stages) & 1); ++t) __nanosleep(64);
+      __syncwarp();
+      issued = i + 1;
+      if (++s == stages) {
+        s = 0;
+        phase ^= 1u;
       }
+    }
+    if (leader && *abort_flag) {
+      // Loads that were issued still write into this block's shared memory: wait for them.
+      for (int i = max(0, issued - stages); i < issued; ++i)
+        for (uint32_t t = 0; t < WAIT_LIMIT && !mbar_try_wait(full_bar(i % stages), (i / stages) & 1); ++t) __nanosleep(64);
     }
     __syncwarp();
     if (CLUSTER) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");

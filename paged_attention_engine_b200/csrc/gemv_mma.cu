@@ -49,6 +49,8 @@ namespace {
 using pae_tcgen05::mbar_expect_tx;
 using pae_tcgen05::mbar_init;
 using pae_tcgen05::mbar_try_wait;
+using pae_tcgen05::elect_one;
+using pae_tcgen05::uniform_warp;
 using pae_tcgen05::encode_tiled;
 using pae_tcgen05::EncodeTiled;
 
@@ -158,7 +160,10 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(const __grid_constant_
   float* token_scale = (float*)(smem + FRONT_BYTES + WARPS * STAGES * 8);   // [TOKENS]
   uint8_t* operand = smem + FRONT_BYTES + WARPS * STAGES * 8 + 64 * 4;   // the normed operand (NORMED)
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // The copies are asked for by an elected lane, from uniform registers: from a branch of one lane each cost the warp some 100 cycles (a layer's
+  // four products at 8 tokens, 1536 wide, 23.0 -> 21.9 us).
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
+  const bool leader = elect_one();
   const int g = lane >> 2, t4 = lane & 3;
   const int tile = SPLIT ? (int)blockIdx.x : (int)blockIdx.x * WARPS + warp;
   const int tiles = KIND == QKV ? (p.n / p.d) * (p.d >> 4) : (is_gate(KIND) ? p.n / 16 : (p.n + ROWS - 1) / ROWS);
@@ -200,7 +205,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(const __grid_constant_
 
   // The first stages' weights before the wait for the kernel before; their activations after it.
   const int early = min(groups, STAGES);
-  if (lane == 0)
+  if (leader)
     for (int i = 0; i < early; ++i) fetch_weights(i);
   // What the epilogue adds comes from weights (the bias) and is asked for now ...
   const bool finishes = live && (!SPLIT || warp == 0);          // this warp runs the epilogue
@@ -231,7 +236,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(const __grid_constant_
     }
   }
   dependent_launch_wait();
-  if (lane == 0)
+  if (leader)
     for (int i = 0; i < early; ++i) fetch_activations(i);
   // ... or from the step (angles and slots, the residual) and is asked for here, a trip to the
   // L2 that the main loop hides: for tokens 8 n + 2 t4 + e.
@@ -369,7 +374,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(const __grid_constant_
       }
     }
     __syncwarp();
-    if (lane == 0 && i + STAGES < groups) {
+    if (leader && i + STAGES < groups) {
       fetch_weights(i + STAGES);
       fetch_activations(i + STAGES);
     }
@@ -548,7 +553,8 @@ int launch_one(const Params& p, const void* w, int tiles, cudaStream_t stream) {
 // does not hold costs further trips to memory one after the other. Measured at 8 tokens (q|k|v, o,
 // gate|up and down of a 1536-wide model in a row, 28 times over, one copy per stage and operand):
 // 23.4 us with 3 stages of 3 chunks, 24.0 us with 2 of 4, 24.4 us with 4 of 2 (not built: the room of 2 of 4), 27.0 us with 2 of 2;
-// with one copy per chunk 25.8 us (2 of 4), 33.1 us (8 of 1), 50.2 us (4 of 1). The first in the
+// with one copy per chunk 25.8 us (2 of 4), 33.1 us (8 of 1), 50.2 us (4 of 1); copies by an elected lane kept the order (22.3, 22.6 and 25.1 us
+// with 3 of 3, 2 of 4 and 2 of 2 for o and down). The first in the
 // order of preference whose blocks all run at once is taken (gate|up alone is fastest with 3 stages
 // of 4; with 9 to 16 tokens the activations' chunks take room beside the weights' and 3 stages of 2
 // fit where 3 of 3 do not), unless `pae_linear_few_tokens_configure` has named one for the kind.
