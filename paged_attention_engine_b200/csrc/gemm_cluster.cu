@@ -479,10 +479,15 @@ int log2_of(int v) { return v <= 1 ? 0 : 1 + log2_of(v >> 1); }
 struct Shape {
   int rows, cluster, stages;
 };
+// A block of a later kernel holds its tensor memory while it waits for the kernels before it. Were it to find room on an SM where a block of the
+// persistent products, which take all of tensor memory, still waits for a third block's part, neither would go on. Two blocks
+// of these beside one of the smallest of those (146 KB) do not fit an SM's 228 KB from 41 KB each on.
+constexpr size_t LEAST_BYTES = 48 * 1024;
 size_t smem_bytes(const Shape& s, int tokens) {
   const size_t stage = (size_t)(s.rows + columns_of(tokens)) * BK * 2;
   const size_t exchange = s.cluster > 1 ? (size_t)s.cluster * ((tokens + s.cluster - 1) / s.cluster) * s.rows * 4 : 0;
-  return 1024 + (s.stages - 1) * stage + (stage > (size_t)A_BYTES ? stage : (size_t)A_BYTES) + exchange + TAIL_BYTES;
+  const size_t bytes = 1024 + (s.stages - 1) * stage + (stage > (size_t)A_BYTES ? stage : (size_t)A_BYTES) + exchange + TAIL_BYTES;
+  return bytes > LEAST_BYTES ? bytes : LEAST_BYTES;
 }
 constexpr int SMEM_PER_BLOCK = 112 * 1024;     // two blocks an SM
 
