@@ -223,12 +223,13 @@ class ModelRunner:
             try:
                 self._capture(slot, ctx)
             except torch.OutOfMemoryError:
-                # No room for the recording's buffers beside the eager step's: such steps stay eager from here on.
+                # No room for the recording's buffers beside the eager step's: such steps stay eager from here on. What the parts
+                # left with `ctx` (the positions' table, the slices' plan) was recorded and never made: the eager step builds its own.
                 self.SHAPE_GRAPHS = 0
                 self.shape_graphs.clear()
+                del ctx, slot
                 torch.cuda.empty_cache()
-                logits, tokens = self._run(ctx)
-                return logits, tokens, ctx.num_tokens
+                return self._eager(entries, sampling)
             slot.num_tokens = ctx.num_tokens
             self.shape_graphs[key] = slot
             while len(self.shape_graphs) > self.SHAPE_GRAPHS:
