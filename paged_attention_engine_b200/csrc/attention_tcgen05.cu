@@ -291,6 +291,7 @@ struct Layout {
   static constexpr int TMEM_COLUMNS = 512;
   static_assert(O_COLUMN + 2 * D <= TMEM_COLUMNS, "two score buffers and two products must fit tensor memory");
   static_assert(SMEM_BYTES <= 227 * 1024, "the block's shared memory");
+  static_assert(SMEM_BYTES >= pae::WHOLE_TENSOR_MEMORY_BYTES, "no block of another cluster with tensor memory beside this one (common.cuh)");
 };
 
 enum Bar : int { Q_FULL = 0, K_FULL = 1, V_FULL = 3, K_EMPTY = 5, V_EMPTY = 7, S_FULL = 9, S_EMPTY = 11, P_READY = 13, O_FULL = 15, O_EMPTY = 17, X_READY = 19, NUM_BARS = 20 };
@@ -299,7 +300,6 @@ template <int D, bool SPLIT>
 __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                   const __grid_constant__ PageMaps maps, const Params p) {
   using L = Layout<D>;
-  dependent_launch_trigger();
   if (threadIdx.x == 0) {         // the descriptors do not depend on the kernel before: fetch them early
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.key_run) : "memory");
@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
   }
   tcgen05_fence_before();
   __syncthreads();
+  dependent_launch_trigger();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
 
@@ -822,7 +823,6 @@ template <int D>
 __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                      const __grid_constant__ PageMaps maps, const Params p) {
   using L = Layout<D>;
-  dependent_launch_trigger();
   if (threadIdx.x == 0) {         // the descriptors do not depend on the kernel before: fetch them early
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.key_run) : "memory");
@@ -868,6 +868,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
   }
   tcgen05_fence_before();
   __syncthreads();
+  dependent_launch_trigger();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
 

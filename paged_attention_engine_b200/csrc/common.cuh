@@ -176,6 +176,16 @@ __device__ __forceinline__ void dependent_launch_prologue() {
 __device__ __forceinline__ void dependent_launch_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dependent_launch_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// TENSOR MEMORY. `tcgen05.alloc` waits, without a limit, until an SM has the columns to give. Two rules keep every such wait finite:
+// - A kernel lets the next one begin (`dependent_launch_trigger`) only when its block holds its columns. So no block that waits for
+//   a kernel before it can hold columns that a block of that kernel is still waiting for.
+// - Blocks of a cluster wait for one another, and one that waits for columns may hold up the others of its cluster, which hold theirs. So no two clusters,
+//   of one stream or of several, may ever want the same columns. Those of the pair products and the wide attention take all 512 and
+//   WHOLE_TENSOR_MEMORY_BYTES of shared memory or more: one to an SM. Those of the cluster products take 128 at most, and so much shared memory that two
+//   at most share an SM, and none shares one with the former. All other blocks that hold columns wait for nothing that wants any.
+constexpr size_t WHOLE_TENSOR_MEMORY_BYTES = 146 * 1024;
+static_assert(2 * (WHOLE_TENSOR_MEMORY_BYTES + 1024) > 228 * 1024, "one to an SM");
+
 inline bool dependent_launch_enabled() {
   static const bool enabled = [] {
     const char* v = std::getenv("PAE_PDL");

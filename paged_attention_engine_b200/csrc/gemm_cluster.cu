@@ -258,7 +258,6 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
   volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
   float* scales = (float*)(tail + 256);
 
-  dependent_launch_trigger();
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
@@ -288,6 +287,7 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
   }
   tcgen05_fence_before();
   __syncthreads();
+  dependent_launch_trigger();
   tcgen05_fence_after();
   // Another block's shared memory may be written once that block has started: the arrival here, whose wait stands before the first store.
   if (CLUSTER) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
@@ -479,15 +479,15 @@ int log2_of(int v) { return v <= 1 ? 0 : 1 + log2_of(v >> 1); }
 struct Shape {
   int rows, cluster, stages;
 };
-// A block of a later kernel holds its tensor memory while it waits for the kernels before it. Were it to find room on an SM where a block of the
-// persistent products, which take all of tensor memory, still waits for a third block's part, neither would go on. Two blocks
-// of these beside one of the smallest of those (146 KB) do not fit an SM's 228 KB from 41 KB each on.
-constexpr size_t LEAST_BYTES = 48 * 1024;
+// What a block of a cluster takes at least: no more than two of them share an SM, and none shares one with a block of the clusters that
+// take all of tensor memory (see TENSOR MEMORY in common.cuh).
+constexpr size_t LEAST_BYTES = 81 * 1024;
+static_assert(LEAST_BYTES + WHOLE_TENSOR_MEMORY_BYTES + 2 * 1024 > 228 * 1024 && 3 * (LEAST_BYTES + 1024) > 228 * 1024, "tensor memory");
 size_t smem_bytes(const Shape& s, int tokens) {
   const size_t stage = (size_t)(s.rows + columns_of(tokens)) * BK * 2;
   const size_t exchange = s.cluster > 1 ? (size_t)s.cluster * ((tokens + s.cluster - 1) / s.cluster) * s.rows * 4 : 0;
   const size_t bytes = 1024 + (s.stages - 1) * stage + (stage > (size_t)A_BYTES ? stage : (size_t)A_BYTES) + exchange + TAIL_BYTES;
-  return bytes > LEAST_BYTES ? bytes : LEAST_BYTES;
+  return s.cluster == 1 || bytes > LEAST_BYTES ? bytes : LEAST_BYTES;
 }
 constexpr int SMEM_PER_BLOCK = 112 * 1024;     // two blocks an SM
 

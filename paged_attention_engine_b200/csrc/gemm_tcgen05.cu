@@ -343,7 +343,6 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
   volatile uint32_t* tmem_holder = (volatile uint32_t*)(generic_base + T::STAGES * T::STAGE_BYTES + 8 * (2 * T::STAGES + 1));
   volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
 
-  dependent_launch_trigger();     // the kernel after this one may begin its own set-up
   if (threadIdx.x == 0) {         // the descriptors do not depend on the kernel before: fetch them early
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
@@ -373,6 +372,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
   }
   tcgen05_fence_before();
   __syncthreads();
+  dependent_launch_trigger();     // the kernel after this one may begin its own set-up: tensor memory is held
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   // Barriers and tensor memory are set up. The WEIGHT operand (A when the rows of the MMA are
@@ -590,7 +590,6 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
   constexpr int P_A_BYTES = PTile<PBN>::A_BYTES;
   constexpr int P_STAGE_BYTES = PTile<PBN>::STAGE_BYTES;
   constexpr int ACC = PTile<PBN>::ACC_COLUMNS;
-  dependent_launch_trigger();
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
@@ -626,6 +625,7 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS) gemm_tcgen05_persistent_ke
   }
   tcgen05_fence_before();
   __syncthreads();
+  dependent_launch_trigger();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   dependent_launch_wait();
@@ -788,6 +788,7 @@ struct PairTile {
   static constexpr int ACC_COLUMNS = 256;
   static constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_BYTES + 1024 + 256;
   static_assert(B_BYTES % 1024 == 0, "stages start on 1024 bytes");
+  static_assert(SMEM_BYTES >= WHOLE_TENSOR_MEMORY_BYTES, "no block of another cluster with tensor memory beside this one (common.cuh)");
 };
 
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
@@ -822,7 +823,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PERSISTENT_THREADS)
                              int tiles_a, int tiles_b) {
   using T = PairTile<PBN>;
   constexpr int STAGES = T::STAGES, ACC = T::ACC_COLUMNS;
-  dependent_launch_trigger();
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
@@ -860,6 +860,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PERSISTENT_THREADS)
   tcgen05_fence_before();
   __syncthreads();
   cluster_sync();                  // the other block's barriers are set up, too
+  dependent_launch_trigger();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
 

@@ -48,3 +48,13 @@ def test_a_many_token_product_loads_nothing_before_the_kernel_before_has_complet
     """Its weights may have been written by the kernel before."""
     (body,) = [body for _, name, body in _kernels() if name == kernel]
     assert 0 < body.index("dependent_launch_wait()") < body.index("tma_load_2d")
+
+
+@pytest.mark.parametrize("kernel", [n for _, n, body in _kernels() if re.search(r"tmem_alloc\(|tcgen05\.alloc", body)])
+def test_the_next_kernel_is_let_go_when_tensor_memory_is_held(kernel):
+    """A block of the next kernel that took columns first would hold them until this kernel has completed, which then waits for them."""
+    for _, name, body in _kernels():
+        if name == kernel:
+            held = body.index("__syncthreads()", re.search(r"tmem_alloc\(|tcgen05\.alloc", body).start())
+            lets_go = [m.start() for m in re.finditer(r"dependent_launch_(?:trigger|prologue)\(\)|launch_dependents", body)]
+            assert lets_go and min(lets_go) > held, name
