@@ -28,6 +28,8 @@
 // the MMAs, 2 between the accumulator and the barrier, 1 in the epilogue; gate|up and down run at 5.2 TB/s between. Sums read from
 // the other blocks' shared memory instead of stored there: a trip there and back behind the barrier, 0.6 us a kernel more (35.4 and 38.1 us);
 // norm weight, bias and residual asked for behind the barrier 1.2 us a kernel more.
+#include <atomic>
+
 #include "tcgen05.cuh"
 
 using namespace pae;
@@ -473,7 +475,11 @@ int log2_of(int v) { return v <= 1 ? 0 : 1 + log2_of(v >> 1); }
 // - two blocks an SM (112 KB each) rather than one with a deeper ring, because the next product's blocks start beside them: q|k|v of
 //   1,536 with 8 blocks a tile, 40 tokens 34.0 with 4 stages, 38.5 with 9. But where the launch leaves a third of the SMs
 //   without a block and a block's K is more than two rings, the deep ring: down of 1,536, 64 tokens 36.7 with 8 stages, 39.9 with 3.
-// - and where the tokens leave a block of two an SM no third stage, fewer blocks with deep rings: width 3,584, 128 tokens 145.6 -> 104.8.
+// - and where the tokens leave a block of two an SM no third stage, or no second, one an SM with a deep ring, and as many blocks a tile as let
+//   every cluster run at once: a cluster lies within a part of the chip whose SMs it need not divide, so 148 SMs take 45 clusters of three,
+//   33 of four, 22 of six, but 15 of seven (`clusters_at_once` asks). A sixteenth cluster of seven ran behind the others: 100 tokens of 1,536, whose
+//   q|k|v has 16 tiles, 42.3 with seven blocks a tile and 37.4 with six; 128 tokens of 2,048 53.6 and 41.2, of 768 38.4 and 27.4, of 5,120 129.2 and
+//   119.6.
 // - gate|up whose tiles fill the SMs by themselves: tiles of 64 rows, while all run at once (280 blocks instead of 140 share the end: 64 tokens
 //   36.0 against 36.6, 40 tokens 34.1 against 34.4).
 struct Shape {
@@ -491,14 +497,48 @@ size_t smem_bytes(const Shape& s, int tokens) {
 }
 constexpr int SMEM_PER_BLOCK = 112 * 1024;     // two blocks an SM
 
+// Stands for the product's kernel in the question below: asked about a kernel that allocates tensor memory, the runtime counts one block an
+// SM whatever the block takes (two of 112 KB share one all the same).
+__global__ void __launch_bounds__(64 + EPILOGUE_THREADS<true>, 2) room_kernel() {}
+
+// Clusters of `cluster` blocks that run at one time on the current device, one block to an SM or two.
+int clusters_at_once(int cluster, bool one_an_sm) {
+  static std::atomic<int> known[64][2][MAX_CLUSTER + 1];
+  int device = 0, count = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) device = 0;
+  const bool kept = device >= 0 && device < 64;
+  if (kept && (count = known[device][one_an_sm][cluster].load(std::memory_order_relaxed)) > 0) return count;
+  const size_t bytes = one_an_sm ? 227 * 1024 : SMEM_PER_BLOCK;
+  static DevicesSet raised;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(cluster);
+  config.blockDim = dim3(64 + EPILOGUE_THREADS<true>);
+  config.dynamicSmemBytes = bytes;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = cluster;
+  attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = 1;
+  if (raise_shared_memory(raised, room_kernel, 227 * 1024, "linear_cluster") != 0 || cudaOccupancyMaxActiveClusters(&count, room_kernel, &config) != cudaSuccess || count < 1) {
+    cudaGetLastError();                                   // not known: half of what the SMs' number would allow
+    return sm_count() * (one_an_sm ? 1 : 2) / (2 * cluster);
+  }
+  if (kept) known[device][one_an_sm][cluster].store(count, std::memory_order_relaxed);
+  return count;
+}
+
 Shape shape_of(int tokens, int n, int k, bool gate) {
   const int k_blocks = (k + BK - 1) / BK, sms = sm_count();
   Shape s{BM, 1, 2};
   const int tiles = (n + BM - 1) / BM;
-  auto blocks_a_tile = [&](int blocks, int most) {
+  // At most `blocks` in all, and all at once.
+  auto blocks_a_tile = [&](int blocks, bool one_an_sm) {
     int c = blocks / tiles;
-    c = c > most ? most : c < 1 ? 1 : c;
-    return c > k_blocks ? k_blocks : c;
+    c = c > MAX_CLUSTER ? MAX_CLUSTER : c < 1 ? 1 : c;
+    c = c > k_blocks ? k_blocks : c;
+    while (c > 1 && clusters_at_once(c, one_an_sm) < tiles) --c;
+    return c;
   };
   auto most_stages = [&](size_t limit) {
     const int per_block = (k_blocks + s.cluster - 1) / s.cluster;
@@ -506,15 +546,14 @@ Shape shape_of(int tokens, int n, int k, bool gate) {
     while (stages < MAX_STAGES && stages < per_block && smem_bytes(Shape{s.rows, s.cluster, stages + 1}, tokens) <= limit) ++stages;
     return stages;
   };
-  s.cluster = blocks_a_tile(sms * 17 / 10, MAX_CLUSTER);
+  s.cluster = blocks_a_tile(sms * 17 / 10, false);
   if (gate && s.cluster == 1 && (n + 63) / 64 <= 2 * sms) s.rows = 64;
   s.stages = most_stages(SMEM_PER_BLOCK);
   const int per_block = (k_blocks + s.cluster - 1) / s.cluster;
-  if (s.cluster > 1 && tiles * s.cluster * 10 <= sms * 7 && per_block > 2 * s.stages) {
+  if (s.cluster > 1 && tiles * s.cluster * 10 <= sms * 7 && per_block > 2 * s.stages && clusters_at_once(s.cluster, true) >= tiles) {
     s.stages = most_stages(227 * 1024);
-  } else if (s.cluster > 1 && s.stages < 3 && per_block >= 3) {
-    s.cluster = blocks_a_tile(sms, 3);
-    if (s.cluster == 3) s.cluster = blocks_a_tile(sms * 76 / 100, MAX_CLUSTER);
+  } else if (s.cluster > 1 && ((s.stages < 3 && per_block >= 3) || smem_bytes(s, tokens) > SMEM_PER_BLOCK)) {
+    s.cluster = blocks_a_tile(sms, true);
     s.stages = most_stages(227 * 1024);
   }
   return s;
@@ -566,6 +605,14 @@ int check_common(const char* what, const void* out, const void* w, const void* x
 PAE_EXPORT int pae_linear_cluster_parts(int tokens, int n, int k) {
   const int rows = shape_of(tokens, n, k, false).rows;
   return (n + rows - 1) / rows;
+}
+
+// Rounds of clusters that a launch takes: 0 without clusters, else 1 unless its shape is wrong.
+PAE_EXPORT int pae_linear_cluster_rounds(int tokens, int n, int k, int gate) {
+  const Shape s = shape_of(tokens, n, k, gate != 0);
+  if (s.cluster == 1) return 0;
+  const int at_once = clusters_at_once(s.cluster, smem_bytes(s, tokens) > SMEM_PER_BLOCK);
+  return ((n + s.rows - 1) / s.rows + at_once - 1) / at_once;
 }
 
 // out[token, n] = x . w[n, k]^T (+ residual[token, n]), bfloat16. With `gamma` also scaled[token, n] = out * gamma and

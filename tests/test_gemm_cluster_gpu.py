@@ -136,6 +136,16 @@ def test_a_chain_of_products_and_norms(ops, tokens):
     ops.check_device_errors()
 
 
+def test_all_clusters_of_a_launch_run_at_once(ops):
+    """One cluster more than the chip takes at a time makes the launch last twice as long."""
+    lib = ops._lib("gemm_cluster")
+    for tokens in TOKENS + [40, 80, 96, 97, 112]:
+        for n in [8, 512, 768, 1024, 1536, 2048, 2304, 2560, 3072, 3584, 4096, 4608, 5120, 6144, 8192, 11008, 16384, 18944, 22016, 37888]:
+            for k in [64, 192, 512, 768, 1024, 1536, 2048, 3584, 8960, 18944]:
+                for gate in (0, 1):
+                    assert lib.pae_linear_cluster_rounds(tokens, n, k, gate) <= 1, (tokens, n, k, gate)
+
+
 def test_what_the_library_refuses(ops):
     lib = ops._lib("gemm_cluster")
     x, w, out = _rand((4, 64), 1), _rand((64, 64), 2), _rand((4, 64), 3)
