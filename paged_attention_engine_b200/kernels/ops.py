@@ -207,9 +207,10 @@ class PendingNorm:
 
 
 class PendingProduct:
-    """x . weight^T + residual of a step of some tens of tokens that has not run: `linear` returns one, and the
+    """x . weight^T + residual of a step of some tens of tokens that has not run: `linear_before_norm` returns one, and the
     `rms_norm` that reads the sum next has the product's own epilogue prepare the norm (`ScaledNorm`), which saves the
-    norm's launch; anything else calls `materialized`, which runs the product alone and keeps its result in `value`."""
+    norm's launch; anything else calls `materialized`, which runs the product alone and keeps its result in `value`. Until then its
+    operand and its residual are not to be written."""
 
     def __init__(self, operand, weight, residual) -> None:
         self.operand, self.weight, self.residual = operand, weight, residual
@@ -632,23 +633,17 @@ def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str 
     before the residual: in the tensor-core product's epilogue or in the sum of its splits, else
     by the activation's own kernel.
 
-    The product of some tens of tokens with a residual is not run before its value or the norm that reads it is asked for (`PendingProduct`).
     The bfloat16 kernels of few tokens (up to 64, or 128 where K is long) or of fewer than 256 columns read `weight` while the kernel
     before them in the stream may still be running, as they do in `linear_swiglu` and `qkv_projection`: a weight that the call just before
     wrote needs another launch, or a synchronisation, in between. Larger products read nothing before that kernel has completed."""
     if activation not in ACTIVATIONS:
         raise KernelError(f"linear: activation '{activation}' (known: gelu_erf, gelu_tanh, relu2)")
-    if (x.shape[0] <= CLUSTER_MAX_TOKENS and activation is None and bias is None and out_dtype in (None, torch.bfloat16)
-            and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.data_ptr() % 16 == 0 and weight.shape[0] <= 65536):
+    if activation is None and _plain_product(x, weight, bias, out_dtype):
         if residual is not None and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0]):
-            operand, residual = _cluster_operand(x), materialized(residual)
-            if operand is not None and residual.dtype == torch.bfloat16 and residual.data_ptr() % 16 == 0:
-                _need(operand[0], "linear: x")
-                _need(weight, "linear: weight")
-                _need(residual, "linear: residual", torch.bfloat16)
-                if tuple(residual.shape) != (x.shape[0], weight.shape[0]):
-                    raise KernelError(f"linear: residual is {tuple(residual.shape)}, the product is [{x.shape[0]}, {weight.shape[0]}]")
-                return PendingProduct(operand, weight, residual)
+            pending = _pending_product(x, weight, residual)
+            if pending is not None:
+                _cluster_product(pending, None)
+                return pending.value
         source, norm_weight, eps = _norm_of(x)
         if (_few_tokens(source, weight.shape[1], norm_weight is not None, RESIDUAL_KIND, weight.shape[0]) and source.dim() == 2 and source.shape[1] == weight.shape[1]
                 and source.is_contiguous() and weight.is_contiguous()):
@@ -699,6 +694,37 @@ def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str 
                                     k, (_code(x)), (_code(weight)), _DTYPE_CODE[out_dtype],
                                     _stream()))
     return out
+
+
+def linear_before_norm(x, weight, bias=None, residual=None, out_dtype=None):
+    """`linear` for a sum that an RMSNorm reads next. The product of some tens of tokens with a residual may come back as a
+    `PendingProduct`, which that norm has run with the norm inside; `materialized` hands out its tensor. x and the residual are not to be
+    written before."""
+    if (residual is not None and _plain_product(x, weight, bias, out_dtype)
+            and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0])):
+        pending = _pending_product(x, weight, residual)
+        if pending is not None:
+            return pending
+    return linear(x, weight, bias, residual, out_dtype)
+
+
+def _plain_product(x, weight, bias, out_dtype) -> bool:
+    """Whether the kernels of few and of some tens of tokens may take a product: bfloat16 without a bias."""
+    return (x.shape[0] <= CLUSTER_MAX_TOKENS and bias is None and out_dtype in (None, torch.bfloat16)
+            and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.data_ptr() % 16 == 0 and weight.shape[0] <= 65536)
+
+
+def _pending_product(x, weight, residual):
+    """The product of sizes that the cluster kernels take, or None when an operand is not theirs."""
+    operand, residual = _cluster_operand(x), materialized(residual)
+    if operand is None or residual.dtype != torch.bfloat16 or residual.data_ptr() % 16:
+        return None
+    _need(operand[0], "linear: x")
+    _need(weight, "linear: weight")
+    _need(residual, "linear: residual", torch.bfloat16)
+    if tuple(residual.shape) != (x.shape[0], weight.shape[0]):
+        raise KernelError(f"linear: residual is {tuple(residual.shape)}, the product is [{x.shape[0]}, {weight.shape[0]}]")
+    return PendingProduct(operand, weight, residual)
 
 
 def _linear_tensor_cores(x, weight, bias, residual, out_dtype, m, n, k, activation: int = 0) -> torch.Tensor:

@@ -115,9 +115,9 @@ def test_a_chain_of_products_and_norms(ops, tokens):
 
     def run():
         before = ops.launches
-        y = ops.linear(a, wo, None, r)
+        y = ops.linear_before_norm(a, wo, None, r)
         normed = ops.rms_norm(y, g1, 1e-6)
-        z = ops.linear(ops.linear_swiglu(normed, wgu), wd, None, ops.materialized(y))
+        z = ops.linear_before_norm(ops.linear_swiglu(normed, wgu), wd, None, ops.materialized(y))
         normed = ops.rms_norm(z, g2, 1e-6)
         q = ops.qkv_projection(normed, wqkv, None, None, None, None, None, heads, kv_heads, d, page)
         stream = ops.materialized(z)
