@@ -342,7 +342,11 @@ def materialized(x):
         return x.value
     if isinstance(x, PendingProduct):
         if x.value is None:
-            _cluster_product(x, None)
+            source, squares, _, _ = x.operand
+            if squares is None and _few_tokens(source, source.shape[1], False, RESIDUAL_KIND, x.weight.shape[0]):
+                x.value = _few_token_product(source, x.weight, x.residual, None, 0.0)
+            else:
+                _cluster_product(x, None)
         return x.value
     if isinstance(x, (PendingNorm, ScaledNorm)):
         if x.value is None:
@@ -478,15 +482,20 @@ def _few_tokens(x: torch.Tensor, k: int, normed: bool = False, kind: int = GATE_
 # 128 weight rows and finishes its tokens itself), with the RMSNorm before it and what follows it inside.
 # False sends such products to the other kernels and their sums (tests compare the two).
 use_cluster_products = True
-# From how many tokens on, by the width of the rows that the norms read. Measured, us, the four products of a layer with
-# their norms in a row, other kernels / these. Width 896: 8 tokens 14.8 / 19.0, 16 19.7 / 19.9, 18 23.6 / 19.8, 64 36.6 / 26.5; 1,536:
-# 8 tokens 23.0 / 27.6, 9 29.0 / 27.5, 16 29.8 / 28.5, 40 43.0 / 30.6, 64 44.4 / 32.9, 100 48.2 / 43.0. From 2,048 on the few-token
-# kernels' blocks no longer all run at once, and these are ahead from one token on: 2,048 1 token 44.7 / 37.6, 8 46.2 / 40.4,
-# 64 58.8 / 49.9; 3,584 83.9 / 79.7, 85.6 / 80.1 and 104.9 / 90.5; 5,120 109.4 / 93.5, 105.6 / 95.9 and 121.5 / 106.8.
+# They take a layer's chain of products and norms, in which each prepares the norm that the next reads; a product whose operand or sum no
+# such norm joins goes to a few-token kernel where one takes it (see `linear`). From how many tokens on, by the width of the rows that the norms
+# read. Measured, us, the four products of a layer with their norms in a row, other kernels / these. Width 896: 8 tokens 13.9 / 19.0, 16 19.7 /
+# 19.9, 17 22.5 / 19.6, 64 35.3 / 24.2; 1,536: 8 tokens 22.4 / 27.6, 9 28.8 / 27.5, 16 29.5 / 28.5, 40 43.3 / 30.1, 64 44.3 / 31.8, 100 47.9 / 37.4.
+# From 2,304 on these are ahead from one token on: 2,304 1 token 27.9 / 23.2 (gate|up of 8,192 rows) and 53.5 / 44.5 (27,648), 8 tokens 28.8 / 25.4 and
+# 55.5 / 47.0; 3,584 83.8 / 78.0 and 86.7 / 80.6, 64 tokens 104.7 / 89.1; 5,120 109.4 / 89.1, 103.7 / 92.5 and 120.4 / 103.4. From 2,048
+# on they are only where gate|up has more rows than the few-token kernel's blocks of 128 and the SMs make: 22,016 rows, 1 token 42.5 / 36.1, 8 43.9 / 38.4;
+# 16,384 rows 29.7 / 30.7 and 30.9 / 32.2; 11,008 rows 25.1 / 25.6 and 25.8 / 27.8.
 CLUSTER_MIN_TOKENS = 9
 CLUSTER_MIN_TOKENS_NARROW = 17        # rows narrower than this:
 CLUSTER_NARROW = 1024
-CLUSTER_WIDE = 2048                   # ... and of rows from this width on, every number of tokens
+CLUSTER_WIDE = 2048                   # ... of rows from this width on, every number of tokens where gate|up has many rows,
+CLUSTER_WIDER = 2304                  # and from this one on always
+FEW_TOKENS_GATE_ROWS = 128
 CLUSTER_MAX_TOKENS = 128
 
 
@@ -639,25 +648,18 @@ def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str 
     if activation not in ACTIVATIONS:
         raise KernelError(f"linear: activation '{activation}' (known: gelu_erf, gelu_tanh, relu2)")
     if activation is None and _plain_product(x, weight, bias, out_dtype):
-        if residual is not None and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0]):
-            pending = _pending_product(x, weight, residual)
-            if pending is not None:
-                _cluster_product(pending, None)
-                return pending.value
-        source, norm_weight, eps = _norm_of(x)
-        if (_few_tokens(source, weight.shape[1], norm_weight is not None, RESIDUAL_KIND, weight.shape[0]) and source.dim() == 2 and source.shape[1] == weight.shape[1]
-                and source.is_contiguous() and weight.is_contiguous()):
-            residual_now = materialized(residual)
-            m, n = source.shape[0], weight.shape[0]
-            if residual_now is not None:
-                _need(residual_now, "linear: residual", torch.bfloat16)
-                if tuple(residual_now.shape) != (m, n):
-                    raise KernelError(f"linear: residual is {tuple(residual_now.shape)}, the product is [{m}, {n}]")
-            out = torch.empty((m, n), dtype=torch.bfloat16, device=source.device)
-            lib = _lib("gemv_mma")
-            _check(lib, lib.pae_linear_few_tokens(_ptr(out), _ptr(source), _ptr(weight), _ptr(residual_now), _ptr(norm_weight),
-                                                  eps, m, n, weight.shape[1], _ptr(_error_flag(source.device)), _stream()))
-            return out
+        # Alone, a product runs as a few-token kernel where one takes it (1,024 x 1,024, 16 tokens: 2.0 us, by clusters 3.1; 2,048 x 5,504, 8
+        # tokens: 5.2 and 6.4); what a cluster's epilogue saves is the norm behind it.
+        clusters = residual is not None and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0])
+        if not (clusters and isinstance(x, ScaledNorm) and x.value is None):
+            source, norm_weight, eps = _norm_of(x)
+            if (_few_tokens(source, weight.shape[1], norm_weight is not None, RESIDUAL_KIND, weight.shape[0]) and source.dim() == 2 and source.shape[1] == weight.shape[1]
+                    and source.is_contiguous() and weight.is_contiguous()):
+                return _few_token_product(source, weight, materialized(residual), norm_weight, eps)
+        pending = _pending_product(x, weight, residual) if clusters else None
+        if pending is not None:
+            _cluster_product(pending, None)
+            return pending.value
     x = materialized(x)
     residual = materialized(residual)
     _need(x, "linear: x")
@@ -701,11 +703,19 @@ def linear_before_norm(x, weight, bias=None, residual=None, out_dtype=None):
     `PendingProduct`, which that norm has run with the norm inside; `materialized` hands out its tensor. x and the residual are not to be
     written before."""
     if (residual is not None and _plain_product(x, weight, bias, out_dtype)
-            and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0])):
+            and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0])
+            and not _few_tokens_layer(x.shape[0], weight.shape[0], x.shape[-1], x.device)):
         pending = _pending_product(x, weight, residual)
         if pending is not None:
             return pending
     return linear(x, weight, bias, residual, out_dtype)
+
+
+def _few_tokens_layer(tokens: int, width: int, k: int, device) -> bool:
+    """Whether the layer of a product of CLUSTER_WIDE rows or some more is faster as few-token kernels. Of the layer's gate|up only the down product knows
+    the rows (2 K); the attention's output product (K the heads' width) runs as a few-token kernel at these widths, and the norm behind it alone where
+    gate|up goes to clusters."""
+    return tokens < CLUSTER_MIN_TOKENS and width < CLUSTER_WIDER and use_few_token_products and (k <= width or 2 * k <= FEW_TOKENS_GATE_ROWS * _sm_count(device))
 
 
 def _plain_product(x, weight, bias, out_dtype) -> bool:
@@ -725,6 +735,19 @@ def _pending_product(x, weight, residual):
     if tuple(residual.shape) != (x.shape[0], weight.shape[0]):
         raise KernelError(f"linear: residual is {tuple(residual.shape)}, the product is [{x.shape[0]}, {weight.shape[0]}]")
     return PendingProduct(operand, weight, residual)
+
+
+def _few_token_product(source, weight, residual, norm_weight, eps) -> torch.Tensor:
+    m, n = source.shape[0], weight.shape[0]
+    if residual is not None:
+        _need(residual, "linear: residual", torch.bfloat16)
+        if tuple(residual.shape) != (m, n):
+            raise KernelError(f"linear: residual is {tuple(residual.shape)}, the product is [{m}, {n}]")
+    out = torch.empty((m, n), dtype=torch.bfloat16, device=source.device)
+    lib = _lib("gemv_mma")
+    _check(lib, lib.pae_linear_few_tokens(_ptr(out), _ptr(source), _ptr(weight), _ptr(residual), _ptr(norm_weight),
+                                          eps, m, n, weight.shape[1], _ptr(_error_flag(source.device)), _stream()))
+    return out
 
 
 def _linear_tensor_cores(x, weight, bias, residual, out_dtype, m, n, k, activation: int = 0) -> torch.Tensor:
@@ -843,27 +866,33 @@ def qkv_projection(x, weight, bias, table, slots, keys, values, num_heads, num_k
     for few tokens fuse the other way round (the split sum runs inside the rotation kernel)."""
     m, k = x.shape
     n = weight.shape[0]
-    # A plain operand of more than 64 tokens keeps the bits of `linear` followed by the rotation (a prompt's first layer only: in
-    # the others the product before has prepared the norm).
-    if (m <= CLUSTER_MAX_TOKENS and (m <= SWAPPED_MAX_TOKENS or isinstance(x, ScaledNorm)) and _cluster_takes(m, n, k, weight, k) and n == (num_heads + 2 * num_kv_heads) * head_dim
+    scaled = isinstance(x, ScaledNorm) and x.value is None
+    if not scaled:
+        source, norm_weight, eps = _norm_of(x)
+        few = _few_tokens(source, k, norm_weight is not None, QKV_KIND, n)
+    # An operand that no product before has prepared goes to a few-token kernel where one takes it (3,072 x 2,048, 8 tokens: 3.2 us, by clusters
+    # 4.6); of more than 64 tokens it keeps the bits of `linear` followed by the rotation.
+    if ((scaled or (not few and m <= SWAPPED_MAX_TOKENS)) and _cluster_takes(m, n, k, weight, k) and n == (num_heads + 2 * num_kv_heads) * head_dim
             and (slots is None or (keys.dtype == torch.bfloat16 and values.dtype == torch.bfloat16))):
         operand = _cluster_operand(x)
         lib = _lib("gemm_cluster")
         if (operand is not None and lib.pae_qkv_cluster_supports(head_dim) and _aligned(bias, table)
                 and (slots is None or _aligned(keys, values))):
-            source, squares, width, eps = operand
-            _need(source, "qkv_projection: x")
+            rows, squares, width, norm_eps = operand
+            _need(rows, "qkv_projection: x")
             _need(weight, "qkv_projection: weight")
             _need_qkv(bias, table, slots, keys, values, m, n, head_dim)
-            out = torch.empty((m, n), dtype=torch.bfloat16, device=source.device)
+            out = torch.empty((m, n), dtype=torch.bfloat16, device=rows.device)
             _set_bounds("gemm_cluster", keys if slots is not None else None)
             _check(lib, lib.pae_qkv_cluster(
-                _ptr(out), _ptr(source), _ptr(weight), _ptr(bias), _ptr(squares), 0 if squares is None else squares.shape[0], width, eps,
+                _ptr(out), _ptr(rows), _ptr(weight), _ptr(bias), _ptr(squares), 0 if squares is None else squares.shape[0], width, norm_eps,
                 _ptr(table), _ptr(slots), _ptr(keys if slots is not None else None), _ptr(values if slots is not None else None), m,
-                num_heads, num_kv_heads, head_dim, page_size, k, _early_weights(m, k), 0, 0, 0, _ptr(_error_flag(source.device)), _stream()))
+                num_heads, num_kv_heads, head_dim, page_size, k, _early_weights(m, k), 0, 0, 0, _ptr(_error_flag(rows.device)), _stream()))
             return out
-    source, norm_weight, eps = _norm_of(x)
-    if (_few_tokens(source, k, norm_weight is not None, QKV_KIND, n) and weight.dtype == torch.bfloat16 and weight.is_contiguous() and weight.data_ptr() % 16 == 0
+    if scaled:
+        source, norm_weight, eps = _norm_of(x)
+        few = _few_tokens(source, k, norm_weight is not None, QKV_KIND, n)
+    if (few and weight.dtype == torch.bfloat16 and weight.is_contiguous() and weight.data_ptr() % 16 == 0
             and n == (num_heads + 2 * num_kv_heads) * head_dim and weight.shape[1] == k and head_dim % 16 == 0
             and (slots is None or (keys.dtype == torch.bfloat16 and values.dtype == torch.bfloat16))):
         _need(source, "qkv_projection: x")
@@ -1124,22 +1153,34 @@ def linear_swiglu(x, weight, gate: str = "silu") -> torch.Tensor:
     tokens the activation runs in the product's epilogue; with few, in the kernel that sums the
     splits; otherwise as a kernel of its own. Gate and up are rounded to the engine dtype first in
     every one of them, so all give the same bits."""
-    if (x.shape[0] <= CLUSTER_MAX_TOKENS and x.dtype == torch.bfloat16 and weight.shape[0] % 32 == 0 and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[1])
-            and not _uneven_gate(x.shape[0], weight.shape[0], x.device)):
+    scaled = isinstance(x, ScaledNorm) and x.value is None
+    takes = (x.dtype == torch.bfloat16 and weight.shape[0] % 32 == 0 and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[1])
+             and not _uneven_gate(x.shape[0], weight.shape[0], x.device))
+    if not scaled:
+        source, norm_weight, eps = _norm_of(x)
+        few = _few_tokens(source, weight.shape[1], norm_weight is not None, GATE_UP_KIND, weight.shape[0])
+        if few and takes and norm_weight is not None and weight.shape[0] > FEW_TOKENS_GATE_ROWS * _sm_count(x.device):
+            few = False
+    # As in `qkv_projection`: an operand that no product before has prepared goes to a few-token kernel where one takes it (11,008 x 2,048, 8 tokens: 9.2 us,
+    # by clusters 10.4), and of more than 64 tokens to the many-token kernel unless K is long (8,192 x 1,024, 100 tokens: 7.6 and 8.7; 11,008
+    # x 2,048 13.7 and 12.7).
+    if takes and (scaled or (not few and (x.shape[0] <= SWAPPED_MAX_TOKENS or weight.shape[1] >= SWAPPED_LONG_K))):
         operand = _cluster_operand(x)
         if operand is not None:
-            source, squares, width, eps = operand
-            m, n, k = source.shape[0], weight.shape[0], weight.shape[1]
-            _need(source, "linear_swiglu: x")
+            rows, squares, width, norm_eps = operand
+            m, n, k = rows.shape[0], weight.shape[0], weight.shape[1]
+            _need(rows, "linear_swiglu: x")
             _need(weight, "linear_swiglu: weight")
-            out = torch.empty((m, n // 2), dtype=torch.bfloat16, device=source.device)
+            out = torch.empty((m, n // 2), dtype=torch.bfloat16, device=rows.device)
             lib = _lib("gemm_cluster")
             _check(lib, lib.pae_linear_swiglu_cluster(
-                _ptr(out), _ptr(source), _ptr(weight), _ptr(squares), 0 if squares is None else squares.shape[0], width, eps, m, n, k,
-                GATE_KINDS[gate], _early_weights(m, k), 0, 0, 0, _ptr(_error_flag(source.device)), _stream()))
+                _ptr(out), _ptr(rows), _ptr(weight), _ptr(squares), 0 if squares is None else squares.shape[0], width, norm_eps, m, n, k,
+                GATE_KINDS[gate], _early_weights(m, k), 0, 0, 0, _ptr(_error_flag(rows.device)), _stream()))
             return out
-    source, norm_weight, eps = _norm_of(x)
-    if (_few_tokens(source, weight.shape[1], norm_weight is not None, GATE_UP_KIND, weight.shape[0]) and weight.dtype == torch.bfloat16 and weight.is_contiguous()
+    if scaled:
+        source, norm_weight, eps = _norm_of(x)
+        few = _few_tokens(source, weight.shape[1], norm_weight is not None, GATE_UP_KIND, weight.shape[0])
+    if (few and weight.dtype == torch.bfloat16 and weight.is_contiguous()
             and weight.data_ptr() % 16 == 0 and weight.shape[0] % 32 == 0 and source.shape[1] == weight.shape[1]):
         _need(source, "linear_swiglu: x")
         out = torch.empty((source.shape[0], weight.shape[0] // 2), dtype=torch.bfloat16, device=source.device)
