@@ -63,6 +63,10 @@ class DecoderModel:
             out += [layer.block, *layer.parts.values()]
         return out
 
+    def plans_decode(self, seqs: int, max_kv_len: int, page_size: int) -> bool:
+        """Whether some part plans the slices of a step of `seqs` single tokens when their contexts are of unequal lengths."""
+        return any(part.plans_decode(seqs, max_kv_len, page_size) for part in self.parts() if hasattr(part, "plans_decode"))
+
     def forward(self, ctx, entry_caches) -> torch.Tensor | None:
         """Runs the step's tokens through every schedule entry; float32 logits
         [wanted, vocab] at `ctx.logit_rows`, or None when nothing is wanted."""

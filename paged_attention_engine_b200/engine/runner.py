@@ -61,9 +61,10 @@ class _DecodeGraph:
 
 
 class ModelRunner:
-    # A graph per (batch size, block-table width, longest context rounded up, sampling, contexts of unequal lengths). They share
-    # one memory pool (they never run at the same time), so a graph costs its launches and little else.
-    MAX_GRAPHS = 512
+    # A graph per (batch size, block-table width, longest context rounded up, sampling, slices planned for contexts of unequal lengths). They share
+    # one memory pool (they never run at the same time), so a graph costs its launches and little else. Batches of up to 256 requests and contexts
+    # of up to 4,096 keys make 44 x 9 of them, and as many again at most where slices are planned.
+    MAX_GRAPHS = 1024
     # A recorded step plans its attention (how the keys are sliced) for a longest context that is
     # fixed in the recording: the true longest context rounded up to a multiple of this many
     # keys, not to the block table's width, which is a power of two (at context 4,097 the table
@@ -89,6 +90,7 @@ class ModelRunner:
         self.use_graphs = (use_graphs and self.runtime.device.type == "cuda" and model.graph_safe
                            and not getattr(self.runtime.ops, "bounds_checked", False))
         self.graphs: dict[tuple[int, int, int, bool, bool], _DecodeGraph] = {}
+        self.planned: dict[tuple[int, int], bool] = {}      # per (batch size, longest context rounded up): whether slices are planned at all
         self.graph_pool = None
         self.capture_stream = None
         self.graph_replays = 0
@@ -142,7 +144,14 @@ class ModelRunner:
         while width * page < longest:
             width *= 2
         bucket = min(width * page, -(-longest // self.KV_BUCKET) * self.KV_BUCKET)
-        return (self.graph_batch(len(entries)), width, bucket, sampling is not None, ragged_contexts(keys, len(entries), bucket))
+        batch = self.graph_batch(len(entries))
+        return (batch, width, bucket, sampling is not None, ragged_contexts(keys, len(entries), bucket) and self._plans_decode(batch, bucket))
+
+    def _plans_decode(self, batch: int, bucket: int) -> bool:
+        plans = self.planned.get((batch, bucket))
+        if plans is None:
+            plans = self.planned[batch, bucket] = self.model.plans_decode(batch, bucket, self.manager.block_size)
+        return plans
 
     def _shape_key(self, entries, sampling) -> tuple | None:
         """The exact shape of a step that is not decode-only (per entry: tokens, start, wanted places,

@@ -968,6 +968,12 @@ use_decode_plans = True
 PLANNED_MIN_TILES = 4000
 
 
+def plans_decode(seqs: int, max_kv_len: int, num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, dtype) -> bool:
+    """Whether `plan_decode` plans the slices of a step of these sizes."""
+    return (use_decode_plans and seqs * num_kv_heads * ((max_kv_len + 15) // 16 + 1) >= PLANNED_MIN_TILES and seqs <= 2048
+            and plain_attention_takes(num_heads, num_kv_heads, head_dim, page_size, dtype))
+
+
 def plan_decode(q_start, kv_len, max_kv_len: int, num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, window: int,
                 dtype) -> None:
     """Plans the slices of a step of single tokens, once a step for all layers of the same kv heads and window: the
@@ -975,8 +981,7 @@ def plan_decode(q_start, kv_len, max_kv_len: int, num_heads: int, num_kv_heads: 
     seqs = kv_len.numel()
     key = (num_kv_heads, head_dim, window)
     tiles = (max_kv_len + 15) // 16 + 1
-    if (not use_decode_plans or seqs * num_kv_heads * tiles < PLANNED_MIN_TILES or seqs > 2048 or key in getattr(kv_len, "decode_plans", {})
-            or not plain_attention_takes(num_heads, num_kv_heads, head_dim, page_size, dtype)):
+    if key in getattr(kv_len, "decode_plans", {}) or not plans_decode(seqs, max_kv_len, num_heads, num_kv_heads, head_dim, page_size, dtype):
         return
     lib = _lib("attention_mma")
     for name, t in (("q_start", q_start), ("kv_len", kv_len)):

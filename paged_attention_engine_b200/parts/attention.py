@@ -67,6 +67,11 @@ class GQAAttention(Part):
         built = self.build_sub_parts(tensors)
         self.position_encoding = built[0] if built else None
 
+    def plans_decode(self, seqs: int, max_kv_len: int, page_size: int) -> bool:
+        """Whether a step of `seqs` single tokens of unequal contexts, planned for `max_kv_len` keys, runs other kernels than one of equal contexts."""
+        plans = getattr(self.ops, "plans_decode", None)
+        return plans is not None and plans(seqs, max_kv_len, self.num_heads, self.num_kv_heads, self.head_dim, page_size, self.runtime.dtype)
+
     def forward(self, ctx, x, residual, cache):
         ops = self.ops
         group = ctx.groups[cache.group]

@@ -58,3 +58,37 @@ def test_a_recording_without_room_leaves_nothing_to_the_eager_step(folder):
     assert len(recorded) == 1 and ran[-1] is not recorded[0]
     assert not hasattr(ran[-1].kv_len, "decode_plans")
     assert torch.equal(got, want)
+
+
+def _keys(runner, contexts_of_steps):
+    """The recordings that decode steps of requests with these contexts ask for."""
+    keys = set()
+    for contexts in contexts_of_steps:
+        runner.manager.num_computed = lambda key, contexts=contexts: contexts[key]
+        keys.add(runner._graph_key([StepEntry(i, (1,), (0,)) for i in range(len(contexts))], None))
+    return keys
+
+
+@pytest.mark.parametrize("plans", [False, True])
+def test_contexts_of_unequal_lengths_get_recordings_of_their_own_only_where_slices_are_planned(folder, plans):
+    runner = _runner(folder, {"a": 0})
+    runner.use_graphs = True
+    asked = []
+    runner.model.plans_decode = lambda seqs, max_kv_len, page_size: (asked.append((seqs, max_kv_len, page_size)), plans and seqs >= 8)[1]
+    # Four requests that grow from 16 to 4,095 keys: a recording per longest context rounded up (256, 512, then every 512).
+    assert len(_keys(runner, [[n] * 4 for n in range(16, 4096)])) == 9
+    assert len(_keys(runner, [[n, 16, 16, 16] for n in range(16, 4096)])) == 9
+    # Sixteen: where they are planned, unequal ones another each.
+    equal = _keys(runner, [[n] * 16 for n in range(400, 4096, 512)])
+    unequal = _keys(runner, [[n] + [16] * 15 for n in range(400, 4096, 512)])
+    assert len(equal) == len(unequal) == 8 and (equal.isdisjoint(unequal) if plans else equal == unequal)
+    assert len(asked) == len(set(asked)), "asked once per size"
+
+
+def test_every_decode_step_of_the_largest_batches_finds_room_for_its_recording(folder):
+    runner = _runner(folder, {"a": 0})
+    runner.use_graphs = True
+    runner.model.plans_decode = lambda *sizes: True
+    steps = [[n] * b for n in range(15, 4096, 64) for b in range(1, 257)]
+    steps += [[n] + [0] * (b - 1) for n in range(15, 4096, 64) for b in range(1, 257)]
+    assert len(_keys(runner, steps)) <= runner.MAX_GRAPHS
