@@ -944,9 +944,13 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
         return true;
       };
       int page0 = first_page;
-      bool ok = load(false, 0, page0);
+      bool ok = true;
+      int keys_issued = 0, values_issued = 0;
+      if (n_tiles > 0) {                                        // a request without a visible key has none: nobody would wait for a copy
+        ok = load(false, 0, page0);
+        keys_issued = 1;
+      }
       int page1 = page_of(1), page2 = page_of(2);               // of tiles t, t + 1, t + 2
-      int keys_issued = 1, values_issued = 0;
       if (n_tiles > 1) {
         ok = ok && load(false, 1, page1);
         keys_issued = 2;

@@ -64,3 +64,20 @@ def test_where_the_pages_lie_changes_no_bit(form, d, page, requests, window):
     want = ref.paged_attention(qkv, keys, values, table, torch.tensor(q_start), torch.tensor([c for c, _ in requests]), torch.tensor(kv_len), **args).float()
     assert (got.cpu().float() - want).abs().max() <= 2.0 ** -6 * max(1.0, float(want.abs().max()))
     ops.check_device_errors()
+
+
+@pytest.mark.parametrize("form", [1, 2, 4])
+def test_a_request_without_a_visible_key_disturbs_nothing(form):
+    """A request of 70 tokens whose length says 0: no copy is made for it, and its neighbours' outputs keep their bits."""
+    from paged_attention_engine_b200.kernels import ops
+
+    heads, kv_heads, d, page = 4, 2, 128, 16
+    gen = torch.Generator().manual_seed(3)
+    qkv = torch.randn((70 + 90, (heads + 2 * kv_heads) * d), generator=gen).to(torch.bfloat16).cuda()
+    keys, values = (torch.randn((12, kv_heads, page, d), generator=gen).to(torch.bfloat16).cuda() for _ in range(2))
+    args = dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=d, page_size=page, max_q_len=90, max_kv_len=90, scale=d ** -0.5, window=0, form=form)
+    table = torch.arange(12, dtype=torch.int32).view(2, 6).cuda()
+    got = ops.paged_attention(qkv, keys, values, table, _i32([0, 70, 160]), _i32([0, 0]), _i32([0, 90]), **args)
+    alone = ops.paged_attention(qkv[70:].contiguous(), keys, values, table[1:].contiguous(), _i32([0, 90]), _i32([0]), _i32([90]), **args)
+    assert torch.equal(got[70:], alone)
+    ops.check_device_errors()
