@@ -657,9 +657,14 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_planned_kernel(const P
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = p.heads / p.kv_heads, g = h / groups;
   const int token = p.q_start[b];
+  const bool single = p.q_start[b + 1] - token == 1;
   const PairSlices pair = a.pairs[(size_t)b * p.kv_heads + g];
   dependent_launch_wait();
-  if (pair.count < 2) return;                 // not a request of one token; or finished by its one warp
+  if (pair.count < 2) {                       // not a request of one token; or finished by its one warp; or one without a key
+    if (pair.count == 0 && single)
+      for (int d = threadIdx.x; d < D; d += blockDim.x) a.out[((size_t)token * p.heads + h) * D + d] = __float2bfloat16_rn(0.f);
+    return;
+  }
   const int slices = min(p.max_slices, pair.count);
   const size_t at = (size_t)(h - g * groups) * a.items + pair.first;
   constexpr int PER_LANE = D / 32;

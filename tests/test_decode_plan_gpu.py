@@ -55,6 +55,25 @@ def test_the_slices_cover_every_request(ops, lengths, window, kv_heads, items, l
     assert length <= 16 * max(least, max(tiles))
 
 
+def test_a_request_without_a_key_leaves_zeros(ops):
+    """As without a plan: no slice is made for it, and its row is written all the same."""
+    heads, kv_heads, d, page, lengths = 4, 2, 64, 16, [70, 0, 33, 1]
+    gen = torch.Generator().manual_seed(5)
+    qkv = torch.randn((4, (heads + 2 * kv_heads) * d), generator=gen).to(torch.bfloat16).cuda()
+    keys, values = (torch.randn((20, kv_heads, page, d), generator=gen).to(torch.bfloat16).cuda() for _ in range(2))
+    table, kv_len = torch.arange(20, dtype=torch.int32).view(4, 5).cuda(), _i32(lengths)
+    q_start, pos0 = _i32([0, 1, 2, 3, 4]), _i32([n - 1 for n in lengths])
+    args = dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=d, page_size=page, max_q_len=1, max_kv_len=70, scale=d ** -0.5, window=0)
+    alone = ops.paged_attention(qkv, keys, values, table, q_start, pos0, kv_len, **args)
+    ops.PLANNED_MIN_TILES = 1
+    ops.plan_decode(q_start, kv_len, 70, heads, kv_heads, d, page, 0, torch.bfloat16)
+    ops.PLANNED_MIN_TILES = 4000
+    torch.full((4, heads * d), float("nan"), dtype=torch.bfloat16, device="cuda")      # what the allocator hands out next
+    got = ops.paged_attention(qkv, keys, values, table, q_start, pos0, kv_len, **args)
+    assert (alone[1] == 0).all() and (got[1] == 0).all() and torch.isfinite(got).all()
+    ops.check_device_errors()
+
+
 @pytest.mark.parametrize("heads,kv_heads,d,page,window", [(12, 2, 128, 16, 0), (28, 4, 128, 16, 0), (8, 8, 64, 32, 0), (4, 1, 32, 16, 90), (12, 2, 128, 48, 300)])
 @pytest.mark.parametrize("lengths", [[1, 900, 17, 16, 33, 2000, 400], [700] * 3 + [5] * 30, [64]])
 def test_attention_over_planned_slices(ops, heads, kv_heads, d, page, window, lengths):
