@@ -36,23 +36,24 @@ def test_the_slices_cover_every_request(ops, lengths, window, kv_heads, items, l
     assert lib.pae_plan_decode(plan.data_ptr(), q_start.data_ptr(), kv_len.data_ptr(), seqs, kv_heads, window, items, least, 0) == 0
     plan = plan.cpu().numpy()
     slices, pairs = plan[: 4 * items].reshape(items, 4), plan[4 * items :].reshape(seqs, kv_heads, 2)
-    used, length = 0, 0
+    # The rule: the shortest slices, in steps of a 32nd and from `least` tiles and an even share on, that are no more than `items`; one a pair at the most.
+    tiles = [(n + 15) // 16 - (max(0, n - window) // 16 if window else 0) for n in lengths]
+    length = max(least, -(-sum(tiles) * kv_heads // items))
+    while sum(-(-t // length) for t in tiles) * kv_heads > items and max(tiles) > length:
+        length += max(1, length // 32)
+    used = 0
     for b, n in enumerate(lengths):
         base = max(0, n - window) // 16 * 16 if window else 0
         for g in range(kv_heads):
             first, count = pairs[b, g]
-            assert count == 0 if n == 0 else count >= 1
+            assert first == used and count == -(-tiles[b] // length)
             at = base
             for request, head, begin, end in slices[first : first + count]:
-                assert (request, head, begin) == (b, g, at) and begin < end <= n
-                length = max(length, int(end - begin))
+                assert (request, head, begin, end) == (b, g, at, min(n, at + 16 * length)) and begin < end
                 at = end
             assert n == 0 or at == n
-            assert first == used
             used += count
     assert used <= items and (slices[used:, 2] >= slices[used:, 3]).all()
-    tiles = [(n + 15) // 16 - (max(0, n - window) // 16 if window else 0) for n in lengths]
-    assert length <= 16 * max(least, max(tiles))
 
 
 def test_a_request_without_a_key_leaves_zeros(ops):
