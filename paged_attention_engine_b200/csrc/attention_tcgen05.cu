@@ -62,7 +62,7 @@ struct Params {
   int table_width, heads, kv_heads, page_size, window, skip_single;
   const int* work_index;  // the requests that this launch works on, one per grid z (null: request z)
   float scale_log2;
-  float slack;            // paired form: a row's reference follows its maximum in steps of more than 2^slack
+  float slack;            // paired form: a row's reference may lie below its maximum by 2^slack (0: it follows every maximum)
   int* error;
 };
 
@@ -708,19 +708,21 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
 // operand there: no trip through shared memory (sixteen-byte stores into the swizzled layout, a proxy fence, and 16 KB that
 // the tensor core reads back), and the softmax never waits for a product unless a reference moves. The thread that issues the MMAs
 // waits for the product of the tile before last before the next scores are written over the probabilities it reads; its warp runs the
-// role together and an elected lane issues, and K is asked for two tiles ahead of its scores (8,192 tokens, 12 heads: 261 -> 235 us). Scale
-// and sum take two scores an instruction. The kernel is bound by the chain of a tile's steps (the special-function
-// units work 38 % of the time, the tensor cores 50 %, issue slots are 32 % busy): 8,192 tokens, 12 heads of 128: 277 -> 258 us (800 TFLOP/s), 28 heads:
-// 596 -> 547 us (880); with the probabilities still in shared memory 266 and 568, without the instructions on pairs 268 and 570.
+// role together and an elected lane issues, and K is asked for two tiles ahead of its scores. Scale and sum take two scores an instruction. 8,192 tokens,
+// 12 heads of 128, us: 277 with the probabilities in shared memory and one score an instruction, 258 without, 235 with K asked for early, 173 with a
+// tile's pages in one box and no look at the maximum (below): 1,190 TFLOP/s, bound by the exponentials and by the tensor cores' turns between two blocks.
 //
-// The reference of a row is its running maximum, but in launches that fill the GPU it only moves when the maximum has grown
-// by more than 2^8 since it was set: probabilities then stay below 256, which float32 sums and
-// the bfloat16 operand hold as well as values below 1, and the output in tensor memory (which
-// must be multiplied by 2^(old - new) whenever the reference moves) is touched on a row's first
-// tiles only. The sum is kept against the same reference, so the quotient is exact softmax. A largest probability that is not
-// 1 is rounded, though: 0.2 to 1.5 % further from 64 bits than the wide form (509 tokens after 512: 0.00229 and 0.00232 of the
-// outputs' norm). Smaller launches, which would otherwise take the wide form, move it with every new maximum: a little closer
-// than the wide form (0.00228) for 0.6 us at 100 tokens (7.9 -> 8.5), 1.5 at 6 requests of 300 (14.1 -> 15.6).
+// The reference of a row is its running maximum, but in launches that fill the GPU it is left behind: probabilities are taken against it
+// without a look at the tile's maximum (which costs a pass over the scores), and while the tile's sum is at most REFERENCE_LIMIT, 2^8, for every row of the warp, that
+// holds: no probability is above 2^8, which float32 sums and the bfloat16 operand hold as well as values below 1. A tile with a larger sum
+// is taken again with all references of the warp moved to their maxima; only then is the output in tensor memory (which must be multiplied by 2^(old - new))
+// touched. The sum is kept against the same reference, so the quotient is exact softmax. A largest probability that is not
+// 1 is rounded, though: 1 % further from 64 bits than the wide form, 2 to 5 % where the maxima grow all along the keys by 2^8 to 2^100
+// in all. The limit is what bounds that: with 2^10 the error is up to 0.6 % larger, with 2^40 up to 2 % (head size 64, 1,500 tokens after
+// 3,000, growth 2^100: 0.002290, 0.002303 and 0.002337 of the outputs' norm; moved where the maximum had grown by 2^8, with a look at every tile's:
+// 0.002304); taking tiles again costs growing maxima 102 -> 111 us (2^8 over 1,500 tokens after 3,000, 28 heads of 128) to 156 (2^100). Smaller launches, which would
+// otherwise take the wide form, move it with every new maximum: a little closer than the wide form (0.00228) for 0.6 us at 100 tokens (7.9 -> 8.5), 1.5 at 6
+// requests of 300 (14.1 -> 15.6).
 // ---------------------------------------------------------------------------------------
 namespace paired {
 
@@ -729,7 +731,7 @@ constexpr int THREADS = 192;        // TMA warp, MMA warp, four softmax warps (o
 constexpr int SOFTMAX_WARPS = 4;
 constexpr int KV_STAGES = 2;
 constexpr float REFERENCE_SLACK = 8.f;   // of launches that fill the GPU; 0 below that (`launch`)
-constexpr float REFERENCE_LIMIT = 1099511627776.f;      // 2^40: a tile's sum beyond it moves the reference
+constexpr float REFERENCE_LIMIT = 256.f; // 2^REFERENCE_SLACK: of a tile's sum against its rows' references
 
 // 64 consecutive float32 columns of this thread's lane of tensor memory.
 __device__ __forceinline__ void tmem_load64(uint32_t address, float* v) {
@@ -1087,9 +1089,10 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
       };
       const uint32_t scores = lane_base + st * L::S_COLUMNS;
       bool taken = false;
+      float slack = p.slack;
       if (p.slack > 0.f && !__any_sync(0xffffffffu, reference == -FLT_MAX)) {
         // Every row has a reference: the probabilities are taken against it without a look at the tile's maximum, the second half
-        // of the scores on its way meanwhile. Should a sum come out beyond REFERENCE_LIMIT (or not a number), the tile is taken again below.
+        // of the scores on its way meanwhile. Should a sum come out above REFERENCE_LIMIT (or not a number), the tile is taken again below.
         float s[32], behind[32];
         tmem_ask32(scores, s);
         tmem_arrived(s);
@@ -1101,6 +1104,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
         const float sum = tile_sum();
         taken = __all_sync(0xffffffffu, sum <= REFERENCE_LIMIT);
         if (taken) row_sum += sum;
+        else slack = 0.f;                  // every row of the warp starts anew from its maximum: the next tiles are taken at once again
       }
       if (!taken) {
         float s[BKEYS];
@@ -1115,7 +1119,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
         }
         float tile_max = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
         if (tile_max != -FLT_MAX) tile_max *= p.scale_log2;        // the scale is positive: max(s) scales with it
-        const bool moves = tile_max > reference + p.slack || (reference == -FLT_MAX && tile_max != -FLT_MAX);
+        const bool moves = tile_max > reference + slack || (reference == -FLT_MAX && tile_max != -FLT_MAX);
         if (__any_sync(0xffffffffu, moves)) {
           // Some row of this warp moves its reference: its sum and its row of O are multiplied
           // by 2^(old - new); the other rows by 1. Reading and writing tensor memory takes the whole warp.
