@@ -75,7 +75,9 @@ struct Params {
   __nv_bfloat16* values;
   int heads, kv_heads, log_d, page_size;
   int* error;
+  int skip_rank, skip_kb;        // self-test of the give-up path only: the block of each cluster, and its k-block, that is never loaded
 };
+constexpr uint32_t SELFTEST_WAIT_LIMIT = 1u << 12;
 
 __device__ __forceinline__ void store_remote(uint32_t address, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(address), "f"(v) : "memory");
@@ -235,11 +237,13 @@ __device__ __forceinline__ void finish(const Params& p, int tile, int column0, i
   }
 }
 
-// Blocks rank 0 .. C - 1 of a cluster (CLUSTER; else C = 1): blockIdx.x = tile * C + rank.
-template <int KIND, bool CLUSTER>
+// Blocks rank 0 .. C - 1 of a cluster (CLUSTER; else C = 1): blockIdx.x = tile * C + rank. SELFTEST: with which a test makes a wait run out, to
+// see the give-up path work.
+template <int KIND, bool CLUSTER, bool SELFTEST = false>
 __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_product_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                      const __grid_constant__ CUtensorMap map_x, const Params p, int cluster) {
   constexpr int EPILOGUE = EPILOGUE_THREADS<CLUSTER>;
+  constexpr uint32_t limit = SELFTEST ? SELFTEST_WAIT_LIMIT : WAIT_LIMIT;
   if (!CLUSTER) cluster = 1;
   extern __shared__ uint8_t raw_smem[];
   const uint32_t raw = smem_u32(raw_smem);
@@ -295,11 +299,13 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
   if (CLUSTER) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   const uint32_t tmem_base = *tmem_holder;
   const int first = min(kb_count, stages);
+  auto skipped = [&](int i) { return SELFTEST && rank == p.skip_rank && i == p.skip_kb; };
   auto load_weights = [&](int i, int s) { tma_load_2d(base + s * stage_bytes, &map_w, full_bar(s), (kb_begin + i) * BK, column0); };
   auto load_tokens = [&](int i, int s) { tma_load_2d(base + s * stage_bytes + a_bytes, &map_x, full_bar(s), (kb_begin + i) * BK, 0); };
   if (warp == 0 && p.early) {
     if (elect_one()) {
       for (int i = 0; i < first; ++i) {
+        if (skipped(i)) continue;
         mbar_expect_tx(full_bar(i), stage_bytes);
         load_weights(i, i);
       }
@@ -320,6 +326,7 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
     const bool leader = elect_one();
     if (leader) {
       for (int i = 0; i < first; ++i) {
+        if (skipped(i)) continue;
         if (!p.early) {
           mbar_expect_tx(full_bar(i), stage_bytes);
           load_weights(i, i);
@@ -331,7 +338,7 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
     int issued = first, s = 0;
     uint32_t phase = 0;
     for (int i = first; i < kb_count; ++i) {
-      if (!mbar_wait_warp(empty_bar(s), phase, abort_flag, p.error, 1)) break;
+      if (!mbar_wait_warp(empty_bar(s), phase, abort_flag, p.error, 1, limit)) break;
       if (leader) {
         mbar_expect_tx(full_bar(s), stage_bytes);
         load_weights(i, s);
@@ -347,6 +354,7 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
     if (leader && *abort_flag) {
       // Loads that were issued still write into this block's shared memory: wait for them.
       for (int i = max(0, issued - stages); i < issued; ++i)
+        if (!skipped(i))
         for (uint32_t t = 0; t < WAIT_LIMIT && !mbar_try_wait(full_bar(i % stages), (i / stages) & 1); ++t) __nanosleep(64);
     }
     __syncwarp();
@@ -362,7 +370,7 @@ __global__ void __launch_bounds__(64 + EPILOGUE_THREADS<CLUSTER>, 2) cluster_pro
       uint32_t phase = 0;
       bool ok = true;
       for (int i = 0; i < kb_count; ++i) {
-        ok = mbar_wait_warp(full_bar(s), phase, abort_flag, p.error, 2);
+        ok = mbar_wait_warp(full_bar(s), phase, abort_flag, p.error, 2, limit);
         if (!ok) break;
         tcgen05_fence_after();
         const uint64_t offset = (uint64_t)(uint32_t)(s * (stage_bytes >> 4)), a = w_first + offset, b = x_first + offset;
@@ -663,6 +671,38 @@ PAE_EXPORT int pae_linear_swiglu_cluster(void* out, const void* x, const void* w
   if (gate_kind == kGateRelu) return launch<GATE_RELU>(p, w, x, k, rows, cluster, stages, s);
   if (gate_kind == kGateGeluTanh) return launch<GATE_GELU>(p, w, x, k, rows, cluster, stages, s);
   return launch<GATE_SILU>(p, w, x, k, rows, cluster, stages, s);
+}
+
+// Self-test of the give-up path: a product of `cluster` blocks a tile in which block `skip_rank` of every cluster never loads its k-block `skip_kb` (one of
+// its first `stages`; nothing is in flight for it). Its wait for the stage runs out after a few thousand polls, the other blocks go on, and all leave.
+PAE_EXPORT int pae_linear_cluster_selftest_giveup(void* out, const void* x, const void* w, int tokens, int n, int k, int cluster, int stages, int skip_rank,
+                                                  int skip_kb, int* error, void* stream) {
+  if (int err = check_common("linear_cluster_selftest_giveup", out, w, x, nullptr, 0, error, tokens, n, k)) return err;
+  Params p{};
+  p.tokens = tokens;
+  p.n = n;
+  p.k_blocks = (k + BK - 1) / BK;
+  p.columns = columns_of(tokens);
+  p.rows = BM;
+  p.stages = stages;
+  p.early = 1;
+  p.out = (__nv_bfloat16*)out;
+  p.error = error;
+  p.skip_rank = skip_rank;
+  p.skip_kb = skip_kb;
+  const Shape s{BM, cluster, stages};
+  const int tiles = (n + BM - 1) / BM;
+  if (cluster < 2 || cluster > MAX_CLUSTER || cluster > p.k_blocks || stages < 2 || stages > MAX_STAGES || smem_bytes(s, tokens) > 227 * 1024 || skip_rank < 0 ||
+      skip_rank >= cluster || skip_kb < 0 || skip_kb >= stages || skip_kb >= p.k_blocks / cluster)
+    return fail(2, "linear_cluster_selftest_giveup: block %d of %d, k-block %d of %d stages", skip_rank, cluster, skip_kb, stages);
+  CUtensorMap map_w, map_x;
+  if (int err = tensor_map(&map_w, w, n, k, BM)) return err;
+  if (int err = tensor_map(&map_x, x, tokens, k, p.columns)) return err;
+  static DevicesSet raised;
+  if (int err = raise_shared_memory(raised, cluster_product_kernel<RESIDUAL, true, true>, 227 * 1024, "linear_cluster_selftest_giveup")) return err;
+  launch_kernel_cluster(cluster_product_kernel<RESIDUAL, true, true>, dim3(tiles * cluster), dim3(64 + EPILOGUE_THREADS<true>), smem_bytes(s, tokens), (cudaStream_t)stream,
+                        (unsigned)cluster, map_w, map_x, p, cluster);
+  return check_launch("linear_cluster_selftest_giveup");
 }
 
 // 1 for head sizes of which a tile of 128 rows holds whole heads.

@@ -146,6 +146,26 @@ def test_all_clusters_of_a_launch_run_at_once(ops):
                     assert lib.pae_linear_cluster_rounds(tokens, n, k, gate) <= 1, (tokens, n, k, gate)
 
 
+@pytest.mark.parametrize("cluster,stages,skip", [(4, 4, (0, 1)), (4, 4, (2, 3)), (2, 8, (1, 5)), (8, 2, (7, 0))])
+def test_a_wait_that_runs_out_in_one_block_of_a_cluster(ops, cluster, stages, skip):
+    """One block of every cluster never loads one of its k-blocks: its wait gives up after a few thousand polls, the cluster's other blocks
+    do their work, all of them end, and the error word says who gave up. The next product is right."""
+    tokens, n, k = 40, 384, 1024
+    x, w = _rand((tokens, k), 20), _rand((n, k), 21, k ** -0.5)
+    out = torch.zeros((tokens, n), dtype=torch.bfloat16, device="cuda")
+    ops.check_device_errors()
+    lib = ops._lib("gemm_cluster")
+    code = lib.pae_linear_cluster_selftest_giveup(_p(out), _p(x), _p(w), tokens, n, k, cluster, stages, *skip, ops.error_flag("cuda:0").data_ptr(), 0)
+    assert code == 0, lib.pae_last_error().decode()
+    torch.cuda.synchronize()                     # the kernel came back by itself
+    assert int(ops.error_flag("cuda:0").item()) == 2, "the MMA issuer's wait is the one that runs out"
+    with pytest.raises(ops.KernelError, match="role code 2"):
+        ops.check_device_errors()
+    got, _, _ = _residual(ops, x, w, None, None, (128, cluster, stages))
+    _near(got, x.double() @ w.double().T)
+    ops.check_device_errors()
+
+
 def test_what_the_library_refuses(ops):
     lib = ops._lib("gemm_cluster")
     x, w, out = _rand((4, 64), 1), _rand((64, 64), 2), _rand((4, 64), 3)
