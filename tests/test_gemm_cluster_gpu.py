@@ -66,20 +66,37 @@ def test_product_with_residual_and_what_the_next_norm_needs(ops, tokens, n, k, s
     ops.check_device_errors()
 
 
+def _squares(x, parts):
+    """The sums of the squares of x's rows over `parts` shares of their columns, as a product before leaves them: [parts, tokens]."""
+    return torch.stack([(share.float() ** 2).sum(1) for share in x.chunk(parts, dim=1)]).contiguous()
+
+
 @pytest.mark.parametrize("gate", ["silu", "relu", "gelu_tanh"])
-@pytest.mark.parametrize("tokens,n,k", [(17, 32, 64), (33, 352, 192), (64, 17920, 128), (65, 37888, 64), (128, 2080, 1536), (100, 544, 8192)])
-def test_gated_product(ops, tokens, n, k, gate):
+@pytest.mark.parametrize("normed", [False, True])
+@pytest.mark.parametrize("tokens,n,k", [(1, 4096, 2048), (8, 7168, 3584), (17, 32, 64), (33, 352, 192), (64, 17920, 128), (65, 37888, 64), (128, 2080, 1536), (100, 544, 8192)])
+def test_gated_product(ops, tokens, n, k, gate, normed):
+    lib = ops._lib("gemm_cluster")
     x, w = _rand((tokens, k), 5), _rand((n, k), 6, k ** -0.5)
-    out = ops.linear_swiglu(x, w, gate=gate)
-    z = (x.double() @ w.double().T).to(torch.bfloat16).double().view(tokens, -1, 2, 16)
+    out = torch.full((tokens, n // 2), float("nan"), dtype=torch.bfloat16, device="cuda")
+    squares = _squares(x, k // 64) if normed else None
+    code = lib.pae_linear_swiglu_cluster(_p(out), _p(x), _p(w), _p(squares), 0 if squares is None else squares.shape[0], k, 1e-5, tokens, n, k, ops.GATE_KINDS[gate], 1,
+                                         0, 0, 0, ops.error_flag("cuda:0").data_ptr(), 0)
+    assert code == 0, lib.pae_last_error().decode()
+    z = x.double() @ w.double().T
+    if normed:
+        z = z * torch.rsqrt((x.double() ** 2).mean(1, keepdim=True) + 1e-5)
+    z = z.to(torch.bfloat16).double().view(tokens, -1, 2, 16)
     act = {"silu": torch.nn.functional.silu, "relu": torch.relu, "gelu_tanh": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}[gate]
     _near(out, (act(z[:, :, 0]) * z[:, :, 1]).reshape(tokens, -1))
     ops.check_device_errors()
 
 
-@pytest.mark.parametrize("tokens", [17, 40, 64, 65, 128])
-@pytest.mark.parametrize("heads,kv_heads,d,k", [(12, 2, 128, 1536), (14, 2, 64, 896), (3, 1, 32, 192), (5, 5, 16, 64)])
-def test_qkv_with_rotation_and_page_write(ops, tokens, heads, kv_heads, d, k):
+@pytest.mark.parametrize("tokens,heads,kv_heads,d,k", [(t, *sizes) for t in (17, 40, 64, 65, 100, 127, 128)
+                                                       for sizes in ((12, 2, 128, 1536), (14, 2, 64, 896), (3, 1, 32, 192), (5, 5, 16, 64))]
+                         + [(1, 16, 4, 128, 2048), (3, 28, 4, 128, 3584), (8, 16, 4, 128, 2048)])
+@pytest.mark.parametrize("normed", [False, True])
+def test_qkv_with_rotation_and_page_write(ops, tokens, heads, kv_heads, d, k, normed):
+    lib = ops._lib("gemm_cluster")
     n, page, pages = (heads + 2 * kv_heads) * d, 16, 10
     x, w = _rand((tokens, k), 7), _rand((n, k), 8, k ** -0.5)
     gen = torch.Generator().manual_seed(9)
@@ -89,8 +106,17 @@ def test_qkv_with_rotation_and_page_write(ops, tokens, heads, kv_heads, d, k):
     slots = slots.cuda()
     keys = torch.zeros((pages, kv_heads, page, d), dtype=torch.bfloat16, device="cuda")
     values = torch.zeros_like(keys)
-    got = ops.qkv_projection(x, w, bias, table, slots, keys, values, heads, kv_heads, d, page).view(tokens, -1, d)
-    y = (x.double() @ w.double().T + bias.double()).to(torch.bfloat16).double().view(tokens, -1, d)
+    got = torch.full((tokens, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    squares = _squares(x, k // 64) if normed else None
+    ops._set_bounds("gemm_cluster", keys)
+    code = lib.pae_qkv_cluster(_p(got), _p(x), _p(w), _p(bias), _p(squares), 0 if squares is None else squares.shape[0], k, 1e-5, _p(table), _p(slots), _p(keys),
+                               _p(values), tokens, heads, kv_heads, d, page, k, 1, 0, 0, 0, ops.error_flag("cuda:0").data_ptr(), 0)
+    assert code == 0, lib.pae_last_error().decode()
+    got = got.view(tokens, -1, d)
+    y = x.double() @ w.double().T
+    if normed:
+        y = y * torch.rsqrt((x.double() ** 2).mean(1, keepdim=True) + 1e-5)
+    y = (y + bias.double()).to(torch.bfloat16).double().view(tokens, -1, d)
     c, s = table.double()[:, None, : d // 2], table.double()[:, None, d // 2 :]
     lo, hi = y[..., : d // 2], y[..., d // 2 :]
     rotated = torch.cat((lo * c - hi * s, hi * c + lo * s), -1)
