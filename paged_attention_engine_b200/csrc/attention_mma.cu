@@ -19,8 +19,7 @@ PAE_EXPORT int pae_decode_blocks_per_wave(int d) {
   static int cached[3] = {0, 0, 0};
   const int which = d == 32 ? 0 : (d == 64 ? 1 : 2);
   if (cached[which] == 0) {
-    int device = 0, sms = 148, per_sm = 0;
-    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    int per_sm = 0;
     const size_t bytes = slices_smem_bytes(d == 32 ? 32 : (d == 64 ? 64 : 128));
     cudaError_t err;
     if (d == 32) {
@@ -33,7 +32,7 @@ PAE_EXPORT int pae_decode_blocks_per_wave(int d) {
       allow_smem(decode_slices_kernel<128>, bytes, "paged_attention_decode");
       err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_slices_kernel<128>, SLICE_WARPS * 32, bytes);
     }
-    cached[which] = (err == cudaSuccess && per_sm > 0 ? per_sm : 1) * sms;
+    cached[which] = (err == cudaSuccess && per_sm > 0 ? per_sm : 1) * multiprocessors();
   }
   return cached[which];
 }

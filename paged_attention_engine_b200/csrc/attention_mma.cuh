@@ -379,26 +379,11 @@ __global__ void __launch_bounds__(SLICE_WARPS * 32) decode_slices_kernel(const D
 constexpr int MERGE_WARPS = 4;
 constexpr int MERGE_DEPTH = 24;      // slices per warp whose partial outputs are in registers at one time
 
+// The block's merge of `slices` parts, part s of which has its output at part_out + s * D, into `out` [D]. `weights`: [max_slices], then [MERGE_WARPS][D].
 template <int D, int DEPTH>
-__global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
-    __nv_bfloat16* __restrict__ out, const float* __restrict__ part_out, const float* __restrict__ part_max,
-    const float* __restrict__ part_sum, const int* __restrict__ q_start, const int* __restrict__ kv_len, int heads, int window,
-    int slice_keys, int max_slices) {
-  // The kernel before this one is the sliced decode kernel of the same call, which has read
-  // the step's integers itself: they are read before the wait.
-  dependent_launch_trigger();
-  extern __shared__ float weights[];          // [max_slices], then [MERGE_WARPS][D]
+__device__ __forceinline__ void merge_parts(__nv_bfloat16* __restrict__ out, const float* __restrict__ part_out, const float* __restrict__ part_max,
+                                            const float* __restrict__ part_sum, int slices, int max_slices, float* weights) {
   __shared__ float reduce[2 * MERGE_WARPS];
-  const int h = blockIdx.x, b = blockIdx.y;
-  const int token = q_start[b];
-  const bool single = q_start[b + 1] - token == 1;
-  const int n_kv = kv_len[b];
-  dependent_launch_wait();
-  if (!single) return;
-  const int first_key = window > 0 ? max(0, n_kv - window) : 0;
-  const int base = (first_key / TILE_KEYS) * TILE_KEYS;
-  const int slices = min(max_slices, (n_kv - base + slice_keys - 1) / slice_keys);
-  const size_t at = ((size_t)b * heads + h) * max_slices;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int PER_LANE = D / 32;
 
@@ -410,7 +395,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
 #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) part[i][j] = 0.f;
     if (s < slices) {
-      const float* from = part_out + (at + s) * D + lane * PER_LANE;
+      const float* from = part_out + (size_t)s * D + lane * PER_LANE;
       if (PER_LANE == 4) {
         const float4 v = *(const float4*)from;
         part[i][0] = v.x; part[i][1] = v.y; part[i][2] = v.z; part[i][3] = v.w;
@@ -422,7 +407,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
   }
   float top = -FLT_MAX;
   for (int s = threadIdx.x; s < slices; s += blockDim.x) {
-    const float m = part_max[at + s];
+    const float m = part_max[s];
     weights[s] = m;
     top = fmaxf(top, m);
   }
@@ -438,7 +423,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
   for (int s = threadIdx.x; s < slices; s += blockDim.x) {
     const float w = exp2f(weights[s] - top);    // this thread wrote weights[s] itself
     weights[s] = w;
-    total += part_sum[at + s] * w;
+    total += part_sum[s] * w;
   }
   total = warp_sum(total);
   if (lane == 0) reduce[MERGE_WARPS + warp] = total;
@@ -463,7 +448,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
   }
   for (int s = warp + DEPTH * MERGE_WARPS; s < slices; s += MERGE_WARPS) {     // more than 96 slices
     const float w = weights[s];
-    const float* from = part_out + (at + s) * D + lane * PER_LANE;
+    const float* from = part_out + (size_t)s * D + lane * PER_LANE;
 #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) acc[j] += from[j] * w;
   }
@@ -475,8 +460,30 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
     float v = 0.f;
 #pragma unroll
     for (int w = 0; w < MERGE_WARPS; ++w) v += across[w * D + d];
-    out[((size_t)token * heads + h) * D + d] = __float2bfloat16_rn(v * inv);
+    out[d] = __float2bfloat16_rn(v * inv);
   }
+}
+
+template <int D, int DEPTH>
+__global__ void __launch_bounds__(MERGE_WARPS * 32) merge_slices_kernel(
+    __nv_bfloat16* __restrict__ out, const float* __restrict__ part_out, const float* __restrict__ part_max,
+    const float* __restrict__ part_sum, const int* __restrict__ q_start, const int* __restrict__ kv_len, int heads, int window,
+    int slice_keys, int max_slices) {
+  // The kernel before this one is the sliced decode kernel of the same call, which has read
+  // the step's integers itself: they are read before the wait.
+  dependent_launch_trigger();
+  extern __shared__ float weights[];          // [max_slices], then [MERGE_WARPS][D]
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int token = q_start[b];
+  const bool single = q_start[b + 1] - token == 1;
+  const int n_kv = kv_len[b];
+  dependent_launch_wait();
+  if (!single) return;
+  const int first_key = window > 0 ? max(0, n_kv - window) : 0;
+  const int base = (first_key / TILE_KEYS) * TILE_KEYS;
+  const int slices = min(max_slices, (n_kv - base + slice_keys - 1) / slice_keys);
+  const size_t at = ((size_t)b * heads + h) * max_slices;
+  merge_parts<D, DEPTH>(out + ((size_t)token * heads + h) * D, part_out + at * D, part_max + at, part_sum + at, slices, max_slices, weights);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -646,15 +653,13 @@ __global__ void __launch_bounds__(SLICE_WARPS * 32) decode_planned_kernel(const 
   });
 }
 
-// The merge of the planned slices: as above, DEPTH parts per warp at one time in registers.
+// The merge of the planned slices.
 template <int D, int DEPTH>
 __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_planned_kernel(const PlannedParams a) {
   dependent_launch_trigger();
   const DecodeParams& p = a.d;
   extern __shared__ float weights[];          // [max_slices], then [MERGE_WARPS][D]
-  __shared__ float reduce[2 * MERGE_WARPS];
   const int h = blockIdx.x, b = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = p.heads / p.kv_heads, g = h / groups;
   const int token = p.q_start[b];
   const bool single = p.q_start[b + 1] - token == 1;
@@ -667,82 +672,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) merge_planned_kernel(const P
   }
   const int slices = min(p.max_slices, pair.count);
   const size_t at = (size_t)(h - g * groups) * a.items + pair.first;
-  constexpr int PER_LANE = D / 32;
-
-  // ---- requests: this warp's first DEPTH partial outputs, then the maxima and sums
-  auto load_part = [&](int s, float* v) {
-    const float* from = p.part_out + (at + s) * D + lane * PER_LANE;
-    if (PER_LANE == 4) {
-      const float4 t = *(const float4*)from;
-      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    } else {
-#pragma unroll
-      for (int j = 0; j < PER_LANE; ++j) v[j] = from[j];
-    }
-  };
-  float part[DEPTH][4];
-#pragma unroll
-  for (int i = 0; i < DEPTH; ++i) {
-    const int s = warp + i * MERGE_WARPS;
-    part[i][0] = part[i][1] = part[i][2] = part[i][3] = 0.f;
-    if (s < slices) load_part(s, part[i]);
-  }
-  float top = -FLT_MAX;
-  for (int s = threadIdx.x; s < slices; s += blockDim.x) {
-    const float m = p.part_max[at + s];
-    weights[s] = m;
-    top = fmaxf(top, m);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-  if (lane == 0) reduce[warp] = top;
-  __syncthreads();
-  top = reduce[0];
-#pragma unroll
-  for (int w = 1; w < MERGE_WARPS; ++w) top = fmaxf(top, reduce[w]);
-
-  float total = 0.f;
-  for (int s = threadIdx.x; s < slices; s += blockDim.x) {
-    const float w = exp2f(weights[s] - top);    // this thread wrote weights[s] itself
-    weights[s] = w;
-    total += p.part_sum[at + s] * w;
-  }
-  total = warp_sum(total);
-  if (lane == 0) reduce[MERGE_WARPS + warp] = total;
-  __syncthreads();                              // the weights of all slices and the warps' sums are in place
-  total = 0.f;
-#pragma unroll
-  for (int w = 0; w < MERGE_WARPS; ++w) total += reduce[MERGE_WARPS + w];
-  const float inv = total > 0.f ? 1.f / total : 0.f;
-
-  // ---- this warp's slices in their order
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int i = 0; i < DEPTH; ++i) {
-    const int s = warp + i * MERGE_WARPS;
-    if (s < slices) {
-      const float w = weights[s];
-#pragma unroll
-      for (int j = 0; j < PER_LANE; ++j) acc[j] += part[i][j] * w;
-    }
-  }
-  for (int s = warp + DEPTH * MERGE_WARPS; s < slices; s += MERGE_WARPS) {
-    float v[4];
-    load_part(s, v);
-    const float w = weights[s];
-#pragma unroll
-    for (int j = 0; j < PER_LANE; ++j) acc[j] += v[j] * w;
-  }
-  float* across = weights + p.max_slices;          // [MERGE_WARPS][D]
-#pragma unroll
-  for (int j = 0; j < PER_LANE; ++j) across[warp * D + lane * PER_LANE + j] = acc[j];
-  __syncthreads();
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float v = 0.f;
-#pragma unroll
-    for (int w = 0; w < MERGE_WARPS; ++w) v += across[w * D + d];
-    a.out[((size_t)token * p.heads + h) * D + d] = __float2bfloat16_rn(v * inv);
-  }
+  merge_parts<D, DEPTH>(a.out + ((size_t)token * p.heads + h) * D, p.part_out + at * D, p.part_max + at, p.part_sum + at, slices, p.max_slices, weights);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -912,9 +842,20 @@ int allow_smem(Kernel kernel, size_t bytes, const char* what) {
 
 inline size_t slices_smem_bytes(int d) { return (size_t)SLICE_WARPS * SLICE_STAGES * 2 * TILE_KEYS * d * 2; }
 
+inline int multiprocessors() {
+  static const int count = [] {
+    int device = 0, n = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) n = 0;
+    return n > 0 ? n : 148;
+  }();
+  return count;
+}
+
 // Which merge: many blocks hold eight slices a warp in registers (64 of them instead of 128), so that more blocks run at once (12 heads of 64
-// requests, 8 slices: 3.0 us instead of 5.2); few blocks with many slices take up to 96 in one trip.
-inline bool merge_in_few_registers(int heads, int seqs, int max_slices) { return (long long)heads * seqs > 4 * 148 || max_slices <= 8 * MERGE_WARPS; }
+// requests, 8 slices: 3.0 us instead of 5.2); few blocks with many slices take up to 96 in one trip. Four blocks of the latter fit an SM.
+inline bool merge_in_few_registers(int heads, int seqs, int max_slices) {
+  return (long long)heads * seqs > 4ll * multiprocessors() || max_slices <= 8 * MERGE_WARPS;
+}
 
 template <int D>
 int launch_decode(const DecodeParams& p, __nv_bfloat16* out, int seqs, cudaStream_t s) {
