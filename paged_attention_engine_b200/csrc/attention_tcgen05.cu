@@ -34,15 +34,15 @@
 //
 // Sizes: head_dim 64 or 128; page sizes 16, 32, 64 or 128; any number of heads and groups.
 // Requests that bring a single token are left to the decode kernel.
-#include <cuda.h>
 
 #include <cfloat>
 #include <mutex>
 #include <unordered_map>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 using namespace pae;
+using namespace pae_tcgen05;
 
 namespace {
 
@@ -50,7 +50,6 @@ constexpr int BQ = 128;             // query rows per block
 constexpr int BKEYS = 128;          // keys per tile
 constexpr int THREADS = 320;         // TMA warp, MMA warp, eight softmax warps (two threads per query row)
 constexpr int SOFTMAX_THREADS = 256;
-constexpr uint32_t WAIT_LIMIT = 1u << 21;
 constexpr float LOG2E = 1.4426950408889634f;
 
 struct Params {
@@ -66,63 +65,8 @@ struct Params {
   int* error;
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(done)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* error, int code) {
-  for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (i > 64) __nanosleep(64);
-  }
-  *abort_flag = 1;
-  atomicCAS(error, 0, code);
-  return false;
-}
-// The same by a whole warp, which goes on together.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* error, int code) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, error, code));
-}
-// True in one lane of a converged warp. The warp that issues MMAs runs its role together and lets this lane issue them: what all lanes
-// hold alike lies in uniform registers, which the instruction takes; issued from a branch of one lane (`if (lane == 0)`) each MMA cost some
-// 110 cycles, more than its work.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t chosen;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "elect.sync _|p, 0xffffffff;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(chosen));
-  return chosen != 0;
-}
-__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
-      : "memory");
 }
 // A box of keys or values: coordinates in a pool seen as [pages][kv heads][D / 64][rows of a page][64].
 __device__ __forceinline__ void tma_load_pages(uint32_t dst, const CUtensorMap* map, uint32_t bar, int row, int half, int head, int page) {
@@ -171,30 +115,6 @@ __device__ __forceinline__ uint32_t value_step(int k, int rows_a_box) {
   const int row = k * 16;
   return (uint32_t)(row + (D / 64 - 1) * (row & -rows_a_box)) * 128;
 }
-__device__ __forceinline__ void tmem_alloc(uint32_t holder, uint32_t columns) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(holder), "r"(columns) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t address, uint32_t columns) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(address), "r"(columns) : "memory");
-}
-__device__ __forceinline__ void tcgen05_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // 32 consecutive float32 columns of this thread's lane of tensor memory.
 __device__ __forceinline__ void tmem_load32(uint32_t address, float* v) {
   uint32_t r[32];
@@ -239,16 +159,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// K-major operand tile with 128-byte swizzle (rows of 64 bfloat16, groups of 8 rows 1024 bytes apart).
-__device__ __forceinline__ uint64_t k_major_descriptor(uint32_t address) {
-  uint64_t d = 0;
-  d |= (uint64_t)((address & 0x3FFFFu) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
 // MN-major operand with 128-byte swizzle: a 128-byte row holds 64 consecutive MN elements of
 // one K index; 8 consecutive K indices are 8 rows (1024 bytes, the stride byte offset); the
 // next 64 MN elements lie `mn_group_bytes` further (the leading byte offset).
@@ -460,8 +370,8 @@ __global__ void __launch_bounds__(THREADS) prefill_tcgen05_kernel(const __grid_c
       const bool leader = elect_one();
       constexpr uint32_t idesc_s = instruction_descriptor(BQ, BKEYS, false);
       constexpr uint32_t idesc_o = instruction_descriptor(BQ, D, true);
-      const uint64_t q_first = k_major_descriptor(base + L::Q_OFFSET), k_first = k_major_descriptor(base + L::K_OFFSET);
-      const uint64_t p_first = k_major_descriptor(base + L::P_OFFSET), v_first = mn_major_descriptor(base + L::V_OFFSET, p.page_size * 128);
+      const uint64_t q_first = smem_descriptor(base + L::Q_OFFSET), k_first = smem_descriptor(base + L::K_OFFSET);
+      const uint64_t p_first = smem_descriptor(base + L::P_OFFSET), v_first = mn_major_descriptor(base + L::V_OFFSET, p.page_size * 128);
       bool ok = mbar_wait_warp(bar(Q_FULL), 0, abort_flag, p.error, 2);
       auto issue_scores = [&](int t) {
         const int st = t & 1;
@@ -983,7 +893,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
       const bool leader = elect_one();
       constexpr uint32_t idesc_s = instruction_descriptor(BQ, BKEYS, false);
       constexpr uint32_t idesc_o = instruction_descriptor(BQ, D, true);
-      const uint64_t q_first = k_major_descriptor(base + L::Q_OFFSET), k_first = k_major_descriptor(base + L::K_OFFSET);
+      const uint64_t q_first = smem_descriptor(base + L::Q_OFFSET), k_first = smem_descriptor(base + L::K_OFFSET);
       const uint64_t v_first = mn_major_descriptor(base + L::V_OFFSET, box_rows * 128);
       bool ok = mbar_wait_warp(bar(Q_FULL), 0, abort_flag, p.error, 2);
       auto issue_scores = [&](int t) {
@@ -1192,22 +1102,6 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_tcgen05_paired_kernel(cons
 }  // namespace paired
 
 // ---------------------------------------------------------------------------------------
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encode_tiled() {
-  static EncodeTiled fn = [] {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult result;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &result) != cudaSuccess ||
-        result != cudaDriverEntryPointSuccess)
-      ptr = nullptr;
-    return (EncodeTiled)ptr;
-  }();
-  return fn;
-}
-
 // A pool [pages, kv_heads, page_size, d] as boxes of `rows` rows of `halves` halves of `run` pages, 128-byte swizzle.
 int page_map(CUtensorMap* out, const void* ptr, long long pages, int kv_heads, int page_size, int d, int rows, int halves, int run) {
   EncodeTiled encode = encode_tiled();
@@ -1258,21 +1152,6 @@ int page_maps(PageMaps* out, const void* keys, const void* values, long long pag
   if (int err = page_map(&out->value_run, values, pages, kv_heads, page_size, d, rows, halves, run)) return err;
   if (cache.size() > 1024) cache.clear();
   cache.emplace(key, *out);
-  return 0;
-}
-
-// [rows, cols] bfloat16 row-major as boxes of 64 columns x box_rows rows, 128-byte swizzle.
-int tensor_map(CUtensorMap* out, const void* ptr, long long rows, int cols, int box_rows) {
-  EncodeTiled encode = encode_tiled();
-  if (encode == nullptr) return fail(101, "paged_attention_tcgen05: the driver does not export cuTensorMapEncodeTiled");
-  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-  const cuuint32_t element_strides[2] = {1, 1};
-  CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, element_strides,
-                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(102, "paged_attention_tcgen05: cuTensorMapEncodeTiled failed with %d", (int)r);
   return 0;
 }
 

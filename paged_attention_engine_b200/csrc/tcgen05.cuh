@@ -210,7 +210,7 @@ inline int tensor_map(CUtensorMap* out, const void* ptr, int rows, int k, int bo
     return 0;
   }
   EncodeTiled encode = encode_tiled();
-  if (encode == nullptr) return fail(101, "linear_tcgen05: the driver does not export cuTensorMapEncodeTiled");
+  if (encode == nullptr) return fail(101, "the driver does not export cuTensorMapEncodeTiled");
   const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
   const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
@@ -218,7 +218,7 @@ inline int tensor_map(CUtensorMap* out, const void* ptr, int rows, int k, int bo
   CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, element_strides,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(102, "linear_tcgen05: cuTensorMapEncodeTiled failed with %d for [%d, %d]", (int)r, rows, k);
+  if (r != CUDA_SUCCESS) return fail(102, "cuTensorMapEncodeTiled failed with %d for a matrix of [%d, %d]", (int)r, rows, k);
   if (cache.size() > 4096) cache.clear();
   cache.emplace(key, *out);
   return 0;

@@ -45,7 +45,7 @@ FAMILIES: dict[str, list[str]] = {
     "gemv_mma": ["gemv_mma.cu", "tcgen05.cuh", "common.cuh"],
     "attention_mma": ["attention_mma.cu", "attention_mma.cuh", "common.cuh"],
     "fused_decode": ["fused_decode.cu", "common.cuh"],
-    "attention_tcgen05": ["attention_tcgen05.cu", "common.cuh"],
+    "attention_tcgen05": ["attention_tcgen05.cu", "tcgen05.cuh", "common.cuh"],
     "norm_act": ["norm_act.cu", "common.cuh"],
     "short_conv": ["short_conv.cu", "common.cuh"],
     "attention_scored": ["attention_scored.cu", "common.cuh"],
