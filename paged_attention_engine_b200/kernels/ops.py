@@ -647,7 +647,7 @@ def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str 
     wrote needs another launch, or a synchronisation, in between. Larger products read nothing before that kernel has completed."""
     if activation not in ACTIVATIONS:
         raise KernelError(f"linear: activation '{activation}' (known: gelu_erf, gelu_tanh, relu2)")
-    if activation is None and _plain_product(x, weight, bias, out_dtype):
+    if activation is None and x.shape[0] <= CLUSTER_MAX_TOKENS and _plain_product(x, weight, bias, out_dtype):
         # Alone, a product runs as a few-token kernel where one takes it (1,024 x 1,024, 16 tokens: 2.0 us, by clusters 3.1; 2,048 x 5,504, 8
         # tokens: 5.2 and 6.4); what a cluster's epilogue saves is the norm behind it.
         clusters = residual is not None and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0])
@@ -702,7 +702,7 @@ def linear_before_norm(x, weight, bias=None, residual=None, out_dtype=None):
     """`linear` for a sum that an RMSNorm reads next. The product of some tens of tokens with a residual may come back as a
     `PendingProduct`, which that norm has run with the norm inside; `materialized` hands out its tensor. x and the residual are not to be
     written before."""
-    if (residual is not None and _plain_product(x, weight, bias, out_dtype)
+    if (x.shape[0] <= CLUSTER_MAX_TOKENS and residual is not None and _plain_product(x, weight, bias, out_dtype)
             and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0])
             and not _few_tokens_layer(x.shape[0], weight.shape[0], x.shape[-1], x.device)):
         pending = _pending_product(x, weight, residual)
@@ -720,8 +720,8 @@ def _few_tokens_layer(tokens: int, width: int, k: int, device) -> bool:
 
 def _plain_product(x, weight, bias, out_dtype) -> bool:
     """Whether the kernels of few and of some tens of tokens may take a product: bfloat16 without a bias."""
-    return (x.shape[0] <= CLUSTER_MAX_TOKENS and bias is None and out_dtype in (None, torch.bfloat16)
-            and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.data_ptr() % 16 == 0 and weight.shape[0] <= 65536)
+    return (bias is None and out_dtype in (None, torch.bfloat16) and weight.dtype == torch.bfloat16 and weight.dim() == 2
+            and weight.data_ptr() % 16 == 0 and weight.shape[0] <= 65536)
 
 
 def _pending_product(x, weight, residual):
@@ -1159,7 +1159,7 @@ def linear_swiglu(x, weight, gate: str = "silu") -> torch.Tensor:
     splits; otherwise as a kernel of its own. Gate and up are rounded to the engine dtype first in
     every one of them, so all give the same bits."""
     scaled = isinstance(x, ScaledNorm) and x.value is None
-    takes = (x.dtype == torch.bfloat16 and weight.shape[0] % 32 == 0 and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[1])
+    takes = (x.shape[0] <= CLUSTER_MAX_TOKENS and x.dtype == torch.bfloat16 and weight.shape[0] % 32 == 0 and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[1])
              and not _uneven_gate(x.shape[0], weight.shape[0], x.device))
     if not scaled:
         source, norm_weight, eps = _norm_of(x)

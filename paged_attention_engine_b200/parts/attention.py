@@ -96,4 +96,4 @@ class GQAAttention(Part):
             ctx.max_q_len, ctx.max_kv_len, self.scale, self.window, num_single=ctx.num_single,
             multi_index=getattr(ctx, "multi_index", None),
         )
-        return self.into_stream(out, self.o_weight, residual)
+        return self.into_stream(out, self.o_weight, None, residual)

@@ -147,17 +147,14 @@ class Part:
         self.spec = spec
         self.runtime = runtime
         self.ops = runtime.ops
+        # x . weight^T (+ bias) + residual, a sublayer's last product. The norm that reads the stream next may run it, so what comes back is a
+        # tensor after `ops.materialized` only.
+        self.into_stream = getattr(runtime.ops, "linear_before_norm", None) or getattr(runtime.ops, "linear", None)
 
     def build_sub_parts(self, tensors: dict[str, torch.Tensor]) -> list[Any]:
         """The parts of `sub_parts`, built, in its order."""
         return [REGISTRIES[registry].get(sub.kind)(sub, tensors, self.runtime)
                 for registry, sub in self.sub_parts(self.spec)]
-
-    def into_stream(self, x, weight, residual, out_dtype=None):
-        """x . weight^T + residual, a sublayer's last product. The norm that reads the stream next may run it, so what comes back is a
-        tensor after `ops.materialized` only."""
-        ops = self.ops
-        return getattr(ops, "linear_before_norm", ops.linear)(x, weight, None, residual, out_dtype=out_dtype)
 
     @classmethod
     def cache_need(cls, spec: PartSpec) -> CacheNeed | None:
@@ -201,7 +198,7 @@ class ProjectedMixer(Part):
         proj = ops.linear(x, self.in_weight, self.in_bias, None, out_dtype=torch.float32)
         out = self.operand(ctx, proj, 0, cache)
         # without a residual (a caller that sums by itself) the output leaves in float32
-        return self.into_stream(out, self.o_weight, residual, out_dtype=residual.dtype if residual is not None else torch.float32)
+        return self.into_stream(out, self.o_weight, None, residual, out_dtype=residual.dtype if residual is not None else torch.float32)
 
 
 class Registry:

@@ -73,4 +73,4 @@ class GeneralDelta(Part):
         out = ops.delta_rule(proj, (0, width, 2 * width, 3 * width), w_pre, self.w0, self.a_bias, 4 * width,
                              self.norm_weight, cache.state, ctx.q_start, ctx.state_slot, ctx.num_seqs, self.num_heads,
                              self.head_dim, self.decay_scale, self.key_eps, self.norm_eps, self.runtime.dtype)
-        return self.into_stream(out, self.o_weight, residual, out_dtype=residual.dtype)
+        return self.into_stream(out, self.o_weight, None, residual, out_dtype=residual.dtype)

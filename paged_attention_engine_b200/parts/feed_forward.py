@@ -47,7 +47,7 @@ class GatedMLP(Part):
             hidden = ops.linear_swiglu(x, self.gate_up_weight, gate=self.activation)
         else:
             hidden = ops.silu_mul(ops.linear(x, self.gate_up_weight, None), gate=self.activation)
-        return self.into_stream(hidden, self.down_weight, residual, out_dtype=residual.dtype if residual is not None else torch.float32)
+        return self.into_stream(hidden, self.down_weight, None, residual, out_dtype=residual.dtype if residual is not None else torch.float32)
 
 
 @FEED_FORWARDS.register("swiglu")
@@ -82,7 +82,7 @@ class DenseMLP(Part):
     def forward(self, ctx, x, residual):
         ops = self.ops
         hidden = ops.linear(x, self.up_weight, None, activation=self.activation)     # the activation in the product's epilogue
-        return self.into_stream(hidden, self.down_weight, residual, out_dtype=residual.dtype if residual is not None else torch.float32)
+        return self.into_stream(hidden, self.down_weight, None, residual, out_dtype=residual.dtype if residual is not None else torch.float32)
 
 
 @FEED_FORWARDS.register("clamped_glu")

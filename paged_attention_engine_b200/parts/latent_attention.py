@@ -156,4 +156,4 @@ class LatentAttention(Part):
         if self.head_gate:
             out = ops.sigmoid_gate(out, proj, gate_off, group=dv)
         # without a residual (a caller that sums by itself) the output leaves in float32
-        return self.into_stream(out, self.o_weight, residual, out_dtype=residual.dtype if residual is not None else torch.float32)
+        return self.into_stream(out, self.o_weight, None, residual, out_dtype=residual.dtype if residual is not None else torch.float32)

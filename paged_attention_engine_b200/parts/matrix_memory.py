@@ -70,4 +70,4 @@ class MatrixMemory(Part):
         out = ops.matrix_memory(proj, (q_off, k_off, v_off, g_off, i_off, i_off + heads), self.i_bias, self.f_bias,
                                 self.norm_weight, cache.state, ctx.q_start, ctx.state_slot, ctx.num_seqs, heads, d, dv,
                                 self.gate_cap, float(d) ** -0.5, self.norm_eps, self.runtime.dtype)
-        return self.into_stream(out, self.o_weight, residual, out_dtype=residual.dtype)
+        return self.into_stream(out, self.o_weight, None, residual, out_dtype=residual.dtype)

@@ -101,4 +101,4 @@ class ScoredWindowAttention(Part):
             self.num_kv_heads, self.head_dim, self.value_dim, cache.page_size, ctx.max_q_len, self.scale, self.softcap,
             self.temp, self.r1, self.r2, self.sink, self.window, self.keep_first, max_kv_len=ctx.max_kv_len,
             num_single=ctx.num_single)
-        return self.into_stream(out, self.o_weight, residual, out_dtype=residual.dtype)
+        return self.into_stream(out, self.o_weight, None, residual, out_dtype=residual.dtype)
