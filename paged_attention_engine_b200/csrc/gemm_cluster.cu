@@ -22,11 +22,11 @@
 // wait for the kernel before (`early`: the few-token products' rule, see launch_kernel). Mostly 112 KB a block, so that
 // two fit an SM and the next product's blocks fill their rings while this one's finish.
 //
-// What bounds it: the chain, then memory. The four products with their norms in a row, before and now: 1,536-wide layers (93.5 MB of
-// weights, 14.3 us at the copy rate) 43.0 -> 30.4 us at 40 tokens, 44.4 -> 32.8 at 64; 3,584-wide (466 MB, 71 us) 104.9 -> 90.4 at
-// 64; of these 3.5 us by issuing the MMAs from uniform registers. Without that, of q|k|v's 6 us at 40 tokens 0.8 pass before the kernel before releases this one, 1.0 until its tokens' first stage is there, 1.0 in
-// the MMAs, 2 between the accumulator and the barrier, 1 in the epilogue; gate|up and down run at 5.2 TB/s between. Sums read from
-// the other blocks' shared memory instead of stored there: a trip there and back behind the barrier, 0.6 us a kernel more (35.4 and 38.1 us);
+// What bounds it: the chain, then memory. The four products with their norms in a row, with split K and summing kernels and so: 1,536-wide layers (93.5 MB of
+// weights, 14.3 us at the copy rate) 43.3 -> 30.1 us at 40 tokens, 44.3 -> 32.0 at 64, 47.9 -> 37.5 at 100; 3,584-wide (466 MB, 71 us) 104.7 -> 89.1 at
+// 64. Of these 3.5 us by issuing the MMAs from uniform registers. A block's time by %clock64, 1,536 wide, 40 tokens, o / q|k|v / down, us after its wait for the
+// kernel before: first stage 0.7 / 0.6 / 1.5, MMAs 0.6 / 1.2 / 3.0, stores to the other blocks 0.7, the cluster's barrier 0.6, epilogue 0.8 / 0.7 / 0.8 (100 tokens: stores 1.4,
+// barrier 0.7 to 0.9). Sums read from the other blocks' shared memory instead of stored there: a trip there and back behind the barrier, 0.6 us a kernel more;
 // norm weight, bias and residual asked for behind the barrier 1.2 us a kernel more.
 #include <atomic>
 

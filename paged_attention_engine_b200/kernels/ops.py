@@ -12,6 +12,7 @@ norm weights float32, indices int32, logits float32.
 from __future__ import annotations
 
 import ctypes
+import functools
 import re
 from ctypes import c_float, c_int, c_void_p
 
@@ -636,11 +637,14 @@ def _tensor_core_shape(x, weight, residual, out_dtype) -> bool:
 ACTIVATIONS = {None: 0, "gelu_erf": 1, "gelu_tanh": 2, "relu2": 3}
 
 
-def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str | None = None) -> torch.Tensor:
+def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str | None = None, before_norm: bool = False) -> torch.Tensor:
     """x [M, K] . weight [N, K]^T (+ bias [N], float32) (+ residual [M, N]) -> [M, N]. `activation`
     ("gelu_erf", "gelu_tanh", "relu2": the square of max(z, 0)) is applied to the product (+ bias), rounded to the output's dtype first,
     before the residual: in the tensor-core product's epilogue or in the sum of its splits, else
     by the activation's own kernel.
+
+    `before_norm`: an RMSNorm reads the sum next. The product of some tens of tokens with a residual may then come back as a `PendingProduct`, which that norm has
+    run with the norm inside; `materialized` hands out its tensor, and x and the residual are not to be written before.
 
     The bfloat16 kernels of few tokens (up to 64, or 128 where K is long) or of fewer than 256 columns read `weight` while the kernel
     before them in the stream may still be running, as they do in `linear_swiglu` and `qkv_projection`: a weight that the call just before
@@ -648,9 +652,13 @@ def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str 
     if activation not in ACTIVATIONS:
         raise KernelError(f"linear: activation '{activation}' (known: gelu_erf, gelu_tanh, relu2)")
     if activation is None and x.shape[0] <= CLUSTER_MAX_TOKENS and _plain_product(x, weight, bias, out_dtype):
+        clusters = residual is not None and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0])
+        if before_norm and clusters and not _few_tokens_layer(x.shape[0], weight.shape[0], x.shape[-1], x.device):
+            pending = _pending_product(x, weight, residual)
+            if pending is not None:
+                return pending
         # Alone, a product runs as a few-token kernel where one takes it (1,024 x 1,024, 16 tokens: 2.0 us, by clusters 3.1; 2,048 x 5,504, 8
         # tokens: 5.2 and 6.4); what a cluster's epilogue saves is the norm behind it.
-        clusters = residual is not None and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0])
         if not (clusters and isinstance(x, ScaledNorm) and x.value is None):
             source, norm_weight, eps = _norm_of(x)
             if (_few_tokens(source, weight.shape[1], norm_weight is not None, RESIDUAL_KIND, weight.shape[0]) and source.dim() == 2 and source.shape[1] == weight.shape[1]
@@ -698,17 +706,8 @@ def linear(x, weight, bias=None, residual=None, out_dtype=None, activation: str 
     return out
 
 
-def linear_before_norm(x, weight, bias=None, residual=None, out_dtype=None):
-    """`linear` for a sum that an RMSNorm reads next. The product of some tens of tokens with a residual may come back as a
-    `PendingProduct`, which that norm has run with the norm inside; `materialized` hands out its tensor. x and the residual are not to be
-    written before."""
-    if (x.shape[0] <= CLUSTER_MAX_TOKENS and residual is not None and _plain_product(x, weight, bias, out_dtype)
-            and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[0])
-            and not _few_tokens_layer(x.shape[0], weight.shape[0], x.shape[-1], x.device)):
-        pending = _pending_product(x, weight, residual)
-        if pending is not None:
-            return pending
-    return linear(x, weight, bias, residual, out_dtype)
+# `linear` for a sum that an RMSNorm reads next (a partial: no frame of its own on the way of every step).
+linear_before_norm = functools.partial(linear, before_norm=True)
 
 
 def _few_tokens_layer(tokens: int, width: int, k: int, device) -> bool:
@@ -861,9 +860,8 @@ fuse_qkv_epilogue = True
 
 def qkv_projection(x, weight, bias, table, slots, keys, values, num_heads, num_kv_heads, head_dim, page_size) -> torch.Tensor:
     """`rotary_qk_cache_write(linear(x, weight, bias), ...)`: q|k|v of the step's tokens, q and k
-    rotated, k and v written to their pages. For more than 64 tokens on the tensor-core path it
-    is one kernel (the product's epilogue rotates and writes); otherwise the two calls, which
-    for few tokens fuse the other way round (the split sum runs inside the rotation kernel)."""
+    rotated, k and v written to their pages. Mostly one kernel, whose epilogue rotates and writes: that of few tokens, of some tens by clusters, or of
+    many; otherwise the two calls, which for few tokens fuse the other way round (the split sum runs inside the rotation kernel)."""
     m, k = x.shape
     n = weight.shape[0]
     scaled = isinstance(x, ScaledNorm) and x.value is None
@@ -1157,10 +1155,11 @@ def linear_swiglu(x, weight, gate: str = "silu") -> torch.Tensor:
     """act(x . Wg^T) (`gate`: "silu", "relu" or "gelu_tanh") * (x . Wu^T) -> [M, I] for a weight from `interleave_gate_up`. With many
     tokens the activation runs in the product's epilogue; with few, in the kernel that sums the
     splits; otherwise as a kernel of its own. Gate and up are rounded to the engine dtype first in
-    every one of them, so all give the same bits."""
+    every one of them."""
+    tokens = x.shape[0]
     scaled = isinstance(x, ScaledNorm) and x.value is None
-    takes = (x.shape[0] <= CLUSTER_MAX_TOKENS and x.dtype == torch.bfloat16 and weight.shape[0] % 32 == 0 and _cluster_takes(x.shape[0], weight.shape[0], x.shape[-1], weight, weight.shape[1])
-             and not _uneven_gate(x.shape[0], weight.shape[0], x.device))
+    takes = (tokens <= CLUSTER_MAX_TOKENS and x.dtype == torch.bfloat16 and weight.shape[0] % 32 == 0
+             and _cluster_takes(tokens, weight.shape[0], x.shape[-1], weight, weight.shape[1]) and not _uneven_gate(tokens, weight.shape[0], x.device))
     if not scaled:
         source, norm_weight, eps = _norm_of(x)
         few = _few_tokens(source, weight.shape[1], norm_weight is not None, GATE_UP_KIND, weight.shape[0])
@@ -1169,7 +1168,7 @@ def linear_swiglu(x, weight, gate: str = "silu") -> torch.Tensor:
     # As in `qkv_projection`: an operand that no product before has prepared goes to a few-token kernel where one takes it (11,008 x 2,048, 8 tokens: 9.2 us,
     # by clusters 10.4), and of more than 64 tokens to the many-token kernel unless K is long (8,192 x 1,024, 100 tokens: 7.6 and 8.7; 11,008
     # x 2,048 13.7 and 12.7).
-    if takes and (scaled or (not few and (x.shape[0] <= SWAPPED_MAX_TOKENS or weight.shape[1] >= SWAPPED_LONG_K))):
+    if takes and (scaled or (not few and (tokens <= SWAPPED_MAX_TOKENS or weight.shape[1] >= SWAPPED_LONG_K))):
         operand = _cluster_operand(x)
         if operand is not None:
             rows, squares, width, norm_eps = operand
