@@ -510,10 +510,12 @@ def _cluster_takes(tokens: int, n: int, k: int, weight, width: int) -> bool:
 
 
 def _uneven_gate(tokens: int, n: int, device) -> bool:
-    """gate|up of more than 64 tokens whose tiles are some more than the SMs: the SMs that get two draw twice the operands (width 2,048, 172
-    tiles, 128 tokens: the layer's products 75.0 us against 70.1 with the many-token kernel throughout)."""
+    """gate|up of more than 64 tokens whose tiles fill a part of a round of blocks. Some more than the SMs: those that get two draw twice the operands
+    (width 2,048, 172 tiles, 128 tokens: the layer's products 75.0 us against 70.1 with the many-token kernel throughout). Some more than two an SM: the rest run alone
+    behind them (100 tokens with the norm before it, 320 tiles of K = 5,120: 91.6 us against 79.3; 344 of 8,192: 142.9 and 126.6; 400 of 5,120: 98.9 and 89.9; but 448 of
+    8,192: 158.0 and 160.1; 592 of 4,096: 105.2 and 107.3)."""
     tiles, sms = -(-n // 128), _sm_count(device)
-    return tokens > 64 and sms < tiles <= sms * 8 // 5
+    return tokens > 64 and (sms < tiles <= sms * 8 // 5 or 2 * sms < tiles <= sms * 14 // 5)
 
 
 def _cluster_operand(x):

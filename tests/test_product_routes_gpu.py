@@ -69,9 +69,10 @@ def test_a_product_alone(ops, ran, tokens, n, k, kernel):
     # few tokens: as few-token kernels while the layer's gate|up runs at once as one
     (8, 1536, 8960, "few few few few"), (8, 2048, 5504, "few few few few"), (8, 2304, 2304, "cluster cluster cluster cluster"),
     (1, 3584, 9472, "cluster cluster cluster cluster"), (8, 2048, 11008, "few cluster cluster cluster"),
-    # some tens, up to the last; gate|up of some more tiles than SMs is the many-token kernel's
+    # some tens, up to the last; gate|up of some more tiles than SMs, or than two an SM, is the many-token kernel's
     (9, 1536, 2048, "cluster cluster cluster cluster"), (16, 896, 1024, "few few few few"), (17, 896, 1024, "cluster cluster cluster cluster"),
     (64, 2048, 11008, "cluster cluster cluster cluster"), (65, 2048, 11008, "cluster other cluster cluster"), (128, 1536, 2048, "cluster cluster cluster cluster"),
+    (64, 2048, 20480, "cluster cluster cluster cluster"), (65, 2048, 20480, "cluster other cluster cluster"), (65, 2048, 28672, "cluster cluster cluster cluster"),
 ])
 def test_a_layers_products(ops, ran, tokens, width, inter, kernels):
     """o, norm, gate|up, down, norm, q|k|v: which kernels run them, and that they compute the layer."""
